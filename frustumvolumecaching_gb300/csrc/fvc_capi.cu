@@ -1240,6 +1240,25 @@ static void apply_settings(const fvc_renderer *r, CacheView &v)
     v.inter_brick = c.use_inter_brick_interpolation ? 1 : 0;
 }
 
+/* The order of a warp's rows (RowWalk): sample by sample where a step along
+ * the ray at the scene's distance is longer than about one and a half pixels
+ * there, so that the 8x4 pixels of a warp at one depth are closer together
+ * than 16 samples of two rays.  Measured, network launch: 1080p of the
+ * 3-cascade scene (4.5 pixels a step) 899 -> 861 us, march 373 -> 348; the
+ * fixed-step box at 256x256 and 960x540 (0.2 and 0.4 pixels a step) is 7 and
+ * 14 % faster ray by ray, the 3-cascade scene at 323x181 (0.8) 1 %. */
+static int rows_by_sample(const RenderParams &p)
+{
+    float d2 = 0.f;
+    const float eye[3] = {p.cam.c2w[3], p.cam.c2w[7], p.cam.c2w[11]};
+    const float lo[3] = {p.scene.aabb_from.x, p.scene.aabb_from.y, p.scene.aabb_from.z};
+    const float hi[3] = {p.scene.aabb_to.x, p.scene.aabb_to.y, p.scene.aabb_to.z};
+    for (int k = 0; k < 3; ++k) d2 += (eye[k] - 0.5f * (lo[k] + hi[k])) * (eye[k] - 0.5f * (lo[k] + hi[k]));
+    const float t = sqrtf(d2);
+    const float step = std::max(p.steps.dt_min, std::min(t * p.steps.cone, p.steps.dt_max));
+    return step * p.cam.fx > 1.5f * t;
+}
+
 static int setup_render_params(fvc_renderer *r, const fvc_raymarch_info *info, float4 *results, uchar4 *image, int4 *counts,
                                RenderParams &p, bool per_view_caches = false)
 {
@@ -1302,6 +1321,7 @@ static int setup_render_params(fvc_renderer *r, const fvc_raymarch_info *info, f
     p.fused_classify = r->fused_classify;
     p.skip_empty = r->skip_empty;
     p.row_target = std::min(r->row_target, r->row_capacity);
+    p.by_sample = rows_by_sample(p);
     return FVC_OK;
 }
 
@@ -1730,7 +1750,7 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
     memset(&f, 0, sizeof(f));
     f.scene = m->dscene; f.steps = p.steps; f.W = W; f.H = H;
     f.states[0] = p.states[0]; f.states[1] = p.states[1];
-    f.ray_rows = p.ray_rows; f.row_t0 = p.row_t0; f.den = x.den; f.lat = x.lat; f.counters = p.counters;
+    f.ray_rows = p.ray_rows; f.by_sample = p.by_sample; f.row_t0 = p.row_t0; f.den = x.den; f.lat = x.lat; f.counters = p.counters;
     f.flag = x.flag; f.set = x.set; f.packed_index = c->d_packed; f.known_ranges = c->d_known; f.voxels = c->d_voxels;
     f.bX = c->bX; f.bY = c->bY; f.bZ = c->bZ; f.dX = c->dX; f.dY = c->dY; f.dZ = c->dZ; f.capacity = c->capacity();
     f.variant = r->settings.interpol_variant;
@@ -2090,6 +2110,7 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
     if ((rc = setup_render_params(r, info, r->d_results, nullptr, nullptr, p))) return rc;
     p.pixel_list = pixels;
     p.n_list = n_rays;
+    p.by_sample = 0; /* the warp's rays are any pixels of the list: only a ray's own samples are close together */
     p.ray_grad = g->d_ray_grad;
     p.row_dout = r->d_row_dout;
     p.grad_res_list = r->d_grad_rows;
@@ -2202,6 +2223,7 @@ static int batch_setup(fvc_renderer *r, const fvc_raymarch_info *infos, int n_vi
     p.views = r->d_views;
     p.view_off = r->d_view_off;
     p.n_views = n_views;
+    p.by_sample = 0; /* a batch's warps are pixel rows, not tiles */
     p.max_iterations = 1 << 14;
     return FVC_OK;
 }

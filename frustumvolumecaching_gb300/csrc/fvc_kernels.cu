@@ -564,12 +564,16 @@ __global__ void __launch_bounds__(128) pr_mark_kernel(PerRayFillParams p, int it
 {
     const int n_alive = p.counters[it & 1];
     const RayState *states = p.states[it & 1];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_alive; i += gridDim.x * blockDim.x) {
-        const int2 rr = p.ray_rows[i];
-        const int id = states[i].cnt.x;
-        float T = states[i].acc.w;
-        for (int k = 0; k < rr.y; ++k) {
-            const int row = rr.x + k;
+    for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
+        const int i = base + threadIdx.x;
+        const bool valid = i < n_alive;
+        const int id = valid ? states[i].cnt.x : 0;
+        float T = valid ? states[i].acc.w : 1.f;
+        bool ended = false;
+        int row;
+        RowWalk walk(valid ? p.ray_rows[i] : make_int2(0, 0), valid, p.by_sample);
+        while (walk.step(row)) {
+            if (row < 0 || ended) continue;
             const float density = expf(__half2float(p.den[row]));
             const float t0 = p.row_t0[row];
             const float dt = calc_step(p.steps, t0);
@@ -580,10 +584,13 @@ __global__ void __launch_bounds__(128) pr_mark_kernel(PerRayFillParams p, int it
                 T *= 1.0f - alpha;
                 int bin;
                 const int b = pr_brick(p, id, tm, bin);
-                if (b < 0) break; /* beyond the frustum depth: pr_write ends the ray here */
+                if (b < 0) { /* beyond the frustum depth: pr_write ends the ray here */
+                    ended = true;
+                    continue;
+                }
                 p.flag[b] = 1;
             }
-            if (T < 1e-4f) break;
+            if (T < 1e-4f) ended = true;
         }
     }
 }
@@ -685,16 +692,20 @@ __global__ void __launch_bounds__(128) pr_write_kernel(PerRayFillParams p, int i
     Voxel *vox = reinterpret_cast<Voxel *>(p.voxels);
     for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
         const int i = base + threadIdx.x;
-        bool alive = false;
+        const bool valid = i < n_alive;
+        bool alive = false, ended = false;
         RayState st;
-        if (i < n_alive) {
+        int id = 0, row;
+        float T = 1.f, term = p.steps.far_;
+        if (valid) {
             st = states[i];
-            const int2 rr = p.ray_rows[i];
-            const int id = st.cnt.x;
-            float T = st.acc.w, term = p.steps.far_;
+            id = st.cnt.x;
+            T = st.acc.w;
             alive = st.cnt2.y == 0; /* the march ended the ray past its far bound */
-            for (int k = 0; k < rr.y; ++k) {
-                const int row = rr.x + k;
+        }
+        RowWalk walk(valid ? p.ray_rows[i] : make_int2(0, 0), valid, p.by_sample);
+        while (walk.step(row)) {
+            if (row >= 0 && !ended) {
                 const float density = expf(fminf(__half2float(p.den[row]), 10.0f));
                 const float t0 = p.row_t0[row];
                 const float dt = calc_step(p.steps, t0);
@@ -708,8 +719,9 @@ __global__ void __launch_bounds__(128) pr_write_kernel(PerRayFillParams p, int i
                     const int packed = b >= 0 ? p.packed_index[b] : -1;
                     if (packed < 0) { /* no slot: the cache overflowed here */
                         alive = false;
+                        ended = true;
                         term = t0;
-                        break;
+                        continue;
                     }
                     const int x = id % p.W, y = id / p.W;
                     const int slot = ((packed >> 20) & 1023) * (p.dY * p.dZ) + ((packed >> 10) & 1023) * p.dZ + (packed & 1023);
@@ -723,10 +735,12 @@ __global__ void __launch_bounds__(128) pr_write_kernel(PerRayFillParams p, int i
                 }
                 if (T < 1e-4f) {
                     alive = false;
+                    ended = true;
                     term = t1;
-                    break;
                 }
             }
+        }
+        if (valid) {
             st.acc.w = T;
             if (!alive) p.known_ranges[id] = term;
         }

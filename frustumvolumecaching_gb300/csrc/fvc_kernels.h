@@ -219,6 +219,68 @@ struct RenderStatsDev {
     unsigned long long n_reason[N_REASONS]; /* composited or dropped rows per REASON_* (cached renderers) */
 };
 
+__device__ __forceinline__ unsigned lanes_below() { unsigned m; asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m)); return m; }
+
+/* the sum of the lower lanes' n (whole warp) */
+__device__ __forceinline__ int lanes_before(int n)
+{
+    int sum = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if ((threadIdx.x & 31) >= (unsigned)o) sum += v;
+    }
+    return sum - n;
+}
+
+/* Where the rows of a sub-iteration lie.  A warp's rows follow each other from
+ * its first row, either ray by ray (a ray's samples adjacent) or, by_sample,
+ * the first sample of every lane that has one, then the second samples, and
+ * so on; a walk over the samples in lockstep finds every row from the lanes'
+ * row counts.  The 32 rows of a network warp are then two rays' runs of
+ * samples, or one sample of an 8x4 pixel tile: whichever is smaller in space
+ * shares more L1 lines in its grid gathers (rows_by_sample, fvc_capi.cu). */
+struct RowWalk {
+    int n, j, next;
+    bool by_sample;
+    __device__ __forceinline__ RowWalk(int2 rr, bool valid, bool by) : n(valid ? rr.y : 0), j(0), next(rr.x), by_sample(by)
+    {
+        if (!by) next += lanes_before(n);
+    }
+    /* the next sample's row of this lane (-1 without one); false when no lane has one */
+    __device__ __forceinline__ bool step(int &row)
+    {
+        const unsigned m = __ballot_sync(0xffffffffu, j < n);
+        row = j < n ? next + (by_sample ? __popc(m & lanes_below()) : j) : -1;
+        if (by_sample) next += __popc(m);
+        ++j;
+        return m != 0u;
+    }
+};
+
+/* A warp's entries of a row list, in the order of its rows: lane's n entries
+ * among the warp's from first on; place() is called by all lanes, sample by
+ * sample, and gives a lane with an entry its place. */
+struct ListWalk {
+    int next;
+    bool by_sample;
+    __device__ __forceinline__ ListWalk(int first, int n, bool by) : next(first), by_sample(by)
+    {
+        if (!by) next += lanes_before(n);
+    }
+    __device__ __forceinline__ int place(bool has)
+    {
+        const int at = next;
+        if (!by_sample) {
+            next += has;
+            return at;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, has);
+        next += __popc(m);
+        return at + __popc(m & lanes_below());
+    }
+};
+
 /* one view's frustum cache with the camera and step grid it was built for */
 struct ViewCache {
     CacheView cache;
@@ -258,7 +320,7 @@ struct RenderParams {
     int render_mode;            /* 0 default, 1 only cache, 2 only resampled */
     /* wavefront buffers */
     RayState *states[2];        /* alive rays, ping-pong between sub-iterations */
-    int2 *ray_rows;             /* per alive ray: first row, number of rows (in t order) */
+    int2 *ray_rows;             /* per alive ray: first row of its warp, its number of rows (in t order; RowWalk) */
     float *row_t0;              /* per row: t0 of the sample */
     int *row_slot;              /* per row: alive slot of its ray */
     uint8_t *row_kind;          /* per row: resample / cache / known empty / skipped */
@@ -268,6 +330,7 @@ struct RenderParams {
     int *res_list, *cache_list; /* row ids of the two network streams */
     int *counters;              /* [0], [1] alive rays (ping-pong), [2] rows, [3] resample, [4] cache */
     int row_capacity;           /* rows per sub-iteration */
+    int by_sample;              /* a warp's rows sample by sample instead of ray by ray (RowWalk) */
     int steps_per_iter;         /* marching steps per ray and sub-iteration */
     int m_tile;                 /* rows per tcgen05 network tile on the plain path: 64, 128 (0 = 128) or 256 */
     int fused_classify;         /* cached renders: classification in the march, one network launch for all rows */
@@ -428,7 +491,8 @@ struct PerRayFillParams {
     DevSteps steps;
     int W, H;
     RayState *states[2];        /* the renderer's alive-ray states (ping-pong) */
-    const int2 *ray_rows;       /* per alive ray: first row, row count */
+    const int2 *ray_rows;       /* per alive ray: first row of its warp, its number of rows (RowWalk) */
+    int by_sample;              /* the order of a warp's rows (RowWalk) */
     const float *row_t0;
     const __half *den;          /* per row: log-density (fp16) */
     const uint4 *lat;           /* per row: latents latent_offset + 0..7 (fp16) */

@@ -57,26 +57,6 @@ constexpr int NET_WARPS = 8;
 __device__ __forceinline__ unsigned lane_lt() { unsigned m; asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m)); return m; }
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
-/* warp-aggregated atomicAdd: every active lane gets its offset */
-__device__ __forceinline__ int warp_alloc(int *ctr, int n)
-{
-    const unsigned act = __activemask();
-    int incl = n;
-    const int lane = lane_id();
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(act, incl, o);
-        if (lane >= o && ((act >> (lane - o)) & 1u)) incl += v;
-    }
-    /* the above scan is valid only for a full warp; fall back to per-lane atomics otherwise */
-    if (act != FULLMASK) return atomicAdd(ctr, n);
-    const int total = __shfl_sync(FULLMASK, incl, 31);
-    int base = 0;
-    if (lane == 31) base = atomicAdd(ctr, total);
-    base = __shfl_sync(FULLMASK, base, 31);
-    return base + incl - n;
-}
-
 /* compensated (Kahan) summation: sum += v with the running error in c */
 __device__ __forceinline__ void kahan_add(float &sum, float &c, float v)
 {
@@ -412,7 +392,7 @@ __device__ __forceinline__ int classify_basic(const RenderParams &p, const Cache
 
 /* Marches every alive ray a fixed number of steps (lanes stay converged),
  * keeping at most S_ROWS occupied samples; the samples become rows
- * (t0, alive slot) that are contiguous and in t order per ray.  The plain
+ * (t0, alive slot) in the warp's order (RowWalk).  The plain
  * renderer also contracts the sample position here; the cached renderer
  * classifies the rows in wf_classify_kernel. */
 #ifndef FVC_RAY_BLOCKS_PER_SM
@@ -484,66 +464,82 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
             }
             dt4.w = t1;
         }
-        const int rbase = warp_alloc(p.counters + 2, n);
-        int n_res = 0, n_hit = 0;
-        uint32_t kinds = 0; /* FUSED: 2 bits per row, its kind */
-        if (FUSED && valid) {
-            /* the cached renderer's classification of this ray's rows (wf_classify_kernel's
-             * non-basic form), with the ray moved into the cache camera once per ray */
-            const ViewCache *vc = p.view_caches ? p.view_caches + states[i].cnt2.w : nullptr;
+        const int n_warp = (int)__reduce_add_sync(FULLMASK, (unsigned)n);
+        int rbase = 0;
+        if (lane_id() == 0 && n_warp) rbase = atomicAdd(p.counters + 2, n_warp);
+        rbase = __shfl_sync(FULLMASK, rbase, 0);
+        RowWalk walk(make_int2(rbase, n), true, p.by_sample);
+        int r;
+        if (FUSED) {
+            /* the cached renderer's classification of the rows (wf_classify_kernel's non-basic
+             * form), with the ray moved into the cache camera once per ray */
+            const ViewCache *vc = p.view_caches && valid ? p.view_caches + states[i].cnt2.w : nullptr;
             const CacheView &C = vc ? vc->cache : p.cache;
             const DevCam &ccam = vc ? vc->ccam : p.ccam;
             const DevSteps &cst = vc ? vc->csteps : p.csteps;
             const float3 o = make_float3(of.x, of.y, of.z), d = make_float3(dt4.x, dt4.y, dt4.z);
             float3 oc, dc;
             transform_ray(ccam.w2c, o, d, oc, dc);
-            for (int s = 0; s < n; ++s) {
-                const float t0 = t0s[s];
-                const float dt = calc_step(p.steps, t0);
-                const float tm = F_MUL(F_ADD(t0, F_ADD(t0, dt)), 0.5f);
-                const float tmh = F_ADD(t0, F_MUL(dt, 0.5f));
-                const int code = classify(p, C, ccam, cst, oc, dc, tm);
-                const int kind = row_kind_of(code);
-                float4 pay = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (kind == KIND_RESAMPLE) {
-                    const float3 pc = contract(p.scene, at(o, d, tmh));
-                    pay = make_float4(pc.x, pc.y, pc.z, 0.f);
-                    ++n_res;
-                } else if (kind == KIND_CACHE) {
-                    float tf2;
-                    const float3 fr = cam2froxel(at(oc, dc, tmh), ccam, cst, tf2);
-                    pay = make_float4(fr.x, fr.y, fr.z, 0.f);
-                    ++n_hit;
+            int n_res = 0, n_hit = 0;
+            uint32_t kinds = 0; /* 2 bits per row, its kind */
+            for (int s = 0; walk.step(r); ++s) {
+                int kind = KIND_SKIP;
+                if (r >= 0) {
+                    const float t0 = t0s[s];
+                    const float dt = calc_step(p.steps, t0);
+                    const float tm = F_MUL(F_ADD(t0, F_ADD(t0, dt)), 0.5f);
+                    const float tmh = F_ADD(t0, F_MUL(dt, 0.5f));
+                    const int code = classify(p, C, ccam, cst, oc, dc, tm);
+                    kind = row_kind_of(code);
+                    float4 pay = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (kind == KIND_RESAMPLE) {
+                        const float3 pc = contract(p.scene, at(o, d, tmh));
+                        pay = make_float4(pc.x, pc.y, pc.z, 0.f);
+                    } else if (kind == KIND_CACHE) {
+                        float tf2;
+                        const float3 fr = cam2froxel(at(oc, dc, tmh), ccam, cst, tf2);
+                        pay = make_float4(fr.x, fr.y, fr.z, 0.f);
+                    }
+                    p.row_t0[r] = t0;
+                    p.row_slot[r] = i;
+                    p.row_pay[r] = pay;
+                    p.row_kind[r] = (uint8_t)code;
+                    kinds |= (uint32_t)kind << (2 * s);
                 }
-                p.row_t0[rbase + s] = t0;
-                p.row_slot[rbase + s] = i;
-                p.row_pay[rbase + s] = pay;
-                p.row_kind[rbase + s] = (uint8_t)code;
-                kinds |= (uint32_t)kind << (2 * s);
+                n_res += kind == KIND_RESAMPLE;
+                n_hit += kind == KIND_CACHE;
             }
-        }
-        if (FUSED) {
             /* the resample rows and the cache rows each go to a list, so that the network's tiles hold one
              * kind of row: a cache row never waits on its tile's hash gathers */
-            int rb = warp_alloc(p.counters + 3, n_res), hb = warp_alloc(p.counters + 4, n_hit);
-            for (int s = 0; s < n && (n_res | n_hit); ++s) {
-                const uint32_t kind = (kinds >> (2 * s)) & 3u;
-                if (kind == KIND_RESAMPLE) p.res_list[rb++] = rbase + s;
-                else if (kind == KIND_CACHE) p.cache_list[hb++] = rbase + s;
+            const int w_res = (int)__reduce_add_sync(FULLMASK, (unsigned)n_res), w_hit = (int)__reduce_add_sync(FULLMASK, (unsigned)n_hit);
+            int rb = 0, hb = 0;
+            if (lane_id() == 0) {
+                if (w_res) rb = atomicAdd(p.counters + 3, w_res);
+                if (w_hit) hb = atomicAdd(p.counters + 4, w_hit);
+            }
+            ListWalk res(__shfl_sync(FULLMASK, rb, 0), n_res, p.by_sample), hit(__shfl_sync(FULLMASK, hb, 0), n_hit, p.by_sample);
+            RowWalk again(make_int2(rbase, n), true, p.by_sample);
+            for (int s = 0; again.step(r); ++s) {
+                const uint32_t kind = r >= 0 ? (kinds >> (2 * s)) & 3u : (uint32_t)KIND_SKIP;
+                const int at_res = res.place(kind == KIND_RESAMPLE), at_hit = hit.place(kind == KIND_CACHE);
+                if (kind == KIND_RESAMPLE) p.res_list[at_res] = r;
+                else if (kind == KIND_CACHE) p.cache_list[at_hit] = r;
+            }
+        } else {
+            for (int s = 0; walk.step(r); ++s) {
+                if (r < 0) continue;
+                const float t0 = t0s[s];
+                p.row_t0[r] = t0;
+                p.row_slot[r] = i;
+                if (!CACHED) {
+                    /* sample_performance_kernel :52-58: midpoint (t0+t1)/2, contracted */
+                    const float tm = F_MUL(F_ADD(t0, F_ADD(t0, calc_step(p.steps, t0))), 0.5f);
+                    const float3 pc = contract(p.scene, at(make_float3(of.x, of.y, of.z), make_float3(dt4.x, dt4.y, dt4.z), tm));
+                    p.row_pay[r] = make_float4(pc.x, pc.y, pc.z, 0.f);
+                }
             }
         }
         if (valid) {
-            for (int s = 0; s < n && !FUSED; ++s) {
-                p.row_t0[rbase + s] = t0s[s];
-                p.row_slot[rbase + s] = i;
-                if (!CACHED) {
-                    /* sample_performance_kernel :52-58: midpoint (t0+t1)/2, contracted */
-                    const float t0 = t0s[s];
-                    const float tm = F_MUL(F_ADD(t0, F_ADD(t0, calc_step(p.steps, t0))), 0.5f);
-                    const float3 pc = contract(p.scene, at(make_float3(of.x, of.y, of.z), make_float3(dt4.x, dt4.y, dt4.z), tm));
-                    p.row_pay[rbase + s] = make_float4(pc.x, pc.y, pc.z, 0.f);
-                }
-            }
             p.ray_rows[i] = make_int2(rbase, n);
             states[i].dt = dt4;
             int4 c = states[i].cnt;
@@ -1637,6 +1633,8 @@ __global__ void __launch_bounds__(128, TC_PREC_CTAS_PER_SM) wf_net_tc_prec_kerne
 /* ------------------------------------------------------------------------- */
 /* composite + compaction                                                    */
 /* ------------------------------------------------------------------------- */
+constexpr int COMP_AHEAD = 4; /* samples of a ray whose rows the compositing loads together */
+
 template <bool CACHED>
 __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int it)
 {
@@ -1649,35 +1647,59 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
         RayState st;
         int n_comp = 0;
         unsigned long long why = 0; /* rows per REASON_* 1..7, 8 bits each (at most S_ROWS rows a ray and sub-iteration) */
+        int2 rr = make_int2(0, 0);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 1.f), comp = make_float4(0.f, 0.f, 0.f, 0.f);
+        int c_res = 0, c_cache = 0, c_drop = 0;
         if (valid) {
             st = cur[i];
-            const int2 rr = p.ray_rows[i];
-            float4 acc = st.acc, comp = st.comp;
-            int c_res = st.cnt.y, c_cache = st.cnt.z, c_drop = st.cnt2.x;
-            float w_res = 0.f, w_cache = 0.f; /* this sub-iteration's contribution weights (DEBUG form, :867-871) */
-            bool term = false;
-            /* rows are in t order: the merge of the resample and cache
-             * streams of accumulate_cache_perf_kernel (:270-304) */
-            for (int j = 0; j < rr.y; ++j) {
-                const int r = rr.x + j;
-                const int code = CACHED ? (int)p.row_kind[r] : KIND_RESAMPLE;
-                const int kind = row_kind_of(code);
-                if (CACHED && kind != KIND_SKIP && row_reason_of(code)) why += 1ull << ((8 * (row_reason_of(code) - 1)) & 63);
+            rr = p.ray_rows[i];
+            acc = st.acc;
+            comp = st.comp;
+            c_res = st.cnt.y;
+            c_cache = st.cnt.z;
+            c_drop = st.cnt2.x;
+        }
+        float w_res = 0.f, w_cache = 0.f; /* this sub-iteration's contribution weights (DEBUG form, :867-871) */
+        bool term = false;
+        /* rows are in t order: the merge of the resample and cache streams of
+         * accumulate_cache_perf_kernel (:270-304); COMP_AHEAD samples are loaded together, before the
+         * first of them is composited */
+        RowWalk walk(rr, valid, p.by_sample);
+        for (bool more = true; more;) {
+            int rs[COMP_AHEAD], codes[COMP_AHEAD];
+            uint2 ovs[COMP_AHEAD];
+            float t0s[COMP_AHEAD];
+#pragma unroll
+            for (int q = 0; q < COMP_AHEAD; ++q) {
+                more = walk.step(rs[q]) && more;
+                if (term) rs[q] = -1;
+                codes[q] = CACHED && rs[q] >= 0 ? (int)p.row_kind[rs[q]] : KIND_RESAMPLE;
+                ovs[q] = make_uint2(0u, 0u);
+                t0s[q] = 0.f;
+                if (rs[q] >= 0) { /* a dropped row's output is not written, and not used */
+                    ovs[q] = p.row_out[rs[q]];
+                    t0s[q] = p.row_t0[rs[q]];
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < COMP_AHEAD; ++q) {
+                if (rs[q] < 0 || term) continue;
+                const int kind = row_kind_of(codes[q]);
+                if (CACHED && kind != KIND_SKIP && row_reason_of(codes[q])) why += 1ull << ((8 * (row_reason_of(codes[q]) - 1)) & 63);
                 if (kind >= KIND_DROP) {
                     c_drop += kind == KIND_DROP;
                     continue;
                 }
                 if (kind == KIND_CACHE) ++c_cache; else ++c_res;
                 ++n_comp;
-                const uint2 ov = p.row_out[r];
-                const float t0 = p.row_t0[r];
+                const uint2 ov = ovs[q];
                 const float2 rg = __half22float2(*reinterpret_cast<const __half2 *>(&ov.x));
                 const float lb = __half2float(__ushort_as_half((unsigned short)(ov.y & 0xffffu)));
                 const float ld = __half2float(__ushort_as_half((unsigned short)(ov.y >> 16)));
-                const float dt = calc_step(p.steps, t0);
+                const float dt = calc_step(p.steps, t0s[q]);
                 /* the basic cache renderer composites a cache row with its looked-up density
                  * (accumulate_cache_render_kernel, src/cache_basic_renderer.cu:255-258) */
-                const float sigma = CACHED && p.basic_cache && kind == KIND_CACHE ? p.row_pay[r].w : expf(ld);
+                const float sigma = CACHED && p.basic_cache && kind == KIND_CACHE ? p.row_pay[rs[q]].w : expf(ld);
                 const float alpha = fminf(1.0f, fmaxf(0.0f, 1.0f - expf(-sigma * dt)));
                 if (alpha > p.scene.alpha_thre) {
                     const float wgt = alpha * acc.w;
@@ -1690,8 +1712,10 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
                         else w_res += wgt;
                     }
                 }
-                if (acc.w < 1e-4f) { term = true; break; }
+                if (acc.w < 1e-4f) term = true;
             }
+        }
+        if (valid) {
             if (CACHED) { /* one ray a pixel: no other thread adds to it in this launch */
                 if (p.contrib_res) p.contrib_res[st.cnt.x] += w_res;
                 if (p.contrib_cache) p.contrib_cache[st.cnt.x] += w_cache;
@@ -1747,14 +1771,20 @@ __global__ void __launch_bounds__(128) wf_composite_bwd_kernel(RenderParams p, i
         int n_res = 0, n_cch = 0;
         int2 rr = make_int2(0, 0);
         uint32_t gmask = 0, cmask = 0;
+        float4 rg = make_float4(0.f, 0.f, 0.f, 0.f);
+        float T = 1.f, xp = 0.f;
         if (valid) {
             st = cur[i];
             rr = p.ray_rows[i];
-            const float4 rg = p.ray_grad[st.cnt.x];
-            float T = st.acc.w, xp = st.acc.x;
-            bool term = false;
-            for (int j = 0; j < rr.y; ++j) {
-                const int r = rr.x + j;
+            rg = p.ray_grad[st.cnt.x];
+            T = st.acc.w;
+            xp = st.acc.x;
+        }
+        bool term = false;
+        int r;
+        RowWalk walk(rr, valid, p.by_sample);
+        for (int j = 0; walk.step(r); ++j) {
+            if (r >= 0) {
                 float4 dout = make_float4(0.f, 0.f, 0.f, 0.f);
                 const int kind = CACHED ? row_kind_of(p.row_kind[r]) : KIND_RESAMPLE;
                 if (!term && kind < KIND_DROP) {
@@ -1784,23 +1814,26 @@ __global__ void __launch_bounds__(128) wf_composite_bwd_kernel(RenderParams p, i
                 }
                 p.row_dout[r] = dout;
             }
+        }
+        if (valid) {
             st.acc.x = xp;
             st.acc.w = T;
             keep = !(term || st.cnt2.y);
         }
         /* list the rows with a gradient per network stream (one atomic per warp and list) */
         auto append = [&](int n, uint32_t mask, int *list, int *counter) {
-            int incl = n;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(FULLMASK, incl, o);
-                if (lane_id() >= o) incl += v;
-            }
-            const int total = __shfl_sync(FULLMASK, incl, 31);
+            const int total = (int)__reduce_add_sync(FULLMASK, (unsigned)n);
+            if (total == 0) return;
             int lb = 0;
-            if (lane_id() == 0 && total) lb = atomicAdd(counter, total);
-            lb = __shfl_sync(FULLMASK, lb, 0) + incl - n;
-            for (uint32_t mm = mask; mm; mm &= mm - 1) list[lb++] = rr.x + __ffs(mm) - 1;
+            if (lane_id() == 0) lb = atomicAdd(counter, total);
+            ListWalk places(__shfl_sync(FULLMASK, lb, 0), n, p.by_sample);
+            int row;
+            RowWalk rows(rr, valid, p.by_sample);
+            for (int j = 0; rows.step(row); ++j) {
+                const bool has = (mask >> j) & 1u;
+                const int at = places.place(has);
+                if (has) list[at] = row;
+            }
         };
         append(n_res, gmask, p.grad_res_list, p.counters + 6);
         if (CACHED) append(n_cch, cmask, p.grad_cache_list, p.counters + 7);
