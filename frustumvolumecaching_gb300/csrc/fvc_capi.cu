@@ -315,6 +315,7 @@ struct fvc_model {
     uint8_t *d_weights_vd = nullptr;        /* VD_WBYTES of K-major tiles (view-dependent models) */
     uint2 *d_weights_fh = nullptr;          /* the first head as W_L1 / W_L2 fragment packs */
     uint8_t *d_bits = nullptr;
+    uint32_t *d_cells = nullptr;            /* the occupancy in 4 x 4 x 2 words (occupied2) */
     __half2 *d_table = nullptr;
     uint2 *d_weights = nullptr;
     uint8_t *d_weights_tc = nullptr;
@@ -324,7 +325,7 @@ struct fvc_model {
     size_t table_entries = 0;
     ~fvc_model()
     {
-        dfree(d_bits); dfree(d_table); dfree(d_weights); dfree(d_weights_tc); dfree(d_bias3);
+        dfree(d_bits); dfree(d_cells); dfree(d_table); dfree(d_weights); dfree(d_weights_tc); dfree(d_bias3);
         dfree(d_weights_tc_bf16); dfree(d_weights_tc_fp8); dfree(d_fp8_iw); dfree(d_weights_vd); dfree(d_weights_fh);
     }
 };
@@ -628,6 +629,13 @@ static int build_model(const JVal &cfg, std::vector<char> &tab, std::vector<char
         const uint32_t x = compact(j), y = compact(j >> 1), z = compact(j >> 2);
         if (occ[lvl * vals + (size_t)x * 16384 + y * 128 + z]) bits[i / 8] |= (uint8_t)(1u << (i % 8));
     }
+    std::vector<uint32_t> cells(vals * s.grid_nlvl / 32, 0);
+    for (size_t i = 0; i < vals * s.grid_nlvl; ++i) {
+        if (!occ[i]) continue;
+        const uint32_t j = (uint32_t)(i % vals);
+        const size_t b = i / vals * vals + occupancy_bit_index(j >> 14, (j >> 7) & 127u, j & 127u);
+        cells[b / 32] |= 1u << (b % 32);
+    }
 
     /* weights -> fragment order */
     auto u16 = [](const std::vector<char> &v, size_t off_h, size_t n) {
@@ -777,6 +785,8 @@ static int build_model(const JVal &cfg, std::vector<char> &tab, std::vector<char
     CU(cudaDeviceGetAttribute(&m.n_sms, cudaDevAttrMultiProcessorCount, m.device));
     int rc;
     if ((rc = dalloc(&m.d_bits, bits.size(), "occupancy bits"))) return rc;
+    if ((rc = dalloc(&m.d_cells, cells.size(), "occupancy cells"))) return rc;
+    CU(cudaMemcpy(m.d_cells, cells.data(), cells.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     if ((rc = dalloc(&m.d_table, (size_t)off * (F / 2), "hash tables"))) return rc;
     if ((rc = dalloc(&m.d_weights, (size_t)W_TOTAL, "weights"))) return rc;
     if ((rc = dalloc(&m.d_bias3, (size_t)64, "bias"))) return rc;
@@ -1269,7 +1279,7 @@ static int setup_render_params(fvc_renderer *r, const fvc_raymarch_info *info, f
     p.steps = dev_steps(info->stepsize_info);
     p.cam = dev_cam_rm(*info);
     p.grid = m->grid;
-    p.bits = m->d_bits; p.table = m->d_table; p.weights = m->d_weights; p.bias3 = m->d_bias3;
+    p.bits = m->d_bits; p.cells = m->d_cells; p.table = m->d_table; p.weights = m->d_weights; p.bias3 = m->d_bias3;
     p.weights_tc = m->d_weights_tc;
     p.use_tc = r->use_tc;
     p.precision = r->precision;
@@ -1633,7 +1643,7 @@ extern "C" int fvc_cache_build(fvc_renderer *r, const fvc_raymarch_info *info)
     CacheBuildParams p;
     memset(&p, 0, sizeof(p));
     p.scene = m->dscene; p.steps = dev_steps(info->stepsize_info); p.cam = dev_cam(info->cam_info); p.grid = m->grid;
-    p.bits = m->d_bits; p.table = m->d_table; p.weights = m->d_weights; p.latent_offset = m->latent_offset;
+    p.bits = m->d_bits; p.cells = m->d_cells; p.table = m->d_table; p.weights = m->d_weights; p.latent_offset = m->latent_offset;
     p.variant = r->settings.interpol_variant;
     p.view_dependent = m->view_dependent;
     p.weights_fh = m->d_weights_fh;
@@ -1858,6 +1868,7 @@ int model_views(const fvc_model *m, RenderParams *p, int *head_hidden, int *n_sm
     p->scene = m->dscene;
     p->grid = m->grid;
     p->bits = m->d_bits;
+    p->cells = m->d_cells;
     p->table = m->d_table;
     p->weights = m->d_weights;
     p->weights_tc = m->d_weights_tc;

@@ -216,6 +216,41 @@ __device__ __forceinline__ void transform_ray(const float *m, float3 o, float3 d
     dc = make_float3(dot4(d.x, d.y, d.z, 0.0f, m), dot4(d.x, d.y, d.z, 0.0f, m + 4), dot4(d.x, d.y, d.z, 0.0f, m + 8));
 }
 
+/* packed fp32 pair arithmetic of sm_100+ (add/sub/fma .f32x2 on a 64-bit register pair) */
+__device__ __forceinline__ unsigned long long f2_bits(float2 a)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+    return r;
+}
+__device__ __forceinline__ float2 f2_from_bits(unsigned long long r)
+{
+    float2 a;
+    asm("mov.b64 {%0,%1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+    return a;
+}
+/* the pair's products, sums and fused products, each rounded to nearest.  A product must not feed a packed sum:
+ * ptxas contracts the two into a packed fused multiply-add, explicit rounding or not (measured: a quarter of random
+ * sums differ); a sum of a rounded product is written with the scalar intrinsics. */
+__device__ __forceinline__ float2 f2_mul(float2 a, float2 b)
+{
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return f2_from_bits(r);
+}
+__device__ __forceinline__ float2 f2_add(float2 a, float2 b)
+{
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return f2_from_bits(r);
+}
+__device__ __forceinline__ float2 f2_fma(float2 a, float2 b, float2 c)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c)));
+    return f2_from_bits(r);
+}
+
 /* --------------------------------------------------------------------- */
 /* occupancy grid (grid_occupied_at<128, true>, include/raymarch_common.h:660-710) */
 /* --------------------------------------------------------------------- */
@@ -266,7 +301,70 @@ __device__ __forceinline__ bool occupied(const DevScene &sc, const uint8_t *__re
     const int ix = cell_of(ax, mip), iy = cell_of(ay, mip), iz = cell_of(az, mip);
     const uint32_t idx = expand_bits3((uint32_t)ix) | (expand_bits3((uint32_t)iy) << 1) | (expand_bits3((uint32_t)iz) << 2);
     const uint32_t bidx = idx / 8u + (uint32_t)((128 * 128 * 128 / 8) * mip);
+    if (bidx >= (uint32_t)(128 * 128 * 128 / 8) * (uint32_t)sc.nlvl) return false; /* cell index 128 in the last cascade */
     return (__ldg(bits + bidx) >> (idx & 7u)) & 1u;
+}
+
+/* The occupancy cells again, as the march reads them: 32-bit words of 4 x 4 x 2
+ * cells (bit x & 3 | (y & 3) << 2 | (z & 1) << 4), words x fastest, then y, then
+ * z, cascade by cascade; filled from the Morton bits' source when a model is
+ * loaded.  A word's index is a sum of the cells' products, where the Morton
+ * index takes 18 shifts, products and masks; a word covers a compact block, so
+ * the rays of a warp still share words and lines. */
+__host__ __device__ __forceinline__ uint32_t occupancy_bit_index(uint32_t x, uint32_t y, uint32_t z)
+{
+    return x + (x >> 2) * 28u + y * 4u + (y >> 2) * 1008u + z * 16u + (z >> 1) * 32736u;
+}
+
+/* occupied() of the points o + tm[0] d and o + tm[1] d (two steps of a ray),
+ * as bits 0 and 1: the same arithmetic and the same outcome, with the two
+ * points' float operations issued as packed pairs.  The bits 2^(7 - mip) of
+ * the cascade's scale come from the exponent of the largest offset mx; adding
+ * 2^23 (2^25) and rounding towards zero leaves a cell coordinate (a quarter of
+ * it; 2^24: a half of it) in the sum's low bits.  A point whose cell
+ * coordinate may round up to 128, beyond the cascade's last cell, or whose
+ * offset is not finite, takes occupied() itself. */
+__device__ __forceinline__ uint32_t occupied2(const DevScene &sc, const uint8_t *__restrict__ bits, const uint32_t *__restrict__ cells,
+                                              float3 o, float3 d, float2 tm)
+{
+    float2 x = make_float2(F_ADD(o.x, F_MUL(tm.x, d.x)), F_ADD(o.x, F_MUL(tm.y, d.x)));
+    float2 y = make_float2(F_ADD(o.y, F_MUL(tm.x, d.y)), F_ADD(o.y, F_MUL(tm.y, d.y)));
+    float2 z = make_float2(F_ADD(o.z, F_MUL(tm.x, d.z)), F_ADD(o.z, F_MUL(tm.y, d.z)));
+    const float2 px = x, py = y, pz = z;
+    if (!sc.normalized) {
+        /* div_rn_by of (p - unit_off) by unit_den */
+        auto unit = [](float2 v, float off, float den, float rcp) {
+            const float2 n = f2_add(v, make_float2(-off, -off)), r = make_float2(rcp, rcp);
+            const float2 q = f2_mul(n, r);
+            return f2_fma(f2_fma(q, make_float2(-den, -den), n), r, q);
+        };
+        x = unit(x, sc.unit_off.x, sc.unit_den.x, sc.unit_rcp.x);
+        y = unit(y, sc.unit_off.y, sc.unit_den.y, sc.unit_rcp.y);
+        z = unit(z, sc.unit_off.z, sc.unit_den.z, sc.unit_rcp.z);
+    }
+    const float2 h = make_float2(-0.5f, -0.5f);
+    x = f2_add(x, h);
+    y = f2_add(y, h);
+    z = f2_add(z, h);
+    auto one = [&](float ax, float ay, float az, float wx, float wy, float wz) -> uint32_t {
+        const float mx = fmaxf(fmaxf(fabsf(ax), fabsf(ay)), fabsf(az));
+        /* 2^(7 - mip) as bits, mip = max(0, exponent field - 125) */
+        const uint32_t sb = min(134u << 23, (259u << 23) - (__float_as_uint(mx) & 0x7f800000u)); /* 259 << 23 needs 32 bits */
+        const float s = __uint_as_float(sb);
+        if (!(__fmaf_rn(mx, s, 64.0f) < 128.0f)) return occupied(sc, bits, make_float3(wx, wy, wz)) ? 1u : 0u;
+        if (sb < (135u - (uint32_t)sc.nlvl) << 23) return 0u; /* outside the last cascade */
+        const float cx = __fmaf_rn(ax, s, 64.0f), cy = __fmaf_rn(ay, s, 64.0f), cz = __fmaf_rn(az, s, 64.0f);
+        const uint32_t ix = __float_as_uint(__fadd_rz(cx, 8388608.0f)), qx = __float_as_uint(__fadd_rz(cx, 33554432.0f));
+        const uint32_t iy = __float_as_uint(__fadd_rz(cy, 8388608.0f)), qy = __float_as_uint(__fadd_rz(cy, 33554432.0f));
+        const uint32_t iz = __float_as_uint(__fadd_rz(cz, 8388608.0f)), qz = __float_as_uint(__fadd_rz(cz, 16777216.0f));
+        /* occupancy_bit_index of the cell, the sums' exponent bits taken out by the constant (mod 2^32), and the
+         * cascade's 2^21 bits: mip = 134 - (sb >> 23) */
+        const uint32_t bias = 0x4B000000u * (1u + 4u + 16u) + 0x4C000000u * (28u + 1008u) + 0x4B800000u * 32736u;
+        uint32_t idx = ix + qx * 28u + iy * 4u + qy * 1008u + iz * 16u + qz * 32736u - bias;
+        idx = (idx & 0x1fffffu) + ((134u << 21) - (sb >> 2));
+        return (__ldg(cells + (idx >> 5)) >> (idx & 31u)) & 1u;
+    };
+    return one(x.x, y.x, z.x, px.x, py.x, pz.x) | (one(x.y, y.y, z.y, px.y, py.y, pz.y) << 1);
 }
 
 /* occupied() plus, for an empty cell, the extent of empty space along the
@@ -372,19 +470,6 @@ __device__ __forceinline__ float3 cam2froxel(float3 c, const DevCam &cam, const 
 /* --------------------------------------------------------------------- */
 /* hash grid (Instant-NGP multiresolution hash encoding)                  */
 /* --------------------------------------------------------------------- */
-/* packed fp32 pair arithmetic of sm_100+ (add/sub/fma .f32x2 on a 64-bit register pair) */
-__device__ __forceinline__ unsigned long long f2_bits(float2 a)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(a.x), "f"(a.y));
-    return r;
-}
-__device__ __forceinline__ float2 f2_from_bits(unsigned long long r)
-{
-    float2 a;
-    asm("mov.b64 {%0,%1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
-    return a;
-}
 /* a + t * (b - a), each step rounded to nearest */
 __device__ __forceinline__ float2 f2_lerp(float2 a, float2 b, float t)
 {

@@ -166,13 +166,18 @@ __global__ void __launch_bounds__(64) cache_search_kernel(CacheBuildParams p)
             float t1 = t_from_step(p.steps, F_ADD((float)(bstep * 8), p.steps.near_i));
             mask = 0;
 #pragma unroll
-            for (int s = 0; s < 8; ++s) {
-                const float t0 = t1;
-                const float dt = calc_step(p.steps, t0);
-                t1 = F_ADD(t0, dt);
-                const float tm = F_MUL(F_ADD(t0, t1), 0.5f);
-                if (tm > cr.far_) cr.alive = 0;
-                else if (occupied(p.scene, p.bits, at(cr.o, cr.d, tm))) mask |= 1u << s;
+            for (int s = 0; s < 8; s += 2) {
+                float tm[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const float t0 = t1;
+                    t1 = F_ADD(t0, calc_step(p.steps, t0));
+                    tm[c] = F_MUL(F_ADD(t0, t1), 0.5f);
+                }
+                /* the midpoints grow: the steps past the far bound are the last ones */
+                const uint32_t in = (tm[0] > cr.far_ ? 0u : 1u) | (tm[1] > cr.far_ ? 0u : 2u);
+                if (in != 3u) cr.alive = 0;
+                if (in) mask |= (occupied2(p.scene, p.bits, p.cells, cr.o, cr.d, make_float2(tm[0], tm[1])) & in) << s;
             }
             if (__syncthreads_or(mask != 0u)) { found = true; break; }
             ++bstep;

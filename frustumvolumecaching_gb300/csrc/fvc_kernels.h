@@ -294,6 +294,7 @@ struct RenderParams {
     DevCam cam;
     DevGrid grid;
     const uint8_t *bits;        /* Morton occupancy bitfield */
+    const uint32_t *cells;      /* the same cells in 4 x 4 x 2 words (occupied2) */
     const __half2 *table;       /* hash tables, F = 2 */
     const uint2 *weights;       /* fragment-ordered MLP weights, W_TOTAL entries */
     const float *bias3;         /* head layer-1 bias from the 1-padding */
@@ -430,6 +431,7 @@ struct CacheBuildParams {
     DevCam cam;
     DevGrid grid;
     const uint8_t *bits;
+    const uint32_t *cells;      /* the same cells in 4 x 4 x 2 words (occupied2) */
     const __half2 *table;
     const uint2 *weights;
     int latent_offset;

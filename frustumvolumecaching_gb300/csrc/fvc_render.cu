@@ -411,11 +411,11 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
      * src/performance_renderer.cu:249 (the host keeps row_target <= row_capacity) */
     const int batch = p.row_target > 0 ? p.row_target : p.row_capacity;
     const int S = max(1, min(S_ROWS, batch / max(1, n_alive)));
+    __shared__ float t0s[S_ROWS][128]; /* the thread's samples, a column each */
     RayState *states = p.states[it & 1];
     for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
         const int i = base + threadIdx.x;
         const bool valid = i < n_alive;
-        float t0s[S_ROWS];
         int n = 0, steps = 0;
         float4 of = make_float4(0, 0, 0, 0), dt4 = make_float4(0, 0, 0, 0);
         bool done = false;
@@ -430,33 +430,44 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
             const float3 inv_d = make_float3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
             float t_free = -1e30f;
             for (int c0 = 0; c0 < p.steps_per_iter; c0 += 4) {
-                float t0c[4], t1c[4];
-                bool past[4], occ[4];
-                float tt = t1;
+                float t0c[5], tm[4];
+                t0c[0] = t1;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    t0c[c] = tt;
-                    const float dtc = calc_step(p.steps, tt);
-                    t1c[c] = F_ADD(tt, dtc);
-                    const float tm = F_MUL(F_ADD(tt, t1c[c]), 0.5f);
-                    past[c] = tm > of.w;
-                    bool oc = false;
-                    if (!past[c] && !(tm < t_free)) {
-                        if (p.skip_empty) oc = occupied_skip(p.scene, p.bits, o, d, inv_d, tm, dtc, t_free);
-                        else oc = occupied(p.scene, p.bits, at(o, d, tm));
+                    t0c[c + 1] = F_ADD(t0c[c], calc_step(p.steps, t0c[c]));
+                    tm[c] = F_MUL(F_ADD(t0c[c], t0c[c + 1]), 0.5f);
+                }
+                uint32_t occ = 0;
+                if (p.skip_empty) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (!(tm[c] > of.w) && !(tm[c] < t_free) &&
+                            occupied_skip(p.scene, p.bits, o, d, inv_d, tm[c], calc_step(p.steps, t0c[c]), t_free))
+                            occ |= 1u << c;
+                } else {
+                    occ = occupied2(p.scene, p.bits, p.cells, o, d, make_float2(tm[0], tm[1])) |
+                          (occupied2(p.scene, p.bits, p.cells, o, d, make_float2(tm[2], tm[3])) << 2);
+                }
+                /* the midpoints grow along the ray, so the last one tells whether the four steps end it */
+                if (!(tm[3] > of.w) && n + __popc(occ) < S) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) { /* an empty step's t0 is overwritten by the next */
+                        t0s[n][threadIdx.x] = t0c[c];
+                        n += (occ >> c) & 1u;
                     }
-                    occ[c] = oc;
-                    tt = t1c[c];
+                    t1 = t0c[4];
+                    steps += 4;
+                    continue;
                 }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     if (!done && n < S) {
                         ++steps;
-                        if (past[c]) {
+                        if (tm[c] > of.w) {
                             done = true;
                         } else {
-                            t1 = t1c[c];
-                            if (occ[c]) t0s[n++] = t0c[c];
+                            t1 = t0c[c + 1];
+                            if ((occ >> c) & 1u) t0s[n++][threadIdx.x] = t0c[c];
                         }
                     }
                 }
@@ -485,7 +496,7 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
             for (int s = 0; walk.step(r); ++s) {
                 int kind = KIND_SKIP;
                 if (r >= 0) {
-                    const float t0 = t0s[s];
+                    const float t0 = t0s[s][threadIdx.x];
                     const float dt = calc_step(p.steps, t0);
                     const float tm = F_MUL(F_ADD(t0, F_ADD(t0, dt)), 0.5f);
                     const float tmh = F_ADD(t0, F_MUL(dt, 0.5f));
@@ -528,7 +539,7 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
         } else {
             for (int s = 0; walk.step(r); ++s) {
                 if (r < 0) continue;
-                const float t0 = t0s[s];
+                const float t0 = t0s[s][threadIdx.x];
                 p.row_t0[r] = t0;
                 p.row_slot[r] = i;
                 if (!CACHED) {
