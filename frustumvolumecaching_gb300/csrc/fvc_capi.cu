@@ -397,6 +397,8 @@ struct PerRayScratch {
     }
 };
 
+constexpr int MARCH_STEPS = 64;
+
 struct fvc_renderer {
     fvc_model *m = nullptr;
     int kind = FVC_RENDERER_PERFORMANCE;
@@ -422,7 +424,8 @@ struct fvc_renderer {
     uint2 *d_row_out = nullptr;
     int *d_res_list = nullptr, *d_cache_list = nullptr;
     int *d_wf_counters = nullptr;
-    int row_capacity = 0;
+    int row_capacity = 0;             /* rows of the buffers: batch_rows for each march window */
+    int batch_rows = 0, windows = 1, ray_stride = 0;
     int last_iterations = 0;
     /* batched views in one graph launch */
     DevCam *d_views = nullptr;
@@ -434,7 +437,7 @@ struct fvc_renderer {
     int graph_head_hidden = 0;
     int graph_kernels = 0;            /* kernels of one loop body + prologue */
     bool last_was_graph = false;
-    int steps_per_iter = 64;          /* marching steps per sub-iteration */
+    int steps_per_iter = MARCH_STEPS; /* marching steps per window */
     int m_tile = 128;                 /* tcgen05 network tile of the plain path (autotuned) */
     /* the autotuner's candidates (fvc_renderer_set_autotune_space); the default is the batched workload's
      * stated space: tcgen05 tiles {64, 128, 256} x compaction batches 2^16..2^20, march lengths 16 and 64 */
@@ -458,7 +461,7 @@ struct fvc_renderer {
         dfree(d_states[0]); dfree(d_states[1]); dfree(d_ray_rows); dfree(d_row_t0); dfree(d_row_slot);
         dfree(d_row_kind); dfree(d_row_pay); dfree(d_row_out); dfree(d_res_list); dfree(d_cache_list); dfree(d_wf_counters);
         dfree(d_row_lat);
-        row_capacity = 0;
+        row_capacity = batch_rows = 0;
     }
     fvc_cache *cache = nullptr, *next = nullptr;
     fvc_cache_settings settings{0, 0, 1, 1, 1, 1};
@@ -1152,6 +1155,26 @@ extern "C" int fvc_renderer_set_stream(fvc_renderer *r, void *s)
     return FVC_OK;
 }
 
+/* March windows of a sub-iteration.  A sub-iteration's launches cost about
+ * 50 us whatever they hold, so an image with few rays marches several windows
+ * (64 steps or 16 samples each) of every ray before its rows go through the
+ * network: about 2^20 rays' worth of windows, at most MAX_WINDOWS (a whole ray
+ * of the 256x256 workload has 28).  Rays that end by opacity inside the
+ * sub-iteration have marched, and sent through the network, up to that many
+ * windows too far; images that fill the chip anyway keep one window, and the
+ * row buffers stay below those of a one-megapixel image.  Measured (us) with
+ * 1 window / 2^16 / 2^18 / 2^20 rays: plain 64x64 1453 / 674 / 630 / 630,
+ * 256x256 2450 / 2311 / 1837 / 1696, per-ray cached 640x360 with opaque
+ * surfaces 6403 / 6244 / 6239 / 5791, training step of 4099 rays 4583 / 4364 /
+ * 2521 / 2059. */
+#ifndef FVC_WINDOW_RAYS
+#define FVC_WINDOW_RAYS (1 << 20)
+#endif
+static int march_windows(size_t n_rays)
+{
+    return (int)std::min<size_t>(MAX_WINDOWS, std::max<size_t>(1, FVC_WINDOW_RAYS / n_rays));
+}
+
 extern "C" int fvc_renderer_resize(fvc_renderer *r, int width, int height)
 {
     CHECK_ARG(r && width > 0 && height > 0, "fvc_renderer_resize: bad arguments");
@@ -1169,11 +1192,14 @@ extern "C" int fvc_renderer_resize(fvc_renderer *r, int width, int height)
     r->release_wavefront();
     /* at least one row per ray: the march gives each alive ray
      * min(16, capacity / alive) rows, so capacity >= rays keeps that >= 1 */
-    const size_t cap = std::max(n, std::min<size_t>(n * 16, (size_t)1 << 25));
+    r->batch_rows = (int)std::max(n, std::min<size_t>(n * 16, (size_t)1 << 25));
+    r->windows = march_windows(n);
+    r->ray_stride = (int)n;
+    const size_t cap = (size_t)r->batch_rows * r->windows;
     const bool cached = is_cache_kind(r->kind);
     if ((rc = dalloc(&r->d_states[0], n, "ray states"))) return rc;
     if ((rc = dalloc(&r->d_states[1], n, "ray states"))) return rc;
-    if ((rc = dalloc(&r->d_ray_rows, n, "ray rows"))) return rc;
+    if ((rc = dalloc(&r->d_ray_rows, n * r->windows, "ray rows"))) return rc;
     if ((rc = dalloc(&r->d_row_t0, cap, "row t0"))) return rc;
     if ((rc = dalloc(&r->d_row_slot, cap, "row slots"))) return rc;
     if ((rc = dalloc(&r->d_row_pay, cap, "row inputs"))) return rc;
@@ -1325,12 +1351,14 @@ static int setup_render_params(fvc_renderer *r, const fvc_raymarch_info *info, f
     p.row_pay = r->d_row_pay; p.row_out = r->d_row_out; p.row_lat = r->d_row_lat;
     p.res_list = r->d_res_list; p.cache_list = r->d_cache_list;
     p.counters = r->d_wf_counters;
-    p.row_capacity = r->row_capacity;
     p.steps_per_iter = r->steps_per_iter;
     p.m_tile = r->m_tile;
     p.fused_classify = r->fused_classify;
     p.skip_empty = r->skip_empty;
-    p.row_target = std::min(r->row_target, r->row_capacity);
+    /* a set compaction batch or march length is one window's */
+    p.batch_rows = r->row_target > 0 ? std::min(r->row_target, r->batch_rows) : r->batch_rows;
+    p.windows = r->row_target > 0 || r->steps_per_iter != MARCH_STEPS ? 1 : r->windows;
+    p.ray_stride = r->ray_stride;
     p.by_sample = rows_by_sample(p);
     return FVC_OK;
 }
@@ -1742,7 +1770,8 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
     c->built = false;
     RenderParams p;
     if ((rc = setup_render_params(r, info, nullptr, nullptr, nullptr, p, true))) return rc;
-    p.steps_per_iter = 1 << 30; /* sample_common_kernel marches until it has its samples */
+    p.steps_per_iter = 1 << 26; /* sample_common_kernel marches until it has its samples */
+    p.windows = 1;
     PerRayScratch &x = r->pr;
     const size_t n_bricks = (size_t)c->bX * c->bY * c->bZ, n_cols = (size_t)c->bX * c->bY, n_rows = (size_t)r->row_capacity;
     if (x.n_bricks < n_bricks || x.n_cols < n_cols || x.n_rows < n_rows) {
@@ -1789,7 +1818,7 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
     int it = 0;
     for (; it < 1000 && n_alive > 0; ++it) { /* MAX_SUBITER */
         const int n_steps = std::min(8, std::max(1, (1 << 21) / n_alive)); /* TARGET_BATCH_SIZE / n_alive */
-        p.row_capacity = n_steps * n_alive;                                 /* the march gives every ray n_steps rows */
+        p.batch_rows = n_steps * n_alive;                                   /* the march gives every ray n_steps rows */
         n_samples += ((long long)n_alive * n_steps + 255) / 256 * 256;     /* next_multiple(batch, 256) */
         CU(cudaMemsetAsync(p.counters + 2, 0, sizeof(int), s));
         CU(launch_fill_march(p, it, n_sms, s));

@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(128) pr_write_kernel(PerRayFillParams p, int i
             st = states[i];
             id = st.cnt.x;
             T = st.acc.w;
-            alive = st.cnt2.y == 0; /* the march ended the ray past its far bound */
+            alive = !window_done(p.ray_rows[i].y); /* the march ended the ray past its far bound */
         }
         RowWalk walk(valid ? p.ray_rows[i] : make_int2(0, 0), valid, p.by_sample);
         while (walk.step(row)) {

@@ -210,7 +210,7 @@ struct __align__(16) RayState {
     float4 acc;   /* rgb, transmittance */
     float4 comp;  /* Kahan compensation of the rgb sums */
     int4 cnt;     /* pixel id, composited resample, composited cache, steps */
-    int4 cnt2;    /* dropped, done flag, samples pushed, - */
+    int4 cnt2;    /* dropped, -, samples pushed (when they are limited), view */
 };
 
 struct RenderStatsDev {
@@ -233,6 +233,15 @@ __device__ __forceinline__ int lanes_before(int n)
     return sum - n;
 }
 
+constexpr int MAX_WINDOWS = 31; /* march windows of a sub-iteration */
+
+/* A ray's share of one march window: its warp's first row and, packed, its
+ * row count, the steps it marched and whether it passed its far bound. */
+__host__ __device__ __forceinline__ int window_pack(int n, int steps, bool done) { return n | (steps << 5) | (int)((done ? 1u : 0u) << 31); }
+__host__ __device__ __forceinline__ int window_rows(int w) { return w & 31; }
+__host__ __device__ __forceinline__ int window_steps(int w) { return (w & 0x7fffffff) >> 5; }
+__host__ __device__ __forceinline__ bool window_done(int w) { return w < 0; }
+
 /* Where the rows of a sub-iteration lie.  A warp's rows follow each other from
  * its first row, either ray by ray (a ray's samples adjacent) or, by_sample,
  * the first sample of every lane that has one, then the second samples, and
@@ -243,7 +252,7 @@ __device__ __forceinline__ int lanes_before(int n)
 struct RowWalk {
     int n, j, next;
     bool by_sample;
-    __device__ __forceinline__ RowWalk(int2 rr, bool valid, bool by) : n(valid ? rr.y : 0), j(0), next(rr.x), by_sample(by)
+    __device__ __forceinline__ RowWalk(int2 rr, bool valid, bool by) : n(valid ? window_rows(rr.y) : 0), j(0), next(rr.x), by_sample(by)
     {
         if (!by) next += lanes_before(n);
     }
@@ -321,7 +330,11 @@ struct RenderParams {
     int render_mode;            /* 0 default, 1 only cache, 2 only resampled */
     /* wavefront buffers */
     RayState *states[2];        /* alive rays, ping-pong between sub-iterations */
-    int2 *ray_rows;             /* per alive ray: first row of its warp, its number of rows (in t order; RowWalk) */
+    int2 *ray_rows;             /* [windows][ray_stride] per alive ray: first row of its warp, window_pack of its share */
+    int windows;                /* march windows (steps_per_iter steps, at most S_ROWS samples) of a sub-iteration */
+    int ray_stride;
+    int batch_rows;             /* rows a window aims at over all rays: samples per ray and window = clamp(batch_rows /
+                                 * alive rays, 1, S_ROWS) */
     float *row_t0;              /* per row: t0 of the sample */
     int *row_slot;              /* per row: alive slot of its ray */
     uint8_t *row_kind;          /* per row: resample / cache / known empty / skipped */
@@ -330,15 +343,12 @@ struct RenderParams {
     uint4 *row_lat;             /* per place in the cache list: the 8 looked-up head inputs from K = latent_offset (fp16) */
     int *res_list, *cache_list; /* row ids of the two network streams */
     int *counters;              /* [0], [1] alive rays (ping-pong), [2] rows, [3] resample, [4] cache */
-    int row_capacity;           /* rows per sub-iteration */
     int by_sample;              /* a warp's rows sample by sample instead of ray by ray (RowWalk) */
     int steps_per_iter;         /* marching steps per ray and sub-iteration */
     int m_tile;                 /* rows per tcgen05 network tile on the plain path: 64, 128 (0 = 128) or 256 */
     int fused_classify;         /* cached renders: classification in the march, one network launch for all rows */
     int skip_empty;             /* the march skips occupancy lookups inside empty cells (exact: occupied_skip) */
     float *contrib_res, *contrib_cache; /* cached renders: per-pixel compositing weight of resample / cache samples (added) */
-    int row_target;             /* compaction batch: rows per sub-iteration the march aims at, samples per ray
-                                 * = clamp(row_target / alive rays, 1, S_ROWS) (0 = row_capacity) */
     int basic_cache;            /* 1: CacheBasicRenderer semantics for the cached rows (classify_basic) */
     int view_dependent;         /* split head (mlp_first_head): first head + SH-difference head input */
     int freq;                   /* the head's positional frequency encoding degree (0, or 4: the TCF_* tile layout) */
@@ -493,7 +503,7 @@ struct PerRayFillParams {
     DevSteps steps;
     int W, H;
     RayState *states[2];        /* the renderer's alive-ray states (ping-pong) */
-    const int2 *ray_rows;       /* per alive ray: first row of its warp, its number of rows (RowWalk) */
+    const int2 *ray_rows;       /* per alive ray: first row of its warp, window_pack of its share (one window) */
     int by_sample;              /* the order of a warp's rows (RowWalk) */
     const float *row_t0;
     const __half *den;          /* per row: log-density (fp16) */

@@ -144,7 +144,9 @@ extern "C" int fvc_render_noalloc(fvc_model *m, const fvc_raymarch_info *info, c
     p.ray_counter = ctl;
     p.guard = ctl + 1;
     p.stats = stats;
-    p.row_capacity = (int)cap;
+    p.batch_rows = (int)cap;
+    p.windows = 1;
+    p.ray_stride = (int)n;
     p.steps_per_iter = 64;
     p.skip_empty = 0;
     p.results = out ? (float4 *)out->results : nullptr;

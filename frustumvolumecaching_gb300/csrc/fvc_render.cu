@@ -40,7 +40,8 @@ namespace fvc {
 
 constexpr unsigned FULLMASK = 0xffffffffu;
 constexpr int S_ROWS = 16;        /* rows per ray and sub-iteration (the reference keeps up to 8) */
-static_assert(S_ROWS < 256, "the compositing kernel counts a ray's rows per miss reason in 8-bit fields");
+static_assert(S_ROWS * MAX_WINDOWS < 512, "the compositing kernel counts a ray's rows per miss reason in 9-bit fields");
+static_assert(S_ROWS < 32, "window_pack holds a window's rows in 5 bits");
 constexpr int NET_WARPS = 8;
 /* tcgen05 network kernel: CTAs resident per SM (launch bound and grid) and
  * hash levels whose gathers are in flight together.  Measured at 1080p on the
@@ -405,164 +406,171 @@ template <bool CACHED, bool FUSED = false>
 __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
 {
     const int n_alive = p.counters[it & 1];
-    if (blockIdx.x == 0 && threadIdx.x == 0) p.counters[(it + 1) & 1] = 0; /* next alive count */
-    /* samples per ray this sub-iteration: the compaction batch (row_target, else the row capacity)
-     * over the alive rays, clamped to [1, S_ROWS] as n_steps_curr_subiter of
-     * src/performance_renderer.cu:249 (the host keeps row_target <= row_capacity) */
-    const int batch = p.row_target > 0 ? p.row_target : p.row_capacity;
-    const int S = max(1, min(S_ROWS, batch / max(1, n_alive)));
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        p.counters[(it + 1) & 1] = 0;        /* next alive count */
+        p.counters[6] = p.counters[7] = 0;   /* the gradient rows of the sub-iteration before are consumed */
+    }
+    /* samples per ray and window: the batch over the alive rays, clamped to [1, S_ROWS] as
+     * n_steps_curr_subiter of src/performance_renderer.cu:249 */
+    const int S = max(1, min(S_ROWS, p.batch_rows / max(1, n_alive)));
     __shared__ float t0s[S_ROWS][128]; /* the thread's samples, a column each */
     RayState *states = p.states[it & 1];
     for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
         const int i = base + threadIdx.x;
         const bool valid = i < n_alive;
-        int n = 0, steps = 0;
         float4 of = make_float4(0, 0, 0, 0), dt4 = make_float4(0, 0, 0, 0);
-        bool done = false;
         if (valid) {
             of = states[i].of;
             dt4 = states[i].dt;
-            const float3 o = make_float3(of.x, of.y, of.z), d = make_float3(dt4.x, dt4.y, dt4.z);
-            float t1 = dt4.w;
-            /* empty-space skipping: steps whose midpoint lies before t_free are in an empty cell
-             * (occupied_skip's conservative DDA bound) and skip the occupancy lookup; the step
-             * sequence and every occupancy outcome stay those of the plain march */
-            const float3 inv_d = make_float3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
-            float t_free = -1e30f;
-            for (int c0 = 0; c0 < p.steps_per_iter; c0 += 4) {
-                float t0c[5], tm[4];
-                t0c[0] = t1;
+        }
+        bool done = !valid;
+        int all_steps = 0, all_rows = 0;
+        for (int w = 0; w < p.windows; ++w) {
+            int n = 0, steps = 0;
+            if (!done) {
+                const float3 o = make_float3(of.x, of.y, of.z), d = make_float3(dt4.x, dt4.y, dt4.z);
+                float t1 = dt4.w;
+                /* empty-space skipping: steps whose midpoint lies before t_free are in an empty cell
+                 * (occupied_skip's conservative DDA bound) and skip the occupancy lookup; the step
+                 * sequence and every occupancy outcome stay those of the plain march */
+                const float3 inv_d = make_float3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
+                float t_free = -1e30f;
+                for (int c0 = 0; c0 < p.steps_per_iter; c0 += 4) {
+                    float t0c[5], tm[4];
+                    t0c[0] = t1;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    t0c[c + 1] = F_ADD(t0c[c], calc_step(p.steps, t0c[c]));
-                    tm[c] = F_MUL(F_ADD(t0c[c], t0c[c + 1]), 0.5f);
-                }
-                uint32_t occ = 0;
-                if (p.skip_empty) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        if (!(tm[c] > of.w) && !(tm[c] < t_free) &&
-                            occupied_skip(p.scene, p.bits, o, d, inv_d, tm[c], calc_step(p.steps, t0c[c]), t_free))
-                            occ |= 1u << c;
-                } else {
-                    occ = occupied2(p.scene, p.bits, p.cells, o, d, make_float2(tm[0], tm[1])) |
-                          (occupied2(p.scene, p.bits, p.cells, o, d, make_float2(tm[2], tm[3])) << 2);
-                }
-                /* the midpoints grow along the ray, so the last one tells whether the four steps end it */
-                if (!(tm[3] > of.w) && n + __popc(occ) < S) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) { /* an empty step's t0 is overwritten by the next */
-                        t0s[n][threadIdx.x] = t0c[c];
-                        n += (occ >> c) & 1u;
+                    for (int c = 0; c < 4; ++c) {
+                        t0c[c + 1] = F_ADD(t0c[c], calc_step(p.steps, t0c[c]));
+                        tm[c] = F_MUL(F_ADD(t0c[c], t0c[c + 1]), 0.5f);
                     }
-                    t1 = t0c[4];
-                    steps += 4;
-                    continue;
-                }
+                    uint32_t occ = 0;
+                    if (p.skip_empty) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    if (!done && n < S) {
-                        ++steps;
-                        if (tm[c] > of.w) {
-                            done = true;
-                        } else {
-                            t1 = t0c[c + 1];
-                            if ((occ >> c) & 1u) t0s[n++][threadIdx.x] = t0c[c];
+                        for (int c = 0; c < 4; ++c)
+                            if (!(tm[c] > of.w) && !(tm[c] < t_free) &&
+                                occupied_skip(p.scene, p.bits, o, d, inv_d, tm[c], calc_step(p.steps, t0c[c]), t_free))
+                                occ |= 1u << c;
+                    } else {
+                        occ = occupied2(p.scene, p.bits, p.cells, o, d, make_float2(tm[0], tm[1])) |
+                              (occupied2(p.scene, p.bits, p.cells, o, d, make_float2(tm[2], tm[3])) << 2);
+                    }
+                    /* the midpoints grow along the ray, so the last one tells whether the four steps end it */
+                    if (!(tm[3] > of.w) && n + __popc(occ) < S) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) { /* an empty step's t0 is overwritten by the next */
+                            t0s[n][threadIdx.x] = t0c[c];
+                            n += (occ >> c) & 1u;
+                        }
+                        t1 = t0c[4];
+                        steps += 4;
+                        continue;
+                    }
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        if (!done && n < S) {
+                            ++steps;
+                            if (tm[c] > of.w) {
+                                done = true;
+                            } else {
+                                t1 = t0c[c + 1];
+                                if ((occ >> c) & 1u) t0s[n++][threadIdx.x] = t0c[c];
+                            }
                         }
                     }
+                    if (done || n >= S) break;
                 }
-                if (done || n >= S) break;
+                dt4.w = t1;
             }
-            dt4.w = t1;
-        }
-        const int n_warp = (int)__reduce_add_sync(FULLMASK, (unsigned)n);
-        int rbase = 0;
-        if (lane_id() == 0 && n_warp) rbase = atomicAdd(p.counters + 2, n_warp);
-        rbase = __shfl_sync(FULLMASK, rbase, 0);
-        RowWalk walk(make_int2(rbase, n), true, p.by_sample);
-        int r;
-        if (FUSED) {
-            /* the cached renderer's classification of the rows (wf_classify_kernel's non-basic
-             * form), with the ray moved into the cache camera once per ray */
-            const ViewCache *vc = p.view_caches && valid ? p.view_caches + states[i].cnt2.w : nullptr;
-            const CacheView &C = vc ? vc->cache : p.cache;
-            const DevCam &ccam = vc ? vc->ccam : p.ccam;
-            const DevSteps &cst = vc ? vc->csteps : p.csteps;
-            const float3 o = make_float3(of.x, of.y, of.z), d = make_float3(dt4.x, dt4.y, dt4.z);
-            float3 oc, dc;
-            transform_ray(ccam.w2c, o, d, oc, dc);
-            int n_res = 0, n_hit = 0;
-            uint32_t kinds = 0; /* 2 bits per row, its kind */
-            for (int s = 0; walk.step(r); ++s) {
-                int kind = KIND_SKIP;
-                if (r >= 0) {
-                    const float t0 = t0s[s][threadIdx.x];
-                    const float dt = calc_step(p.steps, t0);
-                    const float tm = F_MUL(F_ADD(t0, F_ADD(t0, dt)), 0.5f);
-                    const float tmh = F_ADD(t0, F_MUL(dt, 0.5f));
-                    const int code = classify(p, C, ccam, cst, oc, dc, tm);
-                    kind = row_kind_of(code);
-                    float4 pay = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (kind == KIND_RESAMPLE) {
-                        const float3 pc = contract(p.scene, at(o, d, tmh));
-                        pay = make_float4(pc.x, pc.y, pc.z, 0.f);
-                    } else if (kind == KIND_CACHE) {
-                        float tf2;
-                        const float3 fr = cam2froxel(at(oc, dc, tmh), ccam, cst, tf2);
-                        pay = make_float4(fr.x, fr.y, fr.z, 0.f);
+            const int n_warp = (int)__reduce_add_sync(FULLMASK, (unsigned)n);
+            int rbase = 0;
+            if (lane_id() == 0 && n_warp) rbase = atomicAdd(p.counters + 2, n_warp);
+            rbase = __shfl_sync(FULLMASK, rbase, 0);
+            RowWalk walk(make_int2(rbase, window_pack(n, 0, false)), true, p.by_sample);
+            int r;
+            if (FUSED) {
+                /* the cached renderer's classification of the rows (wf_classify_kernel's non-basic
+                 * form), with the ray moved into the cache camera once per ray */
+                const ViewCache *vc = p.view_caches && valid ? p.view_caches + states[i].cnt2.w : nullptr;
+                const CacheView &C = vc ? vc->cache : p.cache;
+                const DevCam &ccam = vc ? vc->ccam : p.ccam;
+                const DevSteps &cst = vc ? vc->csteps : p.csteps;
+                const float3 o = make_float3(of.x, of.y, of.z), d = make_float3(dt4.x, dt4.y, dt4.z);
+                float3 oc, dc;
+                transform_ray(ccam.w2c, o, d, oc, dc);
+                int n_res = 0, n_hit = 0;
+                uint32_t kinds = 0; /* 2 bits per row, its kind */
+                for (int s = 0; walk.step(r); ++s) {
+                    int kind = KIND_SKIP;
+                    if (r >= 0) {
+                        const float t0 = t0s[s][threadIdx.x];
+                        const float dt = calc_step(p.steps, t0);
+                        const float tm = F_MUL(F_ADD(t0, F_ADD(t0, dt)), 0.5f);
+                        const float tmh = F_ADD(t0, F_MUL(dt, 0.5f));
+                        const int code = classify(p, C, ccam, cst, oc, dc, tm);
+                        kind = row_kind_of(code);
+                        float4 pay = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (kind == KIND_RESAMPLE) {
+                            const float3 pc = contract(p.scene, at(o, d, tmh));
+                            pay = make_float4(pc.x, pc.y, pc.z, 0.f);
+                        } else if (kind == KIND_CACHE) {
+                            float tf2;
+                            const float3 fr = cam2froxel(at(oc, dc, tmh), ccam, cst, tf2);
+                            pay = make_float4(fr.x, fr.y, fr.z, 0.f);
+                        }
+                        p.row_t0[r] = t0;
+                        p.row_slot[r] = i;
+                        p.row_pay[r] = pay;
+                        p.row_kind[r] = (uint8_t)code;
+                        kinds |= (uint32_t)kind << (2 * s);
                     }
+                    n_res += kind == KIND_RESAMPLE;
+                    n_hit += kind == KIND_CACHE;
+                }
+                /* the resample rows and the cache rows each go to a list, so that the network's tiles hold one
+                 * kind of row: a cache row never waits on its tile's hash gathers */
+                const int w_res = (int)__reduce_add_sync(FULLMASK, (unsigned)n_res), w_hit = (int)__reduce_add_sync(FULLMASK, (unsigned)n_hit);
+                int rb = 0, hb = 0;
+                if (lane_id() == 0) {
+                    if (w_res) rb = atomicAdd(p.counters + 3, w_res);
+                    if (w_hit) hb = atomicAdd(p.counters + 4, w_hit);
+                }
+                ListWalk res(__shfl_sync(FULLMASK, rb, 0), n_res, p.by_sample), hit(__shfl_sync(FULLMASK, hb, 0), n_hit, p.by_sample);
+                RowWalk again(make_int2(rbase, window_pack(n, 0, false)), true, p.by_sample);
+                for (int s = 0; again.step(r); ++s) {
+                    const uint32_t kind = r >= 0 ? (kinds >> (2 * s)) & 3u : (uint32_t)KIND_SKIP;
+                    const int at_res = res.place(kind == KIND_RESAMPLE), at_hit = hit.place(kind == KIND_CACHE);
+                    if (kind == KIND_RESAMPLE) p.res_list[at_res] = r;
+                    else if (kind == KIND_CACHE) p.cache_list[at_hit] = r;
+                }
+            } else {
+                for (int s = 0; walk.step(r); ++s) {
+                    if (r < 0) continue;
+                    const float t0 = t0s[s][threadIdx.x];
                     p.row_t0[r] = t0;
                     p.row_slot[r] = i;
-                    p.row_pay[r] = pay;
-                    p.row_kind[r] = (uint8_t)code;
-                    kinds |= (uint32_t)kind << (2 * s);
-                }
-                n_res += kind == KIND_RESAMPLE;
-                n_hit += kind == KIND_CACHE;
-            }
-            /* the resample rows and the cache rows each go to a list, so that the network's tiles hold one
-             * kind of row: a cache row never waits on its tile's hash gathers */
-            const int w_res = (int)__reduce_add_sync(FULLMASK, (unsigned)n_res), w_hit = (int)__reduce_add_sync(FULLMASK, (unsigned)n_hit);
-            int rb = 0, hb = 0;
-            if (lane_id() == 0) {
-                if (w_res) rb = atomicAdd(p.counters + 3, w_res);
-                if (w_hit) hb = atomicAdd(p.counters + 4, w_hit);
-            }
-            ListWalk res(__shfl_sync(FULLMASK, rb, 0), n_res, p.by_sample), hit(__shfl_sync(FULLMASK, hb, 0), n_hit, p.by_sample);
-            RowWalk again(make_int2(rbase, n), true, p.by_sample);
-            for (int s = 0; again.step(r); ++s) {
-                const uint32_t kind = r >= 0 ? (kinds >> (2 * s)) & 3u : (uint32_t)KIND_SKIP;
-                const int at_res = res.place(kind == KIND_RESAMPLE), at_hit = hit.place(kind == KIND_CACHE);
-                if (kind == KIND_RESAMPLE) p.res_list[at_res] = r;
-                else if (kind == KIND_CACHE) p.cache_list[at_hit] = r;
-            }
-        } else {
-            for (int s = 0; walk.step(r); ++s) {
-                if (r < 0) continue;
-                const float t0 = t0s[s][threadIdx.x];
-                p.row_t0[r] = t0;
-                p.row_slot[r] = i;
-                if (!CACHED) {
-                    /* sample_performance_kernel :52-58: midpoint (t0+t1)/2, contracted */
-                    const float tm = F_MUL(F_ADD(t0, F_ADD(t0, calc_step(p.steps, t0))), 0.5f);
-                    const float3 pc = contract(p.scene, at(make_float3(of.x, of.y, of.z), make_float3(dt4.x, dt4.y, dt4.z), tm));
-                    p.row_pay[r] = make_float4(pc.x, pc.y, pc.z, 0.f);
+                    if (!CACHED) {
+                        /* sample_performance_kernel :52-58: midpoint (t0+t1)/2, contracted */
+                        const float tm = F_MUL(F_ADD(t0, F_ADD(t0, calc_step(p.steps, t0))), 0.5f);
+                        const float3 pc = contract(p.scene, at(make_float3(of.x, of.y, of.z), make_float3(dt4.x, dt4.y, dt4.z), tm));
+                        p.row_pay[r] = make_float4(pc.x, pc.y, pc.z, 0.f);
+                    }
                 }
             }
+            if (valid) p.ray_rows[(size_t)w * p.ray_stride + i] = make_int2(rbase, window_pack(n, steps, done));
+            all_steps += steps;
+            all_rows += n;
+            /* a warp whose rays have all ended leaves; the compositing stops at its rays' done flags too */
+            if (__all_sync(FULLMASK, done)) break;
         }
         if (valid) {
-            p.ray_rows[i] = make_int2(rbase, n);
-            states[i].dt = dt4;
-            int4 c = states[i].cnt;
-            c.w += steps;
-            states[i].cnt = c;
-            int4 c2 = states[i].cnt2;
-            c2.y = done ? 1 : 0;
-            c2.z += n;
-            states[i].cnt2 = c2;
-            if (p.max_samples_per_ray > 0 && c2.z > p.max_samples_per_ray) atomicOr(p.guard, 1);
+            states[i].dt.w = dt4.w;
+            if (p.max_samples_per_ray > 0) {
+                const int pushed = states[i].cnt2.z + all_rows;
+                states[i].cnt2.z = pushed;
+                if (pushed > p.max_samples_per_ray) atomicOr(p.guard, 1);
+            }
         }
-        const int ws = __reduce_add_sync(FULLMASK, steps);
+        const int ws = __reduce_add_sync(FULLMASK, all_steps);
         if (lane_id() == 0 && ws) atomicAdd(&p.stats->n_steps, (unsigned long long)ws);
     }
 }
@@ -1018,7 +1026,9 @@ __global__ void __launch_bounds__(128, FVC_TC_CTAS_PER_SM) wf_net_tc_kernel(Rend
     TcSmem &S = *reinterpret_cast<TcSmem *>(smem_raw);
     const int n_rows = MODE == 0 ? (LIST ? p.counters[3] : p.counters[2]) : MODE == 1 ? p.counters[4] : p.counters[3];
     const int n_hit = MODE == 2 ? p.counters[4] : 0;
-    if (n_rows == 0 && n_hit == 0) return;
+    const int res_tiles = (n_rows + 127) / 128;
+    const int n_tiles = res_tiles + (n_hit + 127) / 128;
+    if ((int)blockIdx.x >= n_tiles) return; /* a CTA without a tile fetches no weights and allocates no TMEM */
     const int tid = threadIdx.x, warp = tid >> 5;
     /* the weights arrive by one bulk copy on the TMA engine, completing the
      * mbarrier's phase 0; the layers' MMA commits complete the later phases */
@@ -1042,8 +1052,6 @@ __global__ void __launch_bounds__(128, FVC_TC_CTAS_PER_SM) wf_net_tc_kernel(Rend
     uint32_t phase = 0;
     bool ok = mbar_wait(&S.mbar, phase, TC_WAIT_LIMIT);
     phase ^= 1u;
-    const int res_tiles = (n_rows + 127) / 128;
-    const int n_tiles = res_tiles + (n_hit + 127) / 128;
     for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
         int k = tile * 128 + tid, r = -1, kind = KIND_RESAMPLE;
         if (MODE == 2 && tile >= res_tiles) {
@@ -1533,7 +1541,7 @@ __global__ void __launch_bounds__(128, TC_PREC_CTAS_PER_SM) wf_net_tc_prec_kerne
     extern __shared__ __align__(128) unsigned char smem_raw[];
     TcSmem &S = *reinterpret_cast<TcSmem *>(smem_raw);
     const int n_rows = p.counters[2];
-    if (n_rows == 0) return;
+    if ((int)blockIdx.x * 128 >= n_rows) return;
     const int tid = threadIdx.x, warp = tid >> 5;
     const uint8_t *wsrc = PREC == 1 ? p.weights_tc_bf16 : p.weights_tc_fp8;
     const int wbytes = PREC == 1 ? TC_WBYTES : TC8_WBYTES;
@@ -1644,12 +1652,33 @@ __global__ void __launch_bounds__(128, TC_PREC_CTAS_PER_SM) wf_net_tc_prec_kerne
 /* ------------------------------------------------------------------------- */
 /* composite + compaction                                                    */
 /* ------------------------------------------------------------------------- */
+/* counts the sub-iteration's rows and clears their counters */
+__device__ __forceinline__ void reset_row_counters(const RenderParams &p, bool cached)
+{
+    const int rows = p.counters[2], res = p.counters[3], hits = p.counters[4];
+    atomicAdd(&p.stats->n_resamples, (unsigned long long)(cached ? res : rows));
+    atomicAdd(&p.stats->n_cache_hits, (unsigned long long)hits);
+    atomicAdd(&p.stats->n_dropped, (unsigned long long)(cached ? rows - res - hits : 0));
+    p.counters[2] = 0;
+    p.counters[3] = 0;
+    p.counters[4] = 0;
+}
+
+/* the same as a node of the batch graph, where a launch costs little; elsewhere the compositing's first thread does
+ * it: the compositing is the last kernel of a sub-iteration, its network launches have read the counters, and it
+ * reads none of them itself */
+__global__ void wf_reset_rows_kernel(RenderParams p, int cached)
+{
+    if (threadIdx.x == 0) reset_row_counters(p, cached);
+}
+
 constexpr int COMP_AHEAD = 4; /* samples of a ray whose rows the compositing loads together */
 
 template <bool CACHED>
 __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int it)
 {
     const int n_alive = p.counters[it & 1];
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p, CACHED);
     RayState *cur = p.states[it & 1], *nxt = p.states[(it + 1) & 1];
     for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
         const int i = base + threadIdx.x;
@@ -1657,74 +1686,82 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
         bool keep = false;
         RayState st;
         int n_comp = 0;
-        unsigned long long why = 0; /* rows per REASON_* 1..7, 8 bits each (at most S_ROWS rows a ray and sub-iteration) */
-        int2 rr = make_int2(0, 0);
+        unsigned long long why = 0; /* rows per REASON_* 1..7, 9 bits each (at most MAX_WINDOWS * S_ROWS a ray and sub-iteration) */
         float4 acc = make_float4(0.f, 0.f, 0.f, 1.f), comp = make_float4(0.f, 0.f, 0.f, 0.f);
-        int c_res = 0, c_cache = 0, c_drop = 0;
+        int c_res = 0, c_cache = 0, c_drop = 0, c_steps = 0;
         if (valid) {
             st = cur[i];
-            rr = p.ray_rows[i];
             acc = st.acc;
             comp = st.comp;
             c_res = st.cnt.y;
             c_cache = st.cnt.z;
             c_drop = st.cnt2.x;
+            c_steps = st.cnt.w;
         }
         float w_res = 0.f, w_cache = 0.f; /* this sub-iteration's contribution weights (DEBUG form, :867-871) */
-        bool term = false;
-        /* rows are in t order: the merge of the resample and cache streams of
-         * accumulate_cache_perf_kernel (:270-304); COMP_AHEAD samples are loaded together, before the
-         * first of them is composited */
-        RowWalk walk(rr, valid, p.by_sample);
-        for (bool more = true; more;) {
-            int rs[COMP_AHEAD], codes[COMP_AHEAD];
-            uint2 ovs[COMP_AHEAD];
-            float t0s[COMP_AHEAD];
-#pragma unroll
-            for (int q = 0; q < COMP_AHEAD; ++q) {
-                more = walk.step(rs[q]) && more;
-                if (term) rs[q] = -1;
-                codes[q] = CACHED && rs[q] >= 0 ? (int)p.row_kind[rs[q]] : KIND_RESAMPLE;
-                ovs[q] = make_uint2(0u, 0u);
-                t0s[q] = 0.f;
-                if (rs[q] >= 0) { /* a dropped row's output is not written, and not used */
-                    ovs[q] = p.row_out[rs[q]];
-                    t0s[q] = p.row_t0[rs[q]];
-                }
+        bool term = false, done = !valid; /* ended by opacity; the march passed the far bound */
+        for (int w = 0; w < p.windows; ++w) {
+            int2 rr = make_int2(0, 0);
+            if (!done) { /* also of a ray that has ended: the others' rows follow its own */
+                rr = p.ray_rows[(size_t)w * p.ray_stride + i];
+                if (!term) c_steps += window_steps(rr.y);
+                done = window_done(rr.y);
             }
+            /* rows are in t order: the merge of the resample and cache streams of
+             * accumulate_cache_perf_kernel (:270-304); COMP_AHEAD samples are loaded together, before the
+             * first of them is composited */
+            RowWalk walk(rr, true, p.by_sample);
+            for (bool more = true; more;) {
+                int rs[COMP_AHEAD], codes[COMP_AHEAD];
+                uint2 ovs[COMP_AHEAD];
+                float t0s[COMP_AHEAD];
 #pragma unroll
-            for (int q = 0; q < COMP_AHEAD; ++q) {
-                if (rs[q] < 0 || term) continue;
-                const int kind = row_kind_of(codes[q]);
-                if (CACHED && kind != KIND_SKIP && row_reason_of(codes[q])) why += 1ull << ((8 * (row_reason_of(codes[q]) - 1)) & 63);
-                if (kind >= KIND_DROP) {
-                    c_drop += kind == KIND_DROP;
-                    continue;
-                }
-                if (kind == KIND_CACHE) ++c_cache; else ++c_res;
-                ++n_comp;
-                const uint2 ov = ovs[q];
-                const float2 rg = __half22float2(*reinterpret_cast<const __half2 *>(&ov.x));
-                const float lb = __half2float(__ushort_as_half((unsigned short)(ov.y & 0xffffu)));
-                const float ld = __half2float(__ushort_as_half((unsigned short)(ov.y >> 16)));
-                const float dt = calc_step(p.steps, t0s[q]);
-                /* the basic cache renderer composites a cache row with its looked-up density
-                 * (accumulate_cache_render_kernel, src/cache_basic_renderer.cu:255-258) */
-                const float sigma = CACHED && p.basic_cache && kind == KIND_CACHE ? p.row_pay[rs[q]].w : expf(ld);
-                const float alpha = fminf(1.0f, fmaxf(0.0f, 1.0f - expf(-sigma * dt)));
-                if (alpha > p.scene.alpha_thre) {
-                    const float wgt = alpha * acc.w;
-                    kahan_add(acc.x, comp.x, wgt / (1.0f + expf(-rg.x)));
-                    kahan_add(acc.y, comp.y, wgt / (1.0f + expf(-rg.y)));
-                    kahan_add(acc.z, comp.z, wgt / (1.0f + expf(-lb)));
-                    acc.w *= 1.0f - alpha;
-                    if (CACHED) {
-                        if (kind == KIND_CACHE) w_cache += wgt;
-                        else w_res += wgt;
+                for (int q = 0; q < COMP_AHEAD; ++q) {
+                    more = walk.step(rs[q]) && more;
+                    if (term) rs[q] = -1;
+                    codes[q] = CACHED && rs[q] >= 0 ? (int)p.row_kind[rs[q]] : KIND_RESAMPLE;
+                    ovs[q] = make_uint2(0u, 0u);
+                    t0s[q] = 0.f;
+                    if (rs[q] >= 0) { /* a dropped row's output is not written, and not used */
+                        ovs[q] = p.row_out[rs[q]];
+                        t0s[q] = p.row_t0[rs[q]];
                     }
                 }
-                if (acc.w < 1e-4f) term = true;
+#pragma unroll
+                for (int q = 0; q < COMP_AHEAD; ++q) {
+                    if (rs[q] < 0 || term) continue;
+                    const int kind = row_kind_of(codes[q]);
+                    if (CACHED && kind != KIND_SKIP && row_reason_of(codes[q])) why += 1ull << ((9 * (row_reason_of(codes[q]) - 1)) & 63);
+                    if (kind >= KIND_DROP) {
+                        c_drop += kind == KIND_DROP;
+                        continue;
+                    }
+                    if (kind == KIND_CACHE) ++c_cache; else ++c_res;
+                    ++n_comp;
+                    const uint2 ov = ovs[q];
+                    const float2 rg = __half22float2(*reinterpret_cast<const __half2 *>(&ov.x));
+                    const float lb = __half2float(__ushort_as_half((unsigned short)(ov.y & 0xffffu)));
+                    const float ld = __half2float(__ushort_as_half((unsigned short)(ov.y >> 16)));
+                    const float dt = calc_step(p.steps, t0s[q]);
+                    /* the basic cache renderer composites a cache row with its looked-up density
+                     * (accumulate_cache_render_kernel, src/cache_basic_renderer.cu:255-258) */
+                    const float sigma = CACHED && p.basic_cache && kind == KIND_CACHE ? p.row_pay[rs[q]].w : expf(ld);
+                    const float alpha = fminf(1.0f, fmaxf(0.0f, 1.0f - expf(-sigma * dt)));
+                    if (alpha > p.scene.alpha_thre) {
+                        const float wgt = alpha * acc.w;
+                        kahan_add(acc.x, comp.x, wgt / (1.0f + expf(-rg.x)));
+                        kahan_add(acc.y, comp.y, wgt / (1.0f + expf(-rg.y)));
+                        kahan_add(acc.z, comp.z, wgt / (1.0f + expf(-lb)));
+                        acc.w *= 1.0f - alpha;
+                        if (CACHED) {
+                            if (kind == KIND_CACHE) w_cache += wgt;
+                            else w_res += wgt;
+                        }
+                    }
+                    if (acc.w < 1e-4f) term = true;
+                }
             }
+            if (__all_sync(FULLMASK, term || done)) break;
         }
         if (valid) {
             if (CACHED) { /* one ray a pixel: no other thread adds to it in this launch */
@@ -1736,8 +1773,9 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
             st.cnt.y = c_res;
             st.cnt.z = c_cache;
             st.cnt2.x = c_drop;
-            if (term || st.cnt2.y) {
-                write_pixel(p, st.cnt.x, acc, make_int4(c_res, c_cache, c_drop, st.cnt.w));
+            st.cnt.w = c_steps;
+            if (term || done) {
+                write_pixel(p, st.cnt.x, acc, make_int4(c_res, c_cache, c_drop, c_steps));
             } else {
                 keep = true;
             }
@@ -1747,7 +1785,7 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
         if (CACHED && __any_sync(FULLMASK, why != 0)) {
 #pragma unroll
             for (int q = 1; q < N_REASONS; ++q) {
-                const unsigned c = __reduce_add_sync(FULLMASK, (unsigned)(why >> (8 * (q - 1))) & 255u);
+                const unsigned c = __reduce_add_sync(FULLMASK, (unsigned)(why >> (9 * (q - 1))) & 511u);
                 if (lane_id() == 0 && c) atomicAdd(&p.stats->n_reason[q], (unsigned long long)c);
             }
         }
@@ -1773,101 +1811,93 @@ template <bool CACHED>
 __global__ void __launch_bounds__(128) wf_composite_bwd_kernel(RenderParams p, int it)
 {
     const int n_alive = p.counters[it & 1];
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p, CACHED);
     RayState *cur = p.states[it & 1], *nxt = p.states[(it + 1) & 1];
     for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
         const int i = base + threadIdx.x;
         const bool valid = i < n_alive;
         bool keep = false;
         RayState st;
-        int n_res = 0, n_cch = 0;
-        int2 rr = make_int2(0, 0);
-        uint32_t gmask = 0, cmask = 0;
         float4 rg = make_float4(0.f, 0.f, 0.f, 0.f);
         float T = 1.f, xp = 0.f;
         if (valid) {
             st = cur[i];
-            rr = p.ray_rows[i];
             rg = p.ray_grad[st.cnt.x];
             T = st.acc.w;
             xp = st.acc.x;
         }
-        bool term = false;
-        int r;
-        RowWalk walk(rr, valid, p.by_sample);
-        for (int j = 0; walk.step(r); ++j) {
-            if (r >= 0) {
-                float4 dout = make_float4(0.f, 0.f, 0.f, 0.f);
-                const int kind = CACHED ? row_kind_of(p.row_kind[r]) : KIND_RESAMPLE;
-                if (!term && kind < KIND_DROP) {
-                    const uint2 ov = p.row_out[r];
-                    const float t0 = p.row_t0[r];
-                    const float2 lg = __half22float2(*reinterpret_cast<const __half2 *>(&ov.x));
-                    const float lb = __half2float(__ushort_as_half((unsigned short)(ov.y & 0xffffu)));
-                    const float ld = __half2float(__ushort_as_half((unsigned short)(ov.y >> 16)));
-                    const float dt = calc_step(p.steps, t0);
-                    const float sigma = expf(ld);
-                    const float alpha = fminf(1.0f, fmaxf(0.0f, 1.0f - expf(-sigma * dt)));
-                    if (alpha > p.scene.alpha_thre) {
-                        const float c0 = 1.0f / (1.0f + expf(-lg.x)), c1 = 1.0f / (1.0f + expf(-lg.y)),
-                                    c2 = 1.0f / (1.0f + expf(-lb));
-                        const float gc = rg.x * c0 + rg.y * c1 + rg.z * c2;
-                        const float ta = T * alpha;
-                        xp += ta * gc;
-                        const float Tn = T * (1.0f - alpha);
-                        const float dsig = dt * (Tn * gc - (rg.w - xp));
-                        dout = make_float4(rg.x * ta * c0 * (1.0f - c0), rg.y * ta * c1 * (1.0f - c1), rg.z * ta * c2 * (1.0f - c2),
-                                           dsig * sigma);
-                        T = Tn;
-                        if (kind == KIND_CACHE) { cmask |= 1u << j; ++n_cch; }
-                        else { gmask |= 1u << j; ++n_res; }
-                    }
-                    if (T < 1e-4f) term = true;
-                }
-                p.row_dout[r] = dout;
+        bool term = false, done = !valid;
+        for (int w = 0; w < p.windows; ++w) {
+            int n_res = 0, n_cch = 0;
+            uint32_t gmask = 0, cmask = 0;
+            int2 rr = make_int2(0, 0);
+            if (!done) { /* also of a ray that has ended: the others' rows follow its own */
+                rr = p.ray_rows[(size_t)w * p.ray_stride + i];
+                done = window_done(rr.y);
             }
+            int r;
+            RowWalk walk(rr, true, p.by_sample);
+            for (int j = 0; walk.step(r); ++j) {
+                if (r >= 0) {
+                    float4 dout = make_float4(0.f, 0.f, 0.f, 0.f);
+                    const int kind = CACHED ? row_kind_of(p.row_kind[r]) : KIND_RESAMPLE;
+                    if (!term && kind < KIND_DROP) {
+                        const uint2 ov = p.row_out[r];
+                        const float t0 = p.row_t0[r];
+                        const float2 lg = __half22float2(*reinterpret_cast<const __half2 *>(&ov.x));
+                        const float lb = __half2float(__ushort_as_half((unsigned short)(ov.y & 0xffffu)));
+                        const float ld = __half2float(__ushort_as_half((unsigned short)(ov.y >> 16)));
+                        const float dt = calc_step(p.steps, t0);
+                        const float sigma = expf(ld);
+                        const float alpha = fminf(1.0f, fmaxf(0.0f, 1.0f - expf(-sigma * dt)));
+                        if (alpha > p.scene.alpha_thre) {
+                            const float c0 = 1.0f / (1.0f + expf(-lg.x)), c1 = 1.0f / (1.0f + expf(-lg.y)),
+                                        c2 = 1.0f / (1.0f + expf(-lb));
+                            const float gc = rg.x * c0 + rg.y * c1 + rg.z * c2;
+                            const float ta = T * alpha;
+                            xp += ta * gc;
+                            const float Tn = T * (1.0f - alpha);
+                            const float dsig = dt * (Tn * gc - (rg.w - xp));
+                            dout = make_float4(rg.x * ta * c0 * (1.0f - c0), rg.y * ta * c1 * (1.0f - c1), rg.z * ta * c2 * (1.0f - c2),
+                                               dsig * sigma);
+                            T = Tn;
+                            if (kind == KIND_CACHE) { cmask |= 1u << j; ++n_cch; }
+                            else { gmask |= 1u << j; ++n_res; }
+                        }
+                        if (T < 1e-4f) term = true;
+                    }
+                    p.row_dout[r] = dout;
+                }
+            }
+            /* list the rows with a gradient per network stream (one atomic per warp and list) */
+            auto append = [&](int n, uint32_t mask, int *list, int *counter) {
+                const int total = (int)__reduce_add_sync(FULLMASK, (unsigned)n);
+                if (total == 0) return;
+                int lb = 0;
+                if (lane_id() == 0) lb = atomicAdd(counter, total);
+                ListWalk places(__shfl_sync(FULLMASK, lb, 0), n, p.by_sample);
+                int row;
+                RowWalk rows(rr, true, p.by_sample);
+                for (int j = 0; rows.step(row); ++j) {
+                    const bool has = (mask >> j) & 1u;
+                    const int at = places.place(has);
+                    if (has) list[at] = row;
+                }
+            };
+            append(n_res, gmask, p.grad_res_list, p.counters + 6);
+            if (CACHED) append(n_cch, cmask, p.grad_cache_list, p.counters + 7);
+            if (__all_sync(FULLMASK, term || done)) break;
         }
         if (valid) {
             st.acc.x = xp;
             st.acc.w = T;
-            keep = !(term || st.cnt2.y);
+            keep = !(term || done);
         }
-        /* list the rows with a gradient per network stream (one atomic per warp and list) */
-        auto append = [&](int n, uint32_t mask, int *list, int *counter) {
-            const int total = (int)__reduce_add_sync(FULLMASK, (unsigned)n);
-            if (total == 0) return;
-            int lb = 0;
-            if (lane_id() == 0) lb = atomicAdd(counter, total);
-            ListWalk places(__shfl_sync(FULLMASK, lb, 0), n, p.by_sample);
-            int row;
-            RowWalk rows(rr, valid, p.by_sample);
-            for (int j = 0; rows.step(row); ++j) {
-                const bool has = (mask >> j) & 1u;
-                const int at = places.place(has);
-                if (has) list[at] = row;
-            }
-        };
-        append(n_res, gmask, p.grad_res_list, p.counters + 6);
-        if (CACHED) append(n_cch, cmask, p.grad_cache_list, p.counters + 7);
         const unsigned m = __ballot_sync(FULLMASK, keep);
         int nb = 0;
         if (lane_id() == 0 && m) nb = atomicAdd(p.counters + ((it + 1) & 1), __popc(m));
         nb = __shfl_sync(FULLMASK, nb, 0);
         if (keep) nxt[nb + __popc(m & lane_lt())] = st;
-    }
-}
-
-/* resets the row counters after the kernels of the sub-iteration consumed them */
-__global__ void wf_reset_rows_kernel(RenderParams p, int cached)
-{
-    if (threadIdx.x == 0) {
-        atomicAdd(&p.stats->n_resamples, (unsigned long long)(cached ? p.counters[3] : p.counters[2]));
-        atomicAdd(&p.stats->n_cache_hits, (unsigned long long)p.counters[4]);
-        atomicAdd(&p.stats->n_dropped, (unsigned long long)(cached ? p.counters[2] - p.counters[3] - p.counters[4] : 0));
-        p.counters[2] = 0;
-        p.counters[3] = 0;
-        p.counters[4] = 0;
-        p.counters[6] = 0;
-        p.counters[7] = 0;
     }
 }
 
@@ -2120,6 +2150,12 @@ static void launch_plain_net(const RenderParams &p, int it, int n_sms, cudaStrea
     else wf_net_tc_kernel<0, HH, false><<<grid_tc, 128, tc_smem, s>>>(p, it);
 }
 
+/* blocks of the per-ray kernels: no more than the rays fill */
+static inline int ray_grid(int n_rays, int n_sms) { return std::max(1, std::min(n_sms * FVC_RAY_BLOCKS_PER_SM, (n_rays + 127) / 128)); }
+
+/* sub-iterations between two readbacks of the alive count: with more march windows a sub-iteration there are fewer */
+static inline int check_interval(const RenderParams &p, int every) { return p.windows >= 8 ? 1 : p.windows > 1 ? std::min(every, 2) : every; }
+
 template <bool CACHED, int HH>
 static cudaError_t run_frame(const RenderParams &p, int n_sms, cudaStream_t s, int *h_pinned, int check_every, int *n_iter,
                              LaunchLog *log)
@@ -2142,7 +2178,8 @@ static cudaError_t run_frame(const RenderParams &p, int n_sms, cudaStream_t s, i
     if (p.pixel_list) wf_raygen_list_kernel<<<(p.n_list + 255) / 256, 256, 0, s>>>(p);
     else wf_raygen_kernel<<<(n_threads + 255) / 256, 256, 0, s>>>(p);
     ++L.launches;
-    const int grid_ray = n_sms * FVC_RAY_BLOCKS_PER_SM;
+    const int grid_ray = ray_grid(p.pixel_list ? p.n_list : W * H, n_sms);
+    check_every = check_interval(p, check_every);
     const int grid_net = n_sms * 2;
     const size_t net_smem = sizeof(NetSmem);
     const size_t tc_smem = tc_smem_bytes(p.freq);
@@ -2180,8 +2217,7 @@ static cudaError_t run_frame(const RenderParams &p, int n_sms, cudaStream_t s, i
             L.launches += 1;
         }
         wf_composite_kernel<CACHED><<<grid_ray, 128, 0, s>>>(p, it);
-        wf_reset_rows_kernel<<<1, 32, 0, s>>>(p, CACHED ? 1 : 0);
-        L.launches += 2;
+        L.launches += 1;
         if ((it + 1) % check_every == 0) {
             cudaError_t e = cudaMemcpyAsync(h_pinned, p.counters + ((it + 1) & 1), sizeof(int), cudaMemcpyDeviceToHost, s);
             if (e != cudaSuccess) return e;
@@ -2244,7 +2280,7 @@ cudaError_t launch_fill_raygen(const RenderParams &p, cudaStream_t s)
 
 cudaError_t launch_fill_march(const RenderParams &p, int it, int n_sms, cudaStream_t s)
 {
-    wf_march_kernel<false><<<n_sms * FVC_RAY_BLOCKS_PER_SM, 128, 0, s>>>(p, it);
+    wf_march_kernel<false><<<ray_grid(p.cam.W * p.cam.H, n_sms), 128, 0, s>>>(p, it);
     return cudaGetLastError();
 }
 
@@ -2271,7 +2307,8 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
         if (L.ev && L.n_timed < L.cap) cudaEventRecord(L.ev[2 * L.n_timed++ + 1], s);
         else if (L.ev) ++L.n_untimed;
     };
-    const int grid_ray = n_sms * FVC_RAY_BLOCKS_PER_SM;
+    const int grid_ray = ray_grid(p.n_list, n_sms);
+    check_every = check_interval(p, check_every);
     for (int it = 0; it < (1 << 20); ++it) {
         wf_march_kernel<CACHED><<<grid_ray, 128, 0, s>>>(p, it);
         /* the forward kernels of pass 1, so both passes composite the same values */
@@ -2297,8 +2334,7 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
         timed_end();
         if (e == cudaSuccess && CACHED) e = launch_cache_backward(p, b, HH, it, n_sms, s);
         if (e != cudaSuccess) return e;
-        wf_reset_rows_kernel<<<1, 32, 0, s>>>(p, CACHED ? 1 : 0);
-        L.launches += CACHED ? 5 : 4;
+        L.launches += CACHED ? 4 : 3;
         if ((it + 1) % check_every == 0) {
             e = cudaMemcpyAsync(h_pinned, p.counters + ((it + 1) & 1), sizeof(int), cudaMemcpyDeviceToHost, s);
             if (e != cudaSuccess) return e;
@@ -2369,7 +2405,7 @@ static cudaError_t build_batch_graph_t(const RenderParams &p, int n_sms, cudaStr
     int kernels = 1;
     if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        const int grid_ray = n_sms * FVC_RAY_BLOCKS_PER_SM;
+        const int grid_ray = ray_grid(n_rays, n_sms);
         const bool fused = CACHED && fused_cached_path(p);
         for (int it = 0; it < 2; ++it) {
             if (fused) {
