@@ -426,6 +426,7 @@ struct fvc_renderer {
     int *d_wf_counters = nullptr;
     int row_capacity = 0;             /* rows of the buffers: batch_rows for each march window */
     int batch_rows = 0, windows = 1, ray_stride = 0;
+    size_t ray_rows_cap = 0;          /* entries of d_ray_rows */
     int last_iterations = 0;
     /* batched views in one graph launch */
     DevCam *d_views = nullptr;
@@ -453,6 +454,8 @@ struct fvc_renderer {
     float4 *d_row_dout = nullptr;     /* per-row gradients of the differentiable render */
     int *d_grad_rows = nullptr;       /* resample rows with a gradient */
     int *d_grad_cache_rows = nullptr; /* cache rows with a gradient */
+    int *d_list_order = nullptr, *d_list_rank = nullptr, *d_list_bins = nullptr; /* the pixel list by image tile */
+    int list_cap = 0;
     int bwd_capacity = 0;
     LaunchLog log;                    /* kernel accounting of the last render */
     std::vector<cudaEvent_t> events;  /* 2 x 4096 when kernel timing is on */
@@ -462,6 +465,7 @@ struct fvc_renderer {
         dfree(d_row_kind); dfree(d_row_pay); dfree(d_row_out); dfree(d_res_list); dfree(d_cache_list); dfree(d_wf_counters);
         dfree(d_row_lat);
         row_capacity = batch_rows = 0;
+        ray_rows_cap = 0;
     }
     fvc_cache *cache = nullptr, *next = nullptr;
     fvc_cache_settings settings{0, 0, 1, 1, 1, 1};
@@ -478,6 +482,7 @@ struct fvc_renderer {
         if (stream) cudaStreamSynchronize(stream);
         dfree(d_ctl); dfree(d_stats); dfree(d_results); dfree(d_image); dfree(d_counts);
         dfree(d_row_dout); dfree(d_grad_rows); dfree(d_grad_cache_rows);
+        dfree(d_list_order); dfree(d_list_rank); dfree(d_list_bins);
         dfree(d_views); dfree(d_view_off); dfree(d_view_caches);
         if (graph_exec) cudaGraphExecDestroy(graph_exec);
         release_wavefront();
@@ -1175,6 +1180,34 @@ static int march_windows(size_t n_rays)
     return (int)std::min<size_t>(MAX_WINDOWS, std::max<size_t>(1, FVC_WINDOW_RAYS / n_rays));
 }
 
+/* buffers of `cap` sample rows and `windows` per-ray window entries, in place of the renderer's smaller ones */
+static int alloc_rows(fvc_renderer *r, size_t cap, size_t windows)
+{
+    int rc;
+    if (windows > r->ray_rows_cap) {
+        dfree(r->d_ray_rows);
+        r->ray_rows_cap = 0;
+        if ((rc = dalloc(&r->d_ray_rows, windows, "ray rows"))) return rc;
+        r->ray_rows_cap = windows;
+    }
+    if (cap <= (size_t)r->row_capacity) return FVC_OK;
+    dfree(r->d_row_t0); dfree(r->d_row_slot); dfree(r->d_row_pay); dfree(r->d_row_out);
+    dfree(r->d_row_kind); dfree(r->d_res_list); dfree(r->d_cache_list); dfree(r->d_row_lat);
+    r->row_capacity = 0;
+    if ((rc = dalloc(&r->d_row_t0, cap, "row t0"))) return rc;
+    if ((rc = dalloc(&r->d_row_slot, cap, "row slots"))) return rc;
+    if ((rc = dalloc(&r->d_row_pay, cap, "row inputs"))) return rc;
+    if ((rc = dalloc(&r->d_row_out, cap, "row outputs"))) return rc;
+    if (is_cache_kind(r->kind)) {
+        if ((rc = dalloc(&r->d_row_kind, cap, "row kinds"))) return rc;
+        if ((rc = dalloc(&r->d_res_list, cap, "resample list"))) return rc;
+        if ((rc = dalloc(&r->d_cache_list, cap, "cache list"))) return rc;
+        if ((rc = dalloc(&r->d_row_lat, cap, "cache-row head inputs"))) return rc;
+    }
+    r->row_capacity = (int)cap;
+    return FVC_OK;
+}
+
 extern "C" int fvc_renderer_resize(fvc_renderer *r, int width, int height)
 {
     CHECK_ARG(r && width > 0 && height > 0, "fvc_renderer_resize: bad arguments");
@@ -1196,22 +1229,10 @@ extern "C" int fvc_renderer_resize(fvc_renderer *r, int width, int height)
     r->windows = march_windows(n);
     r->ray_stride = (int)n;
     const size_t cap = (size_t)r->batch_rows * r->windows;
-    const bool cached = is_cache_kind(r->kind);
     if ((rc = dalloc(&r->d_states[0], n, "ray states"))) return rc;
     if ((rc = dalloc(&r->d_states[1], n, "ray states"))) return rc;
-    if ((rc = dalloc(&r->d_ray_rows, n * r->windows, "ray rows"))) return rc;
-    if ((rc = dalloc(&r->d_row_t0, cap, "row t0"))) return rc;
-    if ((rc = dalloc(&r->d_row_slot, cap, "row slots"))) return rc;
-    if ((rc = dalloc(&r->d_row_pay, cap, "row inputs"))) return rc;
-    if ((rc = dalloc(&r->d_row_out, cap, "row outputs"))) return rc;
-    if (cached) {
-        if ((rc = dalloc(&r->d_row_kind, cap, "row kinds"))) return rc;
-        if ((rc = dalloc(&r->d_res_list, cap, "resample list"))) return rc;
-        if ((rc = dalloc(&r->d_cache_list, cap, "cache list"))) return rc;
-        if ((rc = dalloc(&r->d_row_lat, cap, "cache-row head inputs"))) return rc;
-    }
+    if ((rc = alloc_rows(r, cap, n * r->windows))) return rc;
     if ((rc = dalloc(&r->d_wf_counters, (size_t)8, "wavefront counters"))) return rc;
-    r->row_capacity = (int)cap;
     r->W = width; r->H = height;
     return FVC_OK;
 }
@@ -1359,6 +1380,7 @@ static int setup_render_params(fvc_renderer *r, const fvc_raymarch_info *info, f
     p.batch_rows = r->row_target > 0 ? std::min(r->row_target, r->batch_rows) : r->batch_rows;
     p.windows = r->row_target > 0 || r->steps_per_iter != MARCH_STEPS ? 1 : r->windows;
     p.ray_stride = r->ray_stride;
+    p.row_capacity = r->row_capacity;
     p.by_sample = rows_by_sample(p);
     return FVC_OK;
 }
@@ -2118,6 +2140,32 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
     std::lock_guard<std::mutex> lk(r->read_mutex);
     fvc_model *m = r->m;
     cudaStream_t s = r->stream;
+    /* Room for whole rays: with every window of a ray in one sub-iteration, pass 2 finds pass 1's rows in place and
+     * neither marches nor runs the networks forward again.  LIST_ROWS rows a ray (the synthetic scenes' rays hold
+     * about 90), at most 2^26 rows and 2^25 windows; rays beyond that wait for a further sub-iteration, and pass 2
+     * then marches again.  Not when a compaction batch or a march length is set. */
+    const bool whole = r->row_target == 0 && r->steps_per_iter == MARCH_STEPS;
+    const int ray_windows = (int)std::min<size_t>(MAX_WINDOWS, std::max<size_t>(1, ((size_t)1 << 25) / n_rays));
+    if (whole) {
+        constexpr size_t LIST_ROWS = 128;
+        const size_t rows = std::max<size_t>(1024, std::min<size_t>((size_t)n_rays * LIST_ROWS, (size_t)1 << 26));
+        const size_t windows = (size_t)n_rays * ray_windows;
+        if (rows > (size_t)r->row_capacity || windows > r->ray_rows_cap) {
+            CU(cudaStreamSynchronize(s));
+            if ((rc = alloc_rows(r, rows, windows))) {
+                r->W = r->H = 0; /* the buffers are gone: the next render allocates its own */
+                return rc;
+            }
+        }
+    }
+    if (r->list_cap < n_rays) {
+        dfree(r->d_list_order); dfree(r->d_list_rank);
+        r->list_cap = 0;
+        if ((rc = dalloc(&r->d_list_order, (size_t)n_rays, "pixel order"))) return rc;
+        if ((rc = dalloc(&r->d_list_rank, (size_t)n_rays, "pixel ranks"))) return rc;
+        if (!r->d_list_bins && (rc = dalloc(&r->d_list_bins, (size_t)LIST_BINS, "pixel tiles"))) return rc;
+        r->list_cap = n_rays;
+    }
     if (r->bwd_capacity != r->row_capacity) {
         dfree(r->d_row_dout); dfree(r->d_grad_rows); dfree(r->d_grad_cache_rows);
         if ((rc = dalloc(&r->d_row_dout, (size_t)r->row_capacity, "row gradients"))) return rc;
@@ -2151,6 +2199,11 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
     p.pixel_list = pixels;
     p.n_list = n_rays;
     p.by_sample = 0; /* the warp's rays are any pixels of the list: only a ray's own samples are close together */
+    if (whole) {
+        p.windows = ray_windows;
+        p.ray_stride = n_rays;
+    }
+    p.list_order = r->d_list_order;
     p.ray_grad = g->d_ray_grad;
     p.row_dout = r->d_row_dout;
     p.grad_res_list = r->d_grad_rows;
@@ -2169,14 +2222,17 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
     CU(cudaMemsetAsync(r->d_ctl, 0, 4 * sizeof(int), s));
     CU(cudaMemsetAsync(r->d_stats, 0, sizeof(RenderStatsDev), s));
     CU(cudaMemsetAsync(r->d_wf_counters, 0, 8 * sizeof(int), s));
+    CU(launch_list_order(p, r->d_list_order, r->d_list_rank, r->d_list_bins, s));
+    r->log.launches += 3;
     CU(render_frame(p, cached, m->head_hidden, m->n_sms, s, r->h_pinned + 8, 4, &r->last_iterations, &r->log));
+    const bool one_round = r->last_iterations == 1;
     /* loss and per-ray dL/dC */
     CU(cudaMemsetAsync(g->d_loss, 0, sizeof(double), s));
     CU(launch_loss(p, b, s));
-    /* pass 2: re-march, compositing adjoint, network adjoint */
+    /* pass 2: re-march, compositing adjoint, network adjoint; over pass 1's rows where one sub-iteration held them */
     r->log.split = r->log.n_timed;
-    CU(cudaMemsetAsync(r->d_wf_counters, 0, 8 * sizeof(int), s));
-    CU(backward_frame(p, b, cached, m->head_hidden, m->n_sms, s, r->h_pinned + 8, 4, &r->log));
+    if (!one_round) CU(cudaMemsetAsync(r->d_wf_counters, 0, 8 * sizeof(int), s));
+    CU(backward_frame(p, b, cached, m->head_hidden, m->n_sms, s, r->h_pinned + 8, 4, one_round, &r->log));
     const float inv = 1.0f / (FVC_LOSS_SCALE * (float)n_rays);
     CU(launch_grad_finalize(g->s_table, g->d_table, g->n_table, inv, m->n_sms, s));
     CU(launch_grad_finalize(g->s_base, g->d_base, g->n_base, inv, m->n_sms, s));

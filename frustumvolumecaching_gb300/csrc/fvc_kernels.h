@@ -236,11 +236,14 @@ __device__ __forceinline__ int lanes_before(int n)
 constexpr int MAX_WINDOWS = 31; /* march windows of a sub-iteration */
 
 /* A ray's share of one march window: its warp's first row and, packed, its
- * row count, the steps it marched and whether it passed its far bound. */
+ * row count, the steps it marched and whether it passed its far bound.  A
+ * ray's windows of a sub-iteration end with one that passed the bound, with
+ * the last, or with one of no steps (no room for its warp's rows). */
 __host__ __device__ __forceinline__ int window_pack(int n, int steps, bool done) { return n | (steps << 5) | (int)((done ? 1u : 0u) << 31); }
 __host__ __device__ __forceinline__ int window_rows(int w) { return w & 31; }
 __host__ __device__ __forceinline__ int window_steps(int w) { return (w & 0x7fffffff) >> 5; }
 __host__ __device__ __forceinline__ bool window_done(int w) { return w < 0; }
+__host__ __device__ __forceinline__ bool window_none(int w) { return w == 0; }
 
 /* Where the rows of a sub-iteration lie.  A warp's rows follow each other from
  * its first row, either ray by ray (a ray's samples adjacent) or, by_sample,
@@ -333,6 +336,7 @@ struct RenderParams {
     int2 *ray_rows;             /* [windows][ray_stride] per alive ray: first row of its warp, window_pack of its share */
     int windows;                /* march windows (steps_per_iter steps, at most S_ROWS samples) of a sub-iteration */
     int ray_stride;
+    int row_capacity;           /* rows of the buffers: a warp whose window does not fit marches it in the next sub-iteration */
     int batch_rows;             /* rows a window aims at over all rays: samples per ray and window = clamp(batch_rows /
                                  * alive rays, 1, S_ROWS) */
     float *row_t0;              /* per row: t0 of the sample */
@@ -365,6 +369,7 @@ struct RenderParams {
     /* differentiable render */
     const int *pixel_list;      /* rays for these pixels (y * W + x) instead of the full image; ray id = list index */
     int n_list;
+    const int *list_order;      /* the order the list's rays are taken in (null: the list's own) */
     const float4 *ray_grad;     /* per ray: dL/dC (loss-scaled) and X_total = g.C + g_T T */
     float4 *row_dout;           /* per row: dL/d rgb logits, dL/d log-density (loss-scaled) */
     int *grad_res_list;         /* rows with a gradient: resample rows (counters[6]) */
@@ -544,8 +549,13 @@ cudaError_t build_batch_graph(const RenderParams &p, bool cached, int head_hidde
                               cudaGraphExec_t *exec, int *n_kernels);
 
 /* differentiable render (fvc_backward.cu): pass 1 is render_frame over p.pixel_list */
+/* pass 2; one_round: pass 1 ended every ray in its only sub-iteration, whose states and rows still stand, so only
+ * the adjoints run */
 cudaError_t backward_frame(const RenderParams &p, const BwdParams &b, bool cached, int head_hidden, int n_sms, cudaStream_t s,
-                           int *h_pinned, int check_every, LaunchLog *log = nullptr);
+                           int *h_pinned, int check_every, bool one_round, LaunchLog *log = nullptr);
+/* orders the pixel list by tiles of the image: order[] from rank[] (n_list) and bins[] (n_bins + 1), n_bins <= LIST_BINS */
+constexpr int LIST_BINS = 16384;
+cudaError_t launch_list_order(const RenderParams &p, int *order, int *rank, int *bins, cudaStream_t s);
 cudaError_t launch_loss(const RenderParams &p, const BwdParams &b, cudaStream_t s);
 cudaError_t launch_net_backward(const RenderParams &p, const BwdParams &b, int head_hidden, int it, int n_sms, cudaStream_t s);
 cudaError_t launch_cache_backward(const RenderParams &p, const BwdParams &b, int head_hidden, int it, int n_sms, cudaStream_t s);

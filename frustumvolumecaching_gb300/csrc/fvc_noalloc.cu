@@ -144,7 +144,7 @@ extern "C" int fvc_render_noalloc(fvc_model *m, const fvc_raymarch_info *info, c
     p.ray_counter = ctl;
     p.guard = ctl + 1;
     p.stats = stats;
-    p.batch_rows = (int)cap;
+    p.row_capacity = p.batch_rows = (int)cap;
     p.windows = 1;
     p.ray_stride = (int)n;
     p.steps_per_iter = 64;

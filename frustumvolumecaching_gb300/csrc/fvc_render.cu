@@ -143,7 +143,8 @@ __global__ void __launch_bounds__(256) wf_raygen_kernel(RenderParams p)
  * results[id] is written for rays that miss the scene box */
 __global__ void __launch_bounds__(256) wf_raygen_list_kernel(RenderParams p)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int at = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = at < p.n_list && p.list_order ? p.list_order[at] : at;
     const int W = p.cam.W, H = p.cam.H;
     const int pix = i < p.n_list ? p.pixel_list[i] : -1;
     const bool valid = pix >= 0 && pix < W * H;
@@ -169,6 +170,64 @@ __global__ void __launch_bounds__(256) wf_raygen_list_kernel(RenderParams p)
         st.cnt2 = make_int4(0, 0, 0, 0);
         p.states[0][base + __popc(m & lane_lt())] = st;
     }
+}
+
+/* The list's rays by image tile (a counting sort: rays per tile and each
+ * ray's place in its tile, the tiles' first places, the order), so that the
+ * rays of neighbouring warps are neighbouring pixels and their gathers and
+ * reductions meet in the L1 and L2.  Tiles of 8 x 8 pixels, larger where the
+ * image has more than LIST_BINS of them; pixels outside the image come last. */
+__device__ __forceinline__ int list_tile(const RenderParams &p, int shift, int n_bins, int pix)
+{
+    if (pix < 0 || pix >= p.cam.W * p.cam.H) return n_bins - 1;
+    return (pix / p.cam.W >> shift) * ((p.cam.W + (1 << shift) - 1) >> shift) + (pix % p.cam.W >> shift);
+}
+
+__global__ void __launch_bounds__(256) list_count_kernel(RenderParams p, int shift, int n_bins, int *bins, int *rank)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < p.n_list) rank[i] = atomicAdd(bins + list_tile(p, shift, n_bins, p.pixel_list[i]), 1);
+}
+
+__global__ void __launch_bounds__(1024) list_scan_kernel(int *bins, int n_bins)
+{
+    __shared__ int sums[32], carry;
+    if (threadIdx.x == 0) carry = 0;
+    for (int c0 = 0; c0 < n_bins; c0 += 1024) {
+        const int b = c0 + threadIdx.x, v = b < n_bins ? bins[b] : 0;
+        const int before = lanes_before(v);
+        if (lane_id() == 31) sums[threadIdx.x >> 5] = before + v;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const int w = sums[threadIdx.x], e = lanes_before(w);
+            sums[threadIdx.x] = carry + e;
+            __syncwarp();
+            if (threadIdx.x == 31) carry += e + w;
+        }
+        __syncthreads();
+        if (b < n_bins) bins[b] = sums[threadIdx.x >> 5] + before;
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(256) list_order_kernel(RenderParams p, int shift, int n_bins, const int *bins, const int *rank, int *order)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < p.n_list) order[bins[list_tile(p, shift, n_bins, p.pixel_list[i])] + rank[i]] = i;
+}
+
+cudaError_t launch_list_order(const RenderParams &p, int *order, int *rank, int *bins, cudaStream_t s)
+{
+    int shift = 3;
+    auto tiles = [&](int n) { return (long long)((n + (1ll << shift) - 1) >> shift); };
+    while (tiles(p.cam.W) * tiles(p.cam.H) + 1 > LIST_BINS) ++shift;
+    const int n_bins = (int)(tiles(p.cam.W) * tiles(p.cam.H)) + 1, blocks = (p.n_list + 255) / 256;
+    cudaError_t e = cudaMemsetAsync(bins, 0, n_bins * sizeof(int), s);
+    if (e != cudaSuccess) return e;
+    list_count_kernel<<<blocks, 256, 0, s>>>(p, shift, n_bins, bins, rank);
+    list_scan_kernel<<<1, 1024, 0, s>>>(bins, n_bins);
+    list_order_kernel<<<blocks, 256, 0, s>>>(p, shift, n_bins, bins, rank, order);
+    return cudaGetLastError();
 }
 
 /* rays of a batch of views (one thread per pixel of the concatenated views) */
@@ -427,6 +486,8 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
         int all_steps = 0, all_rows = 0;
         for (int w = 0; w < p.windows; ++w) {
             int n = 0, steps = 0;
+            const float t_window = dt4.w;
+            const bool done_before = done;
             if (!done) {
                 const float3 o = make_float3(of.x, of.y, of.z), d = make_float3(dt4.x, dt4.y, dt4.z);
                 float t1 = dt4.w;
@@ -483,8 +544,19 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
             }
             const int n_warp = (int)__reduce_add_sync(FULLMASK, (unsigned)n);
             int rbase = 0;
-            if (lane_id() == 0 && n_warp) rbase = atomicAdd(p.counters + 2, n_warp);
+            if (lane_id() == 0 && n_warp) {
+                rbase = atomicAdd(p.counters + 2, n_warp);
+                if (rbase + n_warp > p.row_capacity) { /* no hole: what was added is taken back, and nothing fits meanwhile */
+                    atomicSub(p.counters + 2, n_warp);
+                    rbase = -1;
+                }
+            }
             rbase = __shfl_sync(FULLMASK, rbase, 0);
+            if (rbase < 0) { /* the rays wait at this window's start for the next sub-iteration */
+                if (!done_before) p.ray_rows[(size_t)w * p.ray_stride + i] = make_int2(0, window_pack(0, 0, false));
+                dt4.w = t_window;
+                break;
+            }
             RowWalk walk(make_int2(rbase, window_pack(n, 0, false)), true, p.by_sample);
             int r;
             if (FUSED) {
@@ -1700,12 +1772,14 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
         }
         float w_res = 0.f, w_cache = 0.f; /* this sub-iteration's contribution weights (DEBUG form, :867-871) */
         bool term = false, done = !valid; /* ended by opacity; the march passed the far bound */
+        bool more_windows = true;
         for (int w = 0; w < p.windows; ++w) {
             int2 rr = make_int2(0, 0);
             if (!done) { /* also of a ray that has ended: the others' rows follow its own */
                 rr = p.ray_rows[(size_t)w * p.ray_stride + i];
                 if (!term) c_steps += window_steps(rr.y);
                 done = window_done(rr.y);
+                more_windows = !window_none(rr.y);
             }
             /* rows are in t order: the merge of the resample and cache streams of
              * accumulate_cache_perf_kernel (:270-304); COMP_AHEAD samples are loaded together, before the
@@ -1761,7 +1835,7 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
                     if (acc.w < 1e-4f) term = true;
                 }
             }
-            if (__all_sync(FULLMASK, term || done)) break;
+            if (__all_sync(FULLMASK, term || done || !more_windows)) break;
         }
         if (valid) {
             if (CACHED) { /* one ray a pixel: no other thread adds to it in this launch */
@@ -1826,7 +1900,7 @@ __global__ void __launch_bounds__(128) wf_composite_bwd_kernel(RenderParams p, i
             T = st.acc.w;
             xp = st.acc.x;
         }
-        bool term = false, done = !valid;
+        bool term = false, done = !valid, more_windows = true;
         for (int w = 0; w < p.windows; ++w) {
             int n_res = 0, n_cch = 0;
             uint32_t gmask = 0, cmask = 0;
@@ -1834,6 +1908,7 @@ __global__ void __launch_bounds__(128) wf_composite_bwd_kernel(RenderParams p, i
             if (!done) { /* also of a ray that has ended: the others' rows follow its own */
                 rr = p.ray_rows[(size_t)w * p.ray_stride + i];
                 done = window_done(rr.y);
+                more_windows = !window_none(rr.y);
             }
             int r;
             RowWalk walk(rr, true, p.by_sample);
@@ -1886,7 +1961,7 @@ __global__ void __launch_bounds__(128) wf_composite_bwd_kernel(RenderParams p, i
             };
             append(n_res, gmask, p.grad_res_list, p.counters + 6);
             if (CACHED) append(n_cch, cmask, p.grad_cache_list, p.counters + 7);
-            if (__all_sync(FULLMASK, term || done)) break;
+            if (__all_sync(FULLMASK, term || done || !more_windows)) break;
         }
         if (valid) {
             st.acc.x = xp;
@@ -2289,7 +2364,7 @@ cudaError_t launch_fill_march(const RenderParams &p, int it, int n_sms, cudaStre
  * sub-iteration, then the compositing adjoint and the network adjoint. */
 template <bool CACHED, int HH>
 static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n_sms, cudaStream_t s, int *h_pinned,
-                                int check_every, LaunchLog *log)
+                                int check_every, bool one_round, LaunchLog *log)
 {
     {
         cudaError_t e = ensure_net_attrs<HH>();
@@ -2297,8 +2372,8 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
     }
     LaunchLog local;
     LaunchLog &L = log ? *log : local;
-    wf_raygen_list_kernel<<<(p.n_list + 255) / 256, 256, 0, s>>>(p);
-    ++L.launches;
+    if (!one_round) wf_raygen_list_kernel<<<(p.n_list + 255) / 256, 256, 0, s>>>(p);
+    L.launches += one_round ? 0 : 1;
     /* the network adjoint's launches are timed (when the renderer's kernel timing is on) */
     auto timed_begin = [&]() {
         if (L.ev && L.n_timed < L.cap) cudaEventRecord(L.ev[2 * L.n_timed], s);
@@ -2310,9 +2385,10 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
     const int grid_ray = ray_grid(p.n_list, n_sms);
     check_every = check_interval(p, check_every);
     for (int it = 0; it < (1 << 20); ++it) {
-        wf_march_kernel<CACHED><<<grid_ray, 128, 0, s>>>(p, it);
+        if (!one_round) wf_march_kernel<CACHED><<<grid_ray, 128, 0, s>>>(p, it);
         /* the forward kernels of pass 1, so both passes composite the same values */
-        if (CACHED) {
+        if (one_round) {
+        } else if (CACHED) {
             const size_t tc_smem = tc_smem_bytes(p.freq);
             const int grid_tc = n_sms * FVC_TC_CTAS_PER_SM;
             launch_classify(p, it, n_sms, s);
@@ -2334,7 +2410,8 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
         timed_end();
         if (e == cudaSuccess && CACHED) e = launch_cache_backward(p, b, HH, it, n_sms, s);
         if (e != cudaSuccess) return e;
-        L.launches += CACHED ? 4 : 3;
+        L.launches += 1 + (one_round ? 1 : 2) + (CACHED ? 1 : 0);
+        if (one_round) break;
         if ((it + 1) % check_every == 0) {
             e = cudaMemcpyAsync(h_pinned, p.counters + ((it + 1) & 1), sizeof(int), cudaMemcpyDeviceToHost, s);
             if (e != cudaSuccess) return e;
@@ -2347,13 +2424,13 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
 }
 
 cudaError_t backward_frame(const RenderParams &p, const BwdParams &b, bool cached, int head_hidden, int n_sms, cudaStream_t s,
-                           int *h_pinned, int check_every, LaunchLog *log)
+                           int *h_pinned, int check_every, bool one_round, LaunchLog *log)
 {
     if (cached)
-        return head_hidden == 2 ? run_backward<true, 2>(p, b, n_sms, s, h_pinned, check_every, log)
-                                : run_backward<true, 1>(p, b, n_sms, s, h_pinned, check_every, log);
-    return head_hidden == 2 ? run_backward<false, 2>(p, b, n_sms, s, h_pinned, check_every, log)
-                            : run_backward<false, 1>(p, b, n_sms, s, h_pinned, check_every, log);
+        return head_hidden == 2 ? run_backward<true, 2>(p, b, n_sms, s, h_pinned, check_every, one_round, log)
+                                : run_backward<true, 1>(p, b, n_sms, s, h_pinned, check_every, one_round, log);
+    return head_hidden == 2 ? run_backward<false, 2>(p, b, n_sms, s, h_pinned, check_every, one_round, log)
+                            : run_backward<false, 1>(p, b, n_sms, s, h_pinned, check_every, one_round, log);
 }
 
 template <bool CACHED, int HH>
