@@ -1744,11 +1744,35 @@ __global__ void wf_reset_rows_kernel(RenderParams p, int cached)
     if (threadIdx.x == 0) reset_row_counters(p, cached);
 }
 
-constexpr int COMP_AHEAD = 4; /* samples of a ray whose rows the compositing loads together */
+/* samples of a ray whose rows the compositing loads together */
+#ifndef FVC_COMP_AHEAD_CACHED
+#define FVC_COMP_AHEAD_CACHED 2
+#endif
+constexpr int COMP_AHEAD = 4, COMP_AHEAD_CACHED = FVC_COMP_AHEAD_CACHED;
+
+/* The compositing adjoint takes a window's rows twice.  First the warp
+ * computes every row's factors (opacity and colour), 32 consecutive rows at a
+ * time whoever's they are: coalesced loads, full lanes for the exponentials,
+ * no row waiting on the one before.  Then each lane walks its own ray's rows
+ * in shared memory, and the gradients go out 32 consecutive rows at a time.
+ * One warp's window has at most WARP_ROWS rows.  Measured against a walk that
+ * loaded and evaluated its rows one by one, 4099 rays of the 256x256
+ * workload's scene: 219 -> 166 us.  (The forward compositing gains nothing
+ * from the same: its walk, with three divisions, is the longer part.) */
+constexpr int COMP_THREADS = 64, COMP_WARPS = COMP_THREADS / 32, WARP_ROWS = 32 * S_ROWS;
+
+/* a warp's rows of one window: the first and how many */
+__device__ __forceinline__ void warp_rows(int2 rr, int &first, int &total)
+{
+    const int n = window_rows(rr.y);
+    first = __reduce_max_sync(FULLMASK, n ? rr.x : 0);
+    total = __reduce_add_sync(FULLMASK, n);
+}
 
 template <bool CACHED>
 __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int it)
 {
+    constexpr int AHEAD = CACHED ? COMP_AHEAD_CACHED : COMP_AHEAD;
     const int n_alive = p.counters[it & 1];
     if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p, CACHED);
     RayState *cur = p.states[it & 1], *nxt = p.states[(it + 1) & 1];
@@ -1782,15 +1806,15 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
                 more_windows = !window_none(rr.y);
             }
             /* rows are in t order: the merge of the resample and cache streams of
-             * accumulate_cache_perf_kernel (:270-304); COMP_AHEAD samples are loaded together, before the
+             * accumulate_cache_perf_kernel (:270-304); AHEAD samples are loaded together, before the
              * first of them is composited */
             RowWalk walk(rr, true, p.by_sample);
             for (bool more = true; more;) {
-                int rs[COMP_AHEAD], codes[COMP_AHEAD];
-                uint2 ovs[COMP_AHEAD];
-                float t0s[COMP_AHEAD];
+                int rs[AHEAD], codes[AHEAD];
+                uint2 ovs[AHEAD];
+                float t0s[AHEAD];
 #pragma unroll
-                for (int q = 0; q < COMP_AHEAD; ++q) {
+                for (int q = 0; q < AHEAD; ++q) {
                     more = walk.step(rs[q]) && more;
                     if (term) rs[q] = -1;
                     codes[q] = CACHED && rs[q] >= 0 ? (int)p.row_kind[rs[q]] : KIND_RESAMPLE;
@@ -1802,7 +1826,7 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
                     }
                 }
 #pragma unroll
-                for (int q = 0; q < COMP_AHEAD; ++q) {
+                for (int q = 0; q < AHEAD; ++q) {
                     if (rs[q] < 0 || term) continue;
                     const int kind = row_kind_of(codes[q]);
                     if (CACHED && kind != KIND_SKIP && row_reason_of(codes[q])) why += 1ull << ((9 * (row_reason_of(codes[q]) - 1)) & 63);
@@ -1882,8 +1906,12 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
  * with a gradient are listed per stream: grad_res_list (counters[6]),
  * grad_cache_list (counters[7]). */
 template <bool CACHED>
-__global__ void __launch_bounds__(128) wf_composite_bwd_kernel(RenderParams p, int it)
+__global__ void __launch_bounds__(COMP_THREADS) wf_composite_bwd_kernel(RenderParams p, int it)
 {
+    __shared__ float4 s_vals[COMP_WARPS][WARP_ROWS];  /* opacity and colour, then the row's gradient */
+    __shared__ float2 s_more[COMP_WARPS][WARP_ROWS];  /* step length and density, then .x = 1 for a row with a gradient */
+    float4 *vals = s_vals[threadIdx.x >> 5];
+    float2 *more = s_more[threadIdx.x >> 5];
     const int n_alive = p.counters[it & 1];
     if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p, CACHED);
     RayState *cur = p.states[it & 1], *nxt = p.states[(it + 1) & 1];
@@ -1903,64 +1931,88 @@ __global__ void __launch_bounds__(128) wf_composite_bwd_kernel(RenderParams p, i
         bool term = false, done = !valid, more_windows = true;
         for (int w = 0; w < p.windows; ++w) {
             int n_res = 0, n_cch = 0;
-            uint32_t gmask = 0, cmask = 0;
             int2 rr = make_int2(0, 0);
             if (!done) { /* also of a ray that has ended: the others' rows follow its own */
                 rr = p.ray_rows[(size_t)w * p.ray_stride + i];
                 done = window_done(rr.y);
                 more_windows = !window_none(rr.y);
             }
+            int first, total;
+            warp_rows(rr, first, total);
+#pragma unroll 2
+            for (int k = lane_id(); k < total; k += 32) {
+                const int r = first + k;
+                const uint2 ov = p.row_out[r];
+                const float2 lg = __half22float2(*reinterpret_cast<const __half2 *>(&ov.x));
+                const float lb = __half2float(__ushort_as_half((unsigned short)(ov.y & 0xffffu)));
+                const float ld = __half2float(__ushort_as_half((unsigned short)(ov.y >> 16)));
+                const float dt = calc_step(p.steps, p.row_t0[r]);
+                const float sigma = expf(ld);
+                const bool used = !CACHED || row_kind_of(p.row_kind[r]) < KIND_DROP;
+                /* a dropped row has no output: an opacity below every threshold */
+                vals[k] = make_float4(used ? fminf(1.0f, fmaxf(0.0f, 1.0f - expf(-sigma * dt))) : -1.0f, 1.0f / (1.0f + expf(-lg.x)),
+                                      1.0f / (1.0f + expf(-lg.y)), 1.0f / (1.0f + expf(-lb)));
+                more[k] = make_float2(dt, sigma);
+            }
+            __syncwarp();
             int r;
             RowWalk walk(rr, true, p.by_sample);
-            for (int j = 0; walk.step(r); ++j) {
-                if (r >= 0) {
-                    float4 dout = make_float4(0.f, 0.f, 0.f, 0.f);
-                    const int kind = CACHED ? row_kind_of(p.row_kind[r]) : KIND_RESAMPLE;
-                    if (!term && kind < KIND_DROP) {
-                        const uint2 ov = p.row_out[r];
-                        const float t0 = p.row_t0[r];
-                        const float2 lg = __half22float2(*reinterpret_cast<const __half2 *>(&ov.x));
-                        const float lb = __half2float(__ushort_as_half((unsigned short)(ov.y & 0xffffu)));
-                        const float ld = __half2float(__ushort_as_half((unsigned short)(ov.y >> 16)));
-                        const float dt = calc_step(p.steps, t0);
-                        const float sigma = expf(ld);
-                        const float alpha = fminf(1.0f, fmaxf(0.0f, 1.0f - expf(-sigma * dt)));
-                        if (alpha > p.scene.alpha_thre) {
-                            const float c0 = 1.0f / (1.0f + expf(-lg.x)), c1 = 1.0f / (1.0f + expf(-lg.y)),
-                                        c2 = 1.0f / (1.0f + expf(-lb));
-                            const float gc = rg.x * c0 + rg.y * c1 + rg.z * c2;
-                            const float ta = T * alpha;
-                            xp += ta * gc;
-                            const float Tn = T * (1.0f - alpha);
-                            const float dsig = dt * (Tn * gc - (rg.w - xp));
-                            dout = make_float4(rg.x * ta * c0 * (1.0f - c0), rg.y * ta * c1 * (1.0f - c1), rg.z * ta * c2 * (1.0f - c2),
-                                               dsig * sigma);
-                            T = Tn;
-                            if (kind == KIND_CACHE) { cmask |= 1u << j; ++n_cch; }
-                            else { gmask |= 1u << j; ++n_res; }
-                        }
-                        if (T < 1e-4f) term = true;
+            while (walk.step(r)) {
+                if (r < 0) continue;
+                const int k = r - first;
+                const float4 v = vals[k];
+                const float2 ds = more[k];
+                bool has = false;
+                if (!term && v.x >= 0.0f) {
+                    if (v.x > p.scene.alpha_thre) {
+                        const float gc = rg.x * v.y + rg.y * v.z + rg.z * v.w;
+                        const float ta = T * v.x;
+                        xp += ta * gc;
+                        const float Tn = T * (1.0f - v.x);
+                        const float dsig = ds.x * (Tn * gc - (rg.w - xp));
+                        vals[k] = make_float4(rg.x * ta * v.y * (1.0f - v.y), rg.y * ta * v.z * (1.0f - v.z),
+                                              rg.z * ta * v.w * (1.0f - v.w), dsig * ds.y);
+                        T = Tn;
+                        has = true;
                     }
-                    p.row_dout[r] = dout;
+                    if (T < 1e-4f) term = true;
                 }
+                more[k].x = has ? 1.0f : 0.0f;
             }
-            /* list the rows with a gradient per network stream (one atomic per warp and list) */
-            auto append = [&](int n, uint32_t mask, int *list, int *counter) {
-                const int total = (int)__reduce_add_sync(FULLMASK, (unsigned)n);
-                if (total == 0) return;
-                int lb = 0;
-                if (lane_id() == 0) lb = atomicAdd(counter, total);
-                ListWalk places(__shfl_sync(FULLMASK, lb, 0), n, p.by_sample);
-                int row;
-                RowWalk rows(rr, true, p.by_sample);
-                for (int j = 0; rows.step(row); ++j) {
-                    const bool has = (mask >> j) & 1u;
-                    const int at = places.place(has);
-                    if (has) list[at] = row;
-                }
+            __syncwarp();
+            /* the rows with a gradient: written out, and listed per network stream in the rows' order (one atomic
+             * per warp, window and list) */
+            auto with_gradient = [&](int k, bool &res, bool &hit) {
+                const bool has = k < total && more[k].x != 0.0f;
+                hit = CACHED && has && row_kind_of(p.row_kind[first + k]) == KIND_CACHE;
+                res = has && !hit;
             };
-            append(n_res, gmask, p.grad_res_list, p.counters + 6);
-            if (CACHED) append(n_cch, cmask, p.grad_cache_list, p.counters + 7);
+            for (int k0 = 0; k0 < total; k0 += 32) {
+                bool res, hit;
+                with_gradient(k0 + lane_id(), res, hit);
+                if (res || hit) p.row_dout[first + k0 + lane_id()] = vals[k0 + lane_id()];
+                n_res += __popc(__ballot_sync(FULLMASK, res));
+                if (CACHED) n_cch += __popc(__ballot_sync(FULLMASK, hit));
+            }
+            int rb = 0, hb = 0;
+            if (lane_id() == 0) {
+                if (n_res) rb = atomicAdd(p.counters + 6, n_res);
+                if (n_cch) hb = atomicAdd(p.counters + 7, n_cch);
+            }
+            rb = __shfl_sync(FULLMASK, rb, 0);
+            hb = __shfl_sync(FULLMASK, hb, 0);
+            for (int k0 = 0; k0 < total; k0 += 32) {
+                bool res, hit;
+                with_gradient(k0 + lane_id(), res, hit);
+                const unsigned m0 = __ballot_sync(FULLMASK, res);
+                if (res) p.grad_res_list[rb + __popc(m0 & lane_lt())] = first + k0 + lane_id();
+                rb += __popc(m0);
+                if (!CACHED) continue;
+                const unsigned m1 = __ballot_sync(FULLMASK, hit);
+                if (hit) p.grad_cache_list[hb + __popc(m1 & lane_lt())] = first + k0 + lane_id();
+                hb += __popc(m1);
+            }
+            __syncwarp(); /* the next window overwrites the rows */
             if (__all_sync(FULLMASK, term || done || !more_windows)) break;
         }
         if (valid) {
@@ -2226,7 +2278,10 @@ static void launch_plain_net(const RenderParams &p, int it, int n_sms, cudaStrea
 }
 
 /* blocks of the per-ray kernels: no more than the rays fill */
-static inline int ray_grid(int n_rays, int n_sms) { return std::max(1, std::min(n_sms * FVC_RAY_BLOCKS_PER_SM, (n_rays + 127) / 128)); }
+static inline int ray_grid(int n_rays, int n_sms, int threads = 128)
+{
+    return std::max(1, std::min(n_sms * FVC_RAY_BLOCKS_PER_SM * (128 / threads), (n_rays + threads - 1) / threads));
+}
 
 /* sub-iterations between two readbacks of the alive count: with more march windows a sub-iteration there are fewer */
 static inline int check_interval(const RenderParams &p, int every) { return p.windows >= 8 ? 1 : p.windows > 1 ? std::min(every, 2) : every; }
@@ -2382,7 +2437,7 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
         if (L.ev && L.n_timed < L.cap) cudaEventRecord(L.ev[2 * L.n_timed++ + 1], s);
         else if (L.ev) ++L.n_untimed;
     };
-    const int grid_ray = ray_grid(p.n_list, n_sms);
+    const int grid_ray = ray_grid(p.n_list, n_sms), grid_comp = ray_grid(p.n_list, n_sms, COMP_THREADS);
     check_every = check_interval(p, check_every);
     for (int it = 0; it < (1 << 20); ++it) {
         if (!one_round) wf_march_kernel<CACHED><<<grid_ray, 128, 0, s>>>(p, it);
@@ -2404,7 +2459,7 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
             launch_plain_net<HH>(p, it, n_sms, s);
             L.launches += 1;
         }
-        wf_composite_bwd_kernel<CACHED><<<grid_ray, 128, 0, s>>>(p, it);
+        wf_composite_bwd_kernel<CACHED><<<grid_comp, COMP_THREADS, 0, s>>>(p, it);
         timed_begin();
         cudaError_t e = launch_net_backward(p, b, HH, it, n_sms, s);
         timed_end();
