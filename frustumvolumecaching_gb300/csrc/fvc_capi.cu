@@ -1316,6 +1316,20 @@ static int rows_by_sample(const RenderParams &p)
     return step * p.cam.fx > 1.5f * t;
 }
 
+/* Whether 8 lanes march a ray (wf_march_lanes_kernel): with so few rays that
+ * one lane each leaves the schedulers short of warps, and whole windows of 16
+ * steps a group.  A plain frame of the 256x256 workload's scene, us without /
+ * with: 48x27 532 / 262, 64x64 585 / 321, 128x128 742 / 530, 200x200 1069 /
+ * 955, 256x256 1507 / 1430, 320x240 1407 / 1352; above about 10^5 rays the
+ * chip is full and the doubled instructions cost more than they give. */
+#ifndef FVC_LANES_RAYS
+#define FVC_LANES_RAYS 98304
+#endif
+static int march_by_lanes(const RenderParams &p, size_t n_rays)
+{
+    return n_rays <= FVC_LANES_RAYS && !p.skip_empty && p.steps_per_iter % 16 == 0;
+}
+
 static int setup_render_params(fvc_renderer *r, const fvc_raymarch_info *info, float4 *results, uchar4 *image, int4 *counts,
                                RenderParams &p, bool per_view_caches = false)
 {
@@ -1381,7 +1395,8 @@ static int setup_render_params(fvc_renderer *r, const fvc_raymarch_info *info, f
     p.windows = r->row_target > 0 || r->steps_per_iter != MARCH_STEPS ? 1 : r->windows;
     p.ray_stride = r->ray_stride;
     p.row_capacity = r->row_capacity;
-    p.by_sample = rows_by_sample(p);
+    p.march_lanes = march_by_lanes(p, (size_t)r->W * r->H);
+    p.by_sample = !p.march_lanes && rows_by_sample(p);
     return FVC_OK;
 }
 
@@ -1794,6 +1809,7 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
     if ((rc = setup_render_params(r, info, nullptr, nullptr, nullptr, p, true))) return rc;
     p.steps_per_iter = 1 << 26; /* sample_common_kernel marches until it has its samples */
     p.windows = 1;
+    p.march_lanes = 0;
     PerRayScratch &x = r->pr;
     const size_t n_bricks = (size_t)c->bX * c->bY * c->bZ, n_cols = (size_t)c->bX * c->bY, n_rows = (size_t)r->row_capacity;
     if (x.n_bricks < n_bricks || x.n_cols < n_cols || x.n_rows < n_rows) {
@@ -2204,6 +2220,7 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
         p.ray_stride = n_rays;
     }
     p.list_order = r->d_list_order;
+    p.march_lanes = march_by_lanes(p, n_rays);
     p.ray_grad = g->d_ray_grad;
     p.row_dout = r->d_row_dout;
     p.grad_res_list = r->d_grad_rows;

@@ -348,6 +348,7 @@ struct RenderParams {
     int *res_list, *cache_list; /* row ids of the two network streams */
     int *counters;              /* [0], [1] alive rays (ping-pong), [2] rows, [3] resample, [4] cache */
     int by_sample;              /* a warp's rows sample by sample instead of ray by ray (RowWalk) */
+    int march_lanes;            /* few rays: 8 lanes march a ray (wf_march_lanes_kernel; its rows lie ray by ray) */
     int steps_per_iter;         /* marching steps per ray and sub-iteration */
     int m_tile;                 /* rows per tcgen05 network tile on the plain path: 64, 128 (0 = 128) or 256 */
     int fused_classify;         /* cached renders: classification in the march, one network launch for all rows */

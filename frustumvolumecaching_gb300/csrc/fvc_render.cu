@@ -461,6 +461,39 @@ __device__ __forceinline__ int classify_basic(const RenderParams &p, const Cache
                                   * 32 -> 12.0, 64 -> 11.5, 128 -> 11.6) */
 #endif
 
+/* One sample's row beside its t0 and slot.  FUSED: the cached renderer's
+ * classification (wf_classify_kernel's non-basic form; oc, dc the ray in the
+ * cache camera's frame) and the input of a resample or cache row, the row's
+ * kind returned; else the plain renderer's contracted midpoint (t0 + t1) / 2
+ * (sample_performance_kernel :52-58). */
+template <bool FUSED>
+__device__ __forceinline__ int march_row(const RenderParams &p, const CacheView &C, const DevCam &ccam, const DevSteps &cst, float3 o, float3 d,
+                                         float3 oc, float3 dc, float t0, int r)
+{
+    const float dt = calc_step(p.steps, t0);
+    const float tm = F_MUL(F_ADD(t0, F_ADD(t0, dt)), 0.5f);
+    if (!FUSED) {
+        const float3 pc = contract(p.scene, at(o, d, tm));
+        p.row_pay[r] = make_float4(pc.x, pc.y, pc.z, 0.f);
+        return KIND_RESAMPLE;
+    }
+    const float tmh = F_ADD(t0, F_MUL(dt, 0.5f));
+    const int code = classify(p, C, ccam, cst, oc, dc, tm);
+    const int kind = row_kind_of(code);
+    float4 pay = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (kind == KIND_RESAMPLE) {
+        const float3 pc = contract(p.scene, at(o, d, tmh));
+        pay = make_float4(pc.x, pc.y, pc.z, 0.f);
+    } else if (kind == KIND_CACHE) {
+        float tf2;
+        const float3 fr = cam2froxel(at(oc, dc, tmh), ccam, cst, tf2);
+        pay = make_float4(fr.x, fr.y, fr.z, 0.f);
+    }
+    p.row_pay[r] = pay;
+    p.row_kind[r] = (uint8_t)code;
+    return kind;
+}
+
 template <bool CACHED, bool FUSED = false>
 __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
 {
@@ -575,24 +608,9 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
                     int kind = KIND_SKIP;
                     if (r >= 0) {
                         const float t0 = t0s[s][threadIdx.x];
-                        const float dt = calc_step(p.steps, t0);
-                        const float tm = F_MUL(F_ADD(t0, F_ADD(t0, dt)), 0.5f);
-                        const float tmh = F_ADD(t0, F_MUL(dt, 0.5f));
-                        const int code = classify(p, C, ccam, cst, oc, dc, tm);
-                        kind = row_kind_of(code);
-                        float4 pay = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (kind == KIND_RESAMPLE) {
-                            const float3 pc = contract(p.scene, at(o, d, tmh));
-                            pay = make_float4(pc.x, pc.y, pc.z, 0.f);
-                        } else if (kind == KIND_CACHE) {
-                            float tf2;
-                            const float3 fr = cam2froxel(at(oc, dc, tmh), ccam, cst, tf2);
-                            pay = make_float4(fr.x, fr.y, fr.z, 0.f);
-                        }
                         p.row_t0[r] = t0;
                         p.row_slot[r] = i;
-                        p.row_pay[r] = pay;
-                        p.row_kind[r] = (uint8_t)code;
+                        kind = march_row<true>(p, C, ccam, cst, o, d, oc, dc, t0, r);
                         kinds |= (uint32_t)kind << (2 * s);
                     }
                     n_res += kind == KIND_RESAMPLE;
@@ -620,12 +638,9 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
                     const float t0 = t0s[s][threadIdx.x];
                     p.row_t0[r] = t0;
                     p.row_slot[r] = i;
-                    if (!CACHED) {
-                        /* sample_performance_kernel :52-58: midpoint (t0+t1)/2, contracted */
-                        const float tm = F_MUL(F_ADD(t0, F_ADD(t0, calc_step(p.steps, t0))), 0.5f);
-                        const float3 pc = contract(p.scene, at(make_float3(of.x, of.y, of.z), make_float3(dt4.x, dt4.y, dt4.z), tm));
-                        p.row_pay[r] = make_float4(pc.x, pc.y, pc.z, 0.f);
-                    }
+                    if (!CACHED)
+                        march_row<false>(p, p.cache, p.ccam, p.csteps, make_float3(of.x, of.y, of.z), make_float3(dt4.x, dt4.y, dt4.z),
+                                         make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f), t0, r);
                 }
             }
             if (valid) p.ray_rows[(size_t)w * p.ray_stride + i] = make_int2(rbase, window_pack(n, steps, done));
@@ -644,6 +659,164 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
         }
         const int ws = __reduce_add_sync(FULLMASK, all_steps);
         if (lane_id() == 0 && ws) atomicAdd(&p.stats->n_steps, (unsigned long long)ws);
+    }
+}
+
+/* The march of few rays.  A lane that marches its ray alone leaves most of the
+ * chip's schedulers with one warp or none, each a serial chain of a window's
+ * 64 steps.  Here 8 lanes share a ray: every lane advances the step sequence to
+ * its own two steps of the next 16 (the sequence itself is four dependent
+ * operations a step), looks their cells up, and the group takes the steps the
+ * lone lane would have taken from the ballots of occupied and past steps.  A
+ * block's 32 rays are one warp of the compositing, and their rows lie ray by
+ * ray.  Twice the instructions of the other march, so only where rays are few
+ * (march_by_lanes, fvc_capi.cu): 31 windows of 4099 rays 368 -> 95 us. */
+constexpr int ML_LANES = 8, ML_STEPS = 2 * ML_LANES;
+
+/* bit b of the low 8 bits at 2 b */
+__device__ __forceinline__ uint32_t spread8(uint32_t v)
+{
+    v = (v | (v << 4)) & 0x0f0fu;
+    v = (v | (v << 2)) & 0x3333u;
+    return (v | (v << 1)) & 0x5555u;
+}
+
+template <bool CACHED, bool FUSED>
+__global__ void __launch_bounds__(32 * ML_LANES) wf_march_lanes_kernel(RenderParams p, int it)
+{
+    __shared__ float t0s[32][S_ROWS];
+    __shared__ int s_n[32], s_row[32], s_first;
+    const int n_alive = p.counters[it & 1];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        p.counters[(it + 1) & 1] = 0;
+        p.counters[6] = p.counters[7] = 0;
+    }
+    const int S = max(1, min(S_ROWS, p.batch_rows / max(1, n_alive)));
+    RayState *states = p.states[it & 1];
+    const int q = threadIdx.x / ML_LANES, l = threadIdx.x % ML_LANES, group = lane_id() & ~(ML_LANES - 1);
+    for (int base = blockIdx.x * 32; base < n_alive; base += gridDim.x * 32) {
+        const int i = base + q;
+        const bool valid = i < n_alive;
+        float4 of = make_float4(0, 0, 0, 0), dt4 = make_float4(0, 0, 0, 0);
+        if (valid) {
+            of = states[i].of;
+            dt4 = states[i].dt;
+        }
+        const float3 o = make_float3(of.x, of.y, of.z), d = make_float3(dt4.x, dt4.y, dt4.z);
+        float t1 = dt4.w;
+        bool done = !valid;
+        int all_steps = 0, all_rows = 0;
+        for (int w = 0; w < p.windows; ++w) {
+            int n = 0, steps = 0;
+            const float t_window = t1;
+            const bool done_before = done;
+            for (int c0 = 0; c0 < p.steps_per_iter; c0 += ML_STEPS) {
+                const bool active = !done && n < S; /* uniform in the group */
+                if (!__any_sync(FULLMASK, active)) break;
+                float ta = t1;
+#pragma unroll
+                for (int c = 0; c < ML_STEPS - 2; ++c)
+                    if (c < 2 * l) ta = F_ADD(ta, calc_step(p.steps, ta));
+                const float tb = F_ADD(ta, calc_step(p.steps, ta)), tc = F_ADD(tb, calc_step(p.steps, tb));
+                const float2 tm = make_float2(F_MUL(F_ADD(ta, tb), 0.5f), F_MUL(F_ADD(tb, tc), 0.5f));
+                const uint32_t occ = active ? occupied2(p.scene, p.bits, p.cells, o, d, tm) : 0u;
+                const uint32_t o0 = __ballot_sync(FULLMASK, occ & 1u) >> group, o1 = __ballot_sync(FULLMASK, occ & 2u) >> group;
+                const uint32_t p0 = __ballot_sync(FULLMASK, tm.x > of.w) >> group, p1 = __ballot_sync(FULLMASK, tm.y > of.w) >> group;
+                /* the midpoints grow along the ray: the steps past the far bound are the last ones */
+                const int inside = ML_STEPS - __popc(p0 & 0xffu) - __popc(p1 & 0xffu);
+                uint32_t m = (spread8(o0 & 0xffu) | (spread8(o1 & 0xffu) << 1)) & ((1u << inside) - 1u);
+                int used = ML_STEPS;
+                bool ends = inside < ML_STEPS;
+                if (active && __popc(m) >= S - n) { /* the step that fills the window */
+                    uint32_t rest = m;
+                    for (int k = S - n; k > 1; --k) rest &= rest - 1u;
+                    used = __ffs(rest);
+                    m &= (2u << (used - 1)) - 1u;
+                    ends = false;
+                }
+                const float t_next = __shfl_sync(FULLMASK, (used & 1) ? tb : tc, (used - 1) >> 1, ML_LANES);
+                if (!active) continue;
+                const uint32_t before = (1u << (2 * l)) - 1u;
+                if ((m >> (2 * l)) & 1u) t0s[q][n + __popc(m & before)] = ta;
+                if ((m >> (2 * l)) & 2u) t0s[q][n + __popc(m & (2u * before + 1u))] = tb;
+                n += __popc(m);
+                if (ends) {
+                    steps += inside + 1;
+                    done = true;
+                } else {
+                    steps += used;
+                    t1 = t_next;
+                }
+            }
+            /* the block's rows, ray by ray */
+            if (l == 0) s_n[q] = n;
+            __syncthreads();
+            if (threadIdx.x < 32) {
+                const int mine = s_n[threadIdx.x], before = lanes_before(mine);
+                const int total = __shfl_sync(FULLMASK, before + mine, 31);
+                int first = 0;
+                if (threadIdx.x == 0 && total) {
+                    first = atomicAdd(p.counters + 2, total);
+                    if (first + total > p.row_capacity) {
+                        atomicSub(p.counters + 2, total);
+                        first = -1;
+                    }
+                }
+                first = __shfl_sync(FULLMASK, first, 0);
+                s_row[threadIdx.x] = first + before;
+                if (threadIdx.x == 0) s_first = first;
+            }
+            __syncthreads();
+            const int first = s_first, row = s_row[q];
+            if (first < 0) { /* no room: the rays wait at this window's start for the next sub-iteration */
+                if (l == 0 && !done_before) p.ray_rows[(size_t)w * p.ray_stride + i] = make_int2(0, window_pack(0, 0, false));
+                t1 = t_window;
+                break;
+            }
+            const ViewCache *vc = FUSED && p.view_caches && valid ? p.view_caches + states[i].cnt2.w : nullptr;
+            const CacheView &C = vc ? vc->cache : p.cache;
+            const DevCam &ccam = vc ? vc->ccam : p.ccam;
+            const DevSteps &cst = vc ? vc->csteps : p.csteps;
+            float3 oc = make_float3(0.f, 0.f, 0.f), dc = oc;
+            if (FUSED) transform_ray(ccam.w2c, o, d, oc, dc);
+            for (int s0 = 0; __any_sync(FULLMASK, s0 < n); s0 += ML_LANES) {
+                const int r = row + s0 + l;
+                int kind = KIND_SKIP;
+                if (s0 + l < n) {
+                    const float t0 = t0s[q][s0 + l];
+                    p.row_t0[r] = t0;
+                    p.row_slot[r] = i;
+                    if (FUSED || !CACHED) kind = march_row<FUSED>(p, C, ccam, cst, o, d, oc, dc, t0, r);
+                }
+                if (FUSED) { /* the resample and the cache list, as the other march */
+                    const unsigned m0 = __ballot_sync(FULLMASK, kind == KIND_RESAMPLE), m1 = __ballot_sync(FULLMASK, kind == KIND_CACHE);
+                    int rb = 0, hb = 0;
+                    if (lane_id() == 0) {
+                        if (m0) rb = atomicAdd(p.counters + 3, __popc(m0));
+                        if (m1) hb = atomicAdd(p.counters + 4, __popc(m1));
+                    }
+                    rb = __shfl_sync(FULLMASK, rb, 0);
+                    hb = __shfl_sync(FULLMASK, hb, 0);
+                    if (kind == KIND_RESAMPLE) p.res_list[rb + __popc(m0 & lane_lt())] = r;
+                    else if (kind == KIND_CACHE) p.cache_list[hb + __popc(m1 & lane_lt())] = r;
+                }
+            }
+            if (l == 0 && valid) p.ray_rows[(size_t)w * p.ray_stride + i] = make_int2(first, window_pack(n, steps, done));
+            all_steps += steps;
+            all_rows += n;
+            if (__syncthreads_and(done)) break; /* also: the shared rows are read before the next window's */
+        }
+        if (l == 0 && valid) {
+            states[i].dt.w = t1;
+            if (p.max_samples_per_ray > 0) {
+                const int pushed = states[i].cnt2.z + all_rows;
+                states[i].cnt2.z = pushed;
+                if (pushed > p.max_samples_per_ray) atomicOr(p.guard, 1);
+            }
+        }
+        const int ws = __reduce_add_sync(FULLMASK, l == 0 ? all_steps : 0);
+        if (lane_id() == 0 && ws) atomicAdd(&p.stats->n_steps, (unsigned long long)ws);
+        __syncthreads();
     }
 }
 
@@ -2283,6 +2456,14 @@ static inline int ray_grid(int n_rays, int n_sms, int threads = 128)
     return std::max(1, std::min(n_sms * FVC_RAY_BLOCKS_PER_SM * (128 / threads), (n_rays + threads - 1) / threads));
 }
 
+/* one sub-iteration's march of n_rays rays at most */
+template <bool CACHED, bool FUSED>
+static void launch_march(const RenderParams &p, int it, int n_rays, int n_sms, cudaStream_t s)
+{
+    if (p.march_lanes) wf_march_lanes_kernel<CACHED, FUSED><<<std::max(1, (n_rays + 31) / 32), 32 * ML_LANES, 0, s>>>(p, it);
+    else wf_march_kernel<CACHED, FUSED><<<ray_grid(n_rays, n_sms), 128, 0, s>>>(p, it);
+}
+
 /* sub-iterations between two readbacks of the alive count: with more march windows a sub-iteration there are fewer */
 static inline int check_interval(const RenderParams &p, int every) { return p.windows >= 8 ? 1 : p.windows > 1 ? std::min(every, 2) : every; }
 
@@ -2308,7 +2489,7 @@ static cudaError_t run_frame(const RenderParams &p, int n_sms, cudaStream_t s, i
     if (p.pixel_list) wf_raygen_list_kernel<<<(p.n_list + 255) / 256, 256, 0, s>>>(p);
     else wf_raygen_kernel<<<(n_threads + 255) / 256, 256, 0, s>>>(p);
     ++L.launches;
-    const int grid_ray = ray_grid(p.pixel_list ? p.n_list : W * H, n_sms);
+    const int n_rays = p.pixel_list ? p.n_list : W * H, grid_ray = ray_grid(n_rays, n_sms);
     check_every = check_interval(p, check_every);
     const int grid_net = n_sms * 2;
     const size_t net_smem = sizeof(NetSmem);
@@ -2319,14 +2500,14 @@ static cudaError_t run_frame(const RenderParams &p, int n_sms, cudaStream_t s, i
     const int max_it = 1 << 20;
     for (; it < max_it; ++it) {
         if (fused) {
-            wf_march_kernel<true, true><<<grid_ray, 128, 0, s>>>(p, it);
+            launch_march<true, true>(p, it, n_rays, n_sms, s);
             wf_cache_lookup_kernel<<<n_sms * 8, 256, 0, s>>>(p, it);
             timed_begin();
             wf_net_tc_kernel<2, HH, false><<<grid_tc, 128, tc_smem, s>>>(p, it);
             timed_end();
             L.launches += 3;
         } else {
-            wf_march_kernel<CACHED><<<grid_ray, 128, 0, s>>>(p, it);
+            launch_march<CACHED, false>(p, it, n_rays, n_sms, s);
             ++L.launches;
         }
         if (CACHED && !fused) {
@@ -2437,10 +2618,10 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
         if (L.ev && L.n_timed < L.cap) cudaEventRecord(L.ev[2 * L.n_timed++ + 1], s);
         else if (L.ev) ++L.n_untimed;
     };
-    const int grid_ray = ray_grid(p.n_list, n_sms), grid_comp = ray_grid(p.n_list, n_sms, COMP_THREADS);
+    const int grid_comp = ray_grid(p.n_list, n_sms, COMP_THREADS);
     check_every = check_interval(p, check_every);
     for (int it = 0; it < (1 << 20); ++it) {
-        if (!one_round) wf_march_kernel<CACHED><<<grid_ray, 128, 0, s>>>(p, it);
+        if (!one_round) launch_march<CACHED, false>(p, it, p.n_list, n_sms, s);
         /* the forward kernels of pass 1, so both passes composite the same values */
         if (one_round) {
         } else if (CACHED) {
@@ -2541,12 +2722,12 @@ static cudaError_t build_batch_graph_t(const RenderParams &p, int n_sms, cudaStr
         const bool fused = CACHED && fused_cached_path(p);
         for (int it = 0; it < 2; ++it) {
             if (fused) {
-                wf_march_kernel<true, true><<<grid_ray, 128, 0, s>>>(p, it);
+                launch_march<true, true>(p, it, n_rays, n_sms, s);
                 wf_cache_lookup_kernel<<<n_sms * 8, 256, 0, s>>>(p, it);
                 wf_net_tc_kernel<2, HH, false><<<n_sms * FVC_TC_CTAS_PER_SM, 128, tc_smem_bytes(p.freq), s>>>(p, it);
                 kernels += 2;
             } else {
-                wf_march_kernel<CACHED><<<grid_ray, 128, 0, s>>>(p, it);
+                launch_march<CACHED, false>(p, it, n_rays, n_sms, s);
             }
             if (CACHED && !fused) {
                 const size_t tc_smem = tc_smem_bytes(p.freq);
