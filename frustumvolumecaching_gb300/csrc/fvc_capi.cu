@@ -1728,6 +1728,7 @@ extern "C" int fvc_cache_build(fvc_renderer *r, const fvc_raymarch_info *info)
     p.max_search = c->bZ + 4;
     p.build_rows = b.rows; p.build_den = b.den; p.build_lat = b.lat; p.build_row_of = b.row_of;
     p.build_row_counter = b.counters + 5;
+    p.n_iterations = b.counters + 6;
 
     CU(cudaMemsetAsync(b.counters, 0, 8 * sizeof(int), s));
     CU(cudaMemsetAsync(c->d_packed, 0xff, (size_t)c->bX * c->bY * c->bZ * sizeof(int32_t), s));
@@ -1740,11 +1741,12 @@ extern "C" int fvc_cache_build(fvc_renderer *r, const fvc_raymarch_info *info)
     CU(cudaStreamSynchronize(s));
     int n_alive = r->h_pinned[0];
     long long n_samples = 0;
-    int iter = 0;
     const int max_iter = c->bZ + 8;
-    std::vector<int> dummy;
-    for (; iter < max_iter && n_alive > 0; ++iter) {
-        CU(cudaMemsetAsync(p.build_row_counter, 0, sizeof(int), s));
+    /* Tiles only die, so an alive count read BUILD_CHECK iterations ago still bounds the grids, and iterations past
+     * the last alive tile find nothing to do (a few us each); reading it after every iteration left the GPU idle
+     * for about 20 us a time. */
+    constexpr int BUILD_CHECK = 4;
+    for (int iter = 0; iter < max_iter && n_alive > 0; ++iter) {
         CU(launch_cache_search(p, std::min(n_alive, 1 << 16), s));
         CU(cudaGetLastError());
         /* the density network (fvc_renderer_set_build_network_path); view-dependent models' first head runs
@@ -1761,6 +1763,7 @@ extern "C" int fvc_cache_build(fvc_renderer *r, const fvc_raymarch_info *info)
         n_launches += 5;
         std::swap(p.alive_list, p.alive_list_next);
         std::swap(p.n_alive_tiles, p.n_alive_next);
+        if ((iter + 1) % BUILD_CHECK != 0 && iter + 1 < max_iter) continue;
         CU(cudaMemcpyAsync(r->h_pinned, p.n_alive_tiles, sizeof(int), cudaMemcpyDeviceToHost, s));
         CU(cudaStreamSynchronize(s));
         n_alive = r->h_pinned[0];
@@ -1775,7 +1778,7 @@ extern "C" int fvc_cache_build(fvc_renderer *r, const fvc_raymarch_info *info)
     c->stats.n_bricks_reserved = c->capacity();
     c->stats.n_bricks_set = std::min(demanded, c->capacity());
     c->stats.overflow = demanded > c->capacity();
-    c->stats.n_iterations = iter;
+    c->stats.n_iterations = r->h_pinned[6];
     c->stats.n_launches = n_launches;
     c->stats.n_samples = n_samples;
     c->built = true;

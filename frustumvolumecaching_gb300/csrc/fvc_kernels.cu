@@ -135,20 +135,10 @@ __global__ void __launch_bounds__(64) cache_init_kernel(CacheBuildParams p)
  *                          (accumulateNew_cache_init_second_kernel :289-528);
  * then cache_assign_kernel gives bricks their slots and cache_fill_kernel
  * writes their voxels. */
-__device__ __forceinline__ int tile_block_sum(int v, int *red)
-{
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int w = __reduce_add_sync(FULL, (unsigned)v);
-    __syncthreads();
-    if (lane == 0) red[wid] = w;
-    __syncthreads();
-    return red[0] + red[1];
-}
-
 template <bool VD>
-__global__ void __launch_bounds__(64) cache_search_kernel(CacheBuildParams p)
+__global__ void __launch_bounds__(64, 16) cache_search_kernel(CacheBuildParams p)
 {
-    __shared__ int red[4];
+    __shared__ int2 red[2];
     __shared__ int row_base;
     const int k = threadIdx.x, lane = k & 31, wid = k >> 5;
     const int n_alive_tiles = *p.n_alive_tiles;
@@ -158,12 +148,12 @@ __global__ void __launch_bounds__(64) cache_search_kernel(CacheBuildParams p)
         CacheRay cr = p.rays[(size_t)tile * 64 + k];
         int bstep = p.block_step[tile];
         uint32_t mask = 0;
-        bool found = false;
+        float t_brick = 0.f;
         /* one block-wide vote per depth brick (__syncthreads_or): any ray alive, any sample occupied */
         for (int guard = 0; guard < p.max_search; ++guard) {
             if (!__syncthreads_or(cr.alive)) break;
             if (bstep >= p.bZ) { cr.alive = 0; break; } /* beyond the frustum depth: stop the tile */
-            float t1 = t_from_step(p.steps, F_ADD((float)(bstep * 8), p.steps.near_i));
+            float t1 = t_brick = t_from_step(p.steps, F_ADD((float)(bstep * 8), p.steps.near_i));
             mask = 0;
 #pragma unroll
             for (int s = 0; s < 8; s += 2) {
@@ -179,12 +169,18 @@ __global__ void __launch_bounds__(64) cache_search_kernel(CacheBuildParams p)
                 if (in != 3u) cr.alive = 0;
                 if (in) mask |= (occupied2(p.scene, p.bits, p.cells, cr.o, cr.d, make_float2(tm[0], tm[1])) & in) << s;
             }
-            if (__syncthreads_or(mask != 0u)) { found = true; break; }
+            if (__syncthreads_or(mask != 0u)) break;
             ++bstep;
             if (guard == p.max_search - 1) atomicOr(p.guard, 4);
         }
-        const int total = found ? tile_block_sum(__popc(mask), red) : 0; /* found is block-uniform */
-        const int n_alive = tile_block_sum(cr.alive, red);
+        /* a tile that found no brick holds no sample: its mask is empty */
+        const int cnt = __popc(mask);
+        const int before = lanes_before(cnt); /* of this warp's rays */
+        if (lane == 31) red[wid].x = before + cnt;
+        const int w_alive = __reduce_add_sync(FULL, (unsigned)cr.alive);
+        if (lane == 0) red[wid].y = w_alive;
+        __syncthreads();
+        const int total = red[0].x + red[1].x, n_alive = red[0].y + red[1].y;
         const bool processed = total > 0 && n_alive > 0;
         if (k == 0) {
             p.tile_n_samples[ai] = total;
@@ -192,22 +188,14 @@ __global__ void __launch_bounds__(64) cache_search_kernel(CacheBuildParams p)
             p.tile_alive[tile] = n_alive > 0;
             p.block_step[tile] = bstep;
         }
-        p.rays[(size_t)tile * 64 + k] = cr;
+        p.rays[(size_t)tile * 64 + k].alive = cr.alive;
         if (!processed) continue;
         /* append the brick's samples to the iteration's rows, in (ray, step) order */
-        const int cnt = __popc(mask);
-        int incl = cnt;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int v = __shfl_up_sync(FULL, incl, off);
-            if (lane >= off) incl += v;
-        }
-        if (lane == 31) red[2 + wid] = incl;
         if (k == 0) row_base = atomicAdd(p.build_row_counter, total);
         __syncthreads();
-        int row = row_base + incl - cnt + (wid ? red[2] : 0);
+        int row = row_base + before + (wid ? red[0].x : 0);
         int *rof = p.build_row_of + (size_t)ai * 512;
-        float t1 = t_from_step(p.steps, F_ADD((float)(bstep * 8), p.steps.near_i));
+        float t1 = t_brick;
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
             const float t0 = t1;
@@ -235,11 +223,12 @@ __global__ void __launch_bounds__(128) cache_density_kernel(CacheBuildParams p)
 {
     __shared__ uint2 Wsm[W_L3], Wfh[VD ? W_L3 : 1];
     __shared__ __align__(16) __half tiles[4][32 * TILE_STRIDE];
+    const int n = *p.build_row_counter;
+    if ((int)blockIdx.x * 128 >= n) return; /* no rows: no weights */
     for (int i = threadIdx.x; i < W_L3; i += blockDim.x) Wsm[i] = p.weights[i];
     if (VD)
         for (int i = threadIdx.x; i < W_L3; i += blockDim.x) Wfh[i] = p.weights_fh[i];
     __syncthreads();
-    const int n = *p.build_row_counter;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     __half *tile = tiles[w];
     __half *trow = tile + lane * TILE_STRIDE;
@@ -328,29 +317,41 @@ __global__ void __launch_bounds__(128) cache_composite_kernel(CacheBuildParams p
         const int *rof = p.build_row_of + (size_t)ai * 512;
         const float t1s = t_from_step(p.steps, F_ADD((float)(bstep * 8), p.steps.near_i));
         int visible = 0, alive = 0;
+        /* both rays' 16 row numbers, then their densities, before the first is composited: two memory
+         * latencies a tile instead of two a step */
+        CacheRay cr[2];
+        int rows[2][8];
+        float sigma[2][8];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int k = h * 32 + lane;
-            CacheRay cr = p.rays[(size_t)tile * 64 + k];
+            cr[h] = p.rays[(size_t)tile * 64 + h * 32 + lane];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) rows[h][s] = rof[s * 64 + h * 32 + lane];
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int s = 0; s < 8; ++s) sigma[h][s] = rows[h][s] >= 0 ? __half2float(p.build_den[rows[h][s]]) : 0.f;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
             float t1 = t1s;
-            float T = cr.T;
+            float T = cr[h].T;
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
                 const float t0 = t1;
                 const float dt = calc_step(p.steps, t0);
                 t1 = F_ADD(t0, dt);
                 const float tm = F_MUL(F_ADD(t0, t1), 0.5f);
-                if (tm > cr.far_) { cr.alive = 0; continue; }
-                const int row = rof[s * 64 + k];
-                if (row < 0) continue;
-                const float sigma = expf(__half2float(p.build_den[row]));
-                const float alpha = fminf(1.0f, fmaxf(0.0f, 1.0f - expf(-sigma * dt)));
+                if (tm > cr[h].far_) { cr[h].alive = 0; continue; }
+                if (rows[h][s] < 0) continue;
+                const float alpha = fminf(1.0f, fmaxf(0.0f, 1.0f - expf(-expf(sigma[h][s]) * dt)));
                 if (alpha > p.scene.alpha_thre) { T *= 1.0f - alpha; ++visible; }
-                if (T < 1e-4f) cr.alive = 0;
+                if (T < 1e-4f) cr[h].alive = 0;
             }
-            cr.T = T;
-            alive += cr.alive;
-            p.rays[(size_t)tile * 64 + k] = cr;
+            alive += cr[h].alive;
+            CacheRay *out = p.rays + (size_t)tile * 64 + h * 32 + lane;
+            out->T = T;
+            out->alive = cr[h].alive;
         }
         const int n_visible = (int)__reduce_add_sync(FULL, (unsigned)visible);
         const int n_alive_post = (int)__reduce_add_sync(FULL, (unsigned)alive);
@@ -398,30 +399,88 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int &total, int *s_w)
  * index) order.  Applies the per-tile updates of :518-527 (block step
  * advances unless the allocation overflowed; the tile stays alive while it
  * has alive rays and did not overflow), emits the (tile, slot) fill jobs and
- * the next alive list.  One CTA of 1024 threads. */
+ * the next alive list, counts the iteration and clears the next one's rows.
+ * One CTA of 1024 threads, ASSIGN_TILES consecutive tiles a thread: a scan's
+ * barriers are its whole cost, and 32,400 tiles (1080p) took 32 rounds of
+ * three scans at one tile a thread (100 us), 8 rounds of one now.  A slot's
+ * place among the round's slots is its job's place too, and both lists' counts
+ * go through one scan as the halves of a 64-bit sum; only a round in which the
+ * slots run out, where tiles die, scans the alive tiles again. */
+constexpr int ASSIGN_TILES = 4;
+
+__device__ __forceinline__ unsigned long long block_exclusive_scan64(unsigned long long v, unsigned long long &total, unsigned long long *s_w)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned long long inc = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const unsigned long long u = __shfl_up_sync(FULL, inc, off);
+        if (lane >= off) inc += u;
+    }
+    if (lane == 31) s_w[wid] = inc;
+    __syncthreads();
+    if (wid == 0) {
+        const unsigned long long w = s_w[lane];
+        unsigned long long wi = w;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const unsigned long long u = __shfl_up_sync(FULL, wi, off);
+            if (lane >= off) wi += u;
+        }
+        s_w[lane] = wi - w;
+        if (lane == 31) s_w[32] = wi;
+    }
+    __syncthreads();
+    const unsigned long long excl = s_w[wid] + inc - v;
+    total = s_w[32];
+    __syncthreads();
+    return excl;
+}
+
 __global__ void __launch_bounds__(1024) cache_assign_kernel(CacheBuildParams p)
 {
-    __shared__ int s_w[33];
-    __shared__ int s_slot, s_jobs, s_alive;
-    const int tid = threadIdx.x;
+    __shared__ unsigned long long s_w[33];
     const int n = *p.n_alive_tiles;
-    if (tid == 0) { s_slot = *p.slot_counter; s_jobs = 0; s_alive = 0; }
-    __syncthreads();
-    for (int c0 = 0; c0 < n; c0 += 1024) {
-        const int ai = c0 + tid;
-        const bool valid = ai < n;
-        const int tile = valid ? p.alive_list[ai] : 0;
-        const bool processed = valid && p.tile_processed[ai];
-        const bool need = processed && p.tile_need[ai];
-        int n_need;
-        const int slot = s_slot + block_exclusive_scan(need ? 1 : 0, n_need, s_w);
-        const bool overflow = need && slot >= p.capacity;
-        bool alive_next = false;
-        if (valid) {
-            const int bstep = p.block_step[tile];
-            if (processed) {
-                if (need) {
-                    const int tx = tile % p.bX, ty = tile / p.bX;
+    int slot0 = *p.slot_counter, jobs0 = 0, alive0 = 0; /* the same in every thread */
+    for (int c0 = 0; c0 < n; c0 += 1024 * ASSIGN_TILES) {
+        const int a0 = c0 + threadIdx.x * ASSIGN_TILES;
+        int tile[ASSIGN_TILES];
+        bool processed[ASSIGN_TILES], need[ASSIGN_TILES], stays[ASSIGN_TILES];
+        unsigned long long mine = 0; /* low half: slots needed; high half: tiles alive when every slot is granted */
+#pragma unroll
+        for (int q = 0; q < ASSIGN_TILES; ++q) {
+            const int ai = a0 + q;
+            tile[q] = ai < n ? p.alive_list[ai] : 0;
+            processed[q] = ai < n && p.tile_processed[ai];
+            need[q] = processed[q] && p.tile_need[ai];
+            stays[q] = ai < n && (processed[q] ? p.tile_n_alive[ai] > 0 : p.tile_alive[tile[q]] != 0);
+            mine += (need[q] ? 1ull : 0ull) + (stays[q] ? 1ull << 32 : 0ull);
+        }
+        unsigned long long total;
+        unsigned long long before = block_exclusive_scan64(mine, total, s_w);
+        int slot = slot0 + (int)(before & 0xffffffffull);
+        const int n_need = (int)(total & 0xffffffffull);
+        const bool runs_out = slot0 + n_need > p.capacity; /* block-uniform */
+        if (runs_out) {
+            int sl = slot;
+            mine = 0;
+#pragma unroll
+            for (int q = 0; q < ASSIGN_TILES; ++q) {
+                if (need[q] && sl++ >= p.capacity) stays[q] = false;
+                mine += stays[q] ? 1ull << 32 : 0ull;
+            }
+            before = block_exclusive_scan64(mine, total, s_w);
+        }
+        int apos = alive0 + (int)(before >> 32);
+#pragma unroll
+        for (int q = 0; q < ASSIGN_TILES; ++q) {
+            const int ai = a0 + q;
+            if (ai >= n) break;
+            const bool overflow = need[q] && slot >= p.capacity;
+            if (processed[q]) {
+                const int bstep = p.block_step[tile[q]];
+                if (need[q]) {
+                    const int tx = tile[q] % p.bX, ty = tile[q] / p.bX;
                     if (bstep < p.bZ) {
                         const size_t bidx = ((size_t)bstep * p.bY + ty) * p.bX + tx;
                         if (!overflow) {
@@ -435,27 +494,28 @@ __global__ void __launch_bounds__(1024) cache_assign_kernel(CacheBuildParams p)
                         atomicOr(p.guard, 8);  /* brick beyond the frustum depth */
                     }
                 }
-                p.block_step[tile] = bstep + (overflow ? 0 : 1);
-                alive_next = !overflow && p.tile_n_alive[ai] > 0;
-                p.tile_alive[tile] = alive_next;
-            } else {
-                alive_next = p.tile_alive[tile] != 0;
+                p.block_step[tile[q]] = bstep + (overflow ? 0 : 1);
+                p.tile_alive[tile[q]] = stays[q];
             }
+            if (need[q]) {
+                if (!overflow) {
+                    p.jobs[2 * (jobs0 + slot - slot0)] = ai;
+                    p.jobs[2 * (jobs0 + slot - slot0) + 1] = slot;
+                }
+                ++slot;
+            }
+            if (stays[q]) p.alive_list_next[apos++] = tile[q];
         }
-        const bool job = valid && need && !overflow;
-        int n_job, n_al;
-        const int jpos = s_jobs + block_exclusive_scan(job ? 1 : 0, n_job, s_w);
-        const int apos = s_alive + block_exclusive_scan(alive_next ? 1 : 0, n_al, s_w);
-        if (job) { p.jobs[2 * jpos] = ai; p.jobs[2 * jpos + 1] = slot; }
-        if (alive_next) p.alive_list_next[apos] = tile;
-        __syncthreads();
-        if (tid == 0) { s_slot += n_need; s_jobs += n_job; s_alive += n_al; }
-        __syncthreads();
+        jobs0 += max(0, min(n_need, p.capacity - slot0));
+        slot0 += n_need;
+        alive0 += (int)(total >> 32);
     }
-    if (tid == 0) {
-        *p.slot_counter = s_slot;
-        *p.n_jobs = s_jobs;
-        *p.n_alive_next = s_alive;
+    if (threadIdx.x == 0) {
+        *p.slot_counter = slot0;
+        *p.n_jobs = jobs0;
+        *p.n_alive_next = alive0;
+        *p.build_row_counter = 0;
+        if (n > 0) ++*p.n_iterations;
     }
 }
 

@@ -480,6 +480,7 @@ struct CacheBuildParams {
     uint4 *build_lat;           /* 8 latents (fp16) */
     int *build_row_of;          /* [alive idx][step][ray]: row or -1 */
     int *build_row_counter;
+    int *n_iterations;          /* iterations with alive tiles so far */
 };
 
 /* One frame: ray generation, then sub-iterations of march / network /
