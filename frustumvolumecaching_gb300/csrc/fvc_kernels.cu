@@ -135,26 +135,36 @@ __global__ void __launch_bounds__(64) cache_init_kernel(CacheBuildParams p)
  *                          (accumulateNew_cache_init_second_kernel :289-528);
  * then cache_assign_kernel gives bricks their slots and cache_fill_kernel
  * writes their voxels. */
-template <bool VD>
-__global__ void __launch_bounds__(64, 16) cache_search_kernel(CacheBuildParams p)
+/* G groups of 64 threads, one per ray of the tile: group g examines the depth
+ * brick g past the next, and the tile takes the first one that holds an
+ * occupied sample.  A tile's search is a serial chain over its empty bricks
+ * (up to 36 of them in one iteration of the 3-cascade scene at 323x181), so
+ * with few alive tiles eight bricks are examined at once; with many, all but
+ * the first group's work would be repeated in the next iteration. */
+constexpr int SEARCH_GROUPS = 8;
+
+template <bool VD, int G>
+__global__ void __launch_bounds__(64 * G, G == 1 ? 16 : 2) cache_search_kernel(CacheBuildParams p)
 {
+    __shared__ uint8_t s_flags[2][2 * G]; /* per warp: 1 an occupied sample, 2 a ray alive past the brick */
     __shared__ int2 red[2];
     __shared__ int row_base;
-    const int k = threadIdx.x, lane = k & 31, wid = k >> 5;
+    const int group = threadIdx.x / 64, k = threadIdx.x % 64, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wid = warp & 1;
     const int n_alive_tiles = *p.n_alive_tiles;
     for (int ai = blockIdx.x; ai < n_alive_tiles; ai += gridDim.x) {
         __syncthreads();
         const int tile = p.alive_list[ai];
-        CacheRay cr = p.rays[(size_t)tile * 64 + k];
+        const CacheRay cr = p.rays[(size_t)tile * 64 + k];
         int bstep = p.block_step[tile];
         uint32_t mask = 0;
         float t_brick = 0.f;
-        /* one block-wide vote per depth brick (__syncthreads_or): any ray alive, any sample occupied */
-        for (int guard = 0; guard < p.max_search; ++guard) {
-            if (!__syncthreads_or(cr.alive)) break;
-            if (bstep >= p.bZ) { cr.alive = 0; break; } /* beyond the frustum depth: stop the tile */
-            float t1 = t_brick = t_from_step(p.steps, F_ADD((float)(bstep * 8), p.steps.near_i));
+        bool ray_alive = false; /* past the group's brick: the midpoints grow, so the brick alone tells */
+        int chosen = -1;
+        bool stop = false, alive_before = __syncthreads_or(cr.alive);
+        for (int guard = 0; guard < p.max_search && !stop; ++guard) {
+            float t1 = t_brick = t_from_step(p.steps, F_ADD((float)((bstep + group) * 8), p.steps.near_i));
             mask = 0;
+            ray_alive = cr.alive != 0;
 #pragma unroll
             for (int s = 0; s < 8; s += 2) {
                 float tm[2];
@@ -164,35 +174,51 @@ __global__ void __launch_bounds__(64, 16) cache_search_kernel(CacheBuildParams p
                     t1 = F_ADD(t0, calc_step(p.steps, t0));
                     tm[c] = F_MUL(F_ADD(t0, t1), 0.5f);
                 }
-                /* the midpoints grow: the steps past the far bound are the last ones */
+                /* the steps past the far bound are the last ones */
                 const uint32_t in = (tm[0] > cr.far_ ? 0u : 1u) | (tm[1] > cr.far_ ? 0u : 2u);
-                if (in != 3u) cr.alive = 0;
+                if (in != 3u) ray_alive = false;
                 if (in) mask |= (occupied2(p.scene, p.bits, p.cells, cr.o, cr.d, make_float2(tm[0], tm[1])) & in) << s;
             }
-            if (__syncthreads_or(mask != 0u)) break;
-            ++bstep;
-            if (guard == p.max_search - 1) atomicOr(p.guard, 4);
+            const bool any_occ = __any_sync(FULL, mask != 0u), any_alive = __any_sync(FULL, ray_alive);
+            if (lane == 0) s_flags[guard & 1][warp] = (any_occ ? 1 : 0) | (any_alive ? 2 : 0);
+            __syncthreads();
+            /* the bricks in order, as one group would have met them (the same in every thread) */
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                if (stop) break;
+                const int f = s_flags[guard & 1][2 * g] | s_flags[guard & 1][2 * g + 1];
+                if (!alive_before || bstep >= p.bZ) { /* no ray left, or beyond the frustum depth: the tile stops */
+                    stop = true;
+                } else if (f & 1) {
+                    stop = true;
+                    chosen = g;
+                } else {
+                    ++bstep;
+                    alive_before = f & 2;
+                }
+            }
+            if (!stop && guard == p.max_search - 1 && threadIdx.x == 0) atomicOr(p.guard, 4);
         }
-        /* a tile that found no brick holds no sample: its mask is empty */
+        const bool mine = group == max(chosen, 0); /* the group that goes on with its brick */
+        if (chosen < 0) mask = 0, ray_alive = false;
         const int cnt = __popc(mask);
         const int before = lanes_before(cnt); /* of this warp's rays */
-        if (lane == 31) red[wid].x = before + cnt;
-        const int w_alive = __reduce_add_sync(FULL, (unsigned)cr.alive);
-        if (lane == 0) red[wid].y = w_alive;
+        const int w_alive = __reduce_add_sync(FULL, ray_alive ? 1u : 0u);
+        if (mine && lane == 31) red[wid] = make_int2(before + cnt, w_alive);
         __syncthreads();
         const int total = red[0].x + red[1].x, n_alive = red[0].y + red[1].y;
         const bool processed = total > 0 && n_alive > 0;
-        if (k == 0) {
+        if (mine && k == 0) {
             p.tile_n_samples[ai] = total;
             p.tile_processed[ai] = processed;
             p.tile_alive[tile] = n_alive > 0;
             p.block_step[tile] = bstep;
+            if (processed) row_base = atomicAdd(p.build_row_counter, total);
         }
-        p.rays[(size_t)tile * 64 + k].alive = cr.alive;
-        if (!processed) continue;
-        /* append the brick's samples to the iteration's rows, in (ray, step) order */
-        if (k == 0) row_base = atomicAdd(p.build_row_counter, total);
+        if (mine) p.rays[(size_t)tile * 64 + k].alive = ray_alive;
         __syncthreads();
+        if (!processed || !mine) continue;
+        /* append the brick's samples to the iteration's rows, in (ray, step) order */
         int row = row_base + before + (wid ? red[0].x : 0);
         int *rof = p.build_row_of + (size_t)ai * 512;
         float t1 = t_brick;
@@ -287,10 +313,21 @@ __global__ void __launch_bounds__(128) cache_density_kernel(CacheBuildParams p)
     }
 }
 
+/* grid: the alive tiles, as last known.  Groups of bricks below SEARCH_TILES of them: a search launch of the 3-cascade
+ * scene's build takes, us with 1 / 8 groups, 44 / 30 at 323x181 (943 tiles) and 23 / 11 at 128x128 (256); thresholds of
+ * 1024 to 4096 tiles measured alike. */
+#ifndef FVC_SEARCH_TILES
+#define FVC_SEARCH_TILES 1024
+#endif
 cudaError_t launch_cache_search(const CacheBuildParams &p, int grid, cudaStream_t s)
 {
-    if (p.view_dependent) cache_search_kernel<true><<<grid, 64, 0, s>>>(p);
-    else cache_search_kernel<false><<<grid, 64, 0, s>>>(p);
+    if (grid <= FVC_SEARCH_TILES) {
+        if (p.view_dependent) cache_search_kernel<true, SEARCH_GROUPS><<<grid, 64 * SEARCH_GROUPS, 0, s>>>(p);
+        else cache_search_kernel<false, SEARCH_GROUPS><<<grid, 64 * SEARCH_GROUPS, 0, s>>>(p);
+    } else {
+        if (p.view_dependent) cache_search_kernel<true, 1><<<grid, 64, 0, s>>>(p);
+        else cache_search_kernel<false, 1><<<grid, 64, 0, s>>>(p);
+    }
     return cudaGetLastError();
 }
 
