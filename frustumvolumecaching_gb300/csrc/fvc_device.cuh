@@ -488,115 +488,118 @@ __device__ __forceinline__ float2 f2_lerp(float2 a, float2 b, float t)
  * in flight instead of 8. */
 /* the 4-feature grid (instant-ngp's 8 levels x 4 features): an entry is two
  * half2 (one 8-byte gather per corner), the level's features go to
- * out[2l], out[2l + 1]; levels in groups of LG / 2 */
-template <int LG>
-__device__ __forceinline__ void hash_encode_levels_f4(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, __half2 *out,
-                                                      int l_begin, int l_end)
+ * out[2l], out[2l + 1]: G levels from l0 on */
+template <int G>
+__device__ __forceinline__ void hash_group_f4(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, int l0, __half2 *out)
 {
-    constexpr int G = LG / 2 > 0 ? LG / 2 : 1;
-    for (int l0 = l_begin; l0 < l_end; l0 += G) {
-        uint2 v[G][8];
-        float wx[G], wy[G], wz[G];
+    uint2 v[G][8];
+    float wx[G], wy[G], wz[G];
 #pragma unroll
-        for (int j = 0; j < G; ++j) {
-            const int l = l0 + j;
-            const float sc = g.scale[l];
-            const float px = __fmaf_rn(sc, pos.x, 0.5f), py = __fmaf_rn(sc, pos.y, 0.5f), pz = __fmaf_rn(sc, pos.z, 0.5f);
-            const float fx = floorf(px), fy = floorf(py), fz = floorf(pz);
-            const uint32_t gx = (uint32_t)(int)fx, gy = (uint32_t)(int)fy, gz = (uint32_t)(int)fz;
-            wx[j] = __fsub_rn(px, fx); wy[j] = __fsub_rn(py, fy); wz[j] = __fsub_rn(pz, fz);
-            const uint32_t size = g.size[l];
-            const uint2 *tl = reinterpret_cast<const uint2 *>(table + g.offset[l]);
-            if ((g.dense_mask >> l) & 1u) {
-                const uint32_t r = g.res[l], r2 = g.res2[l];
-                const uint32_t b = gx + gy * r + gz * r2;
+    for (int j = 0; j < G; ++j) {
+        const int l = l0 + j;
+        const float sc = g.scale[l];
+        const float px = __fmaf_rn(sc, pos.x, 0.5f), py = __fmaf_rn(sc, pos.y, 0.5f), pz = __fmaf_rn(sc, pos.z, 0.5f);
+        const float fx = floorf(px), fy = floorf(py), fz = floorf(pz);
+        const uint32_t gx = (uint32_t)(int)fx, gy = (uint32_t)(int)fy, gz = (uint32_t)(int)fz;
+        wx[j] = __fsub_rn(px, fx); wy[j] = __fsub_rn(py, fy); wz[j] = __fsub_rn(pz, fz);
+        const uint32_t size = g.size[l];
+        const uint2 *tl = reinterpret_cast<const uint2 *>(table + g.offset[l]);
+        if ((g.dense_mask >> l) & 1u) {
+            const uint32_t r = g.res[l], r2 = g.res2[l];
+            const uint32_t b = gx + gy * r + gz * r2;
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    uint32_t i = b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u);
-                    if (i >= size) i -= size;
-                    v[j][c] = __ldg(tl + i);
-                }
-            } else {
-                const uint32_t hy0 = gy * 2654435761u, hy1 = (gy + 1u) * 2654435761u;
-                const uint32_t hz0 = gz * 805459861u, hz1 = (gz + 1u) * 805459861u;
-                const uint32_t m = size - 1u;
-#pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    v[j][c] = __ldg(tl + (((gx + ((c & 1) ? 1u : 0u)) ^ ((c & 2) ? hy1 : hy0) ^ ((c & 4) ? hz1 : hz0)) & m));
+            for (int c = 0; c < 8; ++c) {
+                uint32_t i = b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u);
+                if (i >= size) i -= size;
+                v[j][c] = __ldg(tl + i);
             }
+        } else {
+            const uint32_t hy0 = gy * 2654435761u, hy1 = (gy + 1u) * 2654435761u;
+            const uint32_t hz0 = gz * 805459861u, hz1 = (gz + 1u) * 805459861u;
+            const uint32_t m = size - 1u;
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                v[j][c] = __ldg(tl + (((gx + ((c & 1) ? 1u : 0u)) ^ ((c & 2) ? hy1 : hy0) ^ ((c & 4) ? hz1 : hz0)) & m));
         }
+    }
 #pragma unroll
-        for (int j = 0; j < G; ++j) {
+    for (int j = 0; j < G; ++j) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) { /* features 0-1, then 2-3 */
-                float2 e[4];
+        for (int h = 0; h < 2; ++h) { /* features 0-1, then 2-3 */
+            float2 e[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint32_t a = h ? v[j][2 * k].y : v[j][2 * k].x, b = h ? v[j][2 * k + 1].y : v[j][2 * k + 1].x;
-                    e[k] = f2_lerp(__half22float2(*reinterpret_cast<const __half2 *>(&a)),
-                                   __half22float2(*reinterpret_cast<const __half2 *>(&b)), wx[j]);
-                }
-                const float2 g0 = f2_lerp(e[0], e[1], wy[j]), g1 = f2_lerp(e[2], e[3], wy[j]);
-                out[2 * (l0 + j) + h] = __float22half2_rn(f2_lerp(g0, g1, wz[j]));
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t a = h ? v[j][2 * k].y : v[j][2 * k].x, b = h ? v[j][2 * k + 1].y : v[j][2 * k + 1].x;
+                e[k] = f2_lerp(__half22float2(*reinterpret_cast<const __half2 *>(&a)),
+                               __half22float2(*reinterpret_cast<const __half2 *>(&b)), wx[j]);
             }
+            const float2 g0 = f2_lerp(e[0], e[1], wy[j]), g1 = f2_lerp(e[2], e[3], wy[j]);
+            out[2 * j + h] = __float22half2_rn(f2_lerp(g0, g1, wz[j]));
         }
     }
 }
 
+/* LG levels of the 2-feature grid from l0 on: one half2 each */
+template <int LG>
+__device__ __forceinline__ void hash_group_f2(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, int l0, __half2 *out)
+{
+    __half2 v[LG][8];
+    float wx[LG], wy[LG], wz[LG];
+#pragma unroll
+    for (int j = 0; j < LG; ++j) {
+        const int l = l0 + j;
+        const float sc = g.scale[l];
+        const float px = __fmaf_rn(sc, pos.x, 0.5f), py = __fmaf_rn(sc, pos.y, 0.5f), pz = __fmaf_rn(sc, pos.z, 0.5f);
+        const float fx = floorf(px), fy = floorf(py), fz = floorf(pz);
+        const uint32_t gx = (uint32_t)(int)fx, gy = (uint32_t)(int)fy, gz = (uint32_t)(int)fz;
+        wx[j] = __fsub_rn(px, fx); wy[j] = __fsub_rn(py, fy); wz[j] = __fsub_rn(pz, fz);
+        const uint32_t size = g.size[l];
+        const __half2 *tl = table + g.offset[l];
+        if ((g.dense_mask >> l) & 1u) {
+            const uint32_t r = g.res[l], r2 = g.res2[l];
+            const uint32_t b = gx + gy * r + gz * r2;
+            if (b + 1u + r + r2 < size) { /* no corner reaches past the table (all but the grid's far faces) */
+#pragma unroll
+                for (int c = 0; c < 8; ++c) v[j][c] = __ldg(tl + (b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u)));
+            } else {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    uint32_t i = b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u);
+                    if (i >= size) i -= size; /* == i % size: dense indices stay below 2*size */
+                    v[j][c] = __ldg(tl + i);
+                }
+            }
+        } else {
+            const uint32_t hy0 = gy * 2654435761u, hy1 = (gy + 1u) * 2654435761u;
+            const uint32_t hz0 = gz * 805459861u, hz1 = (gz + 1u) * 805459861u;
+            const uint32_t m = size - 1u; /* hashed levels hold 2^log2_T entries */
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                v[j][c] = __ldg(tl + (((gx + ((c & 1) ? 1u : 0u)) ^ ((c & 2) ? hy1 : hy0) ^ ((c & 4) ? hz1 : hz0)) & m));
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < LG; ++j) {
+        /* trilinear interpolation as 7 lerps (x, then y, then z) on both features at once */
+        float2 e[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) e[k] = f2_lerp(__half22float2(v[j][2 * k]), __half22float2(v[j][2 * k + 1]), wx[j]);
+        const float2 g0 = f2_lerp(e[0], e[1], wy[j]), g1 = f2_lerp(e[2], e[3], wy[j]);
+        out[j] = __float22half2_rn(f2_lerp(g0, g1, wz[j]));
+    }
+}
+
+/* levels l_begin .. l_end - 1 into out[] (level l in out[l], or out[2l] and out[2l + 1]), LG half2 at a time */
 template <int LG = 4>
 __device__ __forceinline__ void hash_encode_levels(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, __half2 *out,
                                                    int l_begin, int l_end)
 {
+    constexpr int G = LG / 2 > 0 ? LG / 2 : 1;
     if (g.F == 4) {
-        hash_encode_levels_f4<LG>(g, table, pos, out, l_begin, l_end);
+        for (int l = l_begin; l < l_end; l += G) hash_group_f4<G>(g, table, pos, l, out + 2 * l);
         return;
     }
-    for (int l0 = l_begin; l0 < l_end; l0 += LG) {
-        __half2 v[LG][8];
-        float wx[LG], wy[LG], wz[LG];
-#pragma unroll
-        for (int j = 0; j < LG; ++j) {
-            const int l = l0 + j;
-            const float sc = g.scale[l];
-            const float px = __fmaf_rn(sc, pos.x, 0.5f), py = __fmaf_rn(sc, pos.y, 0.5f), pz = __fmaf_rn(sc, pos.z, 0.5f);
-            const float fx = floorf(px), fy = floorf(py), fz = floorf(pz);
-            const uint32_t gx = (uint32_t)(int)fx, gy = (uint32_t)(int)fy, gz = (uint32_t)(int)fz;
-            wx[j] = __fsub_rn(px, fx); wy[j] = __fsub_rn(py, fy); wz[j] = __fsub_rn(pz, fz);
-            const uint32_t size = g.size[l];
-            const __half2 *tl = table + g.offset[l];
-            if ((g.dense_mask >> l) & 1u) {
-                const uint32_t r = g.res[l], r2 = g.res2[l];
-                const uint32_t b = gx + gy * r + gz * r2;
-                if (b + 1u + r + r2 < size) { /* no corner reaches past the table (all but the grid's far faces) */
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) v[j][c] = __ldg(tl + (b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u)));
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        uint32_t i = b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u);
-                        if (i >= size) i -= size; /* == i % size: dense indices stay below 2*size */
-                        v[j][c] = __ldg(tl + i);
-                    }
-                }
-            } else {
-                const uint32_t hy0 = gy * 2654435761u, hy1 = (gy + 1u) * 2654435761u;
-                const uint32_t hz0 = gz * 805459861u, hz1 = (gz + 1u) * 805459861u;
-                const uint32_t m = size - 1u; /* hashed levels hold 2^log2_T entries */
-#pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    v[j][c] = __ldg(tl + (((gx + ((c & 1) ? 1u : 0u)) ^ ((c & 2) ? hy1 : hy0) ^ ((c & 4) ? hz1 : hz0)) & m));
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < LG; ++j) {
-            /* trilinear interpolation as 7 lerps (x, then y, then z) on both features at once */
-            float2 e[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) e[k] = f2_lerp(__half22float2(v[j][2 * k]), __half22float2(v[j][2 * k + 1]), wx[j]);
-            const float2 g0 = f2_lerp(e[0], e[1], wy[j]), g1 = f2_lerp(e[2], e[3], wy[j]);
-            out[l0 + j] = __float22half2_rn(f2_lerp(g0, g1, wz[j]));
-        }
-    }
+    for (int l = l_begin; l < l_end; l += LG) hash_group_f2<LG>(g, table, pos, l, out + l);
 }
 
 /* all levels of the grid (features of level l in out[l]) */

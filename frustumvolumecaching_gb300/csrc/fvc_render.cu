@@ -1153,9 +1153,6 @@ struct __align__(128) TcSmem {
      * leave the SM its larger L1 share for the hash gathers */
     __align__(128) uint8_t W[TC_WBYTES];
 };
-/* dynamic shared memory of a TcSmem launch */
-static inline size_t tc_smem_bytes(int freq) { return sizeof(TcSmem) + (freq ? (size_t)(TCF_WBYTES - TC_WBYTES) : 0); }
-
 constexpr long long TC_WAIT_LIMIT = 2000000000ll; /* ~1 s of SM clocks */
 constexpr int TC_COLS = 64;
 static_assert(FVC_TC_CTAS_PER_SM * TC_COLS <= 512, "resident CTAs must fit in the SM's 512 TMEM columns");
@@ -1258,160 +1255,250 @@ __device__ __forceinline__ float3 cache_row_position(const RenderParams &p, cons
     return contract(p.scene, at(make_float3(of.x, of.y, of.z), make_float3(dt4.x, dt4.y, dt4.z), t));
 }
 
+/* The network over 128-row tiles, one CTA an SM.  NT_TEAMS teams of 128
+ * threads (thread = row = TMEM lane) take tiles of their own; a team has 96
+ * TMEM columns, 64 of its fp32 accumulator and 32 of its activations, two fp16
+ * a column, which the MMAs read as their A operand: an epilogue's row goes
+ * from registers to tensor memory and never through shared memory.  Shared
+ * memory holds one copy of the weights for all teams, about 21 KB of an SM's
+ * 256, and the rest is L1 for the hash gathers, which bound the kernel.  One
+ * thread of a team issues a layer's MMAs and commits them to the team's
+ * mbarrier; every wait is bounded. */
+#ifndef FVC_NT_TEAMS
+#define FVC_NT_TEAMS 5
+#endif
+#ifndef FVC_NT_HASH_GROUP
+#define FVC_NT_HASH_GROUP 4 /* hash levels whose gathers a thread has in flight together */
+#endif
+constexpr int NT_TEAMS = FVC_NT_TEAMS, NT_THREADS = 128 * NT_TEAMS, NT_TEAM_COLS = 96, NT_A = 64;
+constexpr int NT_COLS = 512;
+static_assert(NT_TEAMS * NT_TEAM_COLS <= NT_COLS, "the teams' columns must fit in the SM's tensor memory");
+struct __align__(128) NtSmem {
+    float bias3[64];
+    uint64_t wbar, mbar[NT_TEAMS];
+    uint32_t tmem_base;
+    __align__(128) uint8_t W[TC_WBYTES]; /* last: TCF_WBYTES for a head with the frequency encoding (nt_smem_bytes) */
+};
+static inline size_t nt_smem_bytes(int freq) { return sizeof(NtSmem) + (freq ? (size_t)(TCF_WBYTES - TC_WBYTES) : 0); }
+
+/* a team's rows are rewritten: this thread's TMEM stores and loads are ordered before the team's next MMA by its
+ * named barrier (1 + team); OR of the failure flags */
+__device__ __forceinline__ bool nt_publish(int team, bool ok)
+{
+    tmem_wait_st();
+    tc_fence_before();
+    uint32_t bad;
+    asm volatile("{\n .reg .pred p, q;\n setp.eq.u32 p, %1, 0;\n bar.red.or.pred q, %2, 128, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(bad)
+                 : "r"(ok ? 1u : 0u), "r"(team + 1)
+                 : "memory");
+    return bad == 0u;
+}
+
+/* 64 accumulator columns of this thread's row -> (+bias) ReLU -> the fp16 row in columns NT_A.. (epi_hidden's arithmetic) */
+__device__ __forceinline__ void nt_epi(uint32_t acc, const float *bias)
+{
+    const __half2 zero = __float2half2_rn(0.0f);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        float v[32];
+        tmem_ld32(acc + 32 * h, v);
+        tmem_wait_ld();
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float2 x = make_float2(v[2 * i], v[2 * i + 1]);
+            if (bias) x = __fadd2_rn(x, make_float2(bias[32 * h + 2 * i], bias[32 * h + 2 * i + 1]));
+            const __half2 r = __hmax2(__float22half2_rn(x), zero);
+            w[i] = *reinterpret_cast<const uint32_t *>(&r);
+        }
+        tmem_st16(acc + NT_A + 16 * h, w);
+    }
+}
+
+/* the row's features into columns NT_A .. NT_A + 15, four half2 at a time: a loop that the compiler keeps, so its code
+ * stays in the instruction cache, and whose results need no array (whole warp) */
+template <bool GENERAL>
+__device__ __forceinline__ void nt_encode(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, uint32_t acc)
+{
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+        __half2 f[4];
+        if (GENERAL && g.F == 4) {
+            hash_group_f4<2>(g, table, pos, 2 * c, f);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j += FVC_NT_HASH_GROUP) hash_group_f2<FVC_NT_HASH_GROUP>(g, table, pos, 4 * c + j, f + j);
+        }
+        __syncwarp();
+        tmem_st4(acc + NT_A + 4 * c, *reinterpret_cast<const uint4 *>(f));
+    }
+}
+
+/* what a thread's row needs from memory before its gathers: its id (-1: none), position and direction */
+struct NtRow {
+    int r;
+    float3 pos, d01;
+};
+
 /* MODE 0: resample rows (the list, or all rows of the plain path); MODE 1: the
  * cache list (head only); MODE 2: both lists of a cached sub-iteration
  * classified by the march in one launch, the resample list's tiles first
  * (hash features, density layers, head), then the cache list's tiles (the
  * head input of each row's lookup, wf_cache_lookup_kernel; head only), so
- * that no tile mixes the two kinds of row. */
-template <int MODE, int HH, bool LIST>
-__global__ void __launch_bounds__(128, FVC_TC_CTAS_PER_SM) wf_net_tc_kernel(RenderParams p, int it)
+ * that no tile mixes the two kinds of row.  GENERAL: the 4-feature grid and
+ * the head with the frequency encoding; without it the kernel is smaller. */
+template <int MODE, int HH, bool LIST, bool GENERAL>
+__global__ void __launch_bounds__(NT_THREADS, 1) wf_net_tc_kernel(RenderParams p, int it)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    TcSmem &S = *reinterpret_cast<TcSmem *>(smem_raw);
+    NtSmem &S = *reinterpret_cast<NtSmem *>(smem_raw);
     const int n_rows = MODE == 0 ? (LIST ? p.counters[3] : p.counters[2]) : MODE == 1 ? p.counters[4] : p.counters[3];
     const int n_hit = MODE == 2 ? p.counters[4] : 0;
     const int res_tiles = (n_rows + 127) / 128;
     const int n_tiles = res_tiles + (n_hit + 127) / 128;
-    if ((int)blockIdx.x >= n_tiles) return; /* a CTA without a tile fetches no weights and allocates no TMEM */
-    const int tid = threadIdx.x, warp = tid >> 5;
-    /* the weights arrive by one bulk copy on the TMA engine, completing the
-     * mbarrier's phase 0; the layers' MMA commits complete the later phases */
+    if ((int)blockIdx.x * NT_TEAMS >= n_tiles) return; /* a CTA without a tile fetches no weights and allocates no TMEM */
+    const int tid = threadIdx.x, warp = tid >> 5, team = tid >> 7, row = tid & 127;
+    const bool freq = GENERAL && p.freq;
     /* the head's input width and tile layout: 32 inputs (TC_*), or 64 with the frequency encoding (TCF_*) */
-    const int HK = p.freq ? 64 : 32;
-    const int wb3 = p.freq ? TCF_B3 : TC_B3, wb4 = p.freq ? TCF_B4 : TC_B4, wb5 = p.freq ? TCF_B5 : TC_B5;
+    const int HK = freq ? 64 : 32;
+    const int wb3 = freq ? TCF_B3 : TC_B3, wb4 = freq ? TCF_B4 : TC_B4, wb5 = freq ? TCF_B5 : TC_B5;
     if (tid == 0) {
-        const int wbytes = p.freq ? TCF_WBYTES : TC_WBYTES;
-        mbar_init(&S.mbar, 1);
-        mbar_arrive_expect_tx(&S.mbar, wbytes);
-        bulk_copy_g2s(S.W, p.weights_tc, wbytes, &S.mbar);
+        /* the weights arrive by one bulk copy on the TMA engine; each team's MMA commits complete its own mbarrier */
+        const int wbytes = freq ? TCF_WBYTES : TC_WBYTES;
+        mbar_init(&S.wbar, 1);
+#pragma unroll
+        for (int t = 0; t < NT_TEAMS; ++t) mbar_init(&S.mbar[t], 1);
+        mbar_arrive_expect_tx(&S.wbar, wbytes);
+        bulk_copy_g2s(S.W, p.weights_tc, wbytes, &S.wbar);
     }
     if (tid < 64) S.bias3[tid] = p.bias3[tid];
-    if (warp == 0) tmem_alloc(&S.tmem_base, TC_COLS);
+    if (warp == 0) tmem_alloc(&S.tmem_base, NT_COLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = S.tmem_base;
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+    const uint32_t tmem0 = S.tmem_base;
+    const uint32_t tmem = tmem0 + (uint32_t)(NT_TEAM_COLS * team);
+    const uint32_t acc = tmem + ((uint32_t)((warp & 3) * 32) << 16); /* this thread's TMEM lane */
+    uint64_t *const mbar = &S.mbar[team];
     const RayState *states = p.states[it & 1];
     uint32_t phase = 0;
-    bool ok = mbar_wait(&S.mbar, phase, TC_WAIT_LIMIT);
-    phase ^= 1u;
-    for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        int k = tile * 128 + tid, r = -1, kind = KIND_RESAMPLE;
-        if (MODE == 2 && tile >= res_tiles) {
-            k = (tile - res_tiles) * 128 + tid;
-            kind = KIND_CACHE;
-            r = k < n_hit ? p.cache_list[k] : -1;
-        } else {
-            r = k < n_rows ? (MODE == 0 ? (LIST ? p.res_list[k] : k) : MODE == 1 ? p.cache_list[k] : p.res_list[k]) : -1;
+    /* one layer's MMAs by the team's first thread, then the bounded wait for their completion */
+    auto layer = [&](const uint8_t *b, int K, int N) {
+        if (row == 0) {
+            tc_fence_after();
+            const uint32_t sbo = (uint32_t)(K / 8) * 128u, id = idesc_f16(128, N, false), b0 = smem_u32(b);
+            for (int kc = 0; kc < K / 16; ++kc)
+                tc_mma_f16_ts(tmem, tmem + NT_A + 8u * kc, umma_desc(b0 + 256u * kc, 128u, sbo), id, kc > 0 ? 1u : 0u);
+            tc_commit(mbar);
         }
+        const bool done = mbar_wait(mbar, phase, TC_WAIT_LIMIT);
+        phase ^= 1u;
+        tc_fence_after();
+        return done;
+    };
+    auto is_cached = [&](int tile) { return MODE == 1 || (MODE == 2 && tile >= res_tiles); };
+    auto load_row = [&](int tile) {
+        NtRow in;
+        in.r = -1;
+        in.pos = in.d01 = make_float3(0.f, 0.f, 0.f);
+        if (tile >= n_tiles) return in;
+        const bool cached = is_cached(tile);
+        const int k = (MODE == 2 && cached ? tile - res_tiles : tile) * 128 + row;
+        if (k >= (MODE == 2 && cached ? n_hit : n_rows)) return in;
+        in.r = cached ? p.cache_list[k] : MODE == 0 && !LIST ? k : p.res_list[k];
+        in.d01 = dir01_of(states, p.row_slot[in.r]);
+        if (!cached) {
+            const float4 pw = p.row_pay[in.r];
+            in.pos = make_float3(pw.x, pw.y, pw.z);
+        }
+        return in;
+    };
+    bool ok = mbar_wait(&S.wbar, 0, TC_WAIT_LIMIT);
+    const int stride = (int)gridDim.x * NT_TEAMS;
+    /* ok may differ between a team's threads only until its next nt_publish, which every thread of the team reaches */
+    int tile = (int)blockIdx.x * NT_TEAMS + team;
+    NtRow in = load_row(tile);
+    for (; tile < n_tiles; tile += stride) {
+        const bool cached = is_cached(tile);
+        const int r = in.r;
+        const float3 d01 = in.d01;
+        uint4 b0 = make_uint4(0u, 0u, 0u, 0u), b1 = b0;
+        float3 fq = in.pos; /* the frequency encoding's position */
+        if (!cached) {
+            /* ---- hash features -> activations (K = 32); a lane without a row encodes the origin ---- */
+            nt_encode<GENERAL>(p.grid, p.table, in.pos, acc);
+        } else if (r >= 0) {
+            /* ---- cache lookup -> head input (log-density, latents); MODE 1 finds it by the place in the list ---- */
+            uint32_t hin[8];
+            const int k = (MODE == 2 ? tile - res_tiles : tile) * 128 + row;
+            cache_head_input(p.row_lat[MODE == 1 ? k : r], p.row_out[r].y >> 16, p.latent_offset, hin);
+            b0 = make_uint4(hin[0], hin[1], hin[2], hin[3]);
+            b1 = make_uint4(hin[4], hin[5], hin[6], hin[7]);
+            if (freq) fq = cache_row_position(p, states, r);
+        }
+        in = load_row(tile + stride); /* in flight under this tile's layers */
+        if (!cached) {
+            if (!(ok = nt_publish(team, ok))) break;
+            /* ---- layer 1: 32 -> 64, ReLU ---- */
+            ok = layer(S.W + TC_B1, 32, 64);
+            nt_epi(acc, nullptr);
+            if (!(ok = nt_publish(team, ok))) break;
+            /* ---- layer 2: 64 -> 16 (log-density, latents) ---- */
+            ok = layer(S.W + TC_B2, 64, 16);
+            float v[16];
+            tmem_ld16(acc, v);
+            tmem_wait_ld();
+            b0 = pack8(v);
+            b1 = pack8(v + 8);
+        }
+        const uint32_t log_density = b0.x & 0xffffu;
+        __syncwarp();
+        tmem_st8(acc + NT_A, b0, b1);
         __half2 sh[8];
-        uint16_t log_density = 0;
-        if (r >= 0) sh16(dir01_of(states, p.row_slot[r]), sh);
-        else for (int q = 0; q < 8; ++q) sh[q] = __floats2half2_rn(0.f, 0.f);
-        if (MODE != 1) {
-            /* ---- hash features -> tile (K = 32); MODE 2 cache rows: the cache lookup ---- */
-            __half2 feat[16];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) feat[q] = __floats2half2_rn(0.f, 0.f);
-            uint32_t hin[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-            if (r >= 0) {
-                const float4 pw = MODE == 2 && kind == KIND_CACHE ? make_float4(0.f, 0.f, 0.f, 0.f) : p.row_pay[r];
-                if (MODE == 2 && kind == KIND_CACHE) {
-                    cache_head_input(p.row_lat[r], p.row_out[r].y >> 16, p.latent_offset, hin);
-                } else {
-                    hash_encode<FVC_TC_HASH_GROUP>(p.grid, p.table, make_float3(pw.x, pw.y, pw.z), feat);
-                }
-            }
-            /* MODE 2: the cache list's tiles skip the density layers (tile is block-uniform) */
-            const bool dense = MODE != 2 || tile < res_tiles;
-            uint4 b0 = make_uint4(hin[0], hin[1], hin[2], hin[3]), b1 = make_uint4(hin[4], hin[5], hin[6], hin[7]);
-            if (dense) {
-#pragma unroll
-                for (int c = 0; c < 4; ++c) st_chunk(S.X, tid, c, 32, *reinterpret_cast<const uint4 *>(feat + 4 * c));
-                if (!(ok = tc_publish(ok))) break;
-                /* ---- layer 1: 32 -> 64, ReLU ---- */
-                ok = tc_run(S, tmem, S.W + TC_B1, 32, 64, phase);
-                epi_hidden(tmem + lane_base, nullptr, S.X, tid);
-                if (!(ok = tc_publish(ok))) break;
-                /* ---- layer 2: 64 -> 16 (log-density, latents) ---- */
-                ok = tc_run(S, tmem, S.W + TC_B2, 64, 16, phase);
-                float v[16];
-                tmem_ld16(tmem + lane_base, v);
-                tmem_wait_ld();
-                if (!(MODE == 2 && kind == KIND_CACHE)) {
-                    b0 = pack8(v);
-                    b1 = pack8(v + 8);
-                }
-            }
-            log_density = (uint16_t)(b0.x & 0xffffu);
-            st_chunk(S.X, tid, 0, HK, b0);
-            st_chunk(S.X, tid, 1, HK, b1);
-        } else {
-            /* ---- cache lookup -> head input (log-density, latents) ---- */
-            __half hin[32];
-            if (r >= 0) {
-                cache_row_input(p, k, r, hin);
-            } else {
-                for (int q = 16; q < 32; ++q) hin[q] = __float2half_rn(0.f);
-            }
-            log_density = __half_as_ushort(hin[16]);
-            st_chunk(S.X, tid, 0, HK, *reinterpret_cast<const uint4 *>(hin + 16));
-            st_chunk(S.X, tid, 1, HK, *reinterpret_cast<const uint4 *>(hin + 24));
-        }
-        st_chunk(S.X, tid, 2, HK, *reinterpret_cast<const uint4 *>(sh));
-        st_chunk(S.X, tid, 3, HK, *reinterpret_cast<const uint4 *>(sh + 4));
-        if (p.freq) {
+        sh16(d01, sh);
+        tmem_st8(acc + NT_A + 8, *reinterpret_cast<const uint4 *>(sh), *reinterpret_cast<const uint4 *>(sh + 4));
+        if (freq) {
             /* the frequency encoding of the row's network input position (include/nerf_network.h:241-246) */
-            uint4 fx = make_uint4(0u, 0u, 0u, 0u), fy = fx, fz = fx;
-            if (r >= 0) {
-                const bool cache_row = MODE == 1 || (MODE == 2 && kind == KIND_CACHE);
-                float3 q;
-                if (cache_row) {
-                    q = cache_row_position(p, states, r);
-                } else {
-                    const float4 pw = p.row_pay[r];
-                    q = make_float3(pw.x, pw.y, pw.z);
-                }
-                fx = freq_chunk(q.x);
-                fy = freq_chunk(q.y);
-                fz = freq_chunk(q.z);
-            }
-            st_chunk(S.X, tid, 4, HK, fx);
-            st_chunk(S.X, tid, 5, HK, fy);
-            st_chunk(S.X, tid, 6, HK, fz);
-            st_chunk(S.X, tid, 7, HK, make_uint4(0u, 0u, 0u, 0u));
+            tmem_st8(acc + NT_A + 16, freq_chunk(fq.x), freq_chunk(fq.y));
+            tmem_st8(acc + NT_A + 24, freq_chunk(fq.z), make_uint4(0u, 0u, 0u, 0u));
         }
-        if (!(ok = tc_publish(ok))) break;
+        if (!(ok = nt_publish(team, ok))) break;
         /* ---- head layer 1: (latents | SH (| frequency)) HK -> 64, bias from the 1-padding, ReLU ---- */
-        ok = tc_run(S, tmem, S.W + wb3, HK, 64, phase);
-        epi_hidden(tmem + lane_base, S.bias3, S.X, tid);
-        if (!(ok = tc_publish(ok))) break;
+        ok = layer(S.W + wb3, HK, 64);
+        nt_epi(acc, S.bias3);
+        if (!(ok = nt_publish(team, ok))) break;
         if (HH == 2) {
             /* ---- head layer 2: 64 -> 64, ReLU ---- */
-            ok = tc_run(S, tmem, S.W + wb4, 64, 64, phase);
-            epi_hidden(tmem + lane_base, nullptr, S.X, tid);
-            if (!(ok = tc_publish(ok))) break;
+            ok = layer(S.W + wb4, 64, 64);
+            nt_epi(acc, nullptr);
+            if (!(ok = nt_publish(team, ok))) break;
         }
-        /* ---- output layer: 64 -> 16 (rgb logits in cols 0..2) ---- */
-        ok = tc_run(S, tmem, S.W + wb5, 64, 16, phase);
-        float o[16];
-        tmem_ld16(tmem + lane_base, o);
+        /* ---- output layer: 64 -> 16 (rgb logits in cols 0..2); the next tile's first MMA overwrites the
+         * accumulator only after its nt_publish, which orders these reads ---- */
+        ok = layer(S.W + wb5, 64, 16);
+        float o[4];
+        tmem_ld4(acc, o);
         tmem_wait_ld();
         if (r >= 0)
-            p.row_out[r] = make_uint2(pack_h2(o[0], o[1]),
-                                      (uint32_t)__half_as_ushort(__float2half_rn(o[2])) | ((uint32_t)log_density << 16));
-        tc_fence_before();
-        if (__syncthreads_or(!ok)) { ok = false; break; }
+            p.row_out[r] = make_uint2(pack_h2(o[0], o[1]), (uint32_t)__half_as_ushort(__float2half_rn(o[2])) | (log_density << 16));
     }
-    if (!ok && tid == 0) atomicOr(p.guard, 16);
+    if (!ok) atomicOr(p.guard, 16);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        tmem_dealloc(tmem, TC_COLS);
+        tmem_dealloc(tmem0, NT_COLS);
     }
+}
+
+/* the kernel for a model's grid and head */
+template <int MODE, int HH, bool LIST>
+static void launch_net_tc(const RenderParams &p, int it, int n_sms, cudaStream_t s)
+{
+    const size_t smem = nt_smem_bytes(p.freq);
+    if (p.freq || p.grid.F == 4) wf_net_tc_kernel<MODE, HH, LIST, true><<<n_sms, NT_THREADS, smem, s>>>(p, it);
+    else wf_net_tc_kernel<MODE, HH, LIST, false><<<n_sms, NT_THREADS, smem, s>>>(p, it);
 }
 
 /* The cache build's density network (NerfNetwork::inferenceLatents on the
@@ -2401,11 +2488,19 @@ static cudaError_t set_net_attrs()
     cudaError_t e = cudaFuncSetAttribute(wf_net_resample_kernel<HH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_resample_kernel<HH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_cache_kernel<HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    const int tsmem = (int)tc_smem_bytes(1); /* the largest launch (a head with the frequency encoding) */
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tc_kernel<0, HH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tc_kernel<0, HH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tc_kernel<1, HH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tc_kernel<2, HH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem);
+    const int tsmem = (int)sizeof(TcSmem), nsmem = (int)nt_smem_bytes(1); /* the largest launch (a head with the frequency encoding) */
+    auto net_attr = [&](auto *kernel) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, nsmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+    };
+    net_attr(wf_net_tc_kernel<0, HH, true, false>);
+    net_attr(wf_net_tc_kernel<0, HH, true, true>);
+    net_attr(wf_net_tc_kernel<0, HH, false, false>);
+    net_attr(wf_net_tc_kernel<0, HH, false, true>);
+    net_attr(wf_net_tc_kernel<1, HH, true, false>);
+    net_attr(wf_net_tc_kernel<1, HH, true, true>);
+    net_attr(wf_net_tc_kernel<2, HH, false, false>);
+    net_attr(wf_net_tc_kernel<2, HH, false, true>);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tcm_kernel<64, HH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcmSmem<64>));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tcm_kernel<256, HH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcmSmem<256>));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tc_prec_kernel<1, HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem);
@@ -2437,17 +2532,15 @@ static inline bool fused_cached_path(const RenderParams &p)
 template <int HH>
 static void launch_plain_net(const RenderParams &p, int it, int n_sms, cudaStream_t s)
 {
-    const size_t tc_smem = tc_smem_bytes(p.freq);
-    const int grid_tc = n_sms * FVC_TC_CTAS_PER_SM;
     if (p.view_dependent) wf_net_vd_kernel<0, HH, false><<<n_sms * 4, 128, sizeof(VdSmem), s>>>(p, it);
     else if (!p.use_tc) wf_net_resample_kernel<HH, false><<<n_sms * 2, NET_WARPS * 32, sizeof(NetSmem), s>>>(p, it);
-    else if (p.precision == 1) wf_net_tc_prec_kernel<1, HH><<<n_sms * TC_PREC_CTAS_PER_SM, 128, tc_smem, s>>>(p, it);
-    else if (p.precision == 2) wf_net_tc_prec_kernel<2, HH><<<n_sms * TC_PREC_CTAS_PER_SM, 128, tc_smem, s>>>(p, it);
+    else if (p.precision == 1) wf_net_tc_prec_kernel<1, HH><<<n_sms * TC_PREC_CTAS_PER_SM, 128, sizeof(TcSmem), s>>>(p, it);
+    else if (p.precision == 2) wf_net_tc_prec_kernel<2, HH><<<n_sms * TC_PREC_CTAS_PER_SM, 128, sizeof(TcSmem), s>>>(p, it);
     else if (p.m_tile == 64)
         wf_net_tcm_kernel<64, HH, false><<<n_sms * tcm_ctas_per_sm<64>(), tcm_threads<64>(), sizeof(TcmSmem<64>), s>>>(p, it);
     else if (p.m_tile == 256)
         wf_net_tcm_kernel<256, HH, false><<<n_sms * tcm_ctas_per_sm<256>(), tcm_threads<256>(), sizeof(TcmSmem<256>), s>>>(p, it);
-    else wf_net_tc_kernel<0, HH, false><<<grid_tc, 128, tc_smem, s>>>(p, it);
+    else launch_net_tc<0, HH, false>(p, it, n_sms, s);
 }
 
 /* blocks of the per-ray kernels: no more than the rays fill */
@@ -2493,8 +2586,6 @@ static cudaError_t run_frame(const RenderParams &p, int n_sms, cudaStream_t s, i
     check_every = check_interval(p, check_every);
     const int grid_net = n_sms * 2;
     const size_t net_smem = sizeof(NetSmem);
-    const size_t tc_smem = tc_smem_bytes(p.freq);
-    const int grid_tc = n_sms * FVC_TC_CTAS_PER_SM; /* <= 8 CTAs x 64 TMEM columns per SM */
     const bool fused = CACHED && fused_cached_path(p);
     int it = 0;
     const int max_it = 1 << 20;
@@ -2503,7 +2594,7 @@ static cudaError_t run_frame(const RenderParams &p, int n_sms, cudaStream_t s, i
             launch_march<true, true>(p, it, n_rays, n_sms, s);
             wf_cache_lookup_kernel<<<n_sms * 8, 256, 0, s>>>(p, it);
             timed_begin();
-            wf_net_tc_kernel<2, HH, false><<<grid_tc, 128, tc_smem, s>>>(p, it);
+            launch_net_tc<2, HH, false>(p, it, n_sms, s);
             timed_end();
             L.launches += 3;
         } else {
@@ -2514,11 +2605,11 @@ static cudaError_t run_frame(const RenderParams &p, int n_sms, cudaStream_t s, i
             launch_classify(p, it, n_sms, s);
             timed_begin();
             if (p.view_dependent) wf_net_vd_kernel<0, HH, true><<<n_sms * 4, 128, sizeof(VdSmem), s>>>(p, it);
-            else if (p.use_tc) wf_net_tc_kernel<0, HH, true><<<grid_tc, 128, tc_smem, s>>>(p, it);
+            else if (p.use_tc) launch_net_tc<0, HH, true>(p, it, n_sms, s);
             else wf_net_resample_kernel<HH, true><<<grid_net, NET_WARPS * 32, net_smem, s>>>(p, it);
             timed_end();
             if (p.view_dependent) wf_net_vd_kernel<1, HH, true><<<n_sms * 4, 128, sizeof(VdSmem), s>>>(p, it);
-            else if (p.use_tc) wf_net_tc_kernel<1, HH, true><<<grid_tc, 128, tc_smem, s>>>(p, it);
+            else if (p.use_tc) launch_net_tc<1, HH, true>(p, it, n_sms, s);
             else wf_net_cache_kernel<HH><<<grid_net, NET_WARPS * 32, net_smem, s>>>(p, it);
             L.launches += 3;
         } else if (!CACHED) {
@@ -2625,12 +2716,10 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
         /* the forward kernels of pass 1, so both passes composite the same values */
         if (one_round) {
         } else if (CACHED) {
-            const size_t tc_smem = tc_smem_bytes(p.freq);
-            const int grid_tc = n_sms * FVC_TC_CTAS_PER_SM;
             launch_classify(p, it, n_sms, s);
             if (p.use_tc) {
-                wf_net_tc_kernel<0, HH, true><<<grid_tc, 128, tc_smem, s>>>(p, it);
-                wf_net_tc_kernel<1, HH, true><<<grid_tc, 128, tc_smem, s>>>(p, it);
+                launch_net_tc<0, HH, true>(p, it, n_sms, s);
+                launch_net_tc<1, HH, true>(p, it, n_sms, s);
             } else {
                 wf_net_resample_kernel<HH, true><<<n_sms * 2, NET_WARPS * 32, sizeof(NetSmem), s>>>(p, it);
                 wf_net_cache_kernel<HH><<<n_sms * 2, NET_WARPS * 32, sizeof(NetSmem), s>>>(p, it);
@@ -2724,21 +2813,19 @@ static cudaError_t build_batch_graph_t(const RenderParams &p, int n_sms, cudaStr
             if (fused) {
                 launch_march<true, true>(p, it, n_rays, n_sms, s);
                 wf_cache_lookup_kernel<<<n_sms * 8, 256, 0, s>>>(p, it);
-                wf_net_tc_kernel<2, HH, false><<<n_sms * FVC_TC_CTAS_PER_SM, 128, tc_smem_bytes(p.freq), s>>>(p, it);
+                launch_net_tc<2, HH, false>(p, it, n_sms, s);
                 kernels += 2;
             } else {
                 launch_march<CACHED, false>(p, it, n_rays, n_sms, s);
             }
             if (CACHED && !fused) {
-                const size_t tc_smem = tc_smem_bytes(p.freq);
-                const int grid_tc = n_sms * FVC_TC_CTAS_PER_SM;
                 launch_classify(p, it, n_sms, s);
                 if (p.view_dependent) {
                     wf_net_vd_kernel<0, HH, true><<<n_sms * 4, 128, sizeof(VdSmem), s>>>(p, it);
                     wf_net_vd_kernel<1, HH, true><<<n_sms * 4, 128, sizeof(VdSmem), s>>>(p, it);
                 } else if (p.use_tc) {
-                    wf_net_tc_kernel<0, HH, true><<<grid_tc, 128, tc_smem, s>>>(p, it);
-                    wf_net_tc_kernel<1, HH, true><<<grid_tc, 128, tc_smem, s>>>(p, it);
+                    launch_net_tc<0, HH, true>(p, it, n_sms, s);
+                    launch_net_tc<1, HH, true>(p, it, n_sms, s);
                 } else {
                     wf_net_resample_kernel<HH, true><<<n_sms * 2, NET_WARPS * 32, sizeof(NetSmem), s>>>(p, it);
                     wf_net_cache_kernel<HH><<<n_sms * 2, NET_WARPS * 32, sizeof(NetSmem), s>>>(p, it);
