@@ -479,6 +479,18 @@ __device__ __forceinline__ float2 f2_lerp(float2 a, float2 b, float t)
     return f2_from_bits(r);
 }
 
+/* One axis of a level's cell: p = fma(scale, x, 0.5), its floor and the
+ * fraction above it.  Rounding p + 1.5 * 2^23 downwards leaves floor(p) in the
+ * sum's low bits (|p| < 2^22), so the floor, the integer and the fraction are
+ * plain additions instead of conversions, which a quarter-rate unit executes. */
+__device__ __forceinline__ uint32_t grid_axis(float scale, float x, float &w)
+{
+    const float p = __fmaf_rn(scale, x, 0.5f);
+    const float t = __fadd_rd(p, 12582912.0f);
+    w = __fsub_rn(p, __fsub_rn(t, 12582912.0f));
+    return __float_as_uint(t) - 0x4B400000u;
+}
+
 /* Encodes one position into 2*n_levels features (fp16) written to
  * out[0 .. 2*n_levels) as half2 per level.  Corner and fraction in float32
  * (p = fma(scale, x, 0.5), floor, subtract); the trilinear interpolation in
@@ -498,10 +510,7 @@ __device__ __forceinline__ void hash_group_f4(const DevGrid &g, const __half2 *_
     for (int j = 0; j < G; ++j) {
         const int l = l0 + j;
         const float sc = g.scale[l];
-        const float px = __fmaf_rn(sc, pos.x, 0.5f), py = __fmaf_rn(sc, pos.y, 0.5f), pz = __fmaf_rn(sc, pos.z, 0.5f);
-        const float fx = floorf(px), fy = floorf(py), fz = floorf(pz);
-        const uint32_t gx = (uint32_t)(int)fx, gy = (uint32_t)(int)fy, gz = (uint32_t)(int)fz;
-        wx[j] = __fsub_rn(px, fx); wy[j] = __fsub_rn(py, fy); wz[j] = __fsub_rn(pz, fz);
+        const uint32_t gx = grid_axis(sc, pos.x, wx[j]), gy = grid_axis(sc, pos.y, wy[j]), gz = grid_axis(sc, pos.z, wz[j]);
         const uint32_t size = g.size[l];
         const uint2 *tl = reinterpret_cast<const uint2 *>(table + g.offset[l]);
         if ((g.dense_mask >> l) & 1u) {
@@ -549,10 +558,7 @@ __device__ __forceinline__ void hash_group_f2(const DevGrid &g, const __half2 *_
     for (int j = 0; j < LG; ++j) {
         const int l = l0 + j;
         const float sc = g.scale[l];
-        const float px = __fmaf_rn(sc, pos.x, 0.5f), py = __fmaf_rn(sc, pos.y, 0.5f), pz = __fmaf_rn(sc, pos.z, 0.5f);
-        const float fx = floorf(px), fy = floorf(py), fz = floorf(pz);
-        const uint32_t gx = (uint32_t)(int)fx, gy = (uint32_t)(int)fy, gz = (uint32_t)(int)fz;
-        wx[j] = __fsub_rn(px, fx); wy[j] = __fsub_rn(py, fy); wz[j] = __fsub_rn(pz, fz);
+        const uint32_t gx = grid_axis(sc, pos.x, wx[j]), gy = grid_axis(sc, pos.y, wy[j]), gz = grid_axis(sc, pos.z, wz[j]);
         const uint32_t size = g.size[l];
         const __half2 *tl = table + g.offset[l];
         if ((g.dense_mask >> l) & 1u) {
