@@ -472,7 +472,8 @@ struct fvc_renderer {
     int render_mode = 0;
     int max_samples = 0;
     int use_tc = 1;                   /* network kernels on tcgen05 (1) or mma.sync (0) */
-    int build_tc = 0;                 /* the cache builds' density network on tcgen05 (1) or mma.sync (0, faster) */
+    int build_tc = -1;                /* the cache builds' density network on tcgen05 (1), mma.sync (0) or by size (-1:
+                                       * build_by_tc); the same voxels */
     int precision = FVC_PRECISION_FP16;
     BuildScratch bs;
     PerRayScratch pr;
@@ -1678,6 +1679,18 @@ static int ensure_build_scratch(fvc_renderer *r, int n_tiles)
     return FVC_OK;
 }
 
+/* The build's density network on tcgen05 (cache_density_tc_kernel) or
+ * mma.sync (cache_density_kernel), by the iteration's rays when the caller has
+ * not chosen: a launch over 32,400 tiles takes 556 us on mma.sync and 480 on
+ * tcgen05, over 943 tiles 16.8 and 18.5 (a tile of 128 rows waits for five
+ * round trips to the tensor cores, a warp of mma.sync for none).  View-dependent
+ * models' first head runs in the warp-level kernel. */
+static bool build_by_tc(const fvc_renderer *r, long long n_rays)
+{
+    if (r->m->view_dependent) return false;
+    return r->build_tc < 0 ? n_rays >= (1 << 18) : r->build_tc == 1;
+}
+
 /* CacheRenderer::initCacheBlockwise, src/cache_renderer.cu:931-1051 */
 extern "C" int fvc_cache_build(fvc_renderer *r, const fvc_raymarch_info *info)
 {
@@ -1751,7 +1764,7 @@ extern "C" int fvc_cache_build(fvc_renderer *r, const fvc_raymarch_info *info)
         CU(cudaGetLastError());
         /* the density network (fvc_renderer_set_build_network_path); view-dependent models' first head runs
          * in the warp-level kernel */
-        if (r->build_tc && !m->view_dependent) CU(launch_cache_density_tc(p, m->d_weights_tc, m->n_sms, s));
+        if (build_by_tc(r, (long long)n_alive * 64)) CU(launch_cache_density_tc(p, m->d_weights_tc, m->n_sms, s));
         else CU(launch_cache_density(p, m->n_sms * 8, s));
         CU(cudaGetLastError());
         cache_composite_kernel<<<std::min((n_alive + 3) / 4, 1 << 16), 128, 0, s>>>(p);
@@ -1864,7 +1877,7 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
         CU(cudaMemsetAsync(p.counters + 2, 0, sizeof(int), s));
         CU(launch_fill_march(p, it, n_sms, s));
         q.dir_states = p.states[it & 1];
-        if (r->build_tc && !m->view_dependent) CU(launch_cache_density_tc(q, m->d_weights_tc, n_sms, s));
+        if (build_by_tc(r, n_alive)) CU(launch_cache_density_tc(q, m->d_weights_tc, n_sms, s));
         else CU(launch_cache_density(q, n_sms * 8, s));
         pr_mark_kernel<<<n_sms * 16, 128, 0, s>>>(f, it);
         pr_count_kernel<<<(int)((n_cols + 255) / 256), 256, 0, s>>>(f);

@@ -1295,7 +1295,46 @@ __device__ __forceinline__ bool nt_publish(int team, bool ok)
     return bad == 0u;
 }
 
-/* 64 accumulator columns of this thread's row -> (+bias) ReLU -> the fp16 row in columns NT_A.. (epi_hidden's arithmetic) */
+__device__ __forceinline__ uint32_t pack_bf2(float a, float b)
+{
+    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t *>(&h);
+}
+
+/* a pair of the network's 16-bit type: fp16 (PREC 0) or bf16 (PREC 1) */
+template <int PREC>
+__device__ __forceinline__ uint32_t nt_pack(float a, float b)
+{
+    return PREC == 1 ? pack_bf2(a, b) : pack_h2(a, b);
+}
+template <int PREC>
+__device__ __forceinline__ uint4 nt_pack8(const float *v)
+{
+    return make_uint4(nt_pack<PREC>(v[0], v[1]), nt_pack<PREC>(v[2], v[3]), nt_pack<PREC>(v[4], v[5]), nt_pack<PREC>(v[6], v[7]));
+}
+/* four fp16 pairs in it */
+template <int PREC>
+__device__ __forceinline__ uint4 nt_from_half(const __half2 *h)
+{
+    if (PREC == 0) return *reinterpret_cast<const uint4 *>(h);
+    uint32_t w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float2 f = __half22float2(h[q]);
+        w[q] = pack_bf2(f.x, f.y);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+/* a network output as stored: in the network's type, then fp16 */
+template <int PREC>
+__device__ __forceinline__ uint32_t nt_out(float v)
+{
+    return (uint32_t)__half_as_ushort(__float2half_rn(PREC == 1 ? __bfloat162float(__float2bfloat16_rn(v)) : v));
+}
+
+/* 64 accumulator columns of this thread's row -> (+bias) ReLU -> the 16-bit row in columns NT_A.. (epi_hidden's arithmetic) */
+template <int PREC>
 __device__ __forceinline__ void nt_epi(uint32_t acc, const float *bias)
 {
     const __half2 zero = __float2half2_rn(0.0f);
@@ -1309,8 +1348,12 @@ __device__ __forceinline__ void nt_epi(uint32_t acc, const float *bias)
         for (int i = 0; i < 16; ++i) {
             float2 x = make_float2(v[2 * i], v[2 * i + 1]);
             if (bias) x = __fadd2_rn(x, make_float2(bias[32 * h + 2 * i], bias[32 * h + 2 * i + 1]));
-            const __half2 r = __hmax2(__float22half2_rn(x), zero);
-            w[i] = *reinterpret_cast<const uint32_t *>(&r);
+            if (PREC == 1) {
+                w[i] = pack_bf2(fmaxf(x.x, 0.0f), fmaxf(x.y, 0.0f));
+            } else {
+                const __half2 r = __hmax2(__float22half2_rn(x), zero);
+                w[i] = *reinterpret_cast<const uint32_t *>(&r);
+            }
         }
         tmem_st16(acc + NT_A + 16 * h, w);
     }
@@ -1318,7 +1361,7 @@ __device__ __forceinline__ void nt_epi(uint32_t acc, const float *bias)
 
 /* the row's features into columns NT_A .. NT_A + 15, four half2 at a time: a loop that the compiler keeps, so its code
  * stays in the instruction cache, and whose results need no array (whole warp) */
-template <bool GENERAL>
+template <bool GENERAL, int PREC>
 __device__ __forceinline__ void nt_encode(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, uint32_t acc)
 {
 #pragma unroll 1
@@ -1331,8 +1374,25 @@ __device__ __forceinline__ void nt_encode(const DevGrid &g, const __half2 *__res
             for (int j = 0; j < 4; j += FVC_NT_HASH_GROUP) hash_group_f2<FVC_NT_HASH_GROUP>(g, table, pos, 4 * c + j, f + j);
         }
         __syncwarp();
-        tmem_st4(acc + NT_A + 4 * c, *reinterpret_cast<const uint4 *>(f));
+        tmem_st4(acc + NT_A + 4 * c, nt_from_half<PREC>(f));
     }
+}
+
+/* one layer: the MMAs by the team's first thread, then the bounded wait for their completion */
+template <int PREC>
+__device__ __forceinline__ bool nt_layer(uint32_t tmem, const uint8_t *w, int K, int N, uint64_t *mbar, uint32_t &phase, bool leader)
+{
+    if (leader) {
+        tc_fence_after();
+        const uint32_t sbo = (uint32_t)(K / 8) * 128u, id = idesc_f16(128, N, PREC == 1), w0 = smem_u32(w);
+        for (int kc = 0; kc < K / 16; ++kc)
+            tc_mma_f16_ts(tmem, tmem + NT_A + 8u * kc, umma_desc(w0 + 256u * kc, 128u, sbo), id, kc > 0 ? 1u : 0u);
+        tc_commit(mbar);
+    }
+    const bool done = mbar_wait(mbar, phase, TC_WAIT_LIMIT);
+    phase ^= 1u;
+    tc_fence_after();
+    return done;
 }
 
 /* what a thread's row needs from memory before its gathers: its id (-1: none), position and direction */
@@ -1347,8 +1407,10 @@ struct NtRow {
  * (hash features, density layers, head), then the cache list's tiles (the
  * head input of each row's lookup, wf_cache_lookup_kernel; head only), so
  * that no tile mixes the two kinds of row.  GENERAL: the 4-feature grid and
- * the head with the frequency encoding; without it the kernel is smaller. */
-template <int MODE, int HH, bool LIST, bool GENERAL>
+ * the head with the frequency encoding; without it the kernel is smaller.
+ * PREC 1: bf16 layers (plain renders): outputs in bf16, stored as fp16 like
+ * the fp16 path. */
+template <int MODE, int HH, bool LIST, bool GENERAL, int PREC = 0>
 __global__ void __launch_bounds__(NT_THREADS, 1) wf_net_tc_kernel(RenderParams p, int it)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1370,7 +1432,7 @@ __global__ void __launch_bounds__(NT_THREADS, 1) wf_net_tc_kernel(RenderParams p
 #pragma unroll
         for (int t = 0; t < NT_TEAMS; ++t) mbar_init(&S.mbar[t], 1);
         mbar_arrive_expect_tx(&S.wbar, wbytes);
-        bulk_copy_g2s(S.W, p.weights_tc, wbytes, &S.wbar);
+        bulk_copy_g2s(S.W, PREC == 1 ? p.weights_tc_bf16 : p.weights_tc, wbytes, &S.wbar);
     }
     if (tid < 64) S.bias3[tid] = p.bias3[tid];
     if (warp == 0) tmem_alloc(&S.tmem_base, NT_COLS);
@@ -1383,20 +1445,7 @@ __global__ void __launch_bounds__(NT_THREADS, 1) wf_net_tc_kernel(RenderParams p
     uint64_t *const mbar = &S.mbar[team];
     const RayState *states = p.states[it & 1];
     uint32_t phase = 0;
-    /* one layer's MMAs by the team's first thread, then the bounded wait for their completion */
-    auto layer = [&](const uint8_t *b, int K, int N) {
-        if (row == 0) {
-            tc_fence_after();
-            const uint32_t sbo = (uint32_t)(K / 8) * 128u, id = idesc_f16(128, N, false), b0 = smem_u32(b);
-            for (int kc = 0; kc < K / 16; ++kc)
-                tc_mma_f16_ts(tmem, tmem + NT_A + 8u * kc, umma_desc(b0 + 256u * kc, 128u, sbo), id, kc > 0 ? 1u : 0u);
-            tc_commit(mbar);
-        }
-        const bool done = mbar_wait(mbar, phase, TC_WAIT_LIMIT);
-        phase ^= 1u;
-        tc_fence_after();
-        return done;
-    };
+    auto layer = [&](const uint8_t *w, int K, int N) { return nt_layer<PREC>(tmem, w, K, N, mbar, phase, row == 0); };
     auto is_cached = [&](int tile) { return MODE == 1 || (MODE == 2 && tile >= res_tiles); };
     auto load_row = [&](int tile) {
         NtRow in;
@@ -1424,10 +1473,11 @@ __global__ void __launch_bounds__(NT_THREADS, 1) wf_net_tc_kernel(RenderParams p
         const int r = in.r;
         const float3 d01 = in.d01;
         uint4 b0 = make_uint4(0u, 0u, 0u, 0u), b1 = b0;
+        uint32_t log_density = 0u; /* fp16 */
         float3 fq = in.pos; /* the frequency encoding's position */
         if (!cached) {
             /* ---- hash features -> activations (K = 32); a lane without a row encodes the origin ---- */
-            nt_encode<GENERAL>(p.grid, p.table, in.pos, acc);
+            nt_encode<GENERAL, PREC>(p.grid, p.table, in.pos, acc);
         } else if (r >= 0) {
             /* ---- cache lookup -> head input (log-density, latents); MODE 1 finds it by the place in the list ---- */
             uint32_t hin[8];
@@ -1442,22 +1492,29 @@ __global__ void __launch_bounds__(NT_THREADS, 1) wf_net_tc_kernel(RenderParams p
             if (!(ok = nt_publish(team, ok))) break;
             /* ---- layer 1: 32 -> 64, ReLU ---- */
             ok = layer(S.W + TC_B1, 32, 64);
-            nt_epi(acc, nullptr);
+            nt_epi<PREC>(acc, nullptr);
             if (!(ok = nt_publish(team, ok))) break;
             /* ---- layer 2: 64 -> 16 (log-density, latents) ---- */
             ok = layer(S.W + TC_B2, 64, 16);
             float v[16];
             tmem_ld16(acc, v);
             tmem_wait_ld();
-            b0 = pack8(v);
-            b1 = pack8(v + 8);
+            log_density = nt_out<PREC>(v[0]);
+            if (PREC == 1) { /* the latents alone */
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (j < p.latent_offset || j >= p.latent_offset + 8) v[j] = 0.f;
+            }
+            b0 = nt_pack8<PREC>(v);
+            b1 = nt_pack8<PREC>(v + 8);
+        } else {
+            log_density = b0.x & 0xffffu;
         }
-        const uint32_t log_density = b0.x & 0xffffu;
         __syncwarp();
         tmem_st8(acc + NT_A, b0, b1);
         __half2 sh[8];
         sh16(d01, sh);
-        tmem_st8(acc + NT_A + 8, *reinterpret_cast<const uint4 *>(sh), *reinterpret_cast<const uint4 *>(sh + 4));
+        tmem_st8(acc + NT_A + 8, nt_from_half<PREC>(sh), nt_from_half<PREC>(sh + 4));
         if (freq) {
             /* the frequency encoding of the row's network input position (include/nerf_network.h:241-246) */
             tmem_st8(acc + NT_A + 16, freq_chunk(fq.x), freq_chunk(fq.y));
@@ -1466,12 +1523,12 @@ __global__ void __launch_bounds__(NT_THREADS, 1) wf_net_tc_kernel(RenderParams p
         if (!(ok = nt_publish(team, ok))) break;
         /* ---- head layer 1: (latents | SH (| frequency)) HK -> 64, bias from the 1-padding, ReLU ---- */
         ok = layer(S.W + wb3, HK, 64);
-        nt_epi(acc, S.bias3);
+        nt_epi<PREC>(acc, S.bias3);
         if (!(ok = nt_publish(team, ok))) break;
         if (HH == 2) {
             /* ---- head layer 2: 64 -> 64, ReLU ---- */
             ok = layer(S.W + wb4, 64, 64);
-            nt_epi(acc, nullptr);
+            nt_epi<PREC>(acc, nullptr);
             if (!(ok = nt_publish(team, ok))) break;
         }
         /* ---- output layer: 64 -> 16 (rgb logits in cols 0..2); the next tile's first MMA overwrites the
@@ -1481,7 +1538,7 @@ __global__ void __launch_bounds__(NT_THREADS, 1) wf_net_tc_kernel(RenderParams p
         tmem_ld4(acc, o);
         tmem_wait_ld();
         if (r >= 0)
-            p.row_out[r] = make_uint2(pack_h2(o[0], o[1]), (uint32_t)__half_as_ushort(__float2half_rn(o[2])) | (log_density << 16));
+            p.row_out[r] = make_uint2(nt_out<PREC>(o[0]) | (nt_out<PREC>(o[1]) << 16), nt_out<PREC>(o[2]) | (log_density << 16));
     }
     if (!ok) atomicOr(p.guard, 16);
     tc_fence_before();
@@ -1493,84 +1550,84 @@ __global__ void __launch_bounds__(NT_THREADS, 1) wf_net_tc_kernel(RenderParams p
 }
 
 /* the kernel for a model's grid and head */
-template <int MODE, int HH, bool LIST>
+template <int MODE, int HH, bool LIST, int PREC = 0>
 static void launch_net_tc(const RenderParams &p, int it, int n_sms, cudaStream_t s)
 {
     const size_t smem = nt_smem_bytes(p.freq);
-    if (p.freq || p.grid.F == 4) wf_net_tc_kernel<MODE, HH, LIST, true><<<n_sms, NT_THREADS, smem, s>>>(p, it);
-    else wf_net_tc_kernel<MODE, HH, LIST, false><<<n_sms, NT_THREADS, smem, s>>>(p, it);
+    if (p.freq || p.grid.F == 4) wf_net_tc_kernel<MODE, HH, LIST, true, PREC><<<n_sms, NT_THREADS, smem, s>>>(p, it);
+    else wf_net_tc_kernel<MODE, HH, LIST, false, PREC><<<n_sms, NT_THREADS, smem, s>>>(p, it);
 }
 
 /* The cache build's density network (NerfNetwork::inferenceLatents on the
  * build rows, src/cache_renderer.cu:1020-1030) on tcgen05: the hash features
- * and the two density layers of wf_net_tc_kernel (same tiles, weights,
+ * and the two density layers of wf_net_tc_kernel (same teams, weights,
  * epilogues and bounded waits), on every row of a build iteration; writes
  * the row's fp16 log-density and its 8 latents from output latent_offset. */
-__global__ void __launch_bounds__(128, FVC_TC_CTAS_PER_SM) cache_density_tc_kernel(CacheBuildParams p, const uint8_t *weights_tc,
-                                                                                     const int *n_rows_ptr)
+template <bool GENERAL>
+__global__ void __launch_bounds__(NT_THREADS, 1) cache_density_tc_kernel(CacheBuildParams p, const uint8_t *weights_tc, const int *n_rows_ptr)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    TcSmem &S = *reinterpret_cast<TcSmem *>(smem_raw);
+    NtSmem &S = *reinterpret_cast<NtSmem *>(smem_raw);
     const int n_rows = *n_rows_ptr;
-    if (n_rows == 0) return;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int n_tiles = (n_rows + 127) / 128;
+    if ((int)blockIdx.x * NT_TEAMS >= n_tiles) return;
+    const int tid = threadIdx.x, warp = tid >> 5, team = tid >> 7, row = tid & 127;
     if (tid == 0) {
-        mbar_init(&S.mbar, 1);
-        mbar_arrive_expect_tx(&S.mbar, TC_WBYTES);
-        bulk_copy_g2s(S.W, weights_tc, TC_WBYTES, &S.mbar);
+        mbar_init(&S.wbar, 1);
+#pragma unroll
+        for (int t = 0; t < NT_TEAMS; ++t) mbar_init(&S.mbar[t], 1);
+        mbar_arrive_expect_tx(&S.wbar, TC_B3);
+        bulk_copy_g2s(S.W, weights_tc, TC_B3, &S.wbar); /* the density layers' tiles */
     }
-    if (warp == 0) tmem_alloc(&S.tmem_base, TC_COLS);
+    if (warp == 0) tmem_alloc(&S.tmem_base, NT_COLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = S.tmem_base;
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+    const uint32_t tmem0 = S.tmem_base, tmem = tmem0 + (uint32_t)(NT_TEAM_COLS * team);
+    const uint32_t acc = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    uint64_t *const mbar = &S.mbar[team];
     uint32_t phase = 0;
-    bool ok = mbar_wait(&S.mbar, phase, TC_WAIT_LIMIT);
-    phase ^= 1u;
-    const int lo = p.latent_offset;
-    const int n_tiles = (n_rows + 127) / 128;
-    for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        const int r = tile * 128 + tid;
-        __half2 feat[16];
-#pragma unroll
-        for (int q = 0; q < 16; ++q) feat[q] = __floats2half2_rn(0.f, 0.f);
-        if (r < n_rows) {
-            const float4 rw = p.build_rows[r];
-            hash_encode<FVC_TC_HASH_GROUP>(p.grid, p.table, make_float3(rw.x, rw.y, rw.z), feat);
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) st_chunk(S.X, tid, c, 32, *reinterpret_cast<const uint4 *>(feat + 4 * c));
-        if (!(ok = tc_publish(ok))) break;
+    bool ok = mbar_wait(&S.wbar, 0, TC_WAIT_LIMIT);
+    const int lo = p.latent_offset, stride = (int)gridDim.x * NT_TEAMS;
+    auto load_pos = [&](int tile) {
+        const int r = tile * 128 + row;
+        const float4 v = r < n_rows ? p.build_rows[r] : make_float4(0.f, 0.f, 0.f, 0.f);
+        return make_float3(v.x, v.y, v.z);
+    };
+    int tile = (int)blockIdx.x * NT_TEAMS + team;
+    float3 pos = load_pos(tile);
+    for (; tile < n_tiles; tile += stride) {
+        const int r = tile * 128 + row;
+        nt_encode<GENERAL, 0>(p.grid, p.table, pos, acc);
+        pos = load_pos(tile + stride); /* in flight under this tile's layers */
+        if (!(ok = nt_publish(team, ok))) break;
         /* ---- layer 1: 32 -> 64, ReLU ---- */
-        ok = tc_run(S, tmem, S.W + TC_B1, 32, 64, phase);
-        epi_hidden(tmem + lane_base, nullptr, S.X, tid);
-        if (!(ok = tc_publish(ok))) break;
-        /* ---- layer 2: 64 -> 16 (log-density, latents) ---- */
-        ok = tc_run(S, tmem, S.W + TC_B2, 64, 16, phase);
+        ok = nt_layer<0>(tmem, S.W + TC_B1, 32, 64, mbar, phase, row == 0);
+        nt_epi<0>(acc, nullptr);
+        if (!(ok = nt_publish(team, ok))) break;
+        /* ---- layer 2: 64 -> 16 (log-density, latents); the next tile's first MMA overwrites the accumulator only
+         * after its nt_publish ---- */
+        ok = nt_layer<0>(tmem, S.W + TC_B2, 64, 16, mbar, phase, row == 0);
         float v[16];
-        tmem_ld16(tmem + lane_base, v);
+        tmem_ld16(acc, v);
         tmem_wait_ld();
         if (r < n_rows) {
-            __half h[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) h[j] = __float2half_rn(v[j]);
-            p.build_den[r] = h[0];
+            p.build_den[r] = __float2half_rn(v[0]);
+            /* latent_offset is 0 or 1 */
+            const uint4 a = pack8(v), b = pack8(v + 8);
+            const uint32_t h[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
             uint32_t lw[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                lw[q] = (uint32_t)__half_as_ushort(h[lo + 2 * q]) | ((uint32_t)__half_as_ushort(h[lo + 2 * q + 1]) << 16);
+            for (int q = 0; q < 4; ++q) lw[q] = lo ? __funnelshift_r(h[q], h[q + 1], 16) : h[q];
             p.build_lat[r] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
         }
-        tc_fence_before();
-        if (__syncthreads_or(!ok)) { ok = false; break; }
     }
-    if (!ok && tid == 0 && p.guard) atomicOr(p.guard, 16);
+    if (!ok && p.guard) atomicOr(p.guard, 16);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        tmem_dealloc(tmem, TC_COLS);
+        tmem_dealloc(tmem0, NT_COLS);
     }
 }
 
@@ -1578,10 +1635,16 @@ cudaError_t launch_cache_density_tc(const CacheBuildParams &p, const uint8_t *we
 {
     static PerDeviceOnce once;
     cudaError_t e = once.run([] {
-        return cudaFuncSetAttribute(cache_density_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem));
+        cudaError_t e = cudaSuccess;
+        for (auto *kernel : {cache_density_tc_kernel<false>, cache_density_tc_kernel<true>}) {
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NtSmem));
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+        }
+        return e;
     });
     if (e != cudaSuccess) return e;
-    cache_density_tc_kernel<<<n_sms * FVC_TC_CTAS_PER_SM, 128, sizeof(TcSmem), s>>>(p, weights_tc, p.build_row_counter);
+    if (p.grid.F == 4) cache_density_tc_kernel<true><<<n_sms, NT_THREADS, sizeof(NtSmem), s>>>(p, weights_tc, p.build_row_counter);
+    else cache_density_tc_kernel<false><<<n_sms, NT_THREADS, sizeof(NtSmem), s>>>(p, weights_tc, p.build_row_counter);
     return cudaGetLastError();
 }
 
@@ -1775,23 +1838,15 @@ __global__ void __launch_bounds__(tcm_threads<MT>(), tcm_ctas_per_sm<MT>()) wf_n
 }
 
 /* ------------------------------------------------------------------------- */
-/* tcgen05 network kernel at reduced precision (plain path, resample rows)   */
+/* tcgen05 network kernel in FP8-E4M3 (plain path, resample rows)            */
 /* ------------------------------------------------------------------------- */
-/* PREC 1, BF16: kind::f16 with bf16 operands; hash features, SH and every
- * layer output are rounded to bf16.
- * PREC 2, FP8-E4M3: kind::f8f6f4 (K = 32 per MMA, the same 8-row x 16-byte
- * core matrices).  Each weight matrix is stored scaled by 448 / amax(W) (per
+/* kind::f8f6f4 (K = 32 per MMA, 8-row x 16-byte core matrices).  Each weight matrix is stored scaled by 448 / amax(W) (per
  * layer, on the host); each activation row is scaled by 448 / amax(row) before
  * its e4m3 conversion.  The thread that owns a row divides both scales out of
  * its fp32 accumulator row in the epilogue.
- * Layer structure, TMEM use, waits and the guard are those of
- * wf_net_tc_kernel; compositing stays fp32. */
-__device__ __forceinline__ uint32_t pack_bf2(float a, float b)
-{
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t *>(&h);
-}
-
+ * One CTA of 128 threads per tile, thread t owning row t and TMEM lane t; the
+ * activations live in one shared tile that each layer rewrites; waits and the
+ * guard are those of wf_net_tc_kernel; compositing stays fp32. */
 __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d)
 {
     const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
@@ -1799,51 +1854,33 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float
     return lo | (hi << 16);
 }
 
-/* writes this thread's row of K values into the operand tile in the kernel's
- * precision; returns the factor that undoes the row's scale (1 for bf16) */
-template <int PREC, int K>
+/* writes this thread's row of K values into the operand tile; returns the factor that undoes the row's scale */
+template <int K>
 __device__ __forceinline__ float put_row(uint8_t *tile, int row, const float *v)
 {
-    if (PREC == 1) {
+    float amax = 0.0f;
 #pragma unroll
-        for (int c = 0; c < K / 8; ++c)
-            *reinterpret_cast<uint4 *>(tile + kmajor_offset(row, 8 * c, K)) =
-                make_uint4(pack_bf2(v[8 * c], v[8 * c + 1]), pack_bf2(v[8 * c + 2], v[8 * c + 3]),
-                           pack_bf2(v[8 * c + 4], v[8 * c + 5]), pack_bf2(v[8 * c + 6], v[8 * c + 7]));
-        return 1.0f;
-    } else {
-        float amax = 0.0f;
+    for (int i = 0; i < K; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    const float sc = amax > 0.0f ? 448.0f / amax : 1.0f;
 #pragma unroll
-        for (int i = 0; i < K; ++i) amax = fmaxf(amax, fabsf(v[i]));
-        const float sc = amax > 0.0f ? 448.0f / amax : 1.0f;
-#pragma unroll
-        for (int c = 0; c < K / 16; ++c) {
-            const float *w = v + 16 * c;
-            *reinterpret_cast<uint4 *>(tile + kmajor_offset8(row, 16 * c, K)) =
-                make_uint4(pack_e4m3x4(w[0] * sc, w[1] * sc, w[2] * sc, w[3] * sc),
-                           pack_e4m3x4(w[4] * sc, w[5] * sc, w[6] * sc, w[7] * sc),
-                           pack_e4m3x4(w[8] * sc, w[9] * sc, w[10] * sc, w[11] * sc),
-                           pack_e4m3x4(w[12] * sc, w[13] * sc, w[14] * sc, w[15] * sc));
-        }
-        return 1.0f / sc;
+    for (int c = 0; c < K / 16; ++c) {
+        const float *w = v + 16 * c;
+        *reinterpret_cast<uint4 *>(tile + kmajor_offset8(row, 16 * c, K)) =
+            make_uint4(pack_e4m3x4(w[0] * sc, w[1] * sc, w[2] * sc, w[3] * sc), pack_e4m3x4(w[4] * sc, w[5] * sc, w[6] * sc, w[7] * sc),
+                       pack_e4m3x4(w[8] * sc, w[9] * sc, w[10] * sc, w[11] * sc),
+                       pack_e4m3x4(w[12] * sc, w[13] * sc, w[14] * sc, w[15] * sc));
     }
+    return 1.0f / sc;
 }
 
-template <int PREC>
-__device__ __forceinline__ bool tc_run_prec(TcSmem &S, uint32_t tmem, const uint8_t *b, int K, int N, uint32_t &phase)
+__device__ __forceinline__ bool tc_run_fp8(TcSmem &S, uint32_t tmem, const uint8_t *b, int K, int N, uint32_t &phase)
 {
     if (threadIdx.x == 0) {
         tc_fence_after();
         const uint32_t a0 = smem_u32(S.X), b0 = smem_u32(b);
-        if (PREC == 1) {
-            const uint32_t sbo = (uint32_t)(K / 8) * 128u, id = idesc_f16(128, N, true);
-            for (int kc = 0; kc < K / 16; ++kc)
-                tc_mma_f16(tmem, umma_desc(a0 + 256u * kc, 128u, sbo), umma_desc(b0 + 256u * kc, 128u, sbo), id, kc > 0 ? 1u : 0u);
-        } else {
-            const uint32_t sbo = (uint32_t)(K / 16) * 128u, id = idesc_f8_e4m3(128, N);
-            for (int kc = 0; kc < K / 32; ++kc)
-                tc_mma_f8(tmem, umma_desc(a0 + 256u * kc, 128u, sbo), umma_desc(b0 + 256u * kc, 128u, sbo), id, kc > 0 ? 1u : 0u);
-        }
+        const uint32_t sbo = (uint32_t)(K / 16) * 128u, id = idesc_f8_e4m3(128, N);
+        for (int kc = 0; kc < K / 32; ++kc)
+            tc_mma_f8(tmem, umma_desc(a0 + 256u * kc, 128u, sbo), umma_desc(b0 + 256u * kc, 128u, sbo), id, kc > 0 ? 1u : 0u);
         tc_commit(&S.mbar);
     }
     const bool ok = mbar_wait(&S.mbar, phase, TC_WAIT_LIMIT);
@@ -1853,8 +1890,7 @@ __device__ __forceinline__ bool tc_run_prec(TcSmem &S, uint32_t tmem, const uint
 }
 
 /* 64 accumulator columns -> scale, (+bias), ReLU -> next operand row */
-template <int PREC>
-__device__ __forceinline__ float epi_hidden_prec(uint32_t taddr, float deq, const float *bias, uint8_t *dst, int row)
+__device__ __forceinline__ float epi_hidden_fp8(uint32_t taddr, float deq, const float *bias, uint8_t *dst, int row)
 {
     float v[64];
     tmem_ld32(taddr, *reinterpret_cast<float(*)[32]>(v));
@@ -1862,37 +1898,32 @@ __device__ __forceinline__ float epi_hidden_prec(uint32_t taddr, float deq, cons
     tmem_wait_ld();
 #pragma unroll
     for (int i = 0; i < 64; ++i) v[i] = fmaxf(v[i] * deq + (bias ? bias[i] : 0.0f), 0.0f);
-    return put_row<PREC, 64>(dst, row, v);
+    return put_row<64>(dst, row, v);
 }
 
-constexpr int TC_PREC_CTAS_PER_SM = 4; /* 128 registers: the fp32 rows of the scaled epilogues */
+constexpr int TC_FP8_CTAS_PER_SM = 4; /* 128 registers: the fp32 rows of the scaled epilogues */
 
-template <int PREC, int HH>
-__global__ void __launch_bounds__(128, TC_PREC_CTAS_PER_SM) wf_net_tc_prec_kernel(RenderParams p, int it)
+template <int HH>
+__global__ void __launch_bounds__(128, TC_FP8_CTAS_PER_SM) wf_net_tc_fp8_kernel(RenderParams p, int it)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     TcSmem &S = *reinterpret_cast<TcSmem *>(smem_raw);
     const int n_rows = p.counters[2];
     if ((int)blockIdx.x * 128 >= n_rows) return;
     const int tid = threadIdx.x, warp = tid >> 5;
-    const uint8_t *wsrc = PREC == 1 ? p.weights_tc_bf16 : p.weights_tc_fp8;
-    const int wbytes = PREC == 1 ? TC_WBYTES : TC8_WBYTES;
     if (tid == 0) { /* the weights by one bulk copy, completing phase 0 (as wf_net_tc_kernel) */
         mbar_init(&S.mbar, 1);
-        mbar_arrive_expect_tx(&S.mbar, (uint32_t)wbytes);
-        bulk_copy_g2s(S.W, wsrc, (uint32_t)wbytes, &S.mbar);
+        mbar_arrive_expect_tx(&S.mbar, TC8_WBYTES);
+        bulk_copy_g2s(S.W, p.weights_tc_fp8, TC8_WBYTES, &S.mbar);
     }
     if (tid < 64) S.bias3[tid] = p.bias3[tid];
     if (warp == 0) tmem_alloc(&S.tmem_base, TC_COLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    float iw[5] = {1.f, 1.f, 1.f, 1.f, 1.f};
-    if (PREC == 2)
+    float iw[5];
 #pragma unroll
-        for (int l = 0; l < 5; ++l) iw[l] = __ldg(p.tc_fp8_iw + l);
-    const int o1 = PREC == 1 ? TC_B1 : TC8_B1, o2 = PREC == 1 ? TC_B2 : TC8_B2, o3 = PREC == 1 ? TC_B3 : TC8_B3,
-              o4 = PREC == 1 ? TC_B4 : TC8_B4, o5 = PREC == 1 ? TC_B5 : TC8_B5;
+    for (int l = 0; l < 5; ++l) iw[l] = __ldg(p.tc_fp8_iw + l);
     const uint32_t tmem = S.tmem_base;
     const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
     const RayState *states = p.states[it & 1];
@@ -1919,13 +1950,13 @@ __global__ void __launch_bounds__(128, TC_PREC_CTAS_PER_SM) wf_net_tc_prec_kerne
             in[2 * q] = f.x;
             in[2 * q + 1] = f.y;
         }
-        float deq = put_row<PREC, 32>(S.X, tid, in);
+        float deq = put_row<32>(S.X, tid, in);
         if (!(ok = tc_publish(ok))) break;
         /* density network */
-        ok = tc_run_prec<PREC>(S, tmem, S.W + o1, 32, 64, phase);
-        deq = epi_hidden_prec<PREC>(tmem + lane_base, deq * iw[0], nullptr, S.X, tid);
+        ok = tc_run_fp8(S, tmem, S.W + TC8_B1, 32, 64, phase);
+        deq = epi_hidden_fp8(tmem + lane_base, deq * iw[0], nullptr, S.X, tid);
         if (!(ok = tc_publish(ok))) break;
-        ok = tc_run_prec<PREC>(S, tmem, S.W + o2, 64, 16, phase);
+        ok = tc_run_fp8(S, tmem, S.W + TC8_B2, 64, 16, phase);
         float o[16];
         tmem_ld16(tmem + lane_base, o);
         tmem_wait_ld();
@@ -1936,7 +1967,7 @@ __global__ void __launch_bounds__(128, TC_PREC_CTAS_PER_SM) wf_net_tc_prec_kerne
         for (int j = 0; j < 16; ++j) {
             const int lat = j - p.latent_offset;
             const float v = o[j] * dq2;
-            in[j] = (lat >= 0 && lat < 8) ? (PREC == 1 ? __bfloat162float(__float2bfloat16_rn(v)) : v) : 0.0f;
+            in[j] = (lat >= 0 && lat < 8) ? v : 0.0f;
         }
         {
             __half2 sh[8];
@@ -1948,27 +1979,25 @@ __global__ void __launch_bounds__(128, TC_PREC_CTAS_PER_SM) wf_net_tc_prec_kerne
                 in[17 + 2 * q] = f.y;
             }
         }
-        deq = put_row<PREC, 32>(S.X, tid, in);
+        deq = put_row<32>(S.X, tid, in);
         if (!(ok = tc_publish(ok))) break;
         /* color head */
-        ok = tc_run_prec<PREC>(S, tmem, S.W + o3, 32, 64, phase);
-        deq = epi_hidden_prec<PREC>(tmem + lane_base, deq * iw[2], S.bias3, S.X, tid);
+        ok = tc_run_fp8(S, tmem, S.W + TC8_B3, 32, 64, phase);
+        deq = epi_hidden_fp8(tmem + lane_base, deq * iw[2], S.bias3, S.X, tid);
         if (!(ok = tc_publish(ok))) break;
         if (HH == 2) {
-            ok = tc_run_prec<PREC>(S, tmem, S.W + o4, 64, 64, phase);
-            deq = epi_hidden_prec<PREC>(tmem + lane_base, deq * iw[3], nullptr, S.X, tid);
+            ok = tc_run_fp8(S, tmem, S.W + TC8_B4, 64, 64, phase);
+            deq = epi_hidden_fp8(tmem + lane_base, deq * iw[3], nullptr, S.X, tid);
             if (!(ok = tc_publish(ok))) break;
         }
-        ok = tc_run_prec<PREC>(S, tmem, S.W + o5, 64, 16, phase);
+        ok = tc_run_fp8(S, tmem, S.W + TC8_B5, 64, 16, phase);
         tmem_ld16(tmem + lane_base, o);
         tmem_wait_ld();
         const float dq5 = deq * iw[4];
-        /* outputs in the network's precision, stored as fp16 like the fp16 path */
-        auto rnd = [](float v) { return PREC == 1 ? __bfloat162float(__float2bfloat16_rn(v)) : v; };
+        /* outputs stored as fp16 like the fp16 path */
         if (r >= 0)
-            p.row_out[r] = make_uint2(pack_h2(rnd(o[0] * dq5), rnd(o[1] * dq5)),
-                                      (uint32_t)__half_as_ushort(__float2half_rn(rnd(o[2] * dq5))) |
-                                          ((uint32_t)__half_as_ushort(__float2half_rn(rnd(log_density))) << 16));
+            p.row_out[r] = make_uint2(pack_h2(o[0] * dq5, o[1] * dq5), (uint32_t)__half_as_ushort(__float2half_rn(o[2] * dq5)) |
+                                                                           ((uint32_t)__half_as_ushort(__float2half_rn(log_density)) << 16));
         tc_fence_before();
         if (__syncthreads_or(!ok)) { ok = false; break; }
     }
@@ -2497,14 +2526,15 @@ static cudaError_t set_net_attrs()
     net_attr(wf_net_tc_kernel<0, HH, true, true>);
     net_attr(wf_net_tc_kernel<0, HH, false, false>);
     net_attr(wf_net_tc_kernel<0, HH, false, true>);
+    net_attr(wf_net_tc_kernel<0, HH, false, false, 1>);
+    net_attr(wf_net_tc_kernel<0, HH, false, true, 1>);
     net_attr(wf_net_tc_kernel<1, HH, true, false>);
     net_attr(wf_net_tc_kernel<1, HH, true, true>);
     net_attr(wf_net_tc_kernel<2, HH, false, false>);
     net_attr(wf_net_tc_kernel<2, HH, false, true>);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tcm_kernel<64, HH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcmSmem<64>));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tcm_kernel<256, HH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcmSmem<256>));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tc_prec_kernel<1, HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tc_prec_kernel<2, HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_tc_fp8_kernel<HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem);
     const int vsmem = (int)sizeof(VdSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_vd_kernel<0, HH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, vsmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_net_vd_kernel<0, HH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, vsmem);
@@ -2534,8 +2564,8 @@ static void launch_plain_net(const RenderParams &p, int it, int n_sms, cudaStrea
 {
     if (p.view_dependent) wf_net_vd_kernel<0, HH, false><<<n_sms * 4, 128, sizeof(VdSmem), s>>>(p, it);
     else if (!p.use_tc) wf_net_resample_kernel<HH, false><<<n_sms * 2, NET_WARPS * 32, sizeof(NetSmem), s>>>(p, it);
-    else if (p.precision == 1) wf_net_tc_prec_kernel<1, HH><<<n_sms * TC_PREC_CTAS_PER_SM, 128, sizeof(TcSmem), s>>>(p, it);
-    else if (p.precision == 2) wf_net_tc_prec_kernel<2, HH><<<n_sms * TC_PREC_CTAS_PER_SM, 128, sizeof(TcSmem), s>>>(p, it);
+    else if (p.precision == 1) launch_net_tc<0, HH, false, 1>(p, it, n_sms, s);
+    else if (p.precision == 2) wf_net_tc_fp8_kernel<HH><<<n_sms * TC_FP8_CTAS_PER_SM, 128, sizeof(TcSmem), s>>>(p, it);
     else if (p.m_tile == 64)
         wf_net_tcm_kernel<64, HH, false><<<n_sms * tcm_ctas_per_sm<64>(), tcm_threads<64>(), sizeof(TcmSmem<64>), s>>>(p, it);
     else if (p.m_tile == 256)

@@ -180,7 +180,7 @@ class Renderer:
         L.check(L.load().fvc_renderer_set_network_path(self.handle, int(bool(use_tcgen05))))
 
     def set_build_network_path(self, use_tcgen05: bool) -> None:
-        """The cache builds' density network: mma.sync (default, faster here) or tcgen05; same slots."""
+        """The cache builds' density network: mma.sync or tcgen05 (default: by the build's size); same slots and voxels."""
         L.check(L.load().fvc_renderer_set_build_network_path(self.handle, int(bool(use_tcgen05))))
 
     def set_empty_space_skipping(self, on: bool) -> None:
