@@ -441,9 +441,6 @@ __global__ void __launch_bounds__(BW_WARPS * 32, 1) wf_net_bwd_kernel(RenderPara
  * once the MMAs that read that tile have completed.
  * TMEM columns: 0..63 layer accumulator; 64..127 dW4; 128..159 dW3;
  * 160..191 dW1; 192..207 dW5^T; 208..223 dW2^T; 224..255 feature gradients. */
-#ifndef FVC_BT_HASH_GROUP
-#define FVC_BT_HASH_GROUP 4 /* hash levels whose gathers are in flight together */
-#endif
 constexpr int BT_COLS = 256;
 constexpr int BT_D0 = 0, BT_DW4 = 64, BT_DW3 = 128, BT_DW1 = 160, BT_DW5T = 192, BT_DW2T = 208, BT_DF = 224;
 constexpr long long BT_WAIT_LIMIT = 2000000000ll; /* ~1 s of SM clocks */
@@ -544,7 +541,7 @@ __device__ __forceinline__ bool bt_publish(bool ok)
 template <int PREC>
 __device__ __forceinline__ void bt_epi_act(uint32_t taddr, uint8_t *dst, int row)
 {
-#pragma unroll
+#pragma unroll 1
     for (int h = 0; h < 2; ++h) {
         float v[32];
         tmem_ld32(taddr + 32 * h, v);
@@ -567,7 +564,7 @@ __device__ __forceinline__ void bt_epi_act(uint32_t taddr, uint8_t *dst, int row
 template <int PREC>
 __device__ __forceinline__ void bt_epi_grad(uint32_t taddr, uint8_t *tile, int row)
 {
-#pragma unroll
+#pragma unroll 1
     for (int h = 0; h < 2; ++h) {
         float v[32];
         tmem_ld32(taddr + 32 * h, v);
@@ -610,6 +607,13 @@ constexpr int SC_PAIR_LEVELS = 10;
  *     {2i, 2i+1} (a hashed level's cell with even x, or adjacent dense
  *     indices) go out as one 16-byte red.global.add.v4.f32.
  * The table receives the same sums with fewer L2 atomics. */
+/* Levels a turn of the scatter's loop, which the compiler keeps, as it does the
+ * encode's over four levels and the epilogues' over two halves: unrolled, the
+ * kernel's warps waited for instructions longer than for anything but the L2
+ * (4.6 of 13 stall cycles an instruction).  A 2^18-ray step of the 256x256
+ * workload's scene, ms: all unrolled 25.4, encode and scatter four levels a
+ * turn 23.9, epilogues halved 23.0, scatter two levels 21.43, one 21.41. */
+constexpr int SC_GROUP = 1;
 template <int NL>
 __device__ __forceinline__ void hash_scatter_levels(const DevGrid &g, float *gt, float3 pos, int l0, const float (&dF)[2 * NL], int lane)
 {
@@ -676,60 +680,13 @@ __device__ __forceinline__ void hash_scatter_levels(const DevGrid &g, float *gt,
     }
 }
 
-__device__ __forceinline__ void tmem_ld_n(uint32_t taddr, float (&v)[16]) { tmem_ld16(taddr, v); }
-__device__ __forceinline__ void tmem_ld_n(uint32_t taddr, float (&v)[32]) { tmem_ld32(taddr, v); }
-
-/* hash_encode restricted to levels l0 .. l0 + NL - 1, LG levels' gathers in
- * flight together; the same arithmetic, so the same features */
-template <int NL, int LG>
-__device__ __forceinline__ void encode_levels(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, int l0, __half2 (&out)[NL])
+/* 2 consecutive columns of this thread's TMEM lane */
+__device__ __forceinline__ void tmem_ld2(uint32_t taddr, float (&v)[2])
 {
-#pragma unroll
-    for (int j0 = 0; j0 < NL; j0 += LG) {
-        __half2 v[LG][8];
-        float wx[LG], wy[LG], wz[LG];
-#pragma unroll
-        for (int j = 0; j < LG; ++j) {
-            const int l = l0 + j0 + j;
-            const float sc = g.scale[l];
-            const float px = __fmaf_rn(sc, pos.x, 0.5f), py = __fmaf_rn(sc, pos.y, 0.5f), pz = __fmaf_rn(sc, pos.z, 0.5f);
-            const float fx = floorf(px), fy = floorf(py), fz = floorf(pz);
-            const uint32_t gx = (uint32_t)(int)fx, gy = (uint32_t)(int)fy, gz = (uint32_t)(int)fz;
-            wx[j] = __fsub_rn(px, fx); wy[j] = __fsub_rn(py, fy); wz[j] = __fsub_rn(pz, fz);
-            const uint32_t size = g.size[l];
-            const __half2 *tl = table + g.offset[l];
-            if ((g.dense_mask >> l) & 1u) {
-                const uint32_t rr = g.res[l], r2 = g.res2[l];
-                const uint32_t b0 = gx + gy * rr + gz * r2;
-                if (b0 + 1u + rr + r2 < size) { /* no corner reaches past the table */
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) v[j][c] = __ldg(tl + (b0 + ((c & 1) ? 1u : 0u) + ((c & 2) ? rr : 0u) + ((c & 4) ? r2 : 0u)));
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        uint32_t i = b0 + ((c & 1) ? 1u : 0u) + ((c & 2) ? rr : 0u) + ((c & 4) ? r2 : 0u);
-                        if (i >= size) i -= size;
-                        v[j][c] = __ldg(tl + i);
-                    }
-                }
-            } else {
-                const uint32_t hy0 = gy * 2654435761u, hy1 = (gy + 1u) * 2654435761u;
-                const uint32_t hz0 = gz * 805459861u, hz1 = (gz + 1u) * 805459861u;
-                const uint32_t m = size - 1u;
-#pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    v[j][c] = __ldg(tl + (((gx + ((c & 1) ? 1u : 0u)) ^ ((c & 2) ? hy1 : hy0) ^ ((c & 4) ? hz1 : hz0)) & m));
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < LG; ++j) {
-            float2 e[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) e[q] = f2_lerp(__half22float2(v[j][2 * q]), __half22float2(v[j][2 * q + 1]), wx[j]);
-            const float2 g0 = f2_lerp(e[0], e[1], wy[j]), g1 = f2_lerp(e[2], e[3], wy[j]);
-            out[j0 + j] = __float22half2_rn(f2_lerp(g0, g1, wz[j]));
-        }
-    }
+    uint32_t r[2];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr) : "memory");
+    v[0] = __uint_as_float(r[0]);
+    v[1] = __uint_as_float(r[1]);
 }
 
 template <int PREC, int HH>
@@ -759,7 +716,10 @@ __global__ void __launch_bounds__(BT_THREADS, 2) wf_net_bwd_tc_kernel(RenderPara
     const uint32_t lrow = tmem + ((uint32_t)((warp & 3) * 32) << 16); /* this thread's TMEM lane */
     const int row = tid & 127;
     const int n_tiles = (n_rows + 127) / 128;
-    const int n_mine = blockIdx.x < n_tiles ? (n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    /* the CTA's tiles follow each other in the list: what its gathers left in L1 serves the next tile, and the CTAs'
+     * reductions into the coarse levels fall on different parts of the scene (4099-ray step 1105 -> 1074 us) */
+    const int tile0 = (int)((long long)n_tiles * blockIdx.x / gridDim.x);
+    const int n_mine = (int)((long long)n_tiles * (blockIdx.x + 1) / gridDim.x) - tile0;
     bool ok = true;
     if (warp >= 4) {
         /* ================= hash warps ================= */
@@ -776,12 +736,10 @@ __global__ void __launch_bounds__(BT_THREADS, 2) wf_net_bwd_tc_kernel(RenderPara
                 /* tile i into buffer i & 1 (its last reader, tile i - 2, finished before df_full of i - 2,
                  * which this loop waited for one iteration ago) */
                 const int bb = i & 1;
-                const int k = ((int)blockIdx.x + i * (int)gridDim.x) * 128 + row;
+                const int k = (tile0 + i) * 128 + row;
                 r = k < n_rows ? p.grad_res_list[k] : -1;
                 float4 dout = make_float4(0.f, 0.f, 0.f, 0.f);
-                __half2 feat[BT_NL], sh[8];
-#pragma unroll
-                for (int q = 0; q < BT_NL; ++q) feat[q] = __floats2half2_rn(0.f, 0.f);
+                __half2 sh[8];
 #pragma unroll
                 for (int q = 0; q < 8; ++q) sh[q] = __floats2half2_rn(0.f, 0.f);
                 if (r >= 0) {
@@ -791,17 +749,20 @@ __global__ void __launch_bounds__(BT_THREADS, 2) wf_net_bwd_tc_kernel(RenderPara
                         dout = p.row_dout[r];
                         sh16(row_dir01(states, p.row_slot[r]), sh);
                     }
-                    encode_levels<BT_NL, FVC_BT_HASH_GROUP>(p.grid, p.table, pos, l0, feat);
                 }
-                uint32_t f[BT_NL];
+                /* a lane without a row encodes the origin; its gradients are zero */
+#pragma unroll 1
+                for (int c = l0 / 4; c < (l0 + BT_NL) / 4; ++c) {
+                    __half2 feat[4];
+                    hash_group_f2<4>(p.grid, p.table, pos, 4 * c, feat);
+                    uint32_t f[4];
 #pragma unroll
-                for (int q = 0; q < BT_NL; ++q) {
-                    const float2 v = __half22float2(feat[q]);
-                    f[q] = PREC == 0 ? *reinterpret_cast<const uint32_t *>(&feat[q]) : T16::pack(v.x, v.y);
+                    for (int q = 0; q < 4; ++q) {
+                        const float2 v = __half22float2(feat[q]);
+                        f[q] = PREC == 0 ? *reinterpret_cast<const uint32_t *>(&feat[q]) : T16::pack(v.x, v.y);
+                    }
+                    bt_st(S.F[bb], row, c, 32, make_uint4(f[0], f[1], f[2], f[3]));
                 }
-#pragma unroll
-                for (int c = 0; c < BT_NL / 4; ++c)
-                    bt_st(S.F[bb], row, l0 / 4 + c, 32, make_uint4(f[4 * c], f[4 * c + 1], f[4 * c + 2], f[4 * c + 3]));
                 if (lead) {
                     uint32_t sv[8];
 #pragma unroll
@@ -823,15 +784,21 @@ __global__ void __launch_bounds__(BT_THREADS, 2) wf_net_bwd_tc_kernel(RenderPara
                 bt_wait_on(&S.df_full, (uint32_t)((i - 1) & 1), ok);
                 ok = __all_sync(FULLMASK, ok); /* the TMEM load and the scatter's shuffles take whole warps */
                 if (!ok) break;
-                float dF[2 * BT_NL];
-                tmem_ld_n(lrow + BT_DF + 2 * l0, dF);
-                tmem_wait_ld();
-                tc_fence_before();
-                mbar_arrive(&S.df_empty);
-                if (r_prev < 0)
+#pragma unroll 1
+                for (int l = l0; l < l0 + BT_NL; l += SC_GROUP) {
+                    float dF[2 * SC_GROUP];
+                    __syncwarp();
+                    tmem_ld2(lrow + BT_DF + 2 * l, dF);
+                    tmem_wait_ld();
+                    if (l + SC_GROUP >= l0 + BT_NL) {
+                        tc_fence_before();
+                        mbar_arrive(&S.df_empty);
+                    }
+                    if (r_prev < 0)
 #pragma unroll
-                    for (int q = 0; q < 2 * BT_NL; ++q) dF[q] = 0.f;
-                hash_scatter_levels<BT_NL>(p.grid, b.g_table, pos_prev, l0, dF, tid & 31);
+                        for (int q = 0; q < 2 * SC_GROUP; ++q) dF[q] = 0.f;
+                    hash_scatter_levels<SC_GROUP>(p.grid, b.g_table, pos_prev, l, dF, tid & 31);
+                }
             }
             r_prev = r;
             pos_prev = pos;
