@@ -1880,9 +1880,9 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
         if (build_by_tc(r, n_alive)) CU(launch_cache_density_tc(q, m->d_weights_tc, n_sms, s));
         else CU(launch_cache_density(q, n_sms * 8, s));
         pr_mark_kernel<<<n_sms * 16, 128, 0, s>>>(f, it);
-        pr_count_kernel<<<(int)((n_cols + 255) / 256), 256, 0, s>>>(f);
+        pr_count_kernel<<<(int)((n_cols + 7) / 8), 256, 0, s>>>(f); /* a warp per column */
         pr_scan_kernel<<<1, 1024, 0, s>>>(f);
-        pr_reserve_kernel<<<(int)((n_cols + 255) / 256), 256, 0, s>>>(f);
+        pr_reserve_kernel<<<(int)((n_cols + 7) / 8), 256, 0, s>>>(f);
         pr_zero_kernel<<<n_sms * 4, 256, 0, s>>>(f);
         pr_write_kernel<<<n_sms * 16, 128, 0, s>>>(f, it);
         CU(cudaGetLastError());
