@@ -1825,7 +1825,6 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
     if ((rc = setup_render_params(r, info, nullptr, nullptr, nullptr, p, true))) return rc;
     p.steps_per_iter = 1 << 26; /* sample_common_kernel marches until it has its samples */
     p.windows = 1;
-    p.march_lanes = 0;
     PerRayScratch &x = r->pr;
     const size_t n_bricks = (size_t)c->bX * c->bY * c->bZ, n_cols = (size_t)c->bX * c->bY, n_rows = (size_t)r->row_capacity;
     if (x.n_bricks < n_bricks || x.n_cols < n_cols || x.n_rows < n_rows) {
@@ -1874,8 +1873,10 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
         const int n_steps = std::min(8, std::max(1, (1 << 21) / n_alive)); /* TARGET_BATCH_SIZE / n_alive */
         p.batch_rows = n_steps * n_alive;                                   /* the march gives every ray n_steps rows */
         n_samples += ((long long)n_alive * n_steps + 255) / 256 * 256;     /* next_multiple(batch, 256) */
+        p.march_lanes = march_by_lanes(p, (size_t)n_alive);
+        p.by_sample = f.by_sample = !p.march_lanes && rows_by_sample(p);
         CU(cudaMemsetAsync(p.counters + 2, 0, sizeof(int), s));
-        CU(launch_fill_march(p, it, n_sms, s));
+        CU(launch_fill_march(p, it, n_alive, n_sms, s));
         q.dir_states = p.states[it & 1];
         if (build_by_tc(r, n_alive)) CU(launch_cache_density_tc(q, m->d_weights_tc, n_sms, s));
         else CU(launch_cache_density(q, n_sms * 8, s));

@@ -2710,9 +2710,9 @@ cudaError_t launch_fill_raygen(const RenderParams &p, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t launch_fill_march(const RenderParams &p, int it, int n_sms, cudaStream_t s)
+cudaError_t launch_fill_march(const RenderParams &p, int it, int n_rays, int n_sms, cudaStream_t s)
 {
-    wf_march_kernel<false><<<ray_grid(p.cam.W * p.cam.H, n_sms), 128, 0, s>>>(p, it);
+    launch_march<false, false>(p, it, n_rays, n_sms, s);
     return cudaGetLastError();
 }
 
