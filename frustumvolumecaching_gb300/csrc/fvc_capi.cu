@@ -1181,6 +1181,17 @@ static int march_windows(size_t n_rays)
     return (int)std::min<size_t>(MAX_WINDOWS, std::max<size_t>(1, FVC_WINDOW_RAYS / n_rays));
 }
 
+/* As the rays of a frame end, its sub-iterations march more windows each, up to
+ * this many rays' worth (SubIter, fvc_kernels.h): fewer of the last ones, which
+ * cost their launches only.  Measured (us) with none / 2^16 / 2^17 / 2^18 /
+ * 2^19 / 2^20: opaque 800x800 frame 10070 / 9804 / 9786 / 9848 / 10129 / 10330,
+ * per-ray cached 640x360 4398 / 4178 / 4205 / 4166 / 4303 / 4330, cached 1080p
+ * 54660 / 54143 / 54129 / 54150 / 54089 / -, plain 1080p and the batch within
+ * 1 %.  Above 2^18 the windows that opaque rays march too far cost more. */
+#ifndef FVC_GROWN_RAYS
+#define FVC_GROWN_RAYS (1 << 18)
+#endif
+
 /* buffers of `cap` sample rows and `windows` per-ray window entries, in place of the renderer's smaller ones */
 static int alloc_rows(fvc_renderer *r, size_t cap, size_t windows)
 {
@@ -1393,10 +1404,13 @@ static int setup_render_params(fvc_renderer *r, const fvc_raymarch_info *info, f
     p.skip_empty = r->skip_empty;
     /* a set compaction batch or march length is one window's */
     p.batch_rows = r->row_target > 0 ? std::min(r->row_target, r->batch_rows) : r->batch_rows;
-    p.windows = r->row_target > 0 || r->steps_per_iter != MARCH_STEPS ? 1 : r->windows;
+    const bool one_window = r->row_target > 0 || r->steps_per_iter != MARCH_STEPS;
+    p.windows = one_window ? 1 : r->windows;
+    p.window_rays = one_window ? 0 : (int)std::min({(size_t)FVC_GROWN_RAYS, r->ray_rows_cap, (size_t)r->row_capacity / 16});
     p.ray_stride = r->ray_stride;
     p.row_capacity = r->row_capacity;
     p.march_lanes = march_by_lanes(p, (size_t)r->W * r->H);
+    p.lanes_rays = march_by_lanes(p, 0) ? FVC_LANES_RAYS : 0;
     p.by_sample = !p.march_lanes && rows_by_sample(p);
     return FVC_OK;
 }
@@ -1825,6 +1839,7 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
     if ((rc = setup_render_params(r, info, nullptr, nullptr, nullptr, p, true))) return rc;
     p.steps_per_iter = 1 << 26; /* sample_common_kernel marches until it has its samples */
     p.windows = 1;
+    p.window_rays = 0;
     PerRayScratch &x = r->pr;
     const size_t n_bricks = (size_t)c->bX * c->bY * c->bZ, n_cols = (size_t)c->bX * c->bY, n_rows = (size_t)r->row_capacity;
     if (x.n_bricks < n_bricks || x.n_cols < n_cols || x.n_rows < n_rows) {
@@ -2231,9 +2246,11 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
     if ((rc = setup_render_params(r, info, r->d_results, nullptr, nullptr, p))) return rc;
     p.pixel_list = pixels;
     p.n_list = n_rays;
+    p.lanes_rays = 0; /* both passes march alike */
     p.by_sample = 0; /* the warp's rays are any pixels of the list: only a ray's own samples are close together */
     if (whole) {
         p.windows = ray_windows;
+        p.window_rays = 0;
         p.ray_stride = n_rays;
     }
     p.list_order = r->d_list_order;

@@ -336,6 +336,8 @@ struct RenderParams {
     int2 *ray_rows;             /* [windows][ray_stride] per alive ray: first row of its warp, window_pack of its share */
     int windows;                /* march windows (steps_per_iter steps, at most S_ROWS samples) of a sub-iteration */
     int ray_stride;
+    int window_rays;            /* 0: `windows` windows in every sub-iteration; else more once the rays are fewer (SubIter) */
+    int lanes_rays;             /* a frame's sub-iterations of no more rays march by lanes (march_by_lanes, fvc_capi.cu) */
     int row_capacity;           /* rows of the buffers: a warp whose window does not fit marches it in the next sub-iteration */
     int batch_rows;             /* rows a window aims at over all rays: samples per ray and window = clamp(batch_rows /
                                  * alive rays, 1, S_ROWS) */
@@ -497,6 +499,23 @@ struct LaunchLog {
     int n_timed = 0;
     int n_untimed = 0;
     int split = -1;  /* fvc_render_backward: timed launches before this index are the forward pass's */
+};
+
+/* The march windows of a sub-iteration of n_alive rays, and the distance of
+ * their entries in ray_rows.  A sub-iteration's launches cost some 50 us however
+ * few rays are left, so the windows grow as the rays end, up to window_rays
+ * rays' worth (FVC_GROWN_RAYS, fvc_capi.cu); no more entries than ray_rows has,
+ * as they lie n_alive apart. */
+struct SubIter {
+    int windows, stride;
+    __host__ __device__ __forceinline__ SubIter(const RenderParams &p, int n_alive) : windows(p.windows), stride(p.ray_stride)
+    {
+        if (p.window_rays > 0 && n_alive > 0) {
+            const int more = p.window_rays / n_alive;
+            if (more > windows) windows = more < MAX_WINDOWS ? more : MAX_WINDOWS;
+            stride = n_alive;
+        }
+    }
 };
 
 /* The per-ray cache fill (CacheRenderer::initCache, src/cache_renderer.cu:

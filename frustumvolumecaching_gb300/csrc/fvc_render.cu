@@ -505,6 +505,7 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
     /* samples per ray and window: the batch over the alive rays, clamped to [1, S_ROWS] as
      * n_steps_curr_subiter of src/performance_renderer.cu:249 */
     const int S = max(1, min(S_ROWS, p.batch_rows / max(1, n_alive)));
+    const SubIter sub(p, n_alive);
     __shared__ float t0s[S_ROWS][128]; /* the thread's samples, a column each */
     RayState *states = p.states[it & 1];
     for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
@@ -517,7 +518,7 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
         }
         bool done = !valid;
         int all_steps = 0, all_rows = 0;
-        for (int w = 0; w < p.windows; ++w) {
+        for (int w = 0; w < sub.windows; ++w) {
             int n = 0, steps = 0;
             const float t_window = dt4.w;
             const bool done_before = done;
@@ -586,7 +587,7 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
             }
             rbase = __shfl_sync(FULLMASK, rbase, 0);
             if (rbase < 0) { /* the rays wait at this window's start for the next sub-iteration */
-                if (!done_before) p.ray_rows[(size_t)w * p.ray_stride + i] = make_int2(0, window_pack(0, 0, false));
+                if (!done_before) p.ray_rows[(size_t)w * sub.stride + i] = make_int2(0, window_pack(0, 0, false));
                 dt4.w = t_window;
                 break;
             }
@@ -643,7 +644,7 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
                                          make_float3(0.f, 0.f, 0.f), make_float3(0.f, 0.f, 0.f), t0, r);
                 }
             }
-            if (valid) p.ray_rows[(size_t)w * p.ray_stride + i] = make_int2(rbase, window_pack(n, steps, done));
+            if (valid) p.ray_rows[(size_t)w * sub.stride + i] = make_int2(rbase, window_pack(n, steps, done));
             all_steps += steps;
             all_rows += n;
             /* a warp whose rays have all ended leaves; the compositing stops at its rays' done flags too */
@@ -692,6 +693,7 @@ __global__ void __launch_bounds__(32 * ML_LANES) wf_march_lanes_kernel(RenderPar
         p.counters[6] = p.counters[7] = 0;
     }
     const int S = max(1, min(S_ROWS, p.batch_rows / max(1, n_alive)));
+    const SubIter sub(p, n_alive);
     RayState *states = p.states[it & 1];
     const int q = threadIdx.x / ML_LANES, l = threadIdx.x % ML_LANES, group = lane_id() & ~(ML_LANES - 1);
     for (int base = blockIdx.x * 32; base < n_alive; base += gridDim.x * 32) {
@@ -706,7 +708,7 @@ __global__ void __launch_bounds__(32 * ML_LANES) wf_march_lanes_kernel(RenderPar
         float t1 = dt4.w;
         bool done = !valid;
         int all_steps = 0, all_rows = 0;
-        for (int w = 0; w < p.windows; ++w) {
+        for (int w = 0; w < sub.windows; ++w) {
             int n = 0, steps = 0;
             const float t_window = t1;
             const bool done_before = done;
@@ -769,7 +771,7 @@ __global__ void __launch_bounds__(32 * ML_LANES) wf_march_lanes_kernel(RenderPar
             __syncthreads();
             const int first = s_first, row = s_row[q];
             if (first < 0) { /* no room: the rays wait at this window's start for the next sub-iteration */
-                if (l == 0 && !done_before) p.ray_rows[(size_t)w * p.ray_stride + i] = make_int2(0, window_pack(0, 0, false));
+                if (l == 0 && !done_before) p.ray_rows[(size_t)w * sub.stride + i] = make_int2(0, window_pack(0, 0, false));
                 t1 = t_window;
                 break;
             }
@@ -801,7 +803,7 @@ __global__ void __launch_bounds__(32 * ML_LANES) wf_march_lanes_kernel(RenderPar
                     else if (kind == KIND_CACHE) p.cache_list[hb + __popc(m1 & lane_lt())] = r;
                 }
             }
-            if (l == 0 && valid) p.ray_rows[(size_t)w * p.ray_stride + i] = make_int2(first, window_pack(n, steps, done));
+            if (l == 0 && valid) p.ray_rows[(size_t)w * sub.stride + i] = make_int2(first, window_pack(n, steps, done));
             all_steps += steps;
             all_rows += n;
             if (__syncthreads_and(done)) break; /* also: the shared rows are read before the next window's */
@@ -2065,6 +2067,7 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
     const int n_alive = p.counters[it & 1];
     if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p, CACHED);
     RayState *cur = p.states[it & 1], *nxt = p.states[(it + 1) & 1];
+    const SubIter sub(p, n_alive);
     for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
         const int i = base + threadIdx.x;
         const bool valid = i < n_alive;
@@ -2086,10 +2089,10 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
         float w_res = 0.f, w_cache = 0.f; /* this sub-iteration's contribution weights (DEBUG form, :867-871) */
         bool term = false, done = !valid; /* ended by opacity; the march passed the far bound */
         bool more_windows = true;
-        for (int w = 0; w < p.windows; ++w) {
+        for (int w = 0; w < sub.windows; ++w) {
             int2 rr = make_int2(0, 0);
             if (!done) { /* also of a ray that has ended: the others' rows follow its own */
-                rr = p.ray_rows[(size_t)w * p.ray_stride + i];
+                rr = p.ray_rows[(size_t)w * sub.stride + i];
                 if (!term) c_steps += window_steps(rr.y);
                 done = window_done(rr.y);
                 more_windows = !window_none(rr.y);
@@ -2204,6 +2207,7 @@ __global__ void __launch_bounds__(COMP_THREADS) wf_composite_bwd_kernel(RenderPa
     const int n_alive = p.counters[it & 1];
     if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p, CACHED);
     RayState *cur = p.states[it & 1], *nxt = p.states[(it + 1) & 1];
+    const SubIter sub(p, n_alive);
     for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
         const int i = base + threadIdx.x;
         const bool valid = i < n_alive;
@@ -2218,11 +2222,11 @@ __global__ void __launch_bounds__(COMP_THREADS) wf_composite_bwd_kernel(RenderPa
             xp = st.acc.x;
         }
         bool term = false, done = !valid, more_windows = true;
-        for (int w = 0; w < p.windows; ++w) {
+        for (int w = 0; w < sub.windows; ++w) {
             int n_res = 0, n_cch = 0;
             int2 rr = make_int2(0, 0);
             if (!done) { /* also of a ray that has ended: the others' rows follow its own */
-                rr = p.ray_rows[(size_t)w * p.ray_stride + i];
+                rr = p.ray_rows[(size_t)w * sub.stride + i];
                 done = window_done(rr.y);
                 more_windows = !window_none(rr.y);
             }
@@ -2588,16 +2592,17 @@ static void launch_march(const RenderParams &p, int it, int n_rays, int n_sms, c
 }
 
 /* sub-iterations between two readbacks of the alive count: with more march windows a sub-iteration there are fewer */
-static inline int check_interval(const RenderParams &p, int every) { return p.windows >= 8 ? 1 : p.windows > 1 ? std::min(every, 2) : every; }
+static inline int check_interval(int windows, int every) { return windows >= 8 ? 1 : windows > 1 ? std::min(every, 2) : every; }
 
 template <bool CACHED, int HH>
-static cudaError_t run_frame(const RenderParams &p, int n_sms, cudaStream_t s, int *h_pinned, int check_every, int *n_iter,
+static cudaError_t run_frame(const RenderParams &params, int n_sms, cudaStream_t s, int *h_pinned, int check_every, int *n_iter,
                              LaunchLog *log)
 {
     {
         cudaError_t e = ensure_net_attrs<HH>();
         if (e != cudaSuccess) return e;
     }
+    RenderParams p = params;
     LaunchLog local;
     LaunchLog &L = log ? *log : local;
     auto timed_begin = [&]() {
@@ -2612,8 +2617,8 @@ static cudaError_t run_frame(const RenderParams &p, int n_sms, cudaStream_t s, i
     if (p.pixel_list) wf_raygen_list_kernel<<<(p.n_list + 255) / 256, 256, 0, s>>>(p);
     else wf_raygen_kernel<<<(n_threads + 255) / 256, 256, 0, s>>>(p);
     ++L.launches;
-    const int n_rays = p.pixel_list ? p.n_list : W * H, grid_ray = ray_grid(n_rays, n_sms);
-    check_every = check_interval(p, check_every);
+    int n_rays = p.pixel_list ? p.n_list : W * H; /* as of the last readback */
+    int next_check = check_interval(SubIter(p, n_rays).windows, check_every);
     const int grid_net = n_sms * 2;
     const size_t net_smem = sizeof(NetSmem);
     const bool fused = CACHED && fused_cached_path(p);
@@ -2648,14 +2653,20 @@ static cudaError_t run_frame(const RenderParams &p, int n_sms, cudaStream_t s, i
             timed_end();
             L.launches += 1;
         }
-        wf_composite_kernel<CACHED><<<grid_ray, 128, 0, s>>>(p, it);
+        wf_composite_kernel<CACHED><<<ray_grid(n_rays, n_sms), 128, 0, s>>>(p, it);
         L.launches += 1;
-        if ((it + 1) % check_every == 0) {
+        if (it + 1 == next_check) {
             cudaError_t e = cudaMemcpyAsync(h_pinned, p.counters + ((it + 1) & 1), sizeof(int), cudaMemcpyDeviceToHost, s);
             if (e != cudaSuccess) return e;
             e = cudaStreamSynchronize(s);
             if (e != cudaSuccess) return e;
-            if (*h_pinned == 0) { ++it; break; }
+            n_rays = *h_pinned;
+            if (n_rays == 0) { ++it; break; }
+            next_check += check_interval(SubIter(p, n_rays).windows, check_every);
+            if (n_rays <= p.lanes_rays) {
+                p.march_lanes = 1;
+                p.by_sample = 0;
+            }
         }
     }
     if (n_iter) *n_iter = it;
@@ -2740,7 +2751,7 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
         else if (L.ev) ++L.n_untimed;
     };
     const int grid_comp = ray_grid(p.n_list, n_sms, COMP_THREADS);
-    check_every = check_interval(p, check_every);
+    check_every = check_interval(p.windows, check_every);
     for (int it = 0; it < (1 << 20); ++it) {
         if (!one_round) launch_march<CACHED, false>(p, it, p.n_list, n_sms, s);
         /* the forward kernels of pass 1, so both passes composite the same values */
