@@ -300,7 +300,21 @@ void dfree(T *&p)
 /* ------------------------------------------------------------------------ */
 /* handles                                                                   */
 /* ------------------------------------------------------------------------ */
+/* The device copies of a network query's inputs and outputs, kept by the model
+ * up to KEEP floats.  An allocation and a release for each of the three cost
+ * more than the network itself (2^19 points: 780 us a call, of it 201 in the
+ * kernel, now 500; 10^4 points 190, now 59).  A query that finds it in use by
+ * another thread, or needs more, has a buffer of its own. */
+struct QueryScratch {
+    static constexpr size_t KEEP = (size_t)1 << 24;
+    std::mutex mutex;
+    float *d = nullptr;
+    size_t cap = 0;
+    ~QueryScratch() { dfree(d); }
+};
+
 struct fvc_model {
+    QueryScratch query;
     int device = 0, n_sms = 0;
     fvc_scene_info scene{};
     fvc_stepsize_info steps{};
@@ -1080,16 +1094,34 @@ static int run_inference(fvc_model *m, const float *pos, const float *dir, int n
     if (m->freq && dir) return fail(FVC_ERR_CONFIG, "network inference evaluates heads without the frequency encoding");
     if (n == 0) return FVC_OK;
     float *dp = nullptr, *dd = nullptr, *d4 = nullptr, *db = nullptr, *df = nullptr;
-    int rc = FVC_OK;
+    struct Part { float **p; size_t floats; } parts[] = {{&dp, 3}, {&dd, dir ? 3u : 0u}, {&d4, out4 ? 4u : 0u}, {&db, base_out ? 16u : 0u},
+                                                         {&df, features ? 32u : 0u}};
+    size_t total = 0;
+    for (const Part &q : parts) total += (q.floats * n + 63) / 64 * 64; /* each from a multiple of 256 bytes, as its own allocation had */
+    float *own = nullptr, *buf = nullptr;
     struct Guard {
-        float **p[5];
-        ~Guard() { for (auto q : p) dfree(*q); }
-    } guard{{&dp, &dd, &d4, &db, &df}};
-    if ((rc = dalloc(&dp, (size_t)3 * n, "inference input"))) return rc;
-    if (dir && (rc = dalloc(&dd, (size_t)3 * n, "inference dir"))) return rc;
-    if (out4 && (rc = dalloc(&d4, (size_t)4 * n, "inference out"))) return rc;
-    if (base_out && (rc = dalloc(&db, (size_t)16 * n, "inference base"))) return rc;
-    if (features && (rc = dalloc(&df, (size_t)32 * n, "inference features"))) return rc;
+        float **p;
+        ~Guard() { dfree(*p); }
+    } guard{&own};
+    std::unique_lock<std::mutex> lk(m->query.mutex, std::try_to_lock);
+    int rc = FVC_OK;
+    if (lk.owns_lock() && total <= QueryScratch::KEEP) {
+        if (total > m->query.cap) {
+            dfree(m->query.d);
+            m->query.cap = 0;
+            if ((rc = dalloc(&m->query.d, total, "inference buffers"))) return rc;
+            m->query.cap = total;
+        }
+        buf = m->query.d;
+    } else {
+        if ((rc = dalloc(&own, total, "inference buffers"))) return rc;
+        buf = own;
+    }
+    for (const Part &q : parts)
+        if (q.floats) {
+            *q.p = buf;
+            buf += (q.floats * n + 63) / 64 * 64;
+        }
     CU(cudaMemcpy(dp, pos, sizeof(float) * 3 * n, cudaMemcpyHostToDevice));
     if (dir) CU(cudaMemcpy(dd, dir, sizeof(float) * 3 * n, cudaMemcpyHostToDevice));
     InferenceParams p;
