@@ -1813,11 +1813,11 @@ extern "C" int fvc_cache_build(fvc_renderer *r, const fvc_raymarch_info *info)
         if (build_by_tc(r, (long long)n_alive * 64)) CU(launch_cache_density_tc(p, m->d_weights_tc, m->n_sms, s));
         else CU(launch_cache_density(p, m->n_sms * 8, s));
         CU(cudaGetLastError());
-        cache_composite_kernel<<<std::min((n_alive + 3) / 4, 1 << 16), 128, 0, s>>>(p);
+        launch_after(cache_composite_kernel, std::min((n_alive + 3) / 4, 1 << 16), 128, 0, s, p);
         CU(cudaGetLastError());
-        cache_assign_kernel<<<1, 1024, 0, s>>>(p);
+        launch_after(cache_assign_kernel, 1, 1024, 0, s, p);
         CU(cudaGetLastError());
-        cache_fill_kernel<<<std::min(n_alive, 8 * m->n_sms), 256, 0, s>>>(p);
+        launch_after(cache_fill_kernel, std::min(n_alive, 8 * m->n_sms), 256, 0, s, p);
         CU(cudaGetLastError());
         n_launches += 5;
         std::swap(p.alive_list, p.alive_list_next);
@@ -1927,12 +1927,12 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
         q.dir_states = p.states[it & 1];
         if (build_by_tc(r, n_alive)) CU(launch_cache_density_tc(q, m->d_weights_tc, n_sms, s));
         else CU(launch_cache_density(q, n_sms * 8, s));
-        pr_mark_kernel<<<n_sms * 16, 128, 0, s>>>(f, it);
-        pr_count_kernel<<<(int)((n_cols + 7) / 8), 256, 0, s>>>(f); /* a warp per column */
-        pr_scan_kernel<<<1, 1024, 0, s>>>(f);
-        pr_reserve_kernel<<<(int)((n_cols + 7) / 8), 256, 0, s>>>(f);
-        pr_zero_kernel<<<n_sms * 4, 256, 0, s>>>(f);
-        pr_write_kernel<<<n_sms * 16, 128, 0, s>>>(f, it);
+        launch_after(pr_mark_kernel, n_sms * 16, 128, 0, s, f, it);
+        launch_after(pr_count_kernel, (int)((n_cols + 7) / 8), 256, 0, s, f); /* a warp per column */
+        launch_after(pr_scan_kernel, 1, 1024, 0, s, f);
+        launch_after(pr_reserve_kernel, (int)((n_cols + 7) / 8), 256, 0, s, f);
+        launch_after(pr_zero_kernel, n_sms * 4, 256, 0, s, f);
+        launch_after(pr_write_kernel, n_sms * 16, 128, 0, s, f, it);
         CU(cudaGetLastError());
         n_launches += 8;
         CU(cudaMemcpyAsync(r->h_pinned, p.counters + ((it + 1) & 1), sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -305,6 +305,16 @@ __device__ __forceinline__ bool occupied(const DevScene &sc, const uint8_t *__re
     return (__ldg(bits + bidx) >> (idx & 7u)) & 1u;
 }
 
+/* First statement of a kernel that launch_after() may launch before the kernel
+ * in front of it on the stream has ended: waits until that one's writes can be
+ * read.  It is the first statement of every thread, so that a kernel has not
+ * ended while the one before it has not.  A kernel launched plainly passes at
+ * once. */
+__device__ __forceinline__ void after_previous()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 /* The occupancy cells again, as the march reads them: 32-bit words of 4 x 4 x 2
  * cells (bit x & 3 | (y & 3) << 2 | (z & 1) << 4), words x fastest, then y, then
  * z, cascade by cascade; filled from the Morton bits' source when a model is

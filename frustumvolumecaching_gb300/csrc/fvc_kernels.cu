@@ -146,6 +146,7 @@ constexpr int SEARCH_GROUPS = 8;
 template <bool VD, int G>
 __global__ void __launch_bounds__(64 * G, G == 1 ? 16 : 2) cache_search_kernel(CacheBuildParams p)
 {
+    after_previous();
     __shared__ uint8_t s_flags[2][2 * G]; /* per warp: 1 an occupied sample, 2 a ray alive past the brick */
     __shared__ int2 red[2];
     __shared__ int row_base;
@@ -247,6 +248,7 @@ __global__ void __launch_bounds__(64 * G, G == 1 ? 16 : 2) cache_search_kernel(C
 template <bool VD>
 __global__ void __launch_bounds__(128) cache_density_kernel(CacheBuildParams p)
 {
+    after_previous();
     __shared__ uint2 Wsm[W_L3], Wfh[VD ? W_L3 : 1];
     __shared__ __align__(16) __half tiles[4][32 * TILE_STRIDE];
     const int n = *p.build_row_counter;
@@ -322,19 +324,16 @@ __global__ void __launch_bounds__(128) cache_density_kernel(CacheBuildParams p)
 cudaError_t launch_cache_search(const CacheBuildParams &p, int grid, cudaStream_t s)
 {
     if (grid <= FVC_SEARCH_TILES) {
-        if (p.view_dependent) cache_search_kernel<true, SEARCH_GROUPS><<<grid, 64 * SEARCH_GROUPS, 0, s>>>(p);
-        else cache_search_kernel<false, SEARCH_GROUPS><<<grid, 64 * SEARCH_GROUPS, 0, s>>>(p);
+        launch_after(p.view_dependent ? cache_search_kernel<true, SEARCH_GROUPS> : cache_search_kernel<false, SEARCH_GROUPS>, grid, 64 * SEARCH_GROUPS, 0, s, p);
     } else {
-        if (p.view_dependent) cache_search_kernel<true, 1><<<grid, 64, 0, s>>>(p);
-        else cache_search_kernel<false, 1><<<grid, 64, 0, s>>>(p);
+        launch_after(p.view_dependent ? cache_search_kernel<true, 1> : cache_search_kernel<false, 1>, grid, 64, 0, s, p);
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_cache_density(const CacheBuildParams &p, int grid, cudaStream_t s)
 {
-    if (p.view_dependent) cache_density_kernel<true><<<grid, 128, 0, s>>>(p);
-    else cache_density_kernel<false><<<grid, 128, 0, s>>>(p);
+    launch_after(p.view_dependent ? cache_density_kernel<true> : cache_density_kernel<false>, grid, 128, 0, s, p);
     return cudaGetLastError();
 }
 
@@ -344,6 +343,7 @@ cudaError_t launch_cache_density(const CacheBuildParams &p, int grid, cudaStream
  * needs a slot (a visible sample). */
 __global__ void __launch_bounds__(128) cache_composite_kernel(CacheBuildParams p)
 {
+    after_previous();
     const int lane = threadIdx.x & 31;
     const int n_alive_tiles = *p.n_alive_tiles;
     const int n_warps = gridDim.x * (blockDim.x >> 5);
@@ -476,6 +476,7 @@ __device__ __forceinline__ unsigned long long block_exclusive_scan64(unsigned lo
 
 __global__ void __launch_bounds__(1024) cache_assign_kernel(CacheBuildParams p)
 {
+    after_previous();
     __shared__ unsigned long long s_w[33];
     const int n = *p.n_alive_tiles;
     int slot0 = *p.slot_counter, jobs0 = 0, alive0 = 0; /* the same in every thread */
@@ -563,6 +564,7 @@ __global__ void __launch_bounds__(1024) cache_assign_kernel(CacheBuildParams p)
  * cache_assign_kernel, which advanced the tile's block step past the brick. */
 __global__ void __launch_bounds__(256) cache_fill_kernel(CacheBuildParams p)
 {
+    after_previous();
     __shared__ float s_dt[8];
     const int n_jobs = *p.n_jobs;
     const bool by_alpha = p.variant == VARIANT_ALPHA || p.variant == VARIANT_ALPHA_INTERMEDIATES;
@@ -664,6 +666,7 @@ __device__ __forceinline__ int pr_brick(const PerRayFillParams &p, int id, float
  * below 1e-4 (unclamped density) */
 __global__ void __launch_bounds__(128) pr_mark_kernel(PerRayFillParams p, int it)
 {
+    after_previous();
     const int n_alive = p.counters[it & 1];
     const RayState *states = p.states[it & 1];
     for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
@@ -704,6 +707,7 @@ __global__ void __launch_bounds__(128) pr_mark_kernel(PerRayFillParams p, int it
  * reservation below; 4 and 14 now). */
 __global__ void __launch_bounds__(256) pr_count_kernel(PerRayFillParams p)
 {
+    after_previous();
     const int n_cols = p.bX * p.bY, lane = threadIdx.x & 31;
     const size_t plane = (size_t)n_cols;
     const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -720,6 +724,7 @@ __global__ void __launch_bounds__(256) pr_count_kernel(PerRayFillParams p)
 /* exclusive scan of the column counts from the slot counter (one CTA of 1024) */
 __global__ void __launch_bounds__(1024) pr_scan_kernel(PerRayFillParams p)
 {
+    after_previous();
     __shared__ int s_w[33];
     __shared__ int s_carry;
     const int n_cols = p.bX * p.bY;
@@ -746,6 +751,7 @@ __global__ void __launch_bounds__(1024) pr_scan_kernel(PerRayFillParams p)
  * marks for the next sub-iteration */
 __global__ void __launch_bounds__(256) pr_reserve_kernel(PerRayFillParams p)
 {
+    after_previous();
     const int n_cols = p.bX * p.bY, lane = threadIdx.x & 31;
     const size_t plane = (size_t)n_cols;
     const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -781,6 +787,7 @@ __global__ void __launch_bounds__(256) pr_reserve_kernel(PerRayFillParams p)
  * setDataArraysZero, src/cache_renderer.cu:854) */
 __global__ void __launch_bounds__(256) pr_zero_kernel(PerRayFillParams p)
 {
+    after_previous();
     const int s0 = min(p.slot_counter[1], p.capacity), s1 = min(p.slot_counter[0], p.capacity);
     uint4 *v = reinterpret_cast<uint4 *>(p.voxels);
     const size_t n = (size_t)(s1 - s0) * 1024;
@@ -798,6 +805,7 @@ __global__ void __launch_bounds__(256) pr_zero_kernel(PerRayFillParams p)
  * into the next alive list. */
 __global__ void __launch_bounds__(128) pr_write_kernel(PerRayFillParams p, int it)
 {
+    after_previous();
     const int n_alive = p.counters[it & 1];
     RayState *states = p.states[it & 1];
     RayState *next = p.states[(it + 1) & 1];

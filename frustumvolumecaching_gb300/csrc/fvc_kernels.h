@@ -233,6 +233,30 @@ __device__ __forceinline__ int lanes_before(int n)
     return sum - n;
 }
 
+/* Launches a kernel that is set up while the kernel in front of it on the stream
+ * ends, and whose first statement is after_previous().  The short kernels of a
+ * build's or a frame's last rounds cost less than the gaps between them (us,
+ * plain launches / these / these with the blocks let in as soon as the kernel in
+ * front has started): cached 323x181 frame 3583 / 3328 / 3465, per-ray cached
+ * 640x360 4157 / 3960 / 4131, opaque 800x800 9848 / 9750 / 9786, plain 64x64
+ * 335 / 327 / 382 (waiting blocks hold registers and shared memory).  The
+ * batch's graph keeps plain launches: it places its kernels itself. */
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A &&...args)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute a = {};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 constexpr int MAX_WINDOWS = 31; /* march windows of a sub-iteration */
 
 /* A ray's share of one march window: its warp's first row and, packed, its

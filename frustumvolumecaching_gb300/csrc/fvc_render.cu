@@ -497,6 +497,7 @@ __device__ __forceinline__ int march_row(const RenderParams &p, const CacheView 
 template <bool CACHED, bool FUSED = false>
 __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
 {
+    after_previous();
     const int n_alive = p.counters[it & 1];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         p.counters[(it + 1) & 1] = 0;        /* next alive count */
@@ -685,6 +686,7 @@ __device__ __forceinline__ uint32_t spread8(uint32_t v)
 template <bool CACHED, bool FUSED>
 __global__ void __launch_bounds__(32 * ML_LANES) wf_march_lanes_kernel(RenderParams p, int it)
 {
+    after_previous();
     __shared__ float t0s[32][S_ROWS];
     __shared__ int s_n[32], s_row[32], s_first;
     const int n_alive = p.counters[it & 1];
@@ -971,6 +973,7 @@ __global__ void __launch_bounds__(256) wf_classify_kernel(RenderParams p, int it
  * row_out.y, which the network kernel's MODE 2 reads for a cache row. */
 __global__ void __launch_bounds__(256) wf_cache_lookup_kernel(RenderParams p, int it)
 {
+    after_previous();
     const int n_rows = p.counters[4];
     const RayState *states = p.states[it & 1];
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n_rows; k += gridDim.x * blockDim.x) {
@@ -1415,6 +1418,7 @@ struct NtRow {
 template <int MODE, int HH, bool LIST, bool GENERAL, int PREC = 0>
 __global__ void __launch_bounds__(NT_THREADS, 1) wf_net_tc_kernel(RenderParams p, int it)
 {
+    after_previous();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     NtSmem &S = *reinterpret_cast<NtSmem *>(smem_raw);
     const int n_rows = MODE == 0 ? (LIST ? p.counters[3] : p.counters[2]) : MODE == 1 ? p.counters[4] : p.counters[3];
@@ -1556,8 +1560,9 @@ template <int MODE, int HH, bool LIST, int PREC = 0>
 static void launch_net_tc(const RenderParams &p, int it, int n_sms, cudaStream_t s)
 {
     const size_t smem = nt_smem_bytes(p.freq);
-    if (p.freq || p.grid.F == 4) wf_net_tc_kernel<MODE, HH, LIST, true, PREC><<<n_sms, NT_THREADS, smem, s>>>(p, it);
-    else wf_net_tc_kernel<MODE, HH, LIST, false, PREC><<<n_sms, NT_THREADS, smem, s>>>(p, it);
+    auto kernel = p.freq || p.grid.F == 4 ? wf_net_tc_kernel<MODE, HH, LIST, true, PREC> : wf_net_tc_kernel<MODE, HH, LIST, false, PREC>;
+    if (p.views) kernel<<<n_sms, NT_THREADS, smem, s>>>(p, it);
+    else launch_after(kernel, n_sms, NT_THREADS, smem, s, p, it);
 }
 
 /* The cache build's density network (NerfNetwork::inferenceLatents on the
@@ -1568,6 +1573,7 @@ static void launch_net_tc(const RenderParams &p, int it, int n_sms, cudaStream_t
 template <bool GENERAL>
 __global__ void __launch_bounds__(NT_THREADS, 1) cache_density_tc_kernel(CacheBuildParams p, const uint8_t *weights_tc, const int *n_rows_ptr)
 {
+    after_previous();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     NtSmem &S = *reinterpret_cast<NtSmem *>(smem_raw);
     const int n_rows = *n_rows_ptr;
@@ -1645,8 +1651,8 @@ cudaError_t launch_cache_density_tc(const CacheBuildParams &p, const uint8_t *we
         return e;
     });
     if (e != cudaSuccess) return e;
-    if (p.grid.F == 4) cache_density_tc_kernel<true><<<n_sms, NT_THREADS, sizeof(NtSmem), s>>>(p, weights_tc, p.build_row_counter);
-    else cache_density_tc_kernel<false><<<n_sms, NT_THREADS, sizeof(NtSmem), s>>>(p, weights_tc, p.build_row_counter);
+    launch_after(p.grid.F == 4 ? cache_density_tc_kernel<true> : cache_density_tc_kernel<false>, n_sms, NT_THREADS, sizeof(NtSmem), s, p, weights_tc,
+                 p.build_row_counter);
     return cudaGetLastError();
 }
 
@@ -2063,6 +2069,7 @@ __device__ __forceinline__ void warp_rows(int2 rr, int &first, int &total)
 template <bool CACHED>
 __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int it)
 {
+    after_previous();
     constexpr int AHEAD = CACHED ? COMP_AHEAD_CACHED : COMP_AHEAD;
     const int n_alive = p.counters[it & 1];
     if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p, CACHED);
@@ -2587,8 +2594,10 @@ static inline int ray_grid(int n_rays, int n_sms, int threads = 128)
 template <bool CACHED, bool FUSED>
 static void launch_march(const RenderParams &p, int it, int n_rays, int n_sms, cudaStream_t s)
 {
-    if (p.march_lanes) wf_march_lanes_kernel<CACHED, FUSED><<<std::max(1, (n_rays + 31) / 32), 32 * ML_LANES, 0, s>>>(p, it);
-    else wf_march_kernel<CACHED, FUSED><<<ray_grid(n_rays, n_sms), 128, 0, s>>>(p, it);
+    auto kernel = p.march_lanes ? wf_march_lanes_kernel<CACHED, FUSED> : wf_march_kernel<CACHED, FUSED>;
+    const int grid = p.march_lanes ? std::max(1, (n_rays + 31) / 32) : ray_grid(n_rays, n_sms), block = p.march_lanes ? 32 * ML_LANES : 128;
+    if (p.views) kernel<<<grid, block, 0, s>>>(p, it);
+    else launch_after(kernel, grid, block, 0, s, p, it);
 }
 
 /* sub-iterations between two readbacks of the alive count: with more march windows a sub-iteration there are fewer */
@@ -2627,7 +2636,7 @@ static cudaError_t run_frame(const RenderParams &params, int n_sms, cudaStream_t
     for (; it < max_it; ++it) {
         if (fused) {
             launch_march<true, true>(p, it, n_rays, n_sms, s);
-            wf_cache_lookup_kernel<<<n_sms * 8, 256, 0, s>>>(p, it);
+            launch_after(wf_cache_lookup_kernel, n_sms * 8, 256, 0, s, p, it);
             timed_begin();
             launch_net_tc<2, HH, false>(p, it, n_sms, s);
             timed_end();
@@ -2653,7 +2662,7 @@ static cudaError_t run_frame(const RenderParams &params, int n_sms, cudaStream_t
             timed_end();
             L.launches += 1;
         }
-        wf_composite_kernel<CACHED><<<ray_grid(n_rays, n_sms), 128, 0, s>>>(p, it);
+        launch_after(wf_composite_kernel<CACHED>, ray_grid(n_rays, n_sms), 128, 0, s, p, it);
         L.launches += 1;
         if (it + 1 == next_check) {
             cudaError_t e = cudaMemcpyAsync(h_pinned, p.counters + ((it + 1) & 1), sizeof(int), cudaMemcpyDeviceToHost, s);
