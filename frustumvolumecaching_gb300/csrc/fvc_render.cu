@@ -2194,6 +2194,122 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
     }
 }
 
+/* The plain compositing of few rays (where 8 lanes march a ray), a block for
+ * the 32 rays of a march block.  A lane that composites its ray alone goes
+ * through some 120 dependent instructions a sample, five exponentials and three
+ * divisions among them, with one warp on a scheduler.  Here the block's 8 warps
+ * take the exponentials of a window's rows, one warp walks the transmittances,
+ * the 8 warps divide, and a warp a channel adds up: the walks keep one product
+ * and one compensated sum a sample.  Every value is that of the other kernel,
+ * from the same operations in the same order (4099 rays of a training step, 31
+ * windows: the step 1083 -> 1023 us; 64x64 frame 326 -> 270; launch_composite
+ * picks it). */
+constexpr int CL_WARPS = 8, CL_ROWS = 32 * S_ROWS + 2 * S_ROWS;
+
+__global__ void __launch_bounds__(32 * CL_WARPS) wf_composite_lanes_kernel(RenderParams p, int it)
+{
+    after_previous();
+    __shared__ float s_w[CL_ROWS], s_c[3][CL_ROWS]; /* a row's opacity, then its weight; its colour's divisors, then the colour */
+    __shared__ int s_used[32];
+    __shared__ float2 s_sum[3][32];
+    const int n_alive = p.counters[it & 1];
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p, false);
+    RayState *cur = p.states[it & 1], *nxt = p.states[(it + 1) & 1];
+    const SubIter sub(p, n_alive);
+    const int warp = threadIdx.x >> 5, lane = lane_id();
+    auto at_row = [](int k) { return k + (k >> 4); }; /* rays of 16 rows apart by an odd number of banks */
+    for (int base = blockIdx.x * 32; base < n_alive; base += gridDim.x * 32) {
+        const int i = base + lane;
+        const bool valid = i < n_alive;
+        float T = 1.f, sum = 0.f, comp = 0.f; /* warp 0: the transmittance; warps 0 to 2: a channel */
+        int c_steps = 0, n_comp = 0;
+        if (valid) {
+            const float4 a = cur[i].acc, c = cur[i].comp;
+            T = a.w;
+            sum = warp == 0 ? a.x : warp == 1 ? a.y : a.z;
+            comp = warp == 0 ? c.x : warp == 1 ? c.y : c.z;
+        }
+        bool term = false, done = !valid, more_windows = true;
+        for (int w = 0; w < sub.windows; ++w) {
+            int2 rr = make_int2(0, 0);
+            if (!done) {
+                rr = p.ray_rows[(size_t)w * sub.stride + i];
+                if (!term) c_steps += window_steps(rr.y);
+                done = window_done(rr.y);
+                more_windows = !window_none(rr.y);
+            }
+            int first, total;
+            warp_rows(rr, first, total);
+            const int n = window_rows(rr.y), before = lanes_before(n);
+            for (int k = threadIdx.x; k < total; k += 32 * CL_WARPS) {
+                const uint2 ov = p.row_out[first + k];
+                const float dt = calc_step(p.steps, p.row_t0[first + k]);
+                const float2 rg = __half22float2(*reinterpret_cast<const __half2 *>(&ov.x));
+                const float lb = __half2float(__ushort_as_half((unsigned short)(ov.y & 0xffffu)));
+                const float ld = __half2float(__ushort_as_half((unsigned short)(ov.y >> 16)));
+                const float sigma = expf(ld);
+                s_w[at_row(k)] = fminf(1.0f, fmaxf(0.0f, 1.0f - expf(-sigma * dt)));
+                s_c[0][at_row(k)] = 1.0f + expf(-rg.x);
+                s_c[1][at_row(k)] = 1.0f + expf(-rg.y);
+                s_c[2][at_row(k)] = 1.0f + expf(-lb);
+            }
+            __syncthreads();
+            if (warp == 0) {
+                int used = 0;
+                for (; used < n && !term; ++used) {
+                    float &a = s_w[at_row(before + used)];
+                    const float alpha = a;
+                    if (alpha > p.scene.alpha_thre) {
+                        a = alpha * T;
+                        T *= 1.0f - alpha;
+                    } else {
+                        a = -1.0f; /* not added */
+                    }
+                    if (T < 1e-4f) term = true;
+                }
+                n_comp += used;
+                s_used[lane] = used;
+            }
+            __syncthreads();
+            for (int k = threadIdx.x; k < total; k += 32 * CL_WARPS) {
+                const float wgt = s_w[at_row(k)];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) s_c[c][at_row(k)] = wgt / s_c[c][at_row(k)];
+            }
+            __syncthreads();
+            if (warp < 3)
+                for (int j = 0, used = s_used[lane]; j < used; ++j)
+                    if (!(s_w[at_row(before + j)] < 0.0f)) kahan_add(sum, comp, s_c[warp][at_row(before + j)]);
+            if (__syncthreads_and(warp != 0 || term || done || !more_windows)) break; /* the rows have been read */
+        }
+        if (warp < 3) s_sum[warp][lane] = make_float2(sum, comp);
+        __syncthreads();
+        if (warp == 0) {
+            bool keep = false;
+            RayState st;
+            if (valid) {
+                st = cur[i];
+                st.acc = make_float4(s_sum[0][lane].x, s_sum[1][lane].x, s_sum[2][lane].x, T);
+                st.comp.x = s_sum[0][lane].y;
+                st.comp.y = s_sum[1][lane].y;
+                st.comp.z = s_sum[2][lane].y;
+                st.cnt.y += n_comp;
+                st.cnt.w += c_steps;
+                if (term || done) write_pixel(p, st.cnt.x, st.acc, make_int4(st.cnt.y, st.cnt.z, st.cnt2.x, st.cnt.w));
+                else keep = true;
+            }
+            const int ws = __reduce_add_sync(FULLMASK, n_comp);
+            if (lane == 0 && ws) atomicAdd(&p.stats->n_samples, (unsigned long long)ws);
+            const unsigned m = __ballot_sync(FULLMASK, keep);
+            int nb = 0;
+            if (lane == 0 && m) nb = atomicAdd(p.counters + ((it + 1) & 1), __popc(m));
+            nb = __shfl_sync(FULLMASK, nb, 0);
+            if (keep) nxt[nb + __popc(m & lane_lt())] = st;
+        }
+        __syncthreads();
+    }
+}
+
 /* Adjoint of front-to-back compositing for this sub-iteration's rows (plain
  * path).  Per ray, in sample order, with g = dL/dC and X_total from the loss
  * kernel, X_prefix in acc.x and T in acc.w of the ray state:
@@ -2600,6 +2716,23 @@ static void launch_march(const RenderParams &p, int it, int n_rays, int n_sms, c
     else launch_after(kernel, grid, block, 0, s, p, it);
 }
 
+/* and its compositing: by blocks where they are few (wf_composite_lanes_kernel; us, a lane a ray / a block for 32 rays, the
+ * 256x256 workload's scene and an opaque unbounded one: 48x27 259 / 202 and 295 / 261, 64x64 308 / 257 and 370 / 333,
+ * 128x128 481 / 431 and 733 / 696, 160x160 616 / 594 and 999 / 978, 200x200 834 / 862 and 1364 / 1365, 256x256
+ * 1234 / 1326 and 1624 / 1668: with more rays every scheduler has warps enough, and the barriers cost) */
+#ifndef FVC_COMP_LANES_RAYS
+#define FVC_COMP_LANES_RAYS 32768
+#endif
+template <bool CACHED>
+static void launch_composite(const RenderParams &p, int it, int n_rays, int n_sms, cudaStream_t s)
+{
+    const bool lanes = !CACHED && p.march_lanes && n_rays <= FVC_COMP_LANES_RAYS;
+    auto kernel = lanes ? wf_composite_lanes_kernel : wf_composite_kernel<CACHED>;
+    const int grid = lanes ? std::max(1, (n_rays + 31) / 32) : ray_grid(n_rays, n_sms), block = lanes ? 32 * CL_WARPS : 128;
+    if (p.views) kernel<<<grid, block, 0, s>>>(p, it);
+    else launch_after(kernel, grid, block, 0, s, p, it);
+}
+
 /* sub-iterations between two readbacks of the alive count: with more march windows a sub-iteration there are fewer */
 static inline int check_interval(int windows, int every) { return windows >= 8 ? 1 : windows > 1 ? std::min(every, 2) : every; }
 
@@ -2662,7 +2795,7 @@ static cudaError_t run_frame(const RenderParams &params, int n_sms, cudaStream_t
             timed_end();
             L.launches += 1;
         }
-        launch_after(wf_composite_kernel<CACHED>, ray_grid(n_rays, n_sms), 128, 0, s, p, it);
+        launch_composite<CACHED>(p, it, n_rays, n_sms, s);
         L.launches += 1;
         if (it + 1 == next_check) {
             cudaError_t e = cudaMemcpyAsync(h_pinned, p.counters + ((it + 1) & 1), sizeof(int), cudaMemcpyDeviceToHost, s);
@@ -2857,7 +2990,6 @@ static cudaError_t build_batch_graph_t(const RenderParams &p, int n_sms, cudaStr
     int kernels = 1;
     if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        const int grid_ray = ray_grid(n_rays, n_sms);
         const bool fused = CACHED && fused_cached_path(p);
         for (int it = 0; it < 2; ++it) {
             if (fused) {
@@ -2885,7 +3017,7 @@ static cudaError_t build_batch_graph_t(const RenderParams &p, int n_sms, cudaStr
                 launch_plain_net<HH>(p, it, n_sms, s);
                 kernels += 1;
             }
-            wf_composite_kernel<CACHED><<<grid_ray, 128, 0, s>>>(p, it);
+            launch_composite<CACHED>(p, it, n_rays, n_sms, s);
             wf_reset_rows_kernel<<<1, 32, 0, s>>>(p, CACHED ? 1 : 0);
             kernels += 3;
         }
