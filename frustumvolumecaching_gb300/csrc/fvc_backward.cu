@@ -680,6 +680,20 @@ __device__ __forceinline__ void hash_scatter_levels(const DevGrid &g, float *gt,
     }
 }
 
+/* Tiles after which a CTA adds its weight gradients to the global blobs and
+ * starts from zero.  The tensor core truncates its sums, so they lose some 5e-7
+ * of their value a tile: summed over a launch of whole rays the weight
+ * gradients of 98305 rays were 1.1e-4 too small.  Relative error of them against
+ * steps of 2048 rays added up in float64, and the training step of 2^18 rays,
+ * with all tiles / 4 / 2 / 1: 4096 rays 4.4e-6 / 1.5e-6 / 8.9e-7 / 8.9e-7, 32768
+ * 4.1e-5 / 1.9e-6 / 1.6e-6 / 2.2e-6, 98305 1.1e-4 / 2.3e-6 / 2.7e-6 / 4.0e-6;
+ * 21.4 / 21.6 / 21.9 / 25.2 ms.  One launch per 64 marched steps, as it was
+ * before whole rays, had 9.1e-7, 2.4e-6 and 6.6e-6. */
+#ifndef FVC_BT_DW_TILES
+#define FVC_BT_DW_TILES 2
+#endif
+constexpr int BT_DW_TILES = FVC_BT_DW_TILES;
+
 /* 2 consecutive columns of this thread's TMEM lane */
 __device__ __forceinline__ void tmem_ld2(uint32_t taddr, float (&v)[2])
 {
@@ -811,7 +825,7 @@ __global__ void __launch_bounds__(BT_THREADS, 2) wf_net_bwd_tc_kernel(RenderPara
         phase ^= 1u;
         ok = bt_publish(ok); /* every decision to leave the loop is taken by all MMA threads together */
         uint8_t *last = HH == 2 ? S.A4 : S.A3;
-        bool acc = false; /* dW accumulators hold this launch's sums */
+        bool acc = false; /* dW accumulators hold the sums of the tiles since they were added to the blobs */
 #define BT_STAGE(...)                                   \
     if (tid == 0) {                                     \
         tc_fence_after();                               \
@@ -908,35 +922,37 @@ __global__ void __launch_bounds__(BT_THREADS, 2) wf_net_bwd_tc_kernel(RenderPara
             phase ^= 1u;
             acc = true;
             ok = bt_publish(ok);
+            /* the accumulators (TMEM lanes 0..63) into the global blobs, and from zero again; the next products wait
+             * for a bt_publish, which comes after these loads */
+            if ((i + 1) % BT_DW_TILES == 0 || i + 1 == n_mine) {
+                if (ok && warp < 2) {
+                    auto add_rows = [&](uint32_t col, float *dst, int width) { /* lane t = output o: dst[o * width + i] */
+#pragma unroll 1
+                        for (int c0 = 0; c0 < width; c0 += 16) {
+                            float v[16];
+                            tmem_ld16(lrow + col + c0, v);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int q = 0; q < 16; q += 4) red_add4(dst + tid * width + c0 + q, v[q], v[q + 1], v[q + 2], v[q + 3]);
+                        }
+                    };
+                    auto add_cols = [&](uint32_t col, float *dst) { /* lane t = input i: dst[o * 64 + i] */
+                        float v[16];
+                        tmem_ld16(lrow + col, v);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int o = 0; o < 16; ++o) atomicAdd(dst + o * 64 + tid, v[o]);
+                    };
+                    if (HH == 2) add_rows(BT_DW4, b.g_head + GH_W4, 64);
+                    add_rows(BT_DW3, b.g_head + GH_W3, 32);
+                    add_rows(BT_DW1, b.g_base + GB_W1, 32);
+                    add_cols(BT_DW5T, b.g_head + b.head_w5);
+                    add_cols(BT_DW2T, b.g_base + GB_W2);
+                }
+                acc = false;
+            }
         }
 #undef BT_STAGE
-        /* the CTA's weight gradients (TMEM lanes 0..63) into the global blobs */
-        if (ok && acc && warp < 2) {
-            float *gh = b.g_head, *gb = b.g_base;
-            auto add_rows = [&](uint32_t col, float *dst, int width) { /* lane t = output o: dst[o * width + i] */
-                for (int c0 = 0; c0 < width; c0 += 32) {
-                    float v[32];
-                    tmem_ld32(lrow + col + c0, v);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int q = 0; q < 32; ++q)
-                        if (v[q] != 0.f) atomicAdd(dst + tid * width + c0 + q, v[q]);
-                }
-            };
-            auto add_cols = [&](uint32_t col, float *dst) { /* lane t = input i: dst[o * 64 + i] */
-                float v[16];
-                tmem_ld16(lrow + col, v);
-                tmem_wait_ld();
-#pragma unroll
-                for (int o = 0; o < 16; ++o)
-                    if (v[o] != 0.f) atomicAdd(dst + o * 64 + tid, v[o]);
-            };
-            if (HH == 2) add_rows(BT_DW4, gh + GH_W4, 64);
-            add_rows(BT_DW3, gh + GH_W3, 32);
-            add_rows(BT_DW1, gb + GB_W1, 32);
-            add_cols(BT_DW5T, gh + b.head_w5);
-            add_cols(BT_DW2T, gb + GB_W2);
-        }
     }
     if (!ok) atomicOr(p.guard, 16);
     tc_fence_before();
