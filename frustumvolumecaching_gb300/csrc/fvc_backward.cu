@@ -680,19 +680,20 @@ __device__ __forceinline__ void hash_scatter_levels(const DevGrid &g, float *gt,
     }
 }
 
-/* Tiles after which a CTA adds its weight gradients to the global blobs and
- * starts from zero.  The tensor core truncates its sums, so they lose some 5e-7
- * of their value a tile: summed over a launch of whole rays the weight
- * gradients of 98305 rays were 1.1e-4 too small.  Relative error of them against
- * steps of 2048 rays added up in float64, and the training step of 2^18 rays,
- * with all tiles / 4 / 2 / 1: 4096 rays 4.4e-6 / 1.5e-6 / 8.9e-7 / 8.9e-7, 32768
- * 4.1e-5 / 1.9e-6 / 1.6e-6 / 2.2e-6, 98305 1.1e-4 / 2.3e-6 / 2.7e-6 / 4.0e-6;
- * 21.4 / 21.6 / 21.9 / 25.2 ms.  One launch per 64 marched steps, as it was
- * before whole rays, had 9.1e-7, 2.4e-6 and 6.6e-6. */
-#ifndef FVC_BT_DW_TILES
-#define FVC_BT_DW_TILES 2
+/* A CTA adds its weight gradients to the global blobs, and starts from zero,
+ * BT_DW_ADDS times, but not more often than every second tile.  The tensor
+ * core truncates its sums, so they lose some 5e-7 of their value a tile, and
+ * each addition to the blobs rounds.  Relative error of the weight gradients
+ * (head layers) against steps of 2048 rays added up in float64, with one
+ * addition a CTA / these / one launch per 64 marched steps (as before the rays
+ * marched whole): 4096 rays 4.4e-6 / 8.6e-7 / 8.9e-7, 32768 4.1e-5 / 1.7e-6 /
+ * 2.3e-6, 98305 1.1e-4 / 3.1e-6 / 6.6e-6, 2^18 - / 9.3e-6 / 2.0e-5.  The
+ * training step of 2^18 rays takes 21.4 ms with one, 21.6 with one every 4
+ * tiles, 21.9 every 2, 25.2 every tile. */
+#ifndef FVC_BT_DW_ADDS
+#define FVC_BT_DW_ADDS 32
 #endif
-constexpr int BT_DW_TILES = FVC_BT_DW_TILES;
+constexpr int BT_DW_ADDS = FVC_BT_DW_ADDS;
 
 /* 2 consecutive columns of this thread's TMEM lane */
 __device__ __forceinline__ void tmem_ld2(uint32_t taddr, float (&v)[2])
@@ -825,6 +826,8 @@ __global__ void __launch_bounds__(BT_THREADS, 2) wf_net_bwd_tc_kernel(RenderPara
         phase ^= 1u;
         ok = bt_publish(ok); /* every decision to leave the loop is taken by all MMA threads together */
         uint8_t *last = HH == 2 ? S.A4 : S.A3;
+        const int dw_tiles = max(2, n_mine / BT_DW_ADDS);
+        int dw_left = dw_tiles;
         bool acc = false; /* dW accumulators hold the sums of the tiles since they were added to the blobs */
 #define BT_STAGE(...)                                   \
     if (tid == 0) {                                     \
@@ -924,7 +927,7 @@ __global__ void __launch_bounds__(BT_THREADS, 2) wf_net_bwd_tc_kernel(RenderPara
             ok = bt_publish(ok);
             /* the accumulators (TMEM lanes 0..63) into the global blobs, and from zero again; the next products wait
              * for a bt_publish, which comes after these loads */
-            if ((i + 1) % BT_DW_TILES == 0 || i + 1 == n_mine) {
+            if (--dw_left == 0 || i + 1 == n_mine) {
                 if (ok && warp < 2) {
                     auto add_rows = [&](uint32_t col, float *dst, int width) { /* lane t = output o: dst[o * width + i] */
 #pragma unroll 1
@@ -950,6 +953,7 @@ __global__ void __launch_bounds__(BT_THREADS, 2) wf_net_bwd_tc_kernel(RenderPara
                     add_cols(BT_DW2T, b.g_base + GB_W2);
                 }
                 acc = false;
+                dw_left = dw_tiles;
             }
         }
 #undef BT_STAGE

@@ -7,17 +7,19 @@
  *   raygen      one thread per pixel: generateRay + AABB clip; rays that hit
  *               enter the alive list (initRayPayloads_split_kernel,
  *               src/renderer.cu:86-134), the others are written out white.
- *   march       one thread per alive ray: up to S occupied samples
- *               (S = clamp(capacity / alive, 1, 8) as the reference's
- *               n_steps), appended as compacted rows; in the cached render
- *               each sample is classified (resample / cache / known empty)
+ *   march       one thread per alive ray (8 lanes where rays are few): one
+ *               or more windows of up to 16 occupied samples (S =
+ *               clamp(batch / alive, 1, 16), the reference's n_steps),
+ *               appended as compacted rows; in the cached render each sample
+ *               is classified (resample / cache / known empty)
  *               (sample_performance_kernel :15-69,
  *               sample_cache_performance_kernel :22-177).
- *   net_*       one warp per 32 rows: hash grid + density net + color head
+ *   net_*       a thread per row, 128-row tiles: hash grid + density net + color head
  *               (resample rows) or trilinear cache lookup + color head (cache
  *               rows) on the tensor cores (NerfNetwork::inference /
  *               inferenceHead, generateNetworkInput_cache_shfl_perf_kernel_cg).
- *   composite   one thread per alive ray: the ray's rows merged by t0 and
+ *   composite   one thread per alive ray (a block for 32 rays where plain
+ *               rays are few): the ray's rows merged by t0 and
  *               composited front to back with early termination; finished
  *               rays are written out, the others compacted into the next
  *               alive list (accumulate_performance_kernel :71-125,
@@ -43,11 +45,12 @@ constexpr int S_ROWS = 16;        /* rows per ray and sub-iteration (the referen
 static_assert(S_ROWS * MAX_WINDOWS < 512, "the compositing kernel counts a ray's rows per miss reason in 9-bit fields");
 static_assert(S_ROWS < 32, "window_pack holds a window's rows in 5 bits");
 constexpr int NET_WARPS = 8;
-/* tcgen05 network kernel: CTAs resident per SM (launch bound and grid) and
- * hash levels whose gathers are in flight together.  Measured at 1080p on the
- * 3-cascade scene (resample-kernel ms per frame, plain / cached path):
- * 6 CTAs + groups of 2 (80 registers, spills) 37.2 / 34.5; 5 + 2: 30.0 / 22.5;
- * 5 + 4 (96 registers): 29.1 / 22.1; 4 + 4: 30.6 / 22.6. */
+/* The one-tile-a-CTA network kernels (64-row tiles, e4m3 layers, view-dependent
+ * models; the default's own constants are NT_*): CTAs resident per SM and hash
+ * levels whose gathers are in flight together.  Measured at 1080p on the
+ * 3-cascade scene with 128-row tiles (resample-kernel ms per frame, plain /
+ * cached path): 6 CTAs + groups of 2 (80 registers, spills) 37.2 / 34.5; 5 + 2:
+ * 30.0 / 22.5; 5 + 4 (96 registers): 29.1 / 22.1; 4 + 4: 30.6 / 22.6. */
 #ifndef FVC_TC_CTAS_PER_SM
 #define FVC_TC_CTAS_PER_SM 5
 #endif
@@ -1137,25 +1140,22 @@ __global__ void __launch_bounds__(NET_WARPS * 32, 2) wf_net_cache_kernel(RenderP
 /* ------------------------------------------------------------------------- */
 /* network over rows on the 5th-generation tensor cores                      */
 /* ------------------------------------------------------------------------- */
-/* One CTA of 128 threads per 128-row tile; thread t owns row t and TMEM lane
- * t.  The activations of a tile live in ONE shared-memory tile in the
- * canonical K-major layout that each layer overwrites in place (a layer's
- * epilogue runs only after its MMA has finished reading the tile); weights
- * stay resident in shared memory; accumulators use 64 TMEM columns (hidden
- * layers in cols 0..63, the 16-wide output layers in cols 0..15 once the
- * previous accumulator has been read).  37 KB of shared memory and 64
- * columns per CTA; FVC_TC_CTAS_PER_SM of them share an SM.  One thread issues each layer's MMAs and
- * commits them to an mbarrier; the CTA waits (bounded), reads its rows back
- * with tcgen05.ld, applies ReLU / fp16 rounding and writes the next layer's
+/* The e4m3 kernel: one CTA of 128 threads per 128-row tile; thread t owns row t
+ * and TMEM lane t.  The activations of a tile live in ONE shared-memory tile in
+ * the canonical K-major layout that each layer overwrites in place (a layer's
+ * epilogue runs only after its MMA has finished reading the tile); weights stay
+ * resident in shared memory; accumulators use 64 TMEM columns (hidden layers in
+ * cols 0..63, the 16-wide output layers in cols 0..15 once the previous
+ * accumulator has been read).  37 KB of shared memory and 64 columns per CTA,
+ * TC_FP8_CTAS_PER_SM of them on an SM.  One thread issues each layer's MMAs and
+ * commits them to the CTA's mbarrier; every thread then reads its row's results
+ * with tcgen05.ld, applies ReLU and rounding and writes the next layer's
  * operand. */
 struct __align__(128) TcSmem {
     uint8_t X[128 * 64 * 2];
     float bias3[64];
     uint64_t mbar;
     uint32_t tmem_base;
-    /* the weight tiles, last: a head with the frequency encoding (TCF_WBYTES) launches with the extra
-     * bytes past the struct (tc_smem_bytes), the others keep the smaller footprint, so that 5 CTAs
-     * leave the SM its larger L1 share for the hash gathers */
     __align__(128) uint8_t W[TC_WBYTES];
 };
 constexpr long long TC_WAIT_LIMIT = 2000000000ll; /* ~1 s of SM clocks */
