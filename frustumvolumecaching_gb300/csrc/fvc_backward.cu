@@ -432,8 +432,8 @@ __global__ void __launch_bounds__(BW_WARPS * 32, 1) wf_net_bwd_kernel(RenderPara
  * groups LBO = C / 8 * 128 bytes apart.  The input-gradient MMAs read the
  * forward weight tiles MN-major as their B = W, so one copy of each weight
  * serves both directions.
- * The weight gradients accumulate in TMEM over every tile the CTA takes and
- * are added to the global blobs once per launch; no shared-memory atomics.
+ * The weight gradients accumulate in TMEM and are added to the global blobs
+ * BT_DW_ADDS times a launch; no shared-memory atomics.
  * The weight-gradient MMAs use M = 128 with their 64 meaningful rows in TMEM
  * lanes 0..63: a 64-column tile read MN-major with M = 128 runs up to 1023
  * bytes past its end, which stays inside the next tile.

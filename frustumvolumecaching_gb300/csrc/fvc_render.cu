@@ -2870,8 +2870,10 @@ cudaError_t launch_fill_march(const RenderParams &p, int it, int n_rays, int n_s
 }
 
 /* Pass 2 of the differentiable render (pass 1 is run_frame over the pixel
- * list, then the loss kernel): the same march and network forward per
- * sub-iteration, then the compositing adjoint and the network adjoint. */
+ * list, then the loss kernel).  one_round: pass 1 took one sub-iteration, and
+ * its rows and their network outputs are still there.  Otherwise the same march
+ * and network forward per sub-iteration.  Then the compositing adjoint and the
+ * network adjoint. */
 template <bool CACHED, int HH>
 static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n_sms, cudaStream_t s, int *h_pinned,
                                 int check_every, bool one_round, LaunchLog *log)
