@@ -1276,7 +1276,7 @@ extern "C" int fvc_renderer_resize(fvc_renderer *r, int width, int height)
     if ((rc = dalloc(&r->d_states[0], n, "ray states"))) return rc;
     if ((rc = dalloc(&r->d_states[1], n, "ray states"))) return rc;
     if ((rc = alloc_rows(r, cap, n * r->windows))) return rc;
-    if ((rc = dalloc(&r->d_wf_counters, (size_t)8, "wavefront counters"))) return rc;
+    if ((rc = dalloc(&r->d_wf_counters, (size_t)N_COUNTERS, "wavefront counters"))) return rc;
     r->W = width; r->H = height;
     return FVC_OK;
 }
@@ -1468,7 +1468,7 @@ static int enqueue_render(fvc_renderer *r, const fvc_raymarch_info *info, float4
     p.contrib_cache = contrib_cache;
     CU(cudaMemsetAsync(r->d_ctl, 0, 4 * sizeof(int), r->stream));
     CU(cudaMemsetAsync(r->d_stats, 0, sizeof(RenderStatsDev), r->stream));
-    CU(cudaMemsetAsync(r->d_wf_counters, 0, 8 * sizeof(int), r->stream));
+    CU(cudaMemsetAsync(r->d_wf_counters, 0, N_COUNTERS * sizeof(int), r->stream));
     reset_launch_log(r);
     r->last_was_graph = false;
     CU(render_frame(p, cached, m->head_hidden, m->n_sms, r->stream, r->h_pinned + 8, 4, &r->last_iterations, &r->log));
@@ -1906,7 +1906,7 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
     CU(cudaMemsetAsync(c->d_packed, 0xff, n_bricks * sizeof(int32_t), s));
     CU(cudaMemsetAsync(r->d_ctl, 0, 4 * sizeof(int), s));
     CU(cudaMemsetAsync(r->d_stats, 0, sizeof(RenderStatsDev), s));
-    CU(cudaMemsetAsync(p.counters, 0, 8 * sizeof(int), s));
+    CU(cudaMemsetAsync(p.counters, 0, N_COUNTERS * sizeof(int), s));
     const int n_sms = m->n_sms;
     pr_known_init_kernel<<<n_sms * 4, 256, 0, s>>>(f);
     CU(launch_fill_raygen(p, s));
@@ -2304,7 +2304,7 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
     /* pass 1: forward render of the listed pixels into d_results */
     CU(cudaMemsetAsync(r->d_ctl, 0, 4 * sizeof(int), s));
     CU(cudaMemsetAsync(r->d_stats, 0, sizeof(RenderStatsDev), s));
-    CU(cudaMemsetAsync(r->d_wf_counters, 0, 8 * sizeof(int), s));
+    CU(cudaMemsetAsync(r->d_wf_counters, 0, N_COUNTERS * sizeof(int), s));
     CU(launch_list_order(p, r->d_list_order, r->d_list_rank, r->d_list_bins, s));
     r->log.launches += 3;
     CU(render_frame(p, cached, m->head_hidden, m->n_sms, s, r->h_pinned + 8, 4, &r->last_iterations, &r->log));
@@ -2314,7 +2314,7 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
     CU(launch_loss(p, b, s));
     /* pass 2: re-march, compositing adjoint, network adjoint; over pass 1's rows where one sub-iteration held them */
     r->log.split = r->log.n_timed;
-    if (!one_round) CU(cudaMemsetAsync(r->d_wf_counters, 0, 8 * sizeof(int), s));
+    if (!one_round) CU(cudaMemsetAsync(r->d_wf_counters, 0, N_COUNTERS * sizeof(int), s));
     CU(backward_frame(p, b, cached, m->head_hidden, m->n_sms, s, r->h_pinned + 8, 4, one_round, &r->log));
     const float inv = 1.0f / (FVC_LOSS_SCALE * (float)n_rays);
     CU(launch_grad_finalize(g->s_table, g->d_table, g->n_table, inv, m->n_sms, s));

@@ -372,7 +372,9 @@ struct RenderParams {
     uint2 *row_out;             /* per row: fp16 logits r, g, b and log-density */
     uint4 *row_lat;             /* per place in the cache list: the 8 looked-up head inputs from K = latent_offset (fp16) */
     int *res_list, *cache_list; /* row ids of the two network streams */
-    int *counters;              /* [0], [1] alive rays (ping-pong), [2] rows, [3] resample, [4] cache */
+    int *counters;              /* N_COUNTERS: [0], [1] alive rays (ping-pong), [2] rows asked for (granted_rows), [3] resample,
+                                 * [4] cache, [5] sub-iterations of the batch graph, [6], [7] rows with a gradient,
+                                 * [8] the rows granted when more were asked for than the buffers hold */
     int by_sample;              /* a warp's rows sample by sample instead of ray by ray (RowWalk) */
     int march_lanes;            /* few rays: 8 lanes march a ray (wf_march_lanes_kernel; its rows lie ray by ray) */
     int steps_per_iter;         /* marching steps per ray and sub-iteration */
@@ -402,6 +404,30 @@ struct RenderParams {
     int *grad_res_list;         /* rows with a gradient: resample rows (counters[6]) */
     int *grad_cache_list;       /*                       cache rows (counters[7]) */
 };
+
+constexpr int N_COUNTERS = 16;
+
+/* A warp's n > 0 rows of a march window: the first of them, or -1 without room
+ * for them all.  The counter only grows during a march, refused requests
+ * included, so after the first refusal every later one is refused too and the
+ * granted rows are [0, that request's base).  (Taking a refused request back
+ * would let a later one in below another that is still to be taken back: the
+ * same rows twice, and rows past the final count.)  A base is no more than the
+ * capacity for the first refused request only, so one warp writes the count. */
+__device__ __forceinline__ int request_rows(const RenderParams &p, int n)
+{
+    const int base = atomicAdd(p.counters + 2, n);
+    if (base + n <= p.row_capacity) return base;
+    if (base <= p.row_capacity) p.counters[8] = base;
+    return -1;
+}
+
+/* the rows that the sub-iteration's march was granted (after its launch) */
+__device__ __forceinline__ int granted_rows(const RenderParams &p)
+{
+    const int asked = p.counters[2];
+    return asked <= p.row_capacity ? asked : p.counters[8];
+}
 
 /* Weights of the backward kernel: fragment packs (mma.sync m16n8k16 B
  * operands, frag_pack order) of each layer W (out x in) for the forward

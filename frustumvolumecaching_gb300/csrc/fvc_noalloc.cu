@@ -129,7 +129,7 @@ extern "C" int fvc_render_noalloc(fvc_model *m, const fvc_raymarch_info *info, c
     p.cam = fvc_internal::cam_view(*info);
     /* carve the scratch: header (counters, statistics) then per-ray arrays */
     unsigned char *cursor = static_cast<unsigned char *>(base);
-    int *ctl = carve<int>(cursor, 16);              /* [0] ray counter, [1] guard, [8..15] sub-iteration counters */
+    int *ctl = carve<int>(cursor, 8 + N_COUNTERS);  /* [0] ray counter, [1] guard, [8..] sub-iteration counters */
     RenderStatsDev *stats = carve<RenderStatsDev>(cursor, 1);
     cursor = static_cast<unsigned char *>(base) + HEADER_BYTES;
     const size_t n = (size_t)n_rays, cap = n * ROWS_PER_RAY;

@@ -582,13 +582,7 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
             }
             const int n_warp = (int)__reduce_add_sync(FULLMASK, (unsigned)n);
             int rbase = 0;
-            if (lane_id() == 0 && n_warp) {
-                rbase = atomicAdd(p.counters + 2, n_warp);
-                if (rbase + n_warp > p.row_capacity) { /* no hole: what was added is taken back, and nothing fits meanwhile */
-                    atomicSub(p.counters + 2, n_warp);
-                    rbase = -1;
-                }
-            }
+            if (lane_id() == 0 && n_warp) rbase = request_rows(p, n_warp);
             rbase = __shfl_sync(FULLMASK, rbase, 0);
             if (rbase < 0) { /* the rays wait at this window's start for the next sub-iteration */
                 if (!done_before) p.ray_rows[(size_t)w * sub.stride + i] = make_int2(0, window_pack(0, 0, false));
@@ -762,13 +756,7 @@ __global__ void __launch_bounds__(32 * ML_LANES) wf_march_lanes_kernel(RenderPar
                 const int mine = s_n[threadIdx.x], before = lanes_before(mine);
                 const int total = __shfl_sync(FULLMASK, before + mine, 31);
                 int first = 0;
-                if (threadIdx.x == 0 && total) {
-                    first = atomicAdd(p.counters + 2, total);
-                    if (first + total > p.row_capacity) {
-                        atomicSub(p.counters + 2, total);
-                        first = -1;
-                    }
-                }
+                if (threadIdx.x == 0 && total) first = request_rows(p, total);
                 first = __shfl_sync(FULLMASK, first, 0);
                 s_row[threadIdx.x] = first + before;
                 if (threadIdx.x == 0) s_first = first;
@@ -896,7 +884,7 @@ __device__ __forceinline__ float3 cache_viewdir01(float3 wp, const DevCam &ccam)
 template <bool VD>
 __global__ void __launch_bounds__(256) wf_classify_kernel(RenderParams p, int it)
 {
-    const int n_rows = p.counters[2];
+    const int n_rows = granted_rows(p);
     const RayState *states = p.states[it & 1];
     for (int base = blockIdx.x * blockDim.x; base < n_rows; base += gridDim.x * blockDim.x) {
         const int r = base + threadIdx.x;
@@ -1031,7 +1019,7 @@ __global__ void __launch_bounds__(NET_WARPS * 32, 2) wf_net_resample_kernel(Rend
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     NetSmem &S = *reinterpret_cast<NetSmem *>(smem_raw);
-    const int n_rows = LIST ? p.counters[3] : p.counters[2];
+    const int n_rows = LIST ? p.counters[3] : granted_rows(p);
     if (n_rows == 0) return;
     for (int i = threadIdx.x; i < W_TOTAL; i += blockDim.x) S.W[i] = p.weights[i];
     for (int i = threadIdx.x; i < 64; i += blockDim.x) S.bias3[i] = p.bias3[i];
@@ -1421,7 +1409,7 @@ __global__ void __launch_bounds__(NT_THREADS, 1) wf_net_tc_kernel(RenderParams p
     after_previous();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     NtSmem &S = *reinterpret_cast<NtSmem *>(smem_raw);
-    const int n_rows = MODE == 0 ? (LIST ? p.counters[3] : p.counters[2]) : MODE == 1 ? p.counters[4] : p.counters[3];
+    const int n_rows = MODE == 0 ? (LIST ? p.counters[3] : granted_rows(p)) : MODE == 1 ? p.counters[4] : p.counters[3];
     const int n_hit = MODE == 2 ? p.counters[4] : 0;
     const int res_tiles = (n_rows + 127) / 128;
     const int n_tiles = res_tiles + (n_hit + 127) / 128;
@@ -1741,7 +1729,7 @@ __global__ void __launch_bounds__(tcm_threads<MT>(), tcm_ctas_per_sm<MT>()) wf_n
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     TcmSmem<MT> &S = *reinterpret_cast<TcmSmem<MT> *>(smem_raw);
-    const int n_rows = LIST ? p.counters[3] : p.counters[2];
+    const int n_rows = LIST ? p.counters[3] : granted_rows(p);
     if (n_rows == 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int trow = MT == 64 ? 16 * warp + (lane & 15) : tid; /* the tile row this thread works on */
@@ -1916,7 +1904,7 @@ __global__ void __launch_bounds__(128, TC_FP8_CTAS_PER_SM) wf_net_tc_fp8_kernel(
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     TcSmem &S = *reinterpret_cast<TcSmem *>(smem_raw);
-    const int n_rows = p.counters[2];
+    const int n_rows = granted_rows(p);
     if ((int)blockIdx.x * 128 >= n_rows) return;
     const int tid = threadIdx.x, warp = tid >> 5;
     if (tid == 0) { /* the weights by one bulk copy, completing phase 0 (as wf_net_tc_kernel) */
@@ -2024,7 +2012,7 @@ __global__ void __launch_bounds__(128, TC_FP8_CTAS_PER_SM) wf_net_tc_fp8_kernel(
 /* counts the sub-iteration's rows and clears their counters */
 __device__ __forceinline__ void reset_row_counters(const RenderParams &p, bool cached)
 {
-    const int rows = p.counters[2], res = p.counters[3], hits = p.counters[4];
+    const int rows = granted_rows(p), res = p.counters[3], hits = p.counters[4];
     atomicAdd(&p.stats->n_resamples, (unsigned long long)(cached ? res : rows));
     atomicAdd(&p.stats->n_cache_hits, (unsigned long long)hits);
     atomicAdd(&p.stats->n_dropped, (unsigned long long)(cached ? rows - res - hits : 0));
@@ -2493,7 +2481,7 @@ __global__ void __launch_bounds__(128, 4) wf_net_vd_kernel(RenderParams p, int i
 {
     extern __shared__ __align__(128) unsigned char vd_smem_raw[];
     VdSmem &S = *reinterpret_cast<VdSmem *>(vd_smem_raw);
-    const int n_rows = MODE == 0 ? (LIST ? p.counters[3] : p.counters[2]) : p.counters[4];
+    const int n_rows = MODE == 0 ? (LIST ? p.counters[3] : granted_rows(p)) : p.counters[4];
     if (n_rows == 0) return;
     const int tid = threadIdx.x, warp = tid >> 5;
     /* the color head's input: K = 48 with the 1-padding, or K = 64 with the frequency encoding */
@@ -2961,7 +2949,7 @@ static cudaError_t build_batch_graph_t(const RenderParams &p, int n_sms, cudaStr
     if (e == cudaSuccess) {
         cudaMemsetAsync(p.ray_counter, 0, 4 * sizeof(int), s);
         cudaMemsetAsync(p.stats, 0, sizeof(RenderStatsDev), s);
-        cudaMemsetAsync(p.counters, 0, 8 * sizeof(int), s);
+        cudaMemsetAsync(p.counters, 0, N_COUNTERS * sizeof(int), s);
         wf_raygen_views_kernel<<<(n_rays + 255) / 256, 256, 0, s>>>(p);
         cudaGraph_t g2 = nullptr;
         e = cudaStreamEndCapture(s, &g2);
