@@ -333,7 +333,8 @@ __host__ __device__ __forceinline__ uint32_t occupancy_bit_index(uint32_t x, uin
  * 2^23 (2^25) and rounding towards zero leaves a cell coordinate (a quarter of
  * it; 2^24: a half of it) in the sum's low bits.  A point whose cell
  * coordinate may round up to 128, beyond the cascade's last cell, or whose
- * offset is not finite, takes occupied() itself. */
+ * largest offset is not finite, takes occupied() itself; the maximum passes
+ * over a NaN beside a number, and the masked index stays inside the cascade. */
 __device__ __forceinline__ uint32_t occupied2(const DevScene &sc, const uint8_t *__restrict__ bits, const uint32_t *__restrict__ cells,
                                               float3 o, float3 d, float2 tm)
 {
@@ -492,13 +493,23 @@ __device__ __forceinline__ float2 f2_lerp(float2 a, float2 b, float t)
 /* One axis of a level's cell: p = fma(scale, x, 0.5), its floor and the
  * fraction above it.  Rounding p + 1.5 * 2^23 downwards leaves floor(p) in the
  * sum's low bits (|p| < 2^22), so the floor, the integer and the fraction are
- * plain additions instead of conversions, which a quarter-rate unit executes. */
+ * plain additions instead of conversions, which a quarter-rate unit executes.
+ * Beyond that, and for a p that is not a number, the cell is any: the level's
+ * index keeps it inside the table (hashed levels mask, dense ones dense_entry),
+ * and the fraction of a NaN is NaN. */
 __device__ __forceinline__ uint32_t grid_axis(float scale, float x, float &w)
 {
     const float p = __fmaf_rn(scale, x, 0.5f);
     const float t = __fadd_rd(p, 12582912.0f);
     w = __fsub_rn(p, __fsub_rn(t, 12582912.0f));
     return __float_as_uint(t) - 0x4B400000u;
+}
+
+/* A dense level's entry: i % size for the indices of [0, 1]^3, which stay below 2 * size (i - size wraps to a large
+ * number for i < size); an entry of the level for any other, as a query's positions are the caller's. */
+__device__ __forceinline__ uint32_t dense_entry(uint32_t i, uint32_t size)
+{
+    return min(min(i, i - size), size - 1u);
 }
 
 /* Encodes one position into 2*n_levels features (fp16) written to
@@ -527,11 +538,8 @@ __device__ __forceinline__ void hash_group_f4(const DevGrid &g, const __half2 *_
             const uint32_t r = g.res[l], r2 = g.res2[l];
             const uint32_t b = gx + gy * r + gz * r2;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                uint32_t i = b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u);
-                if (i >= size) i -= size;
-                v[j][c] = __ldg(tl + i);
-            }
+            for (int c = 0; c < 8; ++c)
+                v[j][c] = __ldg(tl + dense_entry(b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u), size));
         } else {
             const uint32_t hy0 = gy * 2654435761u, hy1 = (gy + 1u) * 2654435761u;
             const uint32_t hz0 = gz * 805459861u, hz1 = (gz + 1u) * 805459861u;
@@ -574,16 +582,13 @@ __device__ __forceinline__ void hash_group_f2(const DevGrid &g, const __half2 *_
         if ((g.dense_mask >> l) & 1u) {
             const uint32_t r = g.res[l], r2 = g.res2[l];
             const uint32_t b = gx + gy * r + gz * r2;
-            if (b + 1u + r + r2 < size) { /* no corner reaches past the table (all but the grid's far faces) */
+            if (b < size - (1u + r + r2)) { /* no corner reaches past the table (all but the grid's far faces) */
 #pragma unroll
                 for (int c = 0; c < 8; ++c) v[j][c] = __ldg(tl + (b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u)));
             } else {
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    uint32_t i = b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u);
-                    if (i >= size) i -= size; /* == i % size: dense indices stay below 2*size */
-                    v[j][c] = __ldg(tl + i);
-                }
+                for (int c = 0; c < 8; ++c)
+                    v[j][c] = __ldg(tl + dense_entry(b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u), size));
             }
         } else {
             const uint32_t hy0 = gy * 2654435761u, hy1 = (gy + 1u) * 2654435761u;
