@@ -465,7 +465,7 @@ def run_backward_bench(args, torch, dev, stream) -> dict:
         launches += bst.n_launches
         adj_ms += bst.timed_adjoint_ms
         adj_launches += bst.n_timed_adjoint_launches
-        adj_rows += bst.n_resamples
+        adj_rows += bst.n_resamples // 2  # both passes' rows
     r.set_kernel_timing(False)
     ms = sum(times) / len(times)
     # the same step with BF16 MLPs

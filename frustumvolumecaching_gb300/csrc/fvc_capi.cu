@@ -442,6 +442,7 @@ struct fvc_renderer {
     int batch_rows = 0, windows = 1, ray_stride = 0;
     size_t ray_rows_cap = 0;          /* entries of d_ray_rows */
     int last_iterations = 0;
+    int last_passes = 1;              /* passes over the last render's rows that its statistics stand for */
     /* batched views in one graph launch */
     DevCam *d_views = nullptr;
     int *d_view_off = nullptr;
@@ -1452,6 +1453,7 @@ static void reset_launch_log(fvc_renderer *r)
     r->log.launches = 0;
     r->log.n_timed = r->log.n_untimed = 0;
     r->log.split = -1;
+    r->last_passes = 1;
     r->log.ev = r->events.empty() ? nullptr : r->events.data();
     r->log.cap = (int)r->events.size() / 2;
 }
@@ -1518,10 +1520,10 @@ extern "C" int fvc_render_stats(fvc_renderer *r, fvc_render_stats_t *o)
     CU(cudaMemcpy(ctl, r->d_ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
     const double n_rays = (double)std::max(1, r->W * r->H);
     o->n_samples = (long long)s.n_samples;
-    o->n_resamples = (long long)s.n_resamples;
-    o->n_cache_hits = (long long)s.n_cache_hits;
-    o->n_dropped = (long long)s.n_dropped;
-    o->n_steps = (long long)s.n_steps;
+    o->n_resamples = (long long)s.n_resamples * r->last_passes;
+    o->n_cache_hits = (long long)s.n_cache_hits * r->last_passes;
+    o->n_dropped = (long long)s.n_dropped * r->last_passes;
+    o->n_steps = (long long)s.n_steps * r->last_passes;
     o->n_rounds = r->last_iterations;
     o->samples_ppx = (double)s.n_samples / n_rays;
     o->guard_flags = ctl[1];
@@ -1894,6 +1896,7 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
     f.bX = c->bX; f.bY = c->bY; f.bZ = c->bZ; f.dX = c->dX; f.dY = c->dY; f.dZ = c->dZ; f.capacity = c->capacity();
     f.variant = r->settings.interpol_variant;
     f.slot_counter = x.slots; f.col_count = x.col_count; f.col_base = x.col_base;
+    f.max_samples_per_ray = p.max_samples_per_ray; f.guard = p.guard; f.stats = p.stats;
     CacheBuildParams q; /* the density network over the sub-iteration's rows */
     memset(&q, 0, sizeof(q));
     q.grid = m->grid; q.table = m->d_table; q.weights = m->d_weights; q.latent_offset = m->latent_offset;
@@ -1906,6 +1909,7 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
     CU(cudaMemsetAsync(c->d_packed, 0xff, n_bricks * sizeof(int32_t), s));
     CU(cudaMemsetAsync(r->d_ctl, 0, 4 * sizeof(int), s));
     CU(cudaMemsetAsync(r->d_stats, 0, sizeof(RenderStatsDev), s));
+    r->last_passes = 1;
     CU(cudaMemsetAsync(p.counters, 0, N_COUNTERS * sizeof(int), s));
     const int n_sms = m->n_sms;
     pr_known_init_kernel<<<n_sms * 4, 256, 0, s>>>(f);
@@ -2301,6 +2305,7 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
     b.loss_scale = FVC_LOSS_SCALE;
     b.g_lat = cached ? g->s_lat : nullptr;
     reset_launch_log(r);
+    r->last_passes = 2; /* the adjoint goes over the same rows and steps */
     /* pass 1: forward render of the listed pixels into d_results */
     CU(cudaMemsetAsync(r->d_ctl, 0, 4 * sizeof(int), s));
     CU(cudaMemsetAsync(r->d_stats, 0, sizeof(RenderStatsDev), s));

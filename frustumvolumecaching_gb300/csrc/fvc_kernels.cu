@@ -819,13 +819,21 @@ __global__ void __launch_bounds__(128) pr_write_kernel(PerRayFillParams p, int i
         RayState st;
         int id = 0, row;
         float T = 1.f, term = p.steps.far_;
+        int2 rr = make_int2(0, 0);
         if (valid) {
             st = states[i];
+            rr = p.ray_rows[i];
             id = st.cnt.x;
             T = st.acc.w;
-            alive = !window_done(p.ray_rows[i].y); /* the march ended the ray past its far bound */
+            alive = !window_done(rr.y); /* the march ended the ray past its far bound */
+            if (p.max_samples_per_ray > 0) {
+                st.cnt2.z += window_rows(rr.y);
+                if (st.cnt2.z > p.max_samples_per_ray) atomicOr(p.guard, 1);
+            }
         }
-        RowWalk walk(valid ? p.ray_rows[i] : make_int2(0, 0), valid, p.by_sample);
+        const int ws = __reduce_add_sync(0xffffffffu, window_steps(rr.y));
+        if ((threadIdx.x & 31) == 0 && ws) atomicAdd(&p.stats->n_steps, (unsigned long long)ws);
+        RowWalk walk(rr, valid, p.by_sample);
         while (walk.step(row)) {
             if (row >= 0 && !ended) {
                 const float density = expf(fminf(__half2float(p.den[row]), 10.0f));

@@ -594,6 +594,9 @@ struct PerRayFillParams {
     int *slot_counter;          /* [0] slots reserved so far (overflowing ones included), [1] its value before this
                                    sub-iteration */
     int *col_count, *col_base;  /* per brick column (bY x bX) */
+    int max_samples_per_ray;    /* 0 = unlimited */
+    int *guard;
+    RenderStatsDev *stats;
 };
 
 __global__ void pr_known_init_kernel(PerRayFillParams p);

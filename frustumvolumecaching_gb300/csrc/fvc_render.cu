@@ -521,7 +521,6 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
             dt4 = states[i].dt;
         }
         bool done = !valid;
-        int all_steps = 0, all_rows = 0;
         for (int w = 0; w < sub.windows; ++w) {
             int n = 0, steps = 0;
             const float t_window = dt4.w;
@@ -643,21 +642,10 @@ __global__ void __launch_bounds__(128) wf_march_kernel(RenderParams p, int it)
                 }
             }
             if (valid) p.ray_rows[(size_t)w * sub.stride + i] = make_int2(rbase, window_pack(n, steps, done));
-            all_steps += steps;
-            all_rows += n;
             /* a warp whose rays have all ended leaves; the compositing stops at its rays' done flags too */
             if (__all_sync(FULLMASK, done)) break;
         }
-        if (valid) {
-            states[i].dt.w = dt4.w;
-            if (p.max_samples_per_ray > 0) {
-                const int pushed = states[i].cnt2.z + all_rows;
-                states[i].cnt2.z = pushed;
-                if (pushed > p.max_samples_per_ray) atomicOr(p.guard, 1);
-            }
-        }
-        const int ws = __reduce_add_sync(FULLMASK, all_steps);
-        if (lane_id() == 0 && ws) atomicAdd(&p.stats->n_steps, (unsigned long long)ws);
+        if (valid) states[i].dt.w = dt4.w;
     }
 }
 
@@ -706,7 +694,6 @@ __global__ void __launch_bounds__(32 * ML_LANES) wf_march_lanes_kernel(RenderPar
         const float3 o = make_float3(of.x, of.y, of.z), d = make_float3(dt4.x, dt4.y, dt4.z);
         float t1 = dt4.w;
         bool done = !valid;
-        int all_steps = 0, all_rows = 0;
         for (int w = 0; w < sub.windows; ++w) {
             int n = 0, steps = 0;
             const float t_window = t1;
@@ -797,20 +784,9 @@ __global__ void __launch_bounds__(32 * ML_LANES) wf_march_lanes_kernel(RenderPar
                 }
             }
             if (l == 0 && valid) p.ray_rows[(size_t)w * sub.stride + i] = make_int2(first, window_pack(n, steps, done));
-            all_steps += steps;
-            all_rows += n;
             if (__syncthreads_and(done)) break; /* also: the shared rows are read before the next window's */
         }
-        if (l == 0 && valid) {
-            states[i].dt.w = t1;
-            if (p.max_samples_per_ray > 0) {
-                const int pushed = states[i].cnt2.z + all_rows;
-                states[i].cnt2.z = pushed;
-                if (pushed > p.max_samples_per_ray) atomicOr(p.guard, 1);
-            }
-        }
-        const int ws = __reduce_add_sync(FULLMASK, l == 0 ? all_steps : 0);
-        if (lane_id() == 0 && ws) atomicAdd(&p.stats->n_steps, (unsigned long long)ws);
+        if (l == 0 && valid) states[i].dt.w = t1;
         __syncthreads();
     }
 }
@@ -2009,24 +1985,36 @@ __global__ void __launch_bounds__(128, TC_FP8_CTAS_PER_SM) wf_net_tc_fp8_kernel(
 /* ------------------------------------------------------------------------- */
 /* composite + compaction                                                    */
 /* ------------------------------------------------------------------------- */
-/* counts the sub-iteration's rows and clears their counters */
-__device__ __forceinline__ void reset_row_counters(const RenderParams &p, bool cached)
-{
-    const int rows = granted_rows(p), res = p.counters[3], hits = p.counters[4];
-    atomicAdd(&p.stats->n_resamples, (unsigned long long)(cached ? res : rows));
-    atomicAdd(&p.stats->n_cache_hits, (unsigned long long)hits);
-    atomicAdd(&p.stats->n_dropped, (unsigned long long)(cached ? rows - res - hits : 0));
-    p.counters[2] = 0;
-    p.counters[3] = 0;
-    p.counters[4] = 0;
-}
+/* clears the sub-iteration's row counters */
+__device__ __forceinline__ void reset_row_counters(const RenderParams &p) { p.counters[2] = p.counters[3] = p.counters[4] = 0; }
 
 /* the same as a node of the batch graph, where a launch costs little; elsewhere the compositing's first thread does
  * it: the compositing is the last kernel of a sub-iteration, its network launches have read the counters, and it
  * reads none of them itself */
-__global__ void wf_reset_rows_kernel(RenderParams p, int cached)
+__global__ void wf_reset_rows_kernel(RenderParams p)
 {
-    if (threadIdx.x == 0) reset_row_counters(p, cached);
+    if (threadIdx.x == 0) reset_row_counters(p);
+}
+
+/* What a warp's rays add to the statistics: per ray the samples composited,
+ * and the steps and rows (resample rows, cache rows) of its march windows up
+ * to the one it ended in, so that the counts do not depend on how many windows
+ * a sub-iteration marches past a ray's end (whole warp). */
+__device__ __forceinline__ void add_stats(const RenderParams &p, int n_comp, int steps, int rows, int res, int hits)
+{
+    const int c = __reduce_add_sync(FULLMASK, n_comp), s = __reduce_add_sync(FULLMASK, steps), r = __reduce_add_sync(FULLMASK, rows);
+    const int q = __reduce_add_sync(FULLMASK, res), h = __reduce_add_sync(FULLMASK, hits);
+    static_assert(offsetof(RenderStatsDev, n_steps) == 4 * sizeof(unsigned long long), "the first five fields, a lane each");
+    const int l = lane_id(), v = l == 0 ? c : l == 1 ? q : l == 2 ? h : l == 3 ? r - q - h : s;
+    if (l < 5 && v) atomicAdd(&p.stats->n_samples + l, (unsigned long long)v);
+}
+
+/* the rows of the windows a ray has marched, when they are limited */
+__device__ __forceinline__ void limit_samples(const RenderParams &p, RayState &st, int rows)
+{
+    if (p.max_samples_per_ray <= 0) return;
+    st.cnt2.z += rows;
+    if (st.cnt2.z > p.max_samples_per_ray) atomicOr(p.guard, 1);
 }
 
 /* samples of a ray whose rows the compositing loads together */
@@ -2055,12 +2043,12 @@ __device__ __forceinline__ void warp_rows(int2 rr, int &first, int &total)
 }
 
 template <bool CACHED>
-__global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int it)
+__global__ void __launch_bounds__(128, CACHED ? 7 : 6) wf_composite_kernel(RenderParams p, int it)
 {
     after_previous();
     constexpr int AHEAD = CACHED ? COMP_AHEAD_CACHED : COMP_AHEAD;
     const int n_alive = p.counters[it & 1];
-    if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p, CACHED);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p);
     RayState *cur = p.states[it & 1], *nxt = p.states[(it + 1) & 1];
     const SubIter sub(p, n_alive);
     for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
@@ -2068,10 +2056,12 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
         const bool valid = i < n_alive;
         bool keep = false;
         RayState st;
-        int n_comp = 0;
         unsigned long long why = 0; /* rows per REASON_* 1..7, 9 bits each (at most MAX_WINDOWS * S_ROWS a ray and sub-iteration) */
         float4 acc = make_float4(0.f, 0.f, 0.f, 1.f), comp = make_float4(0.f, 0.f, 0.f, 0.f);
         int c_res = 0, c_cache = 0, c_drop = 0, c_steps = 0;
+        /* rows of the windows up to the one the ray ended in, and of the latter's those behind the ray's end: resample rows
+         * from bit 10, cache rows from bit 20 (at most MAX_WINDOWS * S_ROWS each) */
+        uint32_t seen = 0;
         if (valid) {
             st = cur[i];
             acc = st.acc;
@@ -2086,9 +2076,13 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
         bool more_windows = true;
         for (int w = 0; w < sub.windows; ++w) {
             int2 rr = make_int2(0, 0);
+            const bool live = !term; /* at the window's start */
             if (!done) { /* also of a ray that has ended: the others' rows follow its own */
                 rr = p.ray_rows[(size_t)w * sub.stride + i];
-                if (!term) c_steps += window_steps(rr.y);
+                if (live) {
+                    c_steps += window_steps(rr.y);
+                    seen += window_rows(rr.y);
+                }
                 done = window_done(rr.y);
                 more_windows = !window_none(rr.y);
             }
@@ -2103,26 +2097,29 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
 #pragma unroll
                 for (int q = 0; q < AHEAD; ++q) {
                     more = walk.step(rs[q]) && more;
-                    if (term) rs[q] = -1;
+                    if (CACHED ? !live : term) rs[q] = -1; /* the rows behind a ray's end still count by kind */
                     codes[q] = CACHED && rs[q] >= 0 ? (int)p.row_kind[rs[q]] : KIND_RESAMPLE;
                     ovs[q] = make_uint2(0u, 0u);
                     t0s[q] = 0.f;
-                    if (rs[q] >= 0) { /* a dropped row's output is not written, and not used */
+                    if (rs[q] >= 0 && !term) { /* a dropped row's output is not written, and not used */
                         ovs[q] = p.row_out[rs[q]];
                         t0s[q] = p.row_t0[rs[q]];
                     }
                 }
 #pragma unroll
                 for (int q = 0; q < AHEAD; ++q) {
-                    if (rs[q] < 0 || term) continue;
+                    if (rs[q] < 0) continue;
                     const int kind = row_kind_of(codes[q]);
+                    if (term) {
+                        seen += kind == KIND_RESAMPLE ? 1u << 10 : kind == KIND_CACHE ? 1u << 20 : 0u;
+                        continue;
+                    }
                     if (CACHED && kind != KIND_SKIP && row_reason_of(codes[q])) why += 1ull << ((9 * (row_reason_of(codes[q]) - 1)) & 63);
                     if (kind >= KIND_DROP) {
                         c_drop += kind == KIND_DROP;
                         continue;
                     }
                     if (kind == KIND_CACHE) ++c_cache; else ++c_res;
-                    ++n_comp;
                     const uint2 ov = ovs[q];
                     const float2 rg = __half22float2(*reinterpret_cast<const __half2 *>(&ov.x));
                     const float lb = __half2float(__ushort_as_half((unsigned short)(ov.y & 0xffffu)));
@@ -2155,18 +2152,24 @@ __global__ void __launch_bounds__(128) wf_composite_kernel(RenderParams p, int i
             }
             st.acc = acc;
             st.comp = comp;
-            st.cnt.y = c_res;
-            st.cnt.z = c_cache;
+            /* the counts become this sub-iteration's */
+            c_res -= st.cnt.y;
+            c_cache -= st.cnt.z;
+            c_steps -= st.cnt.w;
+            st.cnt.y += c_res;
+            st.cnt.z += c_cache;
+            st.cnt.w += c_steps;
             st.cnt2.x = c_drop;
-            st.cnt.w = c_steps;
+            limit_samples(p, st, seen & 1023u);
             if (term || done) {
-                write_pixel(p, st.cnt.x, acc, make_int4(c_res, c_cache, c_drop, c_steps));
+                write_pixel(p, st.cnt.x, acc, make_int4(st.cnt.y, st.cnt.z, c_drop, st.cnt.w));
             } else {
                 keep = true;
             }
         }
-        const int ws = __reduce_add_sync(FULLMASK, n_comp);
-        if (lane_id() == 0 && ws) atomicAdd(&p.stats->n_samples, (unsigned long long)ws);
+        const int n_rows = seen & 1023u;
+        add_stats(p, c_res + c_cache, c_steps, n_rows, CACHED ? c_res + (int)(seen >> 10 & 1023u) : n_rows,
+                  CACHED ? c_cache + (int)(seen >> 20) : 0);
         if (CACHED && __any_sync(FULLMASK, why != 0)) {
 #pragma unroll
             for (int q = 1; q < N_REASONS; ++q) {
@@ -2201,7 +2204,7 @@ __global__ void __launch_bounds__(32 * CL_WARPS) wf_composite_lanes_kernel(Rende
     __shared__ int s_used[32];
     __shared__ float2 s_sum[3][32];
     const int n_alive = p.counters[it & 1];
-    if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p, false);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p);
     RayState *cur = p.states[it & 1], *nxt = p.states[(it + 1) & 1];
     const SubIter sub(p, n_alive);
     const int warp = threadIdx.x >> 5, lane = lane_id();
@@ -2210,7 +2213,7 @@ __global__ void __launch_bounds__(32 * CL_WARPS) wf_composite_lanes_kernel(Rende
         const int i = base + lane;
         const bool valid = i < n_alive;
         float T = 1.f, sum = 0.f, comp = 0.f; /* warp 0: the transmittance; warps 0 to 2: a channel */
-        int c_steps = 0, n_comp = 0;
+        int c_steps = 0, n_comp = 0, n_rows = 0;
         if (valid) {
             const float4 a = cur[i].acc, c = cur[i].comp;
             T = a.w;
@@ -2222,7 +2225,10 @@ __global__ void __launch_bounds__(32 * CL_WARPS) wf_composite_lanes_kernel(Rende
             int2 rr = make_int2(0, 0);
             if (!done) {
                 rr = p.ray_rows[(size_t)w * sub.stride + i];
-                if (!term) c_steps += window_steps(rr.y);
+                if (!term) {
+                    c_steps += window_steps(rr.y);
+                    n_rows += window_rows(rr.y);
+                }
                 done = window_done(rr.y);
                 more_windows = !window_none(rr.y);
             }
@@ -2283,11 +2289,11 @@ __global__ void __launch_bounds__(32 * CL_WARPS) wf_composite_lanes_kernel(Rende
                 st.comp.z = s_sum[2][lane].y;
                 st.cnt.y += n_comp;
                 st.cnt.w += c_steps;
+                limit_samples(p, st, n_rows);
                 if (term || done) write_pixel(p, st.cnt.x, st.acc, make_int4(st.cnt.y, st.cnt.z, st.cnt2.x, st.cnt.w));
                 else keep = true;
             }
-            const int ws = __reduce_add_sync(FULLMASK, n_comp);
-            if (lane == 0 && ws) atomicAdd(&p.stats->n_samples, (unsigned long long)ws);
+            add_stats(p, n_comp, c_steps, n_rows, n_rows, 0);
             const unsigned m = __ballot_sync(FULLMASK, keep);
             int nb = 0;
             if (lane == 0 && m) nb = atomicAdd(p.counters + ((it + 1) & 1), __popc(m));
@@ -2316,7 +2322,7 @@ __global__ void __launch_bounds__(COMP_THREADS) wf_composite_bwd_kernel(RenderPa
     float4 *vals = s_vals[threadIdx.x >> 5];
     float2 *more = s_more[threadIdx.x >> 5];
     const int n_alive = p.counters[it & 1];
-    if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p, CACHED);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !p.views) reset_row_counters(p);
     RayState *cur = p.states[it & 1], *nxt = p.states[(it + 1) & 1];
     const SubIter sub(p, n_alive);
     for (int base = blockIdx.x * blockDim.x; base < n_alive; base += gridDim.x * blockDim.x) {
@@ -3008,7 +3014,7 @@ static cudaError_t build_batch_graph_t(const RenderParams &p, int n_sms, cudaStr
                 kernels += 1;
             }
             launch_composite<CACHED>(p, it, n_rays, n_sms, s);
-            wf_reset_rows_kernel<<<1, 32, 0, s>>>(p, CACHED ? 1 : 0);
+            wf_reset_rows_kernel<<<1, 32, 0, s>>>(p);
             kernels += 3;
         }
         wf_loop_cond_kernel<<<1, 1, 0, s>>>(p, handle);

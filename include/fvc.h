@@ -137,6 +137,8 @@ typedef struct fvc_cache fvc_cache;
 typedef struct {
     double samples_ppx;              /* evaluated samples per pixel          */
     long long n_samples;             /* samples evaluated (resample + cache) */
+    /* Of each ray's march windows (64 steps or 16 samples) up to the one it
+     * ended in; fvc_render_backward: of both passes. */
     long long n_resamples;           /* samples through the full network     */
     long long n_cache_hits;          /* samples served from the cache        */
     long long n_dropped;             /* known-empty cache voxels skipped     */
