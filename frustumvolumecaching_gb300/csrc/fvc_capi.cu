@@ -471,16 +471,28 @@ struct fvc_renderer {
     int *d_grad_cache_rows = nullptr; /* cache rows with a gradient */
     int *d_list_order = nullptr, *d_list_rank = nullptr, *d_list_bins = nullptr; /* the pixel list by image tile */
     int list_cap = 0;
-    int bwd_capacity = 0;
+    int bwd_capacity = 0;             /* entries of d_row_dout and of the gradient row lists */
+    size_t rows_refused = SIZE_MAX;   /* a differentiable step's rows that there was no memory for */
     LaunchLog log;                    /* kernel accounting of the last render */
     std::vector<cudaEvent_t> events;  /* 2 x 4096 when kernel timing is on */
+    void release_rows()
+    {
+        dfree(d_ray_rows); dfree(d_row_t0); dfree(d_row_slot); dfree(d_row_kind); dfree(d_row_pay); dfree(d_row_out);
+        dfree(d_res_list); dfree(d_cache_list); dfree(d_row_lat);
+        row_capacity = 0;
+        ray_rows_cap = 0;
+    }
+    void release_adjoint()
+    {
+        dfree(d_row_dout); dfree(d_grad_rows); dfree(d_grad_cache_rows);
+        bwd_capacity = 0;
+    }
     void release_wavefront()
     {
-        dfree(d_states[0]); dfree(d_states[1]); dfree(d_ray_rows); dfree(d_row_t0); dfree(d_row_slot);
-        dfree(d_row_kind); dfree(d_row_pay); dfree(d_row_out); dfree(d_res_list); dfree(d_cache_list); dfree(d_wf_counters);
-        dfree(d_row_lat);
-        row_capacity = batch_rows = 0;
-        ray_rows_cap = 0;
+        release_rows();
+        dfree(d_states[0]); dfree(d_states[1]); dfree(d_wf_counters);
+        batch_rows = 0;
+        rows_refused = SIZE_MAX;
     }
     fvc_cache *cache = nullptr, *next = nullptr;
     fvc_cache_settings settings{0, 0, 1, 1, 1, 1};
@@ -497,7 +509,7 @@ struct fvc_renderer {
     {
         if (stream) cudaStreamSynchronize(stream);
         dfree(d_ctl); dfree(d_stats); dfree(d_results); dfree(d_image); dfree(d_counts);
-        dfree(d_row_dout); dfree(d_grad_rows); dfree(d_grad_cache_rows);
+        release_adjoint();
         dfree(d_list_order); dfree(d_list_rank); dfree(d_list_bins);
         dfree(d_views); dfree(d_view_off); dfree(d_view_caches);
         if (graph_exec) cudaGraphExecDestroy(graph_exec);
@@ -1253,11 +1265,60 @@ static int alloc_rows(fvc_renderer *r, size_t cap, size_t windows)
     return FVC_OK;
 }
 
+/* the resized renderer's rows: every window's, or one window's without the memory for them */
+static int alloc_frame_rows(fvc_renderer *r, size_t n_rays)
+{
+    int rc = alloc_rows(r, (size_t)r->batch_rows * r->windows, n_rays * r->windows);
+    if (rc && r->windows > 1) {
+        r->release_rows();
+        r->windows = 1;
+        rc = alloc_rows(r, (size_t)r->batch_rows, n_rays);
+    }
+    return rc;
+}
+
+static int alloc_adjoint(fvc_renderer *r)
+{
+    if (r->bwd_capacity == r->row_capacity) return FVC_OK;
+    r->release_adjoint();
+    int rc;
+    if ((rc = dalloc(&r->d_row_dout, (size_t)r->row_capacity, "row gradients"))) return rc;
+    if ((rc = dalloc(&r->d_grad_rows, (size_t)r->row_capacity, "gradient rows"))) return rc;
+    if ((rc = dalloc(&r->d_grad_cache_rows, (size_t)r->row_capacity, "gradient rows"))) return rc;
+    r->bwd_capacity = r->row_capacity;
+    return FVC_OK;
+}
+
+/* Buffers of a differentiable step, which would have `rows` rows and `windows` windows (0: those of a frame).  Without
+ * the memory for that many it has a frame's, and then one window's; the step marches in more sub-iterations, and the
+ * renderer does not ask again until it is resized.  granted: whether the step has what it would. */
+static int alloc_step_rows(fvc_renderer *r, size_t rows, size_t windows, bool &granted)
+{
+    const size_t n_rays = (size_t)r->W * r->H;
+    granted = rows > 0 && rows < r->rows_refused;
+    const bool grow = granted && (rows > (size_t)r->row_capacity || windows > r->ray_rows_cap);
+    if (grow || r->bwd_capacity != r->row_capacity) CU(cudaStreamSynchronize(r->stream)); /* the buffers may be in use */
+    int rc = grow ? alloc_rows(r, rows, windows) : FVC_OK;
+    if (!rc) rc = alloc_adjoint(r);
+    for (int turn = 0; rc == FVC_ERR_OOM && turn < 2; ++turn) {
+        if (rows > 0) r->rows_refused = std::min(r->rows_refused, rows);
+        granted = false;
+        if (turn > 0) r->windows = 1;
+        r->release_rows();
+        r->release_adjoint();
+        rc = alloc_frame_rows(r, n_rays);
+        if (!rc) rc = alloc_adjoint(r);
+    }
+    if (rc) r->W = r->H = 0; /* the next call allocates its own */
+    return rc;
+}
+
 extern "C" int fvc_renderer_resize(fvc_renderer *r, int width, int height)
 {
     CHECK_ARG(r && width > 0 && height > 0, "fvc_renderer_resize: bad arguments");
     if (width == r->W && height == r->H) return FVC_OK;
     CU(cudaStreamSynchronize(r->stream));
+    r->W = r->H = 0; /* until every buffer is there */
     dfree(r->d_results); dfree(r->d_image); dfree(r->d_counts);
     const size_t n = (size_t)width * height;
     int rc;
@@ -1273,10 +1334,9 @@ extern "C" int fvc_renderer_resize(fvc_renderer *r, int width, int height)
     r->batch_rows = (int)std::max(n, std::min<size_t>(n * 16, (size_t)1 << 25));
     r->windows = march_windows(n);
     r->ray_stride = (int)n;
-    const size_t cap = (size_t)r->batch_rows * r->windows;
     if ((rc = dalloc(&r->d_states[0], n, "ray states"))) return rc;
     if ((rc = dalloc(&r->d_states[1], n, "ray states"))) return rc;
-    if ((rc = alloc_rows(r, cap, n * r->windows))) return rc;
+    if ((rc = alloc_frame_rows(r, n))) return rc;
     if ((rc = dalloc(&r->d_wf_counters, (size_t)N_COUNTERS, "wavefront counters"))) return rc;
     r->W = width; r->H = height;
     return FVC_OK;
@@ -2227,21 +2287,13 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
     /* Room for whole rays: with every window of a ray in one sub-iteration, pass 2 finds pass 1's rows in place and
      * neither marches nor runs the networks forward again.  LIST_ROWS rows a ray (the synthetic scenes' rays hold
      * about 90), at most 2^26 rows and 2^25 windows; rays beyond that wait for a further sub-iteration, and pass 2
-     * then marches again.  Not when a compaction batch or a march length is set. */
-    const bool whole = r->row_target == 0 && r->steps_per_iter == MARCH_STEPS;
+     * then marches again.  Not when a compaction batch or a march length is set, or without the memory. */
+    constexpr size_t LIST_ROWS = 128;
     const int ray_windows = (int)std::min<size_t>(MAX_WINDOWS, std::max<size_t>(1, ((size_t)1 << 25) / n_rays));
-    if (whole) {
-        constexpr size_t LIST_ROWS = 128;
-        const size_t rows = std::max<size_t>(1024, std::min<size_t>((size_t)n_rays * LIST_ROWS, (size_t)1 << 26));
-        const size_t windows = (size_t)n_rays * ray_windows;
-        if (rows > (size_t)r->row_capacity || windows > r->ray_rows_cap) {
-            CU(cudaStreamSynchronize(s));
-            if ((rc = alloc_rows(r, rows, windows))) {
-                r->W = r->H = 0; /* the buffers are gone: the next render allocates its own */
-                return rc;
-            }
-        }
-    }
+    const bool may_hold = r->row_target == 0 && r->steps_per_iter == MARCH_STEPS;
+    const size_t rows = may_hold ? std::max<size_t>(1024, std::min<size_t>((size_t)n_rays * LIST_ROWS, (size_t)1 << 26)) : 0;
+    bool whole = false;
+    if ((rc = alloc_step_rows(r, rows, (size_t)n_rays * ray_windows, whole))) return rc;
     if (r->list_cap < n_rays) {
         dfree(r->d_list_order); dfree(r->d_list_rank);
         r->list_cap = 0;
@@ -2249,13 +2301,6 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
         if ((rc = dalloc(&r->d_list_rank, (size_t)n_rays, "pixel ranks"))) return rc;
         if (!r->d_list_bins && (rc = dalloc(&r->d_list_bins, (size_t)LIST_BINS, "pixel tiles"))) return rc;
         r->list_cap = n_rays;
-    }
-    if (r->bwd_capacity != r->row_capacity) {
-        dfree(r->d_row_dout); dfree(r->d_grad_rows); dfree(r->d_grad_cache_rows);
-        if ((rc = dalloc(&r->d_row_dout, (size_t)r->row_capacity, "row gradients"))) return rc;
-        if ((rc = dalloc(&r->d_grad_rows, (size_t)r->row_capacity, "gradient rows"))) return rc;
-        if ((rc = dalloc(&r->d_grad_cache_rows, (size_t)r->row_capacity, "gradient rows"))) return rc;
-        r->bwd_capacity = r->row_capacity;
     }
     if (cached) {
         if (!r->cache || !r->cache->built) return fail(FVC_ERR_CACHE_UNINIT, "Cache is not initialized!");
@@ -2275,6 +2320,7 @@ extern "C" int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_rayma
     }
     if (g->ray_cap < n_rays) {
         dfree(g->d_ray_grad);
+        g->ray_cap = 0;
         if ((rc = dalloc(&g->d_ray_grad, (size_t)n_rays, "ray gradients"))) return rc;
         g->ray_cap = n_rays;
     }

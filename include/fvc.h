@@ -271,7 +271,11 @@ int fvc_model_debug_encode(fvc_model *m, const float *pos, int n, float *feature
 /* ------------------------------------------------------------------------ */
 int fvc_renderer_create(fvc_model *m, int kind, fvc_renderer **out);
 void fvc_renderer_destroy(fvc_renderer *r);
-/* resizeRenderbuffers(int2), src/performance_renderer.cu:186-212. */
+/* resizeRenderbuffers(int2), src/performance_renderer.cu:186-212.  A renderer
+ * keeps 16 sample rows a ray for each march window of a sub-iteration (about
+ * 2^20 rays' worth of windows, at most 31), 32 bytes a row and 57 for a cache
+ * renderer: about 0.5 and 1 GB up to a million rays.  Without the memory for
+ * them it has one window's. */
 int fvc_renderer_resize(fvc_renderer *r, int width, int height);
 /* Use the caller's CUDA stream (cudaStream_t as void*; NULL = internal stream). */
 int fvc_renderer_set_stream(fvc_renderer *r, void *cuda_stream);
@@ -538,8 +542,12 @@ int fvc_grad_cache_latents(fvc_grad *g, float *latents, size_t *n);
  * white-background pixel of writeImageBuffer_performance_kernel
  * (src/performance_renderer.cu:127-149) against device target [n_rays x 3].
  * Adds dL/dparam to g, writes L to *loss_out and, if pred is non-null, the
- * forward (C, T) per ray to device pred [n_rays x 4].  The forward is
- * recomputed per sub-iteration instead of stored.  Synchronous. */
+ * forward (C, T) per ray to device pred [n_rays x 4].  The forward's
+ * rows are kept for the adjoint where one sub-iteration holds them: the
+ * renderer keeps up to 128 rows a ray, at most 2^26, of 56 bytes (81 for a
+ * cache renderer; 3.8 and 5.4 GB) until it is resized.  Beyond that, or
+ * without the memory, the forward is recomputed per sub-iteration.
+ * Synchronous. */
 int fvc_render_backward(fvc_renderer *r, fvc_grad *g, const fvc_raymarch_info *info, const int32_t *pixels, int n_rays,
                         const float *target, double *loss_out, float *pred);
 
