@@ -1908,6 +1908,9 @@ extern "C" int fvc_cache_build(fvc_renderer *r, const fvc_raymarch_info *info)
     return FVC_OK;
 }
 
+/* samples a ray and sub-iteration of the fill: TARGET_BATCH_SIZE / alive rays, 1 to 8 */
+constexpr int FILL_STEPS = 8, FILL_ROWS = 1 << 21;
+
 /* CacheRenderer::initCache, src/cache_renderer.cu:848-928: the per-ray fill
  * of the "next" cache.  The cache camera's rays march like a plain render,
  * TARGET_BATCH_SIZE / alive (1..8) occupied samples per ray and sub-iteration;
@@ -1935,7 +1938,10 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
     p.windows = 1;
     p.window_rays = 0;
     PerRayScratch &x = r->pr;
-    const size_t n_bricks = (size_t)c->bX * c->bY * c->bZ, n_cols = (size_t)c->bX * c->bY, n_rows = (size_t)r->row_capacity;
+    const size_t n_bricks = (size_t)c->bX * c->bY * c->bZ, n_cols = (size_t)c->bX * c->bY;
+    /* the rows that a sub-iteration can have, whatever the renderer's buffers hold */
+    const size_t n_pix = (size_t)W * H, n_rows = std::max(n_pix, std::min(n_pix * FILL_STEPS, (size_t)FILL_ROWS));
+    p.row_capacity = (int)n_rows;
     if (x.n_bricks < n_bricks || x.n_cols < n_cols || x.n_rows < n_rows) {
         x.release();
         if ((rc = dalloc(&x.flag, n_bricks, "fill brick marks"))) return rc;
@@ -1981,7 +1987,7 @@ extern "C" int fvc_cache_build_per_ray(fvc_renderer *r, const fvc_raymarch_info 
     long long n_samples = 0;
     int it = 0;
     for (; it < 1000 && n_alive > 0; ++it) { /* MAX_SUBITER */
-        const int n_steps = std::min(8, std::max(1, (1 << 21) / n_alive)); /* TARGET_BATCH_SIZE / n_alive */
+        const int n_steps = std::min(FILL_STEPS, std::max(1, FILL_ROWS / n_alive));
         p.batch_rows = n_steps * n_alive;                                   /* the march gives every ray n_steps rows */
         n_samples += ((long long)n_alive * n_steps + 255) / 256 * 256;     /* next_multiple(batch, 256) */
         p.march_lanes = march_by_lanes(p, (size_t)n_alive);

@@ -2,7 +2,8 @@
 rays' whole rows takes a frame's rows and marches in more sub-iterations, and a
 resize without the memory for every march window takes one window's; both give
 the same results.  A step whose other buffers fail, and a resize that fails,
-leave the renderer usable at any size."""
+leave the renderer usable at any size.  A per-ray cache fill allocates for its
+own rows, not for those a step has left the renderer with."""
 import numpy as np
 import pytest
 
@@ -104,3 +105,25 @@ def test_failed_resize_then_the_size_before(loader):
         buf = fvc.RenderBuffer((32, 24))
         r.render(fvc.raymarch_info(small, loader.stepsize_info), buf)
         np.testing.assert_array_equal(buf.results.view(np.uint32), ref.results.view(np.uint32))
+
+
+def test_fill_after_a_step_allocates_for_its_own_rows(loader):
+    torch = pytest.importorskip("torch")
+    W = H = 512
+    info = fvc.raymarch_info(small_camera(1001, W, H), loader.stepsize_info)
+    r = fvc.CachePerformanceRenderer(loader.scene_info, loader.occupancy_grid_morton_bitfield, loader.nerf_network, fvc.Cache(), fvc.Cache())
+    r.setCacheSettings(fvc.default_cache_settings())
+    for _ in range(2):
+        r.resizeCache((W, H), loader.stepsize_info)
+        r.swapCache()
+    r.initCacheBlockwise(info)
+    r.swapCache()
+    pix = torch.arange(W * H, dtype=torch.int32, device="cuda")
+    tgt = torch.zeros((W * H, 3), dtype=torch.float32, device="cuda")
+    r.render_backward(info, pix, tgt, fvc.Gradients(loader.nerf_network))  # 2^25 rows
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    r.initCache(info)
+    # 2^21 rows of 18 bytes (38 MB) and a few bytes a brick; for 2^25 rows it would be 604 MB
+    assert free - torch.cuda.mem_get_info()[0] < 150 << 20
+    assert r._init_stats.n_bricks_set > 0
