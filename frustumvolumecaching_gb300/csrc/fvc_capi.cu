@@ -2096,7 +2096,7 @@ extern "C" int fvc_renderer_set_network_path(fvc_renderer *r, int use_tcgen05)
 
 extern "C" int fvc_renderer_set_build_network_path(fvc_renderer *r, int use_tcgen05)
 {
-    CHECK_ARG(r && (use_tcgen05 == 0 || use_tcgen05 == 1), "fvc_renderer_set_build_network_path: bad arguments");
+    CHECK_ARG(r && use_tcgen05 >= -1 && use_tcgen05 <= 1, "fvc_renderer_set_build_network_path: bad arguments");
     r->build_tc = use_tcgen05;
     return FVC_OK;
 }

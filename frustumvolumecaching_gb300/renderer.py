@@ -179,9 +179,10 @@ class Renderer:
         """tcgen05 (default) or mma.sync network kernels."""
         L.check(L.load().fvc_renderer_set_network_path(self.handle, int(bool(use_tcgen05))))
 
-    def set_build_network_path(self, use_tcgen05: bool) -> None:
-        """The cache builds' density network: mma.sync or tcgen05 (default: by the build's size); same slots and voxels."""
-        L.check(L.load().fvc_renderer_set_build_network_path(self.handle, int(bool(use_tcgen05))))
+    def set_build_network_path(self, use_tcgen05: bool | None) -> None:
+        """The cache builds' density network: mma.sync, tcgen05 or (None, the default) by the build's size; same slots and voxels."""
+        path = -1 if use_tcgen05 is None else int(bool(use_tcgen05))
+        L.check(L.load().fvc_renderer_set_build_network_path(self.handle, path))
 
     def set_empty_space_skipping(self, on: bool) -> None:
         """Occupancy lookups once per empty cell (default) or every step; identical results."""

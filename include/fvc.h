@@ -329,7 +329,7 @@ int fvc_renderer_set_max_samples_per_ray(fvc_renderer *r, int max_samples);
 int fvc_renderer_set_network_path(fvc_renderer *r, int use_tcgen05);
 /* Density network of the cache builds (the blockwise build and the per-ray
  * fill; inferenceLatents, src/cache_renderer.cu:1020-1030, :893-900):
- * 0 = warp-level mma.sync, 1 = tcgen05; by default the library takes tcgen05
+ * 0 = warp-level mma.sync, 1 = tcgen05, -1 (the default) = by size: tcgen05
  * for iterations of many rays and mma.sync, whose tiles wait for no round trip
  * to the tensor cores, for few.
  * View-dependent models build on mma.sync.  Slots, known ranges and isset
