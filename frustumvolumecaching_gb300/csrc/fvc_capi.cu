@@ -329,7 +329,7 @@ struct fvc_model {
     uint8_t *d_weights_vd = nullptr;        /* VD_WBYTES of K-major tiles (view-dependent models) */
     uint2 *d_weights_fh = nullptr;          /* the first head as W_L1 / W_L2 fragment packs */
     uint8_t *d_bits = nullptr;
-    uint32_t *d_cells = nullptr;            /* the occupancy in 4 x 4 x 2 words (occupied2) */
+    uint32_t *d_cells = nullptr;            /* the occupancy in 4 x 4 x 2 words, from d_bits in every render (occupied2) */
     __half2 *d_table = nullptr;
     uint2 *d_weights = nullptr;
     uint8_t *d_weights_tc = nullptr;
@@ -665,13 +665,6 @@ static int build_model(const JVal &cfg, std::vector<char> &tab, std::vector<char
         const uint32_t x = compact(j), y = compact(j >> 1), z = compact(j >> 2);
         if (occ[lvl * vals + (size_t)x * 16384 + y * 128 + z]) bits[i / 8] |= (uint8_t)(1u << (i % 8));
     }
-    std::vector<uint32_t> cells(vals * s.grid_nlvl / 32, 0);
-    for (size_t i = 0; i < vals * s.grid_nlvl; ++i) {
-        if (!occ[i]) continue;
-        const uint32_t j = (uint32_t)(i % vals);
-        const size_t b = i / vals * vals + occupancy_bit_index(j >> 14, (j >> 7) & 127u, j & 127u);
-        cells[b / 32] |= 1u << (b % 32);
-    }
 
     /* weights -> fragment order */
     auto u16 = [](const std::vector<char> &v, size_t off_h, size_t n) {
@@ -821,8 +814,7 @@ static int build_model(const JVal &cfg, std::vector<char> &tab, std::vector<char
     CU(cudaDeviceGetAttribute(&m.n_sms, cudaDevAttrMultiProcessorCount, m.device));
     int rc;
     if ((rc = dalloc(&m.d_bits, bits.size(), "occupancy bits"))) return rc;
-    if ((rc = dalloc(&m.d_cells, cells.size(), "occupancy cells"))) return rc;
-    CU(cudaMemcpy(m.d_cells, cells.data(), cells.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    if ((rc = dalloc(&m.d_cells, (size_t)CELL_WORDS * s.grid_nlvl, "occupancy cells"))) return rc;
     if ((rc = dalloc(&m.d_table, (size_t)off * (F / 2), "hash tables"))) return rc;
     if ((rc = dalloc(&m.d_weights, (size_t)W_TOTAL, "weights"))) return rc;
     if ((rc = dalloc(&m.d_bias3, (size_t)64, "bias"))) return rc;
@@ -1854,7 +1846,7 @@ extern "C" int fvc_cache_build(fvc_renderer *r, const fvc_raymarch_info *info)
     CU(cudaMemsetAsync(b.counters, 0, 8 * sizeof(int), s));
     CU(cudaMemsetAsync(c->d_packed, 0xff, (size_t)c->bX * c->bY * c->bZ * sizeof(int32_t), s));
     int n_launches = 2;
-    cache_init_kernel<<<n_tiles, 64, 0, s>>>(p);
+    cache_init_kernel<<<n_tiles + cell_blocks(p.scene.nlvl, 64), 64, 0, s>>>(p, n_tiles);
     CU(cudaGetLastError());
     cache_compact_kernel<<<1, 1024, 0, s>>>(p, n_tiles);
     CU(cudaGetLastError());

@@ -317,13 +317,35 @@ __device__ __forceinline__ void after_previous()
 
 /* The occupancy cells again, as the march reads them: 32-bit words of 4 x 4 x 2
  * cells (bit x & 3 | (y & 3) << 2 | (z & 1) << 4), words x fastest, then y, then
- * z, cascade by cascade; filled from the Morton bits' source when a model is
- * loaded.  A word's index is a sum of the cells' products, where the Morton
- * index takes 18 shifts, products and masks; a word covers a compact block, so
- * the rays of a warp still share words and lines. */
-__host__ __device__ __forceinline__ uint32_t occupancy_bit_index(uint32_t x, uint32_t y, uint32_t z)
+ * z, cascade by cascade: bit x + (x >> 2) 28 + y 4 + (y >> 2) 1008 + z 16 +
+ * (z >> 1) 32736 of a cascade.  A word's index is a sum of the cells' products,
+ * where the Morton index takes 18 shifts, products and masks; a word covers a
+ * compact block, so the rays of a warp still share words and lines.
+ *
+ * The Morton bits are the model's, and a program may write them (their address
+ * is fvc_model_properties'), so every frame, batch, step and build takes the
+ * words from them, in blocks of its first kernel beside those of its rays.  A
+ * word's 32 cells are those of one Morton word, with the bits of their index
+ * (x0 y0 z0 x1 y1) in the order x0 x1 y0 y1 z0: three exchanges of two of
+ * them.  Several streams write the same values. */
+constexpr int CELL_WORDS = 128 * 128 * 128 / 32; /* of a cascade */
+
+/* a word a thread: blocks of 256 or fewer threads divide a cascade's words */
+__host__ __device__ inline int cell_blocks(int nlvl, int threads) { return nlvl * CELL_WORDS / threads; }
+
+__device__ __forceinline__ void cells_from_bits(const uint8_t *bits, uint32_t *cells, int block)
 {
-    return x + (x >> 2) * 28u + y * 4u + (y >> 2) * 1008u + z * 16u + (z >> 1) * 32736u;
+    const uint32_t i = (uint32_t)block * blockDim.x + threadIdx.x;
+    uint32_t w = reinterpret_cast<const uint32_t *>(bits)[i / CELL_WORDS * CELL_WORDS + (expand_bits3(i & 31u) << 1 | expand_bits3(i >> 5 & 31u) << 2 |
+                                                                                        expand_bits3(i >> 10 & 63u))];
+    auto exchange = [&](int shift, uint32_t mask) {
+        const uint32_t t = (w >> shift ^ w) & mask;
+        w ^= t ^ t << shift;
+    };
+    exchange(6, 0x00cc00ccu);
+    exchange(4, 0x00f000f0u);
+    exchange(8, 0x0000ff00u);
+    cells[i] = w;
 }
 
 /* occupied() of the points o + tm[0] d and o + tm[1] d (two steps of a ray),
@@ -368,7 +390,7 @@ __device__ __forceinline__ uint32_t occupied2(const DevScene &sc, const uint8_t 
         const uint32_t ix = __float_as_uint(__fadd_rz(cx, 8388608.0f)), qx = __float_as_uint(__fadd_rz(cx, 33554432.0f));
         const uint32_t iy = __float_as_uint(__fadd_rz(cy, 8388608.0f)), qy = __float_as_uint(__fadd_rz(cy, 33554432.0f));
         const uint32_t iz = __float_as_uint(__fadd_rz(cz, 8388608.0f)), qz = __float_as_uint(__fadd_rz(cz, 16777216.0f));
-        /* occupancy_bit_index of the cell, the sums' exponent bits taken out by the constant (mod 2^32), and the
+        /* the cell's bit, the sums' exponent bits taken out by the constant (mod 2^32), and the
          * cascade's 2^21 bits: mip = 134 - (sb >> 23) */
         const uint32_t bias = 0x4B000000u * (1u + 4u + 16u) + 0x4C000000u * (28u + 1008u) + 0x4B800000u * 32736u;
         uint32_t idx = ix + qx * 28u + iy * 4u + qy * 1008u + iz * 16u + qz * 32736u - bias;

@@ -94,10 +94,15 @@ cudaError_t launch_inference(const InferenceParams &p, int head_hidden, int n_sm
 /* ------------------------------------------------------------------------- */
 
 /* initPayloads_cache_init_kernel, src/cache_renderer.cu:18-81: one CTA of
- * 64 threads per 8x8 tile. */
-__global__ void __launch_bounds__(64) cache_init_kernel(CacheBuildParams p)
+ * 64 threads per 8x8 tile; the blocks past the tiles' write the occupancy
+ * cells. */
+__global__ void __launch_bounds__(64) cache_init_kernel(CacheBuildParams p, int n_tiles)
 {
     const int tile = blockIdx.x;
+    if (tile >= n_tiles) {
+        cells_from_bits(p.bits, p.cells, tile - n_tiles);
+        return;
+    }
     const int k = threadIdx.x;
     const int tx = tile % p.bX, ty = tile / p.bX;
     const int px = tx * 8 + (k & 7), py = ty * 8 + (k >> 3);

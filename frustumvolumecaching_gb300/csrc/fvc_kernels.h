@@ -330,7 +330,7 @@ struct RenderParams {
     DevCam cam;
     DevGrid grid;
     const uint8_t *bits;        /* Morton occupancy bitfield */
-    const uint32_t *cells;      /* the same cells in 4 x 4 x 2 words (occupied2) */
+    uint32_t *cells;            /* the same cells in 4 x 4 x 2 words (occupied2), written from them by the first kernel */
     const __half2 *table;       /* hash tables, F = 2 */
     const uint2 *weights;       /* fragment-ordered MLP weights, W_TOTAL entries */
     const float *bias3;         /* head layer-1 bias from the 1-padding */
@@ -499,7 +499,7 @@ struct CacheBuildParams {
     DevCam cam;
     DevGrid grid;
     const uint8_t *bits;
-    const uint32_t *cells;      /* the same cells in 4 x 4 x 2 words (occupied2) */
+    uint32_t *cells;            /* the same cells in 4 x 4 x 2 words (occupied2), written from them by the first kernel */
     const __half2 *table;
     const uint2 *weights;
     int latent_offset;
@@ -636,7 +636,7 @@ cudaError_t launch_cache_backward(const RenderParams &p, const BwdParams &b, int
 cudaError_t launch_grad_finalize(float *scratch, float *out, size_t n, float inv_scale, int n_sms, cudaStream_t s);
 cudaError_t launch_inference(const InferenceParams &p, int head_hidden, int n_sms, cudaStream_t s);
 
-__global__ void cache_init_kernel(CacheBuildParams p);
+__global__ void cache_init_kernel(CacheBuildParams p, int n_tiles);
 cudaError_t launch_cache_search(const CacheBuildParams &p, int grid, cudaStream_t s);
 cudaError_t launch_cache_density(const CacheBuildParams &p, int grid, cudaStream_t s);
 /* the density network of a build iteration on tcgen05 (models without a first head) */

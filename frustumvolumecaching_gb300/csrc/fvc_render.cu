@@ -106,13 +106,31 @@ __device__ __forceinline__ float start_t1(const DevCam &c, const DevSteps &st, f
     return F_ADD(start, F_MUL(calc_step(st, start), toff));
 }
 
+/* The first `cells` blocks of a ray generation write the occupancy cells
+ * (cells_from_bits); true for them. */
+__device__ __forceinline__ bool write_cells(const RenderParams &p, int cells)
+{
+    if ((int)blockIdx.x >= cells) return false;
+    cells_from_bits(p.bits, p.cells, blockIdx.x);
+    return true;
+}
+
+/* blocks of 256 threads for n rays' threads and the cells, which come first */
+template <class Kernel>
+static void launch_raygen(Kernel kernel, const RenderParams &p, int n, cudaStream_t s)
+{
+    const int cells = cell_blocks(p.scene.nlvl, 256);
+    kernel<<<cells + (n + 255) / 256, 256, 0, s>>>(p, cells);
+}
+
 /* Pixels are visited in 8x4 tiles per warp so that a warp's rays are
  * neighbours (coherent marching and gathers). */
-__global__ void __launch_bounds__(256) wf_raygen_kernel(RenderParams p)
+__global__ void __launch_bounds__(256) wf_raygen_kernel(RenderParams p, int cells)
 {
+    if (write_cells(p, cells)) return;
     const int W = p.cam.W, H = p.cam.H;
     const int tiles_x = (W + 7) / 8, tiles_y = (H + 3) / 4;
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int gid = (blockIdx.x - cells) * blockDim.x + threadIdx.x;
     const int tile = gid >> 5, lane = lane_id();
     if (tile >= tiles_x * tiles_y) return;
     const int x = (tile % tiles_x) * 8 + (lane & 7), y = (tile / tiles_x) * 4 + (lane >> 3);
@@ -144,9 +162,10 @@ __global__ void __launch_bounds__(256) wf_raygen_kernel(RenderParams p)
 
 /* rays for a list of pixels (differentiable render): ray id = list index,
  * results[id] is written for rays that miss the scene box */
-__global__ void __launch_bounds__(256) wf_raygen_list_kernel(RenderParams p)
+__global__ void __launch_bounds__(256) wf_raygen_list_kernel(RenderParams p, int cells)
 {
-    const int at = blockIdx.x * blockDim.x + threadIdx.x;
+    if (write_cells(p, cells)) return;
+    const int at = (blockIdx.x - cells) * blockDim.x + threadIdx.x;
     const int i = at < p.n_list && p.list_order ? p.list_order[at] : at;
     const int W = p.cam.W, H = p.cam.H;
     const int pix = i < p.n_list ? p.pixel_list[i] : -1;
@@ -234,9 +253,10 @@ cudaError_t launch_list_order(const RenderParams &p, int *order, int *rank, int 
 }
 
 /* rays of a batch of views (one thread per pixel of the concatenated views) */
-__global__ void __launch_bounds__(256) wf_raygen_views_kernel(RenderParams p)
+__global__ void __launch_bounds__(256) wf_raygen_views_kernel(RenderParams p, int cells)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (write_cells(p, cells)) return;
+    const int i = (blockIdx.x - cells) * blockDim.x + threadIdx.x;
     const int n = p.view_off[p.n_views];
     const bool valid = i < n;
     bool hits = false;
@@ -2750,8 +2770,8 @@ static cudaError_t run_frame(const RenderParams &params, int n_sms, cudaStream_t
     };
     const int W = p.cam.W, H = p.cam.H;
     const int n_threads = ((W + 7) / 8) * ((H + 3) / 4) * 32;
-    if (p.pixel_list) wf_raygen_list_kernel<<<(p.n_list + 255) / 256, 256, 0, s>>>(p);
-    else wf_raygen_kernel<<<(n_threads + 255) / 256, 256, 0, s>>>(p);
+    if (p.pixel_list) launch_raygen(wf_raygen_list_kernel, p, p.n_list, s);
+    else launch_raygen(wf_raygen_kernel, p, n_threads, s);
     ++L.launches;
     int n_rays = p.pixel_list ? p.n_list : W * H; /* as of the last readback */
     int next_check = check_interval(SubIter(p, n_rays).windows, check_every);
@@ -2853,7 +2873,7 @@ cudaError_t launch_wait_selftest(long long limit_cycles, long long *d_out, cudaS
 cudaError_t launch_fill_raygen(const RenderParams &p, cudaStream_t s)
 {
     const int n_threads = ((p.cam.W + 7) / 8) * ((p.cam.H + 3) / 4) * 32;
-    wf_raygen_kernel<<<(n_threads + 255) / 256, 256, 0, s>>>(p);
+    launch_raygen(wf_raygen_kernel, p, n_threads, s);
     return cudaGetLastError();
 }
 
@@ -2878,7 +2898,7 @@ static cudaError_t run_backward(const RenderParams &p, const BwdParams &b, int n
     }
     LaunchLog local;
     LaunchLog &L = log ? *log : local;
-    if (!one_round) wf_raygen_list_kernel<<<(p.n_list + 255) / 256, 256, 0, s>>>(p);
+    if (!one_round) launch_raygen(wf_raygen_list_kernel, p, p.n_list, s);
     L.launches += one_round ? 0 : 1;
     /* the network adjoint's launches are timed (when the renderer's kernel timing is on) */
     auto timed_begin = [&]() {
@@ -2956,7 +2976,7 @@ static cudaError_t build_batch_graph_t(const RenderParams &p, int n_sms, cudaStr
         cudaMemsetAsync(p.ray_counter, 0, 4 * sizeof(int), s);
         cudaMemsetAsync(p.stats, 0, sizeof(RenderStatsDev), s);
         cudaMemsetAsync(p.counters, 0, N_COUNTERS * sizeof(int), s);
-        wf_raygen_views_kernel<<<(n_rays + 255) / 256, 256, 0, s>>>(p);
+        launch_raygen(wf_raygen_views_kernel, p, n_rays, s);
         cudaGraph_t g2 = nullptr;
         e = cudaStreamEndCapture(s, &g2);
     }
