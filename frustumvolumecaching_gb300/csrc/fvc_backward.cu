@@ -769,7 +769,8 @@ __global__ void __launch_bounds__(BT_THREADS, 2) wf_net_bwd_tc_kernel(RenderPara
 #pragma unroll 1
                 for (int c = l0 / 4; c < (l0 + BT_NL) / 4; ++c) {
                     __half2 feat[4];
-                    hash_group_f2<4>(p.grid, p.table, pos, 4 * c, feat);
+                    if (p.grid.wide) hash_group_f2<4, true>(p.grid, p.table, pos, 4 * c, feat);
+                    else hash_group_f2<4, false>(p.grid, p.table, pos, 4 * c, feat);
                     uint32_t f[4];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {

@@ -629,6 +629,7 @@ static int build_model(const JVal &cfg, std::vector<char> &tab, std::vector<char
     g.n_levels = n_levels;
     g.F = F;
     g.dense_mask = 0;
+    g.wide = 0;
     const JVal &ls = enc["fvc_level_scales"];
     const float log2b = std::log2(b);
     uint32_t off = 0;
@@ -641,6 +642,7 @@ static int build_model(const JVal &cfg, std::vector<char> &tab, std::vector<char
         const uint32_t size = (uint32_t)std::min<uint64_t>(n, 1ull << log2T);
         g.scale[l] = scale; g.res[l] = res; g.res2[l] = res * res; g.size[l] = size; g.offset[l] = off * (uint32_t)(F / 2);
         if ((uint64_t)res * res * res <= size) g.dense_mask |= 1u << l;
+        if (scale >= WIDE_SCALE) g.wide = 1;
         off += size;
     }
     m.table_entries = off;

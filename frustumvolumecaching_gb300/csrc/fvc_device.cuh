@@ -55,6 +55,7 @@ constexpr int MAX_LEVELS = 16;
 struct DevGrid {
     int n_levels;
     int F;                /* features per level: 2 (16 levels) or 4 (8 levels); offset[] counts half2 */
+    int wide;             /* a level's cells reach 2^22 (grid_axis) */
     uint32_t dense_mask;
     float scale[MAX_LEVELS];
     uint32_t res[MAX_LEVELS], res2[MAX_LEVELS], size[MAX_LEVELS], offset[MAX_LEVELS];
@@ -516,12 +517,21 @@ __device__ __forceinline__ float2 f2_lerp(float2 a, float2 b, float t)
  * fraction above it.  Rounding p + 1.5 * 2^23 downwards leaves floor(p) in the
  * sum's low bits (|p| < 2^22), so the floor, the integer and the fraction are
  * plain additions instead of conversions, which a quarter-rate unit executes.
- * Beyond that, and for a p that is not a number, the cell is any: the level's
+ * A grid with finer levels than that is WIDE and converts.  Beyond 2^22
+ * otherwise, and for a p that is not a number, the cell is any: the level's
  * index keeps it inside the table (hashed levels mask, dense ones dense_entry),
  * and the fraction of a NaN is NaN. */
+constexpr float WIDE_SCALE = 4194303.0f; /* scale * 1 + 0.5 stays below 2^22 */
+
+template <bool WIDE>
 __device__ __forceinline__ uint32_t grid_axis(float scale, float x, float &w)
 {
     const float p = __fmaf_rn(scale, x, 0.5f);
+    if (WIDE) {
+        const float f = floorf(p);
+        w = __fsub_rn(p, f);
+        return (uint32_t)(int)f;
+    }
     const float t = __fadd_rd(p, 12582912.0f);
     w = __fsub_rn(p, __fsub_rn(t, 12582912.0f));
     return __float_as_uint(t) - 0x4B400000u;
@@ -544,7 +554,7 @@ __device__ __forceinline__ uint32_t dense_entry(uint32_t i, uint32_t size)
 /* the 4-feature grid (instant-ngp's 8 levels x 4 features): an entry is two
  * half2 (one 8-byte gather per corner), the level's features go to
  * out[2l], out[2l + 1]: G levels from l0 on */
-template <int G>
+template <int G, bool WIDE>
 __device__ __forceinline__ void hash_group_f4(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, int l0, __half2 *out)
 {
     uint2 v[G][8];
@@ -553,7 +563,7 @@ __device__ __forceinline__ void hash_group_f4(const DevGrid &g, const __half2 *_
     for (int j = 0; j < G; ++j) {
         const int l = l0 + j;
         const float sc = g.scale[l];
-        const uint32_t gx = grid_axis(sc, pos.x, wx[j]), gy = grid_axis(sc, pos.y, wy[j]), gz = grid_axis(sc, pos.z, wz[j]);
+        const uint32_t gx = grid_axis<WIDE>(sc, pos.x, wx[j]), gy = grid_axis<WIDE>(sc, pos.y, wy[j]), gz = grid_axis<WIDE>(sc, pos.z, wz[j]);
         const uint32_t size = g.size[l];
         const uint2 *tl = reinterpret_cast<const uint2 *>(table + g.offset[l]);
         if ((g.dense_mask >> l) & 1u) {
@@ -589,7 +599,7 @@ __device__ __forceinline__ void hash_group_f4(const DevGrid &g, const __half2 *_
 }
 
 /* LG levels of the 2-feature grid from l0 on: one half2 each */
-template <int LG>
+template <int LG, bool WIDE>
 __device__ __forceinline__ void hash_group_f2(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, int l0, __half2 *out)
 {
     __half2 v[LG][8];
@@ -598,7 +608,7 @@ __device__ __forceinline__ void hash_group_f2(const DevGrid &g, const __half2 *_
     for (int j = 0; j < LG; ++j) {
         const int l = l0 + j;
         const float sc = g.scale[l];
-        const uint32_t gx = grid_axis(sc, pos.x, wx[j]), gy = grid_axis(sc, pos.y, wy[j]), gz = grid_axis(sc, pos.z, wz[j]);
+        const uint32_t gx = grid_axis<WIDE>(sc, pos.x, wx[j]), gy = grid_axis<WIDE>(sc, pos.y, wy[j]), gz = grid_axis<WIDE>(sc, pos.z, wz[j]);
         const uint32_t size = g.size[l];
         const __half2 *tl = table + g.offset[l];
         if ((g.dense_mask >> l) & 1u) {
@@ -633,16 +643,23 @@ __device__ __forceinline__ void hash_group_f2(const DevGrid &g, const __half2 *_
 }
 
 /* levels l_begin .. l_end - 1 into out[] (level l in out[l], or out[2l] and out[2l + 1]), LG half2 at a time */
+template <int LG, bool WIDE>
+__device__ __forceinline__ void hash_encode_range(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, __half2 *out, int l_begin,
+                                                  int l_end)
+{
+    constexpr int G = LG / 2 > 0 ? LG / 2 : 1;
+    if (g.F == 4) {
+        for (int l = l_begin; l < l_end; l += G) hash_group_f4<G, WIDE>(g, table, pos, l, out + 2 * l);
+        return;
+    }
+    for (int l = l_begin; l < l_end; l += LG) hash_group_f2<LG, WIDE>(g, table, pos, l, out + l);
+}
 template <int LG = 4>
 __device__ __forceinline__ void hash_encode_levels(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, __half2 *out,
                                                    int l_begin, int l_end)
 {
-    constexpr int G = LG / 2 > 0 ? LG / 2 : 1;
-    if (g.F == 4) {
-        for (int l = l_begin; l < l_end; l += G) hash_group_f4<G>(g, table, pos, l, out + 2 * l);
-        return;
-    }
-    for (int l = l_begin; l < l_end; l += LG) hash_group_f2<LG>(g, table, pos, l, out + l);
+    if (g.wide) hash_encode_range<LG, true>(g, table, pos, out, l_begin, l_end);
+    else hash_encode_range<LG, false>(g, table, pos, out, l_begin, l_end);
 }
 
 /* all levels of the grid (features of level l in out[l]) */

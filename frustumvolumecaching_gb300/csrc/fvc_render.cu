@@ -1357,10 +1357,13 @@ __device__ __forceinline__ void nt_encode(const DevGrid &g, const __half2 *__res
     for (int c = 0; c < 4; ++c) {
         __half2 f[4];
         if (GENERAL && g.F == 4) {
-            hash_group_f4<2>(g, table, pos, 2 * c, f);
+            if (g.wide) hash_group_f4<2, true>(g, table, pos, 2 * c, f);
+            else hash_group_f4<2, false>(g, table, pos, 2 * c, f);
+        } else if (GENERAL && g.wide) {
+            hash_group_f2<4, true>(g, table, pos, 4 * c, f);
         } else {
 #pragma unroll
-            for (int j = 0; j < 4; j += FVC_NT_HASH_GROUP) hash_group_f2<FVC_NT_HASH_GROUP>(g, table, pos, 4 * c + j, f + j);
+            for (int j = 0; j < 4; j += FVC_NT_HASH_GROUP) hash_group_f2<FVC_NT_HASH_GROUP, false>(g, table, pos, 4 * c + j, f + j);
         }
         __syncwarp();
         tmem_st4(acc + NT_A + 4 * c, nt_from_half<PREC>(f));
@@ -1395,8 +1398,9 @@ struct NtRow {
  * classified by the march in one launch, the resample list's tiles first
  * (hash features, density layers, head), then the cache list's tiles (the
  * head input of each row's lookup, wf_cache_lookup_kernel; head only), so
- * that no tile mixes the two kinds of row.  GENERAL: the 4-feature grid and
- * the head with the frequency encoding; without it the kernel is smaller.
+ * that no tile mixes the two kinds of row.  GENERAL: the 4-feature grid, WIDE
+ * levels (grid_axis) and the head with the frequency encoding; without it the
+ * kernel is smaller.
  * PREC 1: bf16 layers (plain renders): outputs in bf16, stored as fp16 like
  * the fp16 path. */
 template <int MODE, int HH, bool LIST, bool GENERAL, int PREC = 0>
@@ -1544,7 +1548,7 @@ template <int MODE, int HH, bool LIST, int PREC = 0>
 static void launch_net_tc(const RenderParams &p, int it, int n_sms, cudaStream_t s)
 {
     const size_t smem = nt_smem_bytes(p.freq);
-    auto kernel = p.freq || p.grid.F == 4 ? wf_net_tc_kernel<MODE, HH, LIST, true, PREC> : wf_net_tc_kernel<MODE, HH, LIST, false, PREC>;
+    auto kernel = p.freq || p.grid.F == 4 || p.grid.wide ? wf_net_tc_kernel<MODE, HH, LIST, true, PREC> : wf_net_tc_kernel<MODE, HH, LIST, false, PREC>;
     if (p.views) kernel<<<n_sms, NT_THREADS, smem, s>>>(p, it);
     else launch_after(kernel, n_sms, NT_THREADS, smem, s, p, it);
 }
@@ -1635,7 +1639,7 @@ cudaError_t launch_cache_density_tc(const CacheBuildParams &p, const uint8_t *we
         return e;
     });
     if (e != cudaSuccess) return e;
-    launch_after(p.grid.F == 4 ? cache_density_tc_kernel<true> : cache_density_tc_kernel<false>, n_sms, NT_THREADS, sizeof(NtSmem), s, p, weights_tc,
+    launch_after(p.grid.F == 4 || p.grid.wide ? cache_density_tc_kernel<true> : cache_density_tc_kernel<false>, n_sms, NT_THREADS, sizeof(NtSmem), s, p, weights_tc,
                  p.build_row_counter);
     return cudaGetLastError();
 }
