@@ -55,7 +55,7 @@ constexpr int MAX_LEVELS = 16;
 struct DevGrid {
     int n_levels;
     int F;                /* features per level: 2 (16 levels) or 4 (8 levels); offset[] counts half2 */
-    int wide;             /* a level's cells reach 2^22 (grid_axis) */
+    int wide;             /* a level has 2^21 cells an axis or more (grid_axis) */
     uint32_t dense_mask;
     float scale[MAX_LEVELS];
     uint32_t res[MAX_LEVELS], res2[MAX_LEVELS], size[MAX_LEVELS], offset[MAX_LEVELS];
@@ -517,11 +517,11 @@ __device__ __forceinline__ float2 f2_lerp(float2 a, float2 b, float t)
  * fraction above it.  Rounding p + 1.5 * 2^23 downwards leaves floor(p) in the
  * sum's low bits (|p| < 2^22), so the floor, the integer and the fraction are
  * plain additions instead of conversions, which a quarter-rate unit executes.
- * A grid with finer levels than that is WIDE and converts.  Beyond 2^22
- * otherwise, and for a p that is not a number, the cell is any: the level's
- * index keeps it inside the table (hashed levels mask, dense ones dense_entry),
- * and the fraction of a NaN is NaN. */
-constexpr float WIDE_SCALE = 4194303.0f; /* scale * 1 + 0.5 stays below 2^22 */
+ * Grids of finer levels and a query's positions outside the grid are WIDE and
+ * convert (hash_encode_any).  For a p beyond 2^22 or not a number the cell is
+ * any otherwise: the level's index keeps it inside the table (hashed levels
+ * mask, dense ones dense_entry), and the fraction of a NaN is NaN. */
+constexpr float WIDE_SCALE = 2097152.0f; /* scale * x + 0.5 stays below 2^22 up to x = 2 */
 
 template <bool WIDE>
 __device__ __forceinline__ uint32_t grid_axis(float scale, float x, float &w)
@@ -537,11 +537,14 @@ __device__ __forceinline__ uint32_t grid_axis(float scale, float x, float &w)
     return __float_as_uint(t) - 0x4B400000u;
 }
 
-/* A dense level's entry: i % size for the indices of [0, 1]^3, which stay below 2 * size (i - size wraps to a large
- * number for i < size); an entry of the level for any other, as a query's positions are the caller's. */
+/* A dense level's entry, i % size: the indices of [0, 1]^3 stay below 2 * size, and i - size wraps to a large number for
+ * i < size; without WIDE any other index gives an entry of the level. */
+template <bool WIDE>
 __device__ __forceinline__ uint32_t dense_entry(uint32_t i, uint32_t size)
 {
-    return min(min(i, i - size), size - 1u);
+    const uint32_t e = min(i, i - size);
+    if (WIDE) return e < size ? e : i % size;
+    return min(e, size - 1u);
 }
 
 /* Encodes one position into 2*n_levels features (fp16) written to
@@ -571,7 +574,7 @@ __device__ __forceinline__ void hash_group_f4(const DevGrid &g, const __half2 *_
             const uint32_t b = gx + gy * r + gz * r2;
 #pragma unroll
             for (int c = 0; c < 8; ++c)
-                v[j][c] = __ldg(tl + dense_entry(b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u), size));
+                v[j][c] = __ldg(tl + dense_entry<WIDE>(b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u), size));
         } else {
             const uint32_t hy0 = gy * 2654435761u, hy1 = (gy + 1u) * 2654435761u;
             const uint32_t hz0 = gz * 805459861u, hz1 = (gz + 1u) * 805459861u;
@@ -620,7 +623,7 @@ __device__ __forceinline__ void hash_group_f2(const DevGrid &g, const __half2 *_
             } else {
 #pragma unroll
                 for (int c = 0; c < 8; ++c)
-                    v[j][c] = __ldg(tl + dense_entry(b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u), size));
+                    v[j][c] = __ldg(tl + dense_entry<WIDE>(b + ((c & 1) ? 1u : 0u) + ((c & 2) ? r : 0u) + ((c & 4) ? r2 : 0u), size));
             }
         } else {
             const uint32_t hy0 = gy * 2654435761u, hy1 = (gy + 1u) * 2654435761u;
@@ -667,6 +670,14 @@ template <int LG = 4>
 __device__ __forceinline__ void hash_encode(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, __half2 *out)
 {
     hash_encode_levels<LG>(g, table, pos, out, 0, g.n_levels);
+}
+
+/* the same at any position, as a query's are the caller's: outside [0, 1]^3 and for a NaN as in a WIDE grid */
+__device__ __forceinline__ void hash_encode_any(const DevGrid &g, const __half2 *__restrict__ table, float3 pos, __half2 *out)
+{
+    const bool inside = fminf(fminf(pos.x, pos.y), pos.z) >= 0.0f && pos.x <= 1.0f && pos.y <= 1.0f && pos.z <= 1.0f;
+    if (g.wide || !inside) hash_encode_range<4, true>(g, table, pos, out, 0, g.n_levels);
+    else hash_encode_range<4, false>(g, table, pos, out, 0, g.n_levels);
 }
 
 /* SH degree 4 (16 values) of a unit_to_01 direction, written as 8 half2.

@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(128) inference_kernel(InferenceParams p)
         __half *trow = tile + lane * TILE_STRIDE;
         if (r < p.n) {
             const float3 pos = make_float3(p.pos[3 * r], p.pos[3 * r + 1], p.pos[3 * r + 2]);
-            hash_encode(p.grid, p.table, pos, reinterpret_cast<__half2 *>(trow));
+            hash_encode_any(p.grid, p.table, pos, reinterpret_cast<__half2 *>(trow));
             if (p.features)
                 for (int j = 0; j < 32; ++j) p.features[32 * r + j] = __half2float(trow[j]);
             if (p.dir) sh16(make_float3(p.dir[3 * r], p.dir[3 * r + 1], p.dir[3 * r + 2]), reinterpret_cast<__half2 *>(trow + 32));
