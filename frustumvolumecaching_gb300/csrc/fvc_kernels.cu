@@ -20,9 +20,6 @@ namespace fvc {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-__device__ __forceinline__ unsigned lanemask_lt() { unsigned m; asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m)); return m; }
-
-
 /* ------------------------------------------------------------------------- */
 /* network at given inputs (testing / occupancy generation)                   */
 /* ------------------------------------------------------------------------- */
@@ -774,7 +771,7 @@ __global__ void __launch_bounds__(256) pr_reserve_kernel(PerRayFillParams p)
         const unsigned m = __ballot_sync(FULL, fresh);
         if (marked) p.flag[b] = 0;
         if (fresh) {
-            const int slot = first + __popc(m & lanemask_lt());
+            const int slot = first + __popc(m & lanes_below());
             if (slot < p.capacity) {
                 const int sx = slot / (p.dY * p.dZ), sy = (slot - sx * p.dY * p.dZ) / p.dZ;
                 const int sz = slot - sx * p.dY * p.dZ - sy * p.dZ;
@@ -883,11 +880,7 @@ __global__ void __launch_bounds__(128) pr_write_kernel(PerRayFillParams p, int i
         int wbase = 0;
         if ((threadIdx.x & 31) == 0 && m) wbase = atomicAdd(p.counters + ((it + 1) & 1), __popc(m));
         wbase = __shfl_sync(0xffffffffu, wbase, 0);
-        if (alive) {
-            unsigned lt;
-            asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-            next[wbase + __popc(m & lt)] = st;
-        }
+        if (alive) next[wbase + __popc(m & lanes_below())] = st;
     }
 }
 

@@ -58,7 +58,6 @@ constexpr int NET_WARPS = 8;
 #define FVC_TC_HASH_GROUP 4
 #endif
 
-__device__ __forceinline__ unsigned lane_lt() { unsigned m; asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m)); return m; }
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
 /* compensated (Kahan) summation: sum += v with the running error in c */
@@ -156,7 +155,7 @@ __global__ void __launch_bounds__(256) wf_raygen_kernel(RenderParams p, int cell
         st.comp = make_float4(0.f, 0.f, 0.f, 0.f);
         st.cnt = make_int4(id, 0, 0, 0);
         st.cnt2 = make_int4(0, 0, 0, 0);
-        p.states[0][base + __popc(m & lane_lt())] = st;
+        p.states[0][base + __popc(m & lanes_below())] = st;
     }
 }
 
@@ -190,7 +189,7 @@ __global__ void __launch_bounds__(256) wf_raygen_list_kernel(RenderParams p, int
         st.comp = make_float4(0.f, 0.f, 0.f, 0.f);
         st.cnt = make_int4(i, 0, 0, 0);
         st.cnt2 = make_int4(0, 0, 0, 0);
-        p.states[0][base + __popc(m & lane_lt())] = st;
+        p.states[0][base + __popc(m & lanes_below())] = st;
     }
 }
 
@@ -288,7 +287,7 @@ __global__ void __launch_bounds__(256) wf_raygen_views_kernel(RenderParams p, in
         st.comp = make_float4(0.f, 0.f, 0.f, 0.f);
         st.cnt = make_int4(i, 0, 0, 0);
         st.cnt2 = make_int4(0, 0, 0, view);
-        p.states[0][base + __popc(m & lane_lt())] = st;
+        p.states[0][base + __popc(m & lanes_below())] = st;
     }
 }
 
@@ -799,8 +798,8 @@ __global__ void __launch_bounds__(32 * ML_LANES) wf_march_lanes_kernel(RenderPar
                     }
                     rb = __shfl_sync(FULLMASK, rb, 0);
                     hb = __shfl_sync(FULLMASK, hb, 0);
-                    if (kind == KIND_RESAMPLE) p.res_list[rb + __popc(m0 & lane_lt())] = r;
-                    else if (kind == KIND_CACHE) p.cache_list[hb + __popc(m1 & lane_lt())] = r;
+                    if (kind == KIND_RESAMPLE) p.res_list[rb + __popc(m0 & lanes_below())] = r;
+                    else if (kind == KIND_CACHE) p.cache_list[hb + __popc(m1 & lanes_below())] = r;
                 }
             }
             if (l == 0 && valid) p.ray_rows[(size_t)w * sub.stride + i] = make_int2(first, window_pack(n, steps, done));
@@ -942,9 +941,9 @@ __global__ void __launch_bounds__(256) wf_classify_kernel(RenderParams p, int it
         }
         b0 = __shfl_sync(FULLMASK, b0, 0);
         b1 = __shfl_sync(FULLMASK, b1, 0);
-        if (kind == KIND_RESAMPLE) p.res_list[b0 + __popc(m0 & lane_lt())] = r;
+        if (kind == KIND_RESAMPLE) p.res_list[b0 + __popc(m0 & lanes_below())] = r;
         if (kind == KIND_CACHE) {
-            const int kc = b1 + __popc(m1 & lane_lt());
+            const int kc = b1 + __popc(m1 & lanes_below());
             p.cache_list[kc] = r;
             p.row_lat[kc] = make_uint4(pack_h2(lat[0], lat[1]), pack_h2(lat[2], lat[3]), pack_h2(lat[4], lat[5]), pack_h2(lat[6], lat[7]));
             p.row_out[r] = make_uint2(0u, (uint32_t)__half_as_ushort(__float2half_rn(logd)) << 16);
@@ -2205,7 +2204,7 @@ __global__ void __launch_bounds__(128, CACHED ? 7 : 6) wf_composite_kernel(Rende
         int nb = 0;
         if (lane_id() == 0 && m) nb = atomicAdd(p.counters + ((it + 1) & 1), __popc(m));
         nb = __shfl_sync(FULLMASK, nb, 0);
-        if (keep) nxt[nb + __popc(m & lane_lt())] = st;
+        if (keep) nxt[nb + __popc(m & lanes_below())] = st;
     }
 }
 
@@ -2322,7 +2321,7 @@ __global__ void __launch_bounds__(32 * CL_WARPS) wf_composite_lanes_kernel(Rende
             int nb = 0;
             if (lane == 0 && m) nb = atomicAdd(p.counters + ((it + 1) & 1), __popc(m));
             nb = __shfl_sync(FULLMASK, nb, 0);
-            if (keep) nxt[nb + __popc(m & lane_lt())] = st;
+            if (keep) nxt[nb + __popc(m & lanes_below())] = st;
         }
         __syncthreads();
     }
@@ -2439,11 +2438,11 @@ __global__ void __launch_bounds__(COMP_THREADS) wf_composite_bwd_kernel(RenderPa
                 bool res, hit;
                 with_gradient(k0 + lane_id(), res, hit);
                 const unsigned m0 = __ballot_sync(FULLMASK, res);
-                if (res) p.grad_res_list[rb + __popc(m0 & lane_lt())] = first + k0 + lane_id();
+                if (res) p.grad_res_list[rb + __popc(m0 & lanes_below())] = first + k0 + lane_id();
                 rb += __popc(m0);
                 if (!CACHED) continue;
                 const unsigned m1 = __ballot_sync(FULLMASK, hit);
-                if (hit) p.grad_cache_list[hb + __popc(m1 & lane_lt())] = first + k0 + lane_id();
+                if (hit) p.grad_cache_list[hb + __popc(m1 & lanes_below())] = first + k0 + lane_id();
                 hb += __popc(m1);
             }
             __syncwarp(); /* the next window overwrites the rows */
@@ -2458,7 +2457,7 @@ __global__ void __launch_bounds__(COMP_THREADS) wf_composite_bwd_kernel(RenderPa
         int nb = 0;
         if (lane_id() == 0 && m) nb = atomicAdd(p.counters + ((it + 1) & 1), __popc(m));
         nb = __shfl_sync(FULLMASK, nb, 0);
-        if (keep) nxt[nb + __popc(m & lane_lt())] = st;
+        if (keep) nxt[nb + __popc(m & lanes_below())] = st;
     }
 }
 
