@@ -33,7 +33,7 @@ def main(argv=None) -> None:
     ap.add_argument("--network", choices=["tc", "mma"], default="tc")
     ap.add_argument("--rays", type=int, default=1 << 16, help="rays per backward step")
     ap.add_argument("--tile", type=int, choices=[64, 128, 256], default=128, help="tcgen05 network tile height (plain path)")
-    ap.add_argument("--batch-rows", type=int, default=0, help="compaction batch, rows per sub-iteration (0: capacity)")
+    ap.add_argument("--batch-rows", type=int, default=0, help="compaction batch, rows of a march window (0: by the image's size)")
     ap.add_argument("--skip", action="store_true", help="empty-space skipping in the march (off by default, as in the library)")
     ap.add_argument("--scene", choices=["c2", "c1"], default="c2",
                     help="c2: the cached workload's scene and camera path; c1: the 256x256 workload's scene, seeded camera")

@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(BW_WARPS * 32, 1) wf_net_bwd_kernel(RenderPara
  * forward weight tiles MN-major as their B = W, so one copy of each weight
  * serves both directions.
  * The weight gradients accumulate in TMEM and are added to the global blobs
- * BT_DW_ADDS times a launch; no shared-memory atomics.
+ * some BT_DW_ADDS times a launch; no shared-memory atomics.
  * The weight-gradient MMAs use M = 128 with their 64 meaningful rows in TMEM
  * lanes 0..63: a 64-column tile read MN-major with M = 128 runs up to 1023
  * bytes past its end, which stays inside the next tile.
@@ -597,6 +597,14 @@ __device__ __forceinline__ void red_add4(float *a, float x, float y, float z, fl
  * wider than about one step) */
 constexpr int SC_PAIR_LEVELS = 10;
 
+/* Levels a turn of the scatter's loop, which the compiler keeps, as it does the
+ * encode's over four levels and the epilogues' over two halves: unrolled, the
+ * kernel's warps waited for instructions longer than for anything but the L2
+ * (4.6 of 13 stall cycles an instruction).  A 2^18-ray step of the 256x256
+ * workload's scene, ms: all unrolled 25.4, encode and scatter four levels a
+ * turn 23.9, epilogues halved 23.0, scatter two levels 21.43, one 21.41. */
+constexpr int SC_GROUP = 1;
+
 /* Adjoint of hash_encode over levels l0 .. l0 + NL - 1 of the 16-level grid,
  * called by all 32 lanes of a warp (rows without a gradient pass zeros).
  * Per level:
@@ -607,13 +615,6 @@ constexpr int SC_PAIR_LEVELS = 10;
  *     {2i, 2i+1} (a hashed level's cell with even x, or adjacent dense
  *     indices) go out as one 16-byte red.global.add.v4.f32.
  * The table receives the same sums with fewer L2 atomics. */
-/* Levels a turn of the scatter's loop, which the compiler keeps, as it does the
- * encode's over four levels and the epilogues' over two halves: unrolled, the
- * kernel's warps waited for instructions longer than for anything but the L2
- * (4.6 of 13 stall cycles an instruction).  A 2^18-ray step of the 256x256
- * workload's scene, ms: all unrolled 25.4, encode and scatter four levels a
- * turn 23.9, epilogues halved 23.0, scatter two levels 21.43, one 21.41. */
-constexpr int SC_GROUP = 1;
 template <int NL>
 __device__ __forceinline__ void hash_scatter_levels(const DevGrid &g, float *gt, float3 pos, int l0, const float (&dF)[2 * NL], int lane)
 {
@@ -681,7 +682,8 @@ __device__ __forceinline__ void hash_scatter_levels(const DevGrid &g, float *gt,
 }
 
 /* A CTA adds its weight gradients to the global blobs, and starts from zero,
- * BT_DW_ADDS times, but not more often than every second tile.  The tensor
+ * after every n-th of its tiles and the last: n = tiles / BT_DW_ADDS rounded
+ * down, at least 2 (so up to half as often again as BT_DW_ADDS).  The tensor
  * core truncates its sums, so they lose some 5e-7 of their value a tile, and
  * each addition to the blobs rounds.  Relative error of the weight gradients
  * (head layers) against steps of 2048 rays added up in float64, with one

@@ -377,7 +377,7 @@ struct RenderParams {
                                  * [8] the rows granted when more were asked for than the buffers hold */
     int by_sample;              /* a warp's rows sample by sample instead of ray by ray (RowWalk) */
     int march_lanes;            /* few rays: 8 lanes march a ray (wf_march_lanes_kernel; its rows lie ray by ray) */
-    int steps_per_iter;         /* marching steps per ray and sub-iteration */
+    int steps_per_iter;         /* marching steps per ray and march window */
     int m_tile;                 /* rows per tcgen05 network tile on the plain path: 64, 128 (0 = 128) or 256 */
     int fused_classify;         /* cached renders: classification in the march, one network launch for all rows */
     int skip_empty;             /* the march skips occupancy lookups inside empty cells (exact: occupied_skip) */
@@ -627,7 +627,8 @@ cudaError_t build_batch_graph(const RenderParams &p, bool cached, int head_hidde
  * the adjoints run */
 cudaError_t backward_frame(const RenderParams &p, const BwdParams &b, bool cached, int head_hidden, int n_sms, cudaStream_t s,
                            int *h_pinned, int check_every, bool one_round, LaunchLog *log = nullptr);
-/* orders the pixel list by tiles of the image: order[] from rank[] (n_list) and bins[] (n_bins + 1), n_bins <= LIST_BINS */
+/* orders the pixel list by tiles of the image: order[] from rank[] (n_list) and bins[] (LIST_BINS; a tile each, and one for
+ * pixels outside the image) */
 constexpr int LIST_BINS = 16384;
 cudaError_t launch_list_order(const RenderParams &p, int *order, int *rank, int *bins, cudaStream_t s);
 cudaError_t launch_loss(const RenderParams &p, const BwdParams &b, cudaStream_t s);

@@ -2750,7 +2750,10 @@ static void launch_composite(const RenderParams &p, int it, int n_rays, int n_sm
     else launch_after(kernel, grid, block, 0, s, p, it);
 }
 
-/* sub-iterations between two readbacks of the alive count: with more march windows a sub-iteration there are fewer */
+/* Sub-iterations between two readbacks of the alive count: with more march windows a sub-iteration there are fewer, and
+ * one too many costs its launches.  us, always every 4 / these: 64x64 287 / 278, 256x256 1357 / 1343, per-ray cached 640x360
+ * 4218 / 4021, larger frames alike; always every one / these: opaque 1283x717 8665 / 8535, plain 1080p 30.92 / 30.67 ms,
+ * smaller frames alike. */
 static inline int check_interval(int windows, int every) { return windows >= 8 ? 1 : windows > 1 ? std::min(every, 2) : every; }
 
 template <bool CACHED, int HH>

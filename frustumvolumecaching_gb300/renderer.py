@@ -180,7 +180,7 @@ class Renderer:
         L.check(L.load().fvc_renderer_set_network_path(self.handle, int(bool(use_tcgen05))))
 
     def set_build_network_path(self, use_tcgen05: bool | None) -> None:
-        """The cache builds' density network: mma.sync, tcgen05 or (None, the default) by the build's size; same slots and voxels."""
+        """The cache builds' density network: mma.sync, tcgen05 or (None, the default) by the build's size; same slots, voxels to fp16 rounding."""
         path = -1 if use_tcgen05 is None else int(bool(use_tcgen05))
         L.check(L.load().fvc_renderer_set_build_network_path(self.handle, path))
 

@@ -307,9 +307,10 @@ typedef struct {
  * PerformanceRenderer::render (src/performance_renderer.cu:214-286) or
  * CachePerformanceRenderer::render (src/cache_performance_renderer.cu:1059-1263).
  * Device pointers.  The sub-iterations are enqueued on the renderer stream;
- * the host reads the alive-ray count back every 4 sub-iterations, so the
- * call returns once the last sub-iteration is enqueued (the final writes may
- * still be in flight on the stream). */
+ * the host reads the alive-ray count back every 4 sub-iterations (every 2 of
+ * more than one march window, each of 8 or more), so the call returns once the
+ * last sub-iteration is enqueued (the final writes may still be in flight on
+ * the stream). */
 int fvc_render_device(fvc_renderer *r, const fvc_raymarch_info *info, const fvc_render_outputs *out);
 /* Same with host pointers: H2D of the previous image (progressive average),
  * render, D2H of the outputs, synchronise. */
@@ -333,15 +334,17 @@ int fvc_renderer_set_network_path(fvc_renderer *r, int use_tcgen05);
  * for iterations of many rays and mma.sync, whose tiles wait for no round trip
  * to the tensor cores, for few.
  * View-dependent models build on mma.sync.  Slots, known ranges and isset
- * flags do not depend on it; voxel values agree to fp16 rounding.  No
- * reference counterpart. */
+ * flags do not depend on it; voxel values agree to fp16 rounding (the two
+ * units add a layer's products in their own order).  No reference
+ * counterpart. */
 int fvc_renderer_set_build_network_path(fvc_renderer *r, int use_tcgen05);
 
 /* Rows per tcgen05 network tile of the plain path (64, 128 or 256; FP16, not
- * view-dependent; default 128) and the compaction batch, the rows per
- * sub-iteration the march aims at (0: the renderer's row capacity, the
- * default; else in [2^10, 2^26], capped at the capacity).  Results do not
- * depend on either: every row's arithmetic is the same. */
+ * view-dependent; default 128) and the compaction batch, the rows per march
+ * window that the march aims at (0, the default: 16 a ray, at most 2^25, in as
+ * many windows a sub-iteration as the image's size gives; else in [2^10, 2^26],
+ * capped at those, and one window).  Results do not depend on either: every
+ * row's arithmetic is the same. */
 int fvc_renderer_set_tiling(fvc_renderer *r, int m_tile, int batch_rows);
 
 /* Cache renderers (CACHE_PERFORMANCE, tcgen05 path, density head): 1 (the
