@@ -49,9 +49,9 @@ BYTES_CACHE_ROW = 16 + 4 + 8 + 28  # per cache row: head input + log-density rea
 SCENE_SIZING = (64, 0.25)  # cache sizing of the scene-sized run: 64 samples per ray, brick sparsity 0.25
 MISS_FIELDS = ("n_miss_outside_fov", "n_miss_outside_depth", "n_miss_before_near", "n_miss_beyond_known",
                "n_drop_brick_unset", "n_drop_voxel_empty")
-# DRAM bytes (read + write) per resample row of that kernel: dram__bytes_read.sum + dram__bytes_write.sum over all
-# its launches of 2 frames of the same scene at 960x540 / the rows they processed (4.616 GB / 116,864,373 rows)
-NET_TRAFFIC_PER_ROW = 39.5
+# DRAM bytes (read + write) per row of that kernel: dram__bytes_read.sum + dram__bytes_write.sum over all its
+# launches of a cached frame of the same scene at 960x540 / the rows they processed (2.459 GB / 57,470,229 rows)
+NET_TRAFFIC_PER_ROW = 42.8
 
 
 def dist_env():
